@@ -83,7 +83,8 @@ def build_runtime(force=False):
     if ref is None:
         if os.path.exists(lib):
             return lib
-        raise RuntimeError("libpolar_rt_cuda.so is not built and the reference headers are absent")
+        print("libpolar_rt_cuda.so left out: it is compiled against the reference's headers, which are absent")
+        return None
     srcs = [os.path.join(rt_dir, f) for f in sorted(os.listdir(rt_dir)) if f.endswith((".cpp", ".cu"))]
     deps = tuple(os.path.join(rt_dir, f) for f in os.listdir(rt_dir)) + _headers()
     if not (force or any(_newer(s, lib, deps) for s in srcs)):
