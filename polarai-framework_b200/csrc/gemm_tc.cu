@@ -82,7 +82,8 @@ template <int BN, int BK, int MT = 1> struct Cfg {
   static constexpr uint32_t kSmemBytes = kTileBytes + 1024 + 256;
   static constexpr uint32_t kTmemCols = 2 * BN;            // two fp32 accumulators
   static constexpr uint32_t kBoxBytes = 32 * BK * 4;       // one MN-major TMA box {32 m/n, BK k}
-  static constexpr int kBBoxRows = BN < 128 ? BN : 128;    // a K-major B slab arrives in boxes of 128 rows
+  static constexpr int kBBoxRows = BN < 128 ? BN : 128;    // B arrives in boxes of 128 rows (columns of the tile)
+  static constexpr int kABoxRows = BM * MT;                // A in one box
 };
 
 struct Params {
@@ -90,6 +91,7 @@ struct Params {
   float* out;
   int a_mn_major;   // left operand stored [k,m]
   int b_mn_major;   // right operand stored [k,n]
+  int a_chunked, b_chunked;   // MN-major through a 3-D map of 32-element chunks (make_map_chunks)
   int passes;       // 3 = fp32-accurate split, 1 = plain TF32 (diagnostic)
   int write_hi;     // split warps also store the masked hi part in place
   int* status;      // this device's status word (pinned host memory, device-visible)
@@ -284,9 +286,16 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           const uint32_t stage = smem_base + s * C::kStageBytes;
           mbar_expect_tx(full_raw(s), C::kABytes + (pc.half ? C::kBBytes / 2 : C::kBBytes));
           const int k0 = (int)(kb * BK);
+          // The TMA unit takes 50-100 ns per instruction whatever its size, so a slab comes in as few
+          // boxes as possible: an MN-major slab, 32-element chunks of BK rows each, in one or two 3-D
+          // boxes of 4 or 8 chunks.  (As one 2-D box per chunk - 16 instructions for a 256 x 256 x 16
+          // slab of a t_f product, 0.85 us - TMA was slower than the slab's three products, 0.8 us:
+          // measured 5.7 TB/s in 2 KB boxes, 17 TB/s in 16 KB ones.)  A contiguous extent that is no
+          // multiple of 32 still takes the 2-D boxes, whose reads TMA cuts off at the extent.
           if (!p.a_mn_major) {
-            for (int h = 0; h < MT; ++h)                               // boxes {BK k, 128 m}
-              tma_load_2d(stage + h * C::kASubBytes, &map_a, full_raw(s), k0, m0 + h * BM);
+            tma_load_2d(stage, &map_a, full_raw(s), k0, m0);           // box {BK k, kTileM m}
+          } else if (p.a_chunked) {
+            tma_load_3d(stage, &map_a, full_raw(s), 0, k0, m0 / 32);  // box {32 m, BK k, kTileM / 32}
           } else {
             for (int c = 0; c < kTileM / 32; ++c)                      // boxes {32 m, BK k}
               tma_load_2d(stage + c * C::kBoxBytes, &map_a, full_raw(s), m0 + 32 * c, k0);
@@ -295,6 +304,10 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           if (!p.b_mn_major) {
             for (int c = 0; c < bn_now / C::kBBoxRows; ++c)            // boxes {BK k, 128 n}
               tma_load_2d(bdst + c * (C::kBBoxRows * BK * 4), &map_b, full_raw(s), k0, n0 + C::kBBoxRows * c);
+          } else if (p.b_chunked) {
+            for (int c = 0; c < bn_now / C::kBBoxRows; ++c)            // boxes {32 n, BK k, 4}
+              tma_load_3d(bdst + c * (C::kBBoxRows * BK * 4), &map_b, full_raw(s), 0, k0,
+                          (n0 + C::kBBoxRows * c) / 32);
           } else {
             for (int c = 0; c < bn_now / 32; ++c)                      // boxes {32 n, BK k}
               tma_load_2d(bdst + c * C::kBoxBytes, &map_b, full_raw(s), n0 + 32 * c, k0);
@@ -511,6 +524,24 @@ int make_map(CUtensorMap* map, const float* base, uint64_t inner, uint64_t outer
   return POLAR_B200_OK;
 }
 
+// The same MN-major matrix as a 3-D map {32 elements of a chunk, rows, chunks}: one box of
+// `box_chunks` chunks lands in shared memory as that many consecutive 2-D boxes.  Whole chunks only:
+// TMA could not cut a box off inside the last one.
+int make_map_chunks(CUtensorMap* map, const float* base, uint64_t chunks, uint64_t outer, uint32_t box_outer,
+                    uint32_t box_chunks, uint64_t pitch) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc) return fail(POLAR_B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  cuuint64_t dims[3] = {32, outer, chunks};
+  cuuint64_t strides[2] = {pitch * 4, 32 * 4};
+  cuuint32_t box[3] = {32, box_outer, box_chunks};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(POLAR_B200_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+  return POLAR_B200_OK;
+}
+
 bool shape_ok(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
               const float* right) {
   // TMA: 16-byte aligned base, row pitch a multiple of 16 bytes.
@@ -660,17 +691,23 @@ static int launch_cfg(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const 
   int* status_word = device_status_word(&rc);
   if (!status_word) return rc;
   CUtensorMap map_a, map_b;
-  // left: stored [m,k] (K-major: inner k, box {BK, 128}) or [k,m] (MN-major: inner m, box {32, BK})
-  rc = tl ? make_map(&map_a, left, m, k, 32, BK, true, BK, left_pitch)
-          : make_map(&map_a, left, k, m, BK, BM, false, BK, left_pitch);
+  const bool a_chunked = tl && (m & 31) == 0, b_chunked = !tr && (n & 31) == 0;
+  // left: stored [m,k] (K-major: inner k, box {BK, tile rows}) or [k,m] (MN-major: 3-D, or inner m, box {32, BK})
+  rc = !tl ? make_map(&map_a, left, k, m, BK, C::kABoxRows, false, BK, left_pitch)
+       : a_chunked ? make_map_chunks(&map_a, left, m / 32, k, BK, C::kABoxRows / 32, left_pitch ? left_pitch : m)
+                   : make_map(&map_a, left, m, k, 32, BK, true, BK, left_pitch);
   if (rc) return rc;
-  // right: stored [n,k] when transposed (K-major: inner k, box {BK, BN}) or [k,n] (MN-major)
-  rc = tr ? make_map(&map_b, right, k, n, BK, C::kBBoxRows, false, BK) : make_map(&map_b, right, n, k, 32, BK, true, BK);
+  // right: stored [n,k] when transposed (K-major: inner k, box {BK, 128}) or [k,n] (MN-major)
+  rc = tr ? make_map(&map_b, right, k, n, BK, C::kBBoxRows, false, BK)
+       : b_chunked ? make_map_chunks(&map_b, right, n / 32, k, BK, C::kBBoxRows / 32, n)
+                   : make_map(&map_b, right, n, k, 32, BK, true, BK);
   if (rc) return rc;
   Params p;
   p.m = m; p.n = n; p.k = k; p.out = out;
   p.a_mn_major = tl ? 1 : 0;
   p.b_mn_major = tr ? 0 : 1;
+  p.a_chunked = a_chunked;
+  p.b_chunked = b_chunked;
   p.passes = passes; p.write_hi = write_hi; p.status = status_word;
   p.wait_ns = wait_limit_ns(2000000000ull);
   p.wide_store = wide_store_enabled() ? 1 : 0;
