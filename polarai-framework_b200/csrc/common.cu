@@ -83,6 +83,44 @@ void device_status_clear_all() {
   for (int d = 0; d < kMaxDevices; ++d) *(volatile int*)(g_status_host + d) = 0;
 }
 
+namespace {
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pool[kMaxDevices] = {nullptr};
+}  // namespace
+
+cudaError_t scratch_alloc(void** p, uint64_t bytes, cudaStream_t stream) {
+  // under stream capture the block belongs to the graph, whatever the pool
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(stream, &capturing);
+  if (e != cudaSuccess) return e;
+  if (capturing != cudaStreamCaptureStatusNone) return cudaMallocAsync(p, bytes, stream);
+  int dev = 0;
+  e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= kMaxDevices) return cudaMallocAsync(p, bytes, stream);
+  cudaMemPool_t pool;
+  {
+    std::lock_guard<std::mutex> guard(g_pool_mutex);
+    if (!g_pool[dev]) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      e = cudaMemPoolCreate(&pool, &props);
+      if (e != cudaSuccess) return e;
+      unsigned long long keep = kScratchKeepBytes;
+      e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return e;
+      }
+      g_pool[dev] = pool;
+    }
+    pool = g_pool[dev];
+  }
+  return cudaMallocFromPoolAsync(p, bytes, pool, stream);
+}
+
 unsigned long long wait_limit_ns(unsigned long long fallback) {
   const unsigned long long v = g_wait_limit_ns.load(std::memory_order_relaxed);
   return v ? v : fallback;
@@ -102,6 +140,17 @@ int polar_b200_check_device_status(void) {
   std::snprintf(msg, sizeof msg, "a bounded device-side wait gave up (code %d)", code);
   clear_error();
   return fail(POLAR_B200_ERR_TIMEOUT, msg);
+}
+int polar_b200_trim_scratch(uint64_t keep_bytes) {
+  using namespace polar_b200;
+  clear_error();
+  std::lock_guard<std::mutex> guard(g_pool_mutex);
+  for (cudaMemPool_t pool : g_pool) {
+    if (!pool) continue;
+    cudaError_t e = cudaMemPoolTrimTo(pool, keep_bytes);
+    if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaMemPoolTrimTo", e);
+  }
+  return POLAR_B200_OK;
 }
 void polar_b200_set_wait_limit_ns(uint64_t ns) { polar_b200::g_wait_limit_ns.store(ns, std::memory_order_relaxed); }
 uint64_t polar_b200_wait_limit_ns(void) { return polar_b200::g_wait_limit_ns.load(std::memory_order_relaxed); }

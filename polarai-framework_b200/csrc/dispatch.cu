@@ -66,12 +66,12 @@ int run_tc(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left
                      splits, epilogue, stream, left_pitch, mt, swap_ab);
   }
   void* ws = nullptr;
-  cudaError_t e = cudaMallocAsync(&ws, need, stream);
-  if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaMallocAsync(workspace)", e);
+  cudaError_t e = scratch_alloc(&ws, need, stream);
+  if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "scratch (workspace)", e);
   int rc = launch_tc(tl, tr, m, n, k, left, right, out, bn, bk, passes, write_hi, static_cast<float*>(ws), splits,
                      epilogue, stream, left_pitch, mt, swap_ab);
-  e = cudaFreeAsync(ws, stream);
-  if (rc == POLAR_B200_OK && e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFreeAsync(workspace)", e);
+  e = scratch_free(ws, stream);
+  if (rc == POLAR_B200_OK && e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "returning scratch", e);
   return rc;
 }
 
@@ -97,13 +97,16 @@ struct SideStream {
   cudaStream_t stream = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
 };
+// A thread that captures a program uses a set apart (use_capture_side_stream): the shared one may be
+// in use by another thread while this one's is part of a capture.
+thread_local bool tls_capturing_program = false;
 SideStream* side_stream() {
-  static SideStream per_device[64];
+  static SideStream shared[64], for_capture[64];
   static std::mutex mu;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   std::lock_guard<std::mutex> g(mu);
-  SideStream& s = per_device[dev];
+  SideStream& s = tls_capturing_program ? for_capture[dev] : shared[dev];
   if (!s.stream) {
     if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) != cudaSuccess ||
@@ -171,6 +174,15 @@ TcChoice tc_choose(uint64_t m, uint64_t n, uint64_t k, bool may_swap) {
   }
   return best;
 }
+
+}  // namespace
+
+bool use_capture_side_stream(bool on) {
+  tls_capturing_program = on;
+  return !on || side_stream() != nullptr;
+}
+
+namespace {
 
 int check_mm(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
              const float* right, float* out) {
@@ -283,8 +295,8 @@ static int tc_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const flo
     if (workspace_bytes < tc_need + rag_need || (reinterpret_cast<uintptr_t>(workspace) & 15))
       return fail(POLAR_B200_ERR_WORKSPACE, "workspace too small or not 16-byte aligned");
   } else {
-    cudaError_t e = cudaMallocAsync(&own, tc_need + rag_need, main_stream);
-    if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaMallocAsync(workspace)", e);
+    cudaError_t e = scratch_alloc(&own, tc_need + rag_need, main_stream);
+    if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "scratch (workspace)", e);
     ws = static_cast<char*>(own);
   }
   // fork: the side stream starts where the caller's stream is now (one fork/join at a time
@@ -313,8 +325,8 @@ static int tc_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const flo
     }
   }
   if (own) {
-    cudaError_t e = cudaFreeAsync(own, main_stream);
-    if (!rc && !rc2 && e != cudaSuccess) rc = fail(POLAR_B200_ERR_CUDA, "cudaFreeAsync(workspace)", e);
+    cudaError_t e = scratch_free(own, main_stream);
+    if (!rc && !rc2 && e != cudaSuccess) rc = fail(POLAR_B200_ERR_CUDA, "returning scratch", e);
   }
   return rc ? rc : rc2;
 }
@@ -361,11 +373,11 @@ static int fmatmul_impl(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, cons
       }
       // No workspace from the caller: take it from the stream-ordered pool.
       void* ws = nullptr;
-      cudaError_t e = cudaMallocAsync(&ws, need, as_stream(stream));
-      if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaMallocAsync(workspace)", e);
+      cudaError_t e = scratch_alloc(&ws, need, as_stream(stream));
+      if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "scratch (workspace)", e);
       rc = launch_skinny(kind, tl, tr, m, n, k, left, right, out, static_cast<float*>(ws), as_stream(stream), nullptr);
-      e = cudaFreeAsync(ws, as_stream(stream));
-      if (rc == POLAR_B200_OK && e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFreeAsync(workspace)", e);
+      e = scratch_free(ws, as_stream(stream));
+      if (rc == POLAR_B200_OK && e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "returning scratch", e);
       return rc;
     }
     default:
@@ -455,11 +467,11 @@ int polar_b200_fdense_grad(uint64_t rows, uint64_t kh, uint64_t n, const float* 
     return launch_dense_grad(h, dz, w, din, dw, static_cast<float*>(workspace), rows, kh, n, st);
   }
   void* ws = nullptr;
-  cudaError_t e = cudaMallocAsync(&ws, need, st);
-  if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaMallocAsync(workspace)", e);
+  cudaError_t e = scratch_alloc(&ws, need, st);
+  if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "scratch (workspace)", e);
   int rc = launch_dense_grad(h, dz, w, din, dw, static_cast<float*>(ws), rows, kh, n, st);
-  e = cudaFreeAsync(ws, st);
-  if (rc == POLAR_B200_OK && e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFreeAsync(workspace)", e);
+  e = scratch_free(ws, st);
+  if (rc == POLAR_B200_OK && e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "returning scratch", e);
   return rc;
 }
 

@@ -17,129 +17,43 @@
 // contraction into FMA), fdivide is IEEE division, fsigmoid and flogloss use
 // the full-precision expf/logf (1 ulp), not the fast intrinsics.
 #include "common.cuh"
+#include "elementwise_ops.cuh"
 
 namespace polar_b200 {
 namespace {
+
+using namespace ew;
 
 constexpr int kThreads = 256;
 constexpr int kCtasPerSm = 4;   // 1024 threads/SM: 64 registers per thread available
 constexpr int kUnroll = 4;      // float4 vectors in flight per input per thread
 
-struct FillOp {
-  float v;
-  __device__ __forceinline__ float operator()(float, float) const { return v; }
-};
-struct CopyOp {
-  __device__ __forceinline__ float operator()(float a, float) const { return a; }
-};
-struct AddOp {
-  float sa, sb;
-  __device__ __forceinline__ float operator()(float a, float b) const {
-    return __fadd_rn(__fmul_rn(a, sa), __fmul_rn(b, sb));
-  }
-};
-struct MulOp {
-  __device__ __forceinline__ float operator()(float a, float b) const { return __fmul_rn(a, b); }
-};
-struct DivOp {
-  __device__ __forceinline__ float operator()(float a, float b) const { return __fdiv_rn(a, b); }
-};
-template <bool CLAMP>
-struct SigmoidOp {
-  __device__ __forceinline__ float operator()(float x, float) const {
-    if (CLAMP) return sigmoid_clamped(x);
-    return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-x)));
-  }
-};
-struct LogLossOp {
-  // out = fl(fl(-y * log(p + eps)) - fl((1 - y) * log(1 - p + eps))), eps = 1e-5: the general
-  // form, two full-precision logarithms (scalar fallback kernel, and soft labels in the
-  // vector kernel below).
-  __device__ __forceinline__ float operator()(float p, float y) const {
-    const float eps = 1e-5f;
-    float t0 = __fmul_rn(-y, logf(__fadd_rn(p, eps)));
-    float t1 = __fmul_rn(__fadd_rn(1.0f, -y), logf(__fadd_rn(__fadd_rn(1.0f, -p), eps)));
-    return __fadd_rn(t0, -t1);
-  }
-};
-// flogloss for labels that are exactly 0 or 1 (what LogLoss is fed): one of the two weights
-// -y and 1-y is then an exact zero, and its product with a logarithm is a signed zero, NaN
-// or NaN - whatever the logarithm's low bits are.  So only the OTHER logarithm needs full
-// precision; the one under the zero weight comes from the special-function unit
-// (lg2.approx), which returns the same NaN / -inf / +inf classes and the same sign.  (The
-// sign of that zero is only visible when the full-precision term is itself zero, i.e. its
-// argument is exactly 1; the two arguments sum to 1 + 2 eps, so the other one is then about
-// 2e-5, far from where an approximate logarithm could have the wrong sign.)  Same bits as
-// the two-logarithm form at roughly 60 % of its instructions - two full logf per element make
-// the builtin issue-bound instead of HBM-bound.  Branch-free, so the unrolled elements
-// interleave.
-__device__ __forceinline__ float logloss_binary(float p, float y) {
-  const float eps = 1e-5f;
-  const float a0 = __fadd_rn(p, eps);
-  const float a1 = __fadd_rn(__fadd_rn(1.0f, -p), eps);
-  const float w0 = -y, w1 = __fadd_rn(1.0f, -y);
-  const bool first = (w1 == 0.0f);                       // y == 1: log(a0) carries the result
-  const float fine = logf(first ? a0 : a1);
-  const float coarse = __logf(first ? a1 : a0);
-  const float t0 = __fmul_rn(w0, first ? fine : coarse);
-  const float t1 = __fmul_rn(w1, first ? coarse : fine);
-  return __fadd_rn(t0, -t1);
-}
-// Extended builtin: the three launches the reference's Sigmoid derivative compiles to
-// (SigmoidOperationInternal.cpp:107-135: fadd(ones,1,s,-1) -> fmul(.,s) -> fmul(grad,.))
-// in one pass, with the same three roundings, so the result is bit-identical.
-struct SigmoidGradOp {
-  __device__ __forceinline__ float operator()(float g, float s) const {
-    return sigmoid_grad_chain(g, s);
-  }
-};
-// Extended builtin: dZ = dL/dP * dP/dZ for LogLoss on a Sigmoid output, the seven launches
-// the reference's derivatives compile to (LogLossOperationInternal.cpp:127-170:
-// fadd(p,1,y,-1), fmul(p,p), fadd(p,1,pp,-1), fdivide; SigmoidOperationInternal.cpp:107-135:
-// fadd(ones,1,p,-1), fmul(.,p), fmul(dLdP,.)) in one pass with the same seven roundings.
-struct SigmoidLogLossGradOp {
-  __device__ __forceinline__ float operator()(float p, float y) const {
-    const float pmy = __fadd_rn(__fmul_rn(p, 1.0f), __fmul_rn(y, -1.0f));
-    const float pp = __fmul_rn(p, p);
-    const float den = __fadd_rn(__fmul_rn(p, 1.0f), __fmul_rn(pp, -1.0f));
-    const float dldp = __fdiv_rn(pmy, den);
-    return sigmoid_grad_chain(dldp, p);
-  }
-};
-struct ScaleByFirstOp {  // fmulconcat: the scalar is read once per thread
-  float g;
-  __device__ __forceinline__ float operator()(float l, float) const { return __fmul_rn(g, l); }
-};
-
 __device__ __forceinline__ float4 ld_stream(const float4* p) { return __ldcs(p); }
 __device__ __forceinline__ void st_stream(float4* p, float4 v) { __stcs(p, v); }
 
-// Per-op tile shape: vectors in flight per input per thread, and CTAs per SM the
-// register budget must allow (flat between 2 and 8 vectors per thread for every builtin
-// served by this template; flogloss has its own kernel below).
-template <class Op> struct Shape { static constexpr int kUnroll = 4, kMinCtas = kCtasPerSm; };
-
+// Vectors in flight per input per thread: kUnroll for streams (flat between 2 and 8 for every
+// builtin), 1 for short vectors (short_vector below).
 // NIN = number of input streams (0, 1 or 2).
-template <int NIN, class Op>
-__global__ void __launch_bounds__(kThreads, Shape<Op>::kMinCtas)
+template <int NIN, int UNROLL, class Op>
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
 ew_vec_kernel(Op op, const float* in0, const float* in1, float* out, uint64_t n) {
-  constexpr int kUnroll = Shape<Op>::kUnroll;
+  pdl_enter();
   const uint64_t nvec = n >> 2;
   const float4* v0 = reinterpret_cast<const float4*>(in0);
   const float4* v1 = reinterpret_cast<const float4*>(in1);
   float4* vo = reinterpret_cast<float4*>(out);
-  const uint64_t tile = (uint64_t)kThreads * kUnroll;
+  const uint64_t tile = (uint64_t)kThreads * UNROLL;
   {
     const uint64_t base = (uint64_t)blockIdx.x * tile;
-    float4 a[kUnroll], b[kUnroll];
+    float4 a[UNROLL], b[UNROLL];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < UNROLL; ++u) {
       uint64_t i = base + (uint64_t)u * kThreads + threadIdx.x;
       if (NIN >= 1 && i < nvec) a[u] = ld_stream(v0 + i);
       if (NIN >= 2 && i < nvec) b[u] = ld_stream(v1 + i);
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < UNROLL; ++u) {
       uint64_t i = base + (uint64_t)u * kThreads + threadIdx.x;
       if (i < nvec) {
         float4 r;
@@ -161,18 +75,19 @@ ew_vec_kernel(Op op, const float* in0, const float* in1, float* out, uint64_t n)
 // flogloss, vector form: one tile per CTA like ew_vec_kernel.  A thread whose labels are all
 // exactly 0 or 1 takes the one-logarithm arithmetic for its whole tile (one branch per
 // thread, uniform for hard labels); any other label sends the thread to the general form.
-constexpr int kLogLossUnroll = 4;
+template <int UNROLL>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 logloss_vec_kernel(const float* predicted, const float* truth, float* out, uint64_t n) {
+  pdl_enter();
   const uint64_t nvec = n >> 2;
   const float4* vp = reinterpret_cast<const float4*>(predicted);
   const float4* vy = reinterpret_cast<const float4*>(truth);
   float4* vo = reinterpret_cast<float4*>(out);
-  const uint64_t base = (uint64_t)blockIdx.x * kThreads * kLogLossUnroll;
-  float4 p[kLogLossUnroll], y[kLogLossUnroll];
+  const uint64_t base = (uint64_t)blockIdx.x * kThreads * UNROLL;
+  float4 p[UNROLL], y[UNROLL];
   bool binary = true;
 #pragma unroll
-  for (int u = 0; u < kLogLossUnroll; ++u) {
+  for (int u = 0; u < UNROLL; ++u) {
     const uint64_t i = base + (uint64_t)u * kThreads + threadIdx.x;
     if (i < nvec) {
       p[u] = ld_stream(vp + i);
@@ -183,14 +98,14 @@ logloss_vec_kernel(const float* predicted, const float* truth, float* out, uint6
     }
   }
 #pragma unroll
-  for (int u = 0; u < kLogLossUnroll; ++u) {
+  for (int u = 0; u < UNROLL; ++u) {
     const float w[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) binary = binary && (w[j] == 0.0f || w[j] == 1.0f);
   }
   LogLossOp general;
 #pragma unroll
-  for (int u = 0; u < kLogLossUnroll; ++u) {
+  for (int u = 0; u < UNROLL; ++u) {
     const uint64_t i = base + (uint64_t)u * kThreads + threadIdx.x;
     float4 r;
     if (binary) {
@@ -215,6 +130,7 @@ logloss_vec_kernel(const float* predicted, const float* truth, float* out, uint6
 template <int NIN, class Op>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 ew_scalar_kernel(Op op, const float* in0, const float* in1, float* out, uint64_t n) {
+  pdl_enter();
   const uint64_t stride = (uint64_t)gridDim.x * kThreads;
   for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride) {
     out[i] = op(NIN >= 1 ? in0[i] : 0.f, NIN >= 2 ? in1[i] : 0.f);
@@ -222,24 +138,26 @@ ew_scalar_kernel(Op op, const float* in0, const float* in1, float* out, uint64_t
 }
 
 // fmulconcat reads its scalar from device memory inside the kernel.
+template <int UNROLL>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 mulconcat_vec_kernel(const float* gradient, const float* local, float* out, uint64_t n) {
+  pdl_enter();
   const float g = gradient[0];
   ScaleByFirstOp op{g};
   const uint64_t nvec = n >> 2;
   const float4* v0 = reinterpret_cast<const float4*>(local);
   float4* vo = reinterpret_cast<float4*>(out);
-  const uint64_t tile = (uint64_t)kThreads * kUnroll;
+  const uint64_t tile = (uint64_t)kThreads * UNROLL;
   {
     const uint64_t base = (uint64_t)blockIdx.x * tile;
-    float4 a[kUnroll];
+    float4 a[UNROLL];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < UNROLL; ++u) {
       uint64_t i = base + (uint64_t)u * kThreads + threadIdx.x;
       if (i < nvec) a[u] = ld_stream(v0 + i);
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < UNROLL; ++u) {
       uint64_t i = base + (uint64_t)u * kThreads + threadIdx.x;
       if (i < nvec) {
         float4 r = {op(a[u].x, 0.f), op(a[u].y, 0.f), op(a[u].z, 0.f), op(a[u].w, 0.f)};
@@ -255,6 +173,7 @@ mulconcat_vec_kernel(const float* gradient, const float* local, float* out, uint
 
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 mulconcat_scalar_kernel(const float* gradient, const float* local, float* out, uint64_t n) {
+  pdl_enter();
   const float g = gradient[0];
   const uint64_t stride = (uint64_t)gridDim.x * kThreads;
   for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride)
@@ -264,6 +183,7 @@ mulconcat_scalar_kernel(const float* gradient, const float* local, float* out, u
 // fsum: per-thread double partials, warp shuffle, one atomicAdd(double) per block.
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 sum_kernel(const float* in, double* sum, uint64_t n, int vec_ok) {
+  pdl_enter();
   double acc = 0.0;
   if (vec_ok) {
     const uint64_t nvec = n >> 2;
@@ -296,6 +216,7 @@ sum_kernel(const float* in, double* sum, uint64_t n, int vec_ok) {
 // (one CTA) adds them in index order and stores the rounded float - the same bits run to run.
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 sum_partials_kernel(const float* in, double* partials, uint64_t n, int vec_ok) {
+  pdl_enter();
   double acc = 0.0;
   const uint64_t stride = (uint64_t)gridDim.x * kThreads;
   if (vec_ok) {
@@ -321,6 +242,7 @@ sum_partials_kernel(const float* in, double* partials, uint64_t n, int vec_ok) {
   }
 }
 __global__ void __launch_bounds__(32) sum_finish_kernel(const double* partials, uint32_t count, float* out) {
+  pdl_enter();
   if (threadIdx.x == 0) {
     double s = 0.0;
     for (uint32_t i = 0; i < count; ++i) s += partials[i];
@@ -335,8 +257,11 @@ unsigned grid_for(uint64_t work_items, uint64_t per_cta) {
   if (need < 1) need = 1;
   return (unsigned)(need < cap ? need : cap);
 }
+// A vector shorter than two tiles of four vectors per thread on every SM runs with one vector per
+// thread: four times as many CTAs, each a quarter as long a chain of loads and stores.
+bool short_vector(uint64_t nvec) { return nvec < 2ull * kThreads * kUnroll * (uint64_t)sm_count(); }
 // One tile per CTA (vector kernels).
-unsigned tiles_for(uint64_t nvec, int unroll = kUnroll) {
+unsigned tiles_for(uint64_t nvec, int unroll) {
   uint64_t per_cta = (uint64_t)kThreads * unroll;
   uint64_t need = (nvec + per_cta - 1) / per_cta;
   return (unsigned)(need < 1 ? 1 : need);
@@ -352,14 +277,12 @@ int launch_ew(const char* name, Op op, const float* in0, const float* in1, float
   if (n > (1ull << 40)) return fail(POLAR_B200_ERR_INVALID, "element count too large");
   LaunchDeviceScope on(stream, out);
   bool vec = aligned16(out) && (NIN < 1 || aligned16(in0)) && (NIN < 2 || aligned16(in1)) && n >= 4;
-  if (vec) {
-    unsigned grid = tiles_for(n >> 2, Shape<Op>::kUnroll);
-    ew_vec_kernel<NIN, Op><<<grid, kThreads, 0, as_stream(stream)>>>(op, in0, in1, out, n);
-  } else {
-    unsigned grid = grid_for(n, kThreads);
-    ew_scalar_kernel<NIN, Op><<<grid, kThreads, 0, as_stream(stream)>>>(op, in0, in1, out, n);
-  }
-  return check_launch(name);
+  if (!vec)
+    return launch(name, ew_scalar_kernel<NIN, Op>, grid_for(n, kThreads), kThreads, 0, as_stream(stream), op, in0, in1, out, n);
+  if (short_vector(n >> 2))
+    return launch(name, ew_vec_kernel<NIN, 1, Op>, tiles_for(n >> 2, 1), kThreads, 0, as_stream(stream), op, in0, in1, out, n);
+  return launch(name, ew_vec_kernel<NIN, kUnroll, Op>, tiles_for(n >> 2, kUnroll), kThreads, 0, as_stream(stream), op, in0,
+                in1, out, n);
 }
 
 }  // namespace
@@ -398,9 +321,11 @@ int polar_b200_flogloss(const float* predicted, const float* groundTruth, float*
       aligned16(groundTruth) && aligned16(out)) {
     clear_error();
     LaunchDeviceScope on(stream, out);
-    logloss_vec_kernel<<<tiles_for(n >> 2, kLogLossUnroll), kThreads, 0, as_stream(stream)>>>(predicted, groundTruth,
-                                                                                            out, n);
-    return check_launch("flogloss");
+    return short_vector(n >> 2)
+               ? launch("flogloss", logloss_vec_kernel<1>, tiles_for(n >> 2, 1), kThreads, 0, as_stream(stream), predicted,
+                        groundTruth, out, n)
+               : launch("flogloss", logloss_vec_kernel<kUnroll>, tiles_for(n >> 2, kUnroll), kThreads, 0, as_stream(stream),
+                        predicted, groundTruth, out, n);
   }
   return launch_ew<2>("flogloss", LogLossOp{}, predicted, groundTruth, out, n, stream);   // null, empty, unaligned
 }
@@ -422,14 +347,15 @@ int polar_b200_fmulconcat(const float* gradient, const float* localDerivative, f
   if (!gradient || !localDerivative || !out) return fail(POLAR_B200_ERR_INVALID, "null device pointer");
   if (n > (1ull << 40)) return fail(POLAR_B200_ERR_INVALID, "element count too large");
   LaunchDeviceScope on(stream, out);
-  if (aligned16(localDerivative) && aligned16(out) && n >= 4) {
-    unsigned grid = tiles_for(n >> 2);
-    mulconcat_vec_kernel<<<grid, kThreads, 0, as_stream(stream)>>>(gradient, localDerivative, out, n);
-  } else {
-    unsigned grid = grid_for(n, kThreads);
-    mulconcat_scalar_kernel<<<grid, kThreads, 0, as_stream(stream)>>>(gradient, localDerivative, out, n);
-  }
-  return check_launch("fmulconcat");
+  cudaStream_t st = as_stream(stream);
+  if (!(aligned16(localDerivative) && aligned16(out) && n >= 4))
+    return launch("fmulconcat", mulconcat_scalar_kernel, grid_for(n, kThreads), kThreads, 0, st, gradient, localDerivative,
+                  out, n);
+  if (short_vector(n >> 2))
+    return launch("fmulconcat", mulconcat_vec_kernel<1>, tiles_for(n >> 2, 1), kThreads, 0, st, gradient, localDerivative,
+                  out, n);
+  return launch("fmulconcat", mulconcat_vec_kernel<kUnroll>, tiles_for(n >> 2, kUnroll), kThreads, 0, st, gradient,
+                localDerivative, out, n);
 }
 
 int polar_b200_fsum(const float* in, double* sum, uint64_t n, void* stream) {
@@ -440,8 +366,7 @@ int polar_b200_fsum(const float* in, double* sum, uint64_t n, void* stream) {
   LaunchDeviceScope on(stream, in);
   int vec_ok = aligned16(in) && n >= 4;
   unsigned grid = grid_for(vec_ok ? (n >> 2) : n, (uint64_t)kThreads * 8);
-  sum_kernel<<<grid, kThreads, 0, as_stream(stream)>>>(in, sum, n, vec_ok);
-  return check_launch("fsum");
+  return launch("fsum", sum_kernel, grid, kThreads, 0, as_stream(stream), in, sum, n, vec_ok);
 }
 
 uint64_t polar_b200_fsum_f32_workspace_bytes(uint64_t n) {
@@ -463,19 +388,15 @@ int polar_b200_fsum_f32(const float* in, float* out, uint64_t n, void* workspace
   double* partials = static_cast<double*>(workspace);
   bool own = false;
   if (!partials) {
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&partials), need, st);
-    if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaMallocAsync(fsum partial sums)", e);
+    cudaError_t e = scratch_alloc(reinterpret_cast<void**>(&partials), need, st);
+    if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "scratch (fsum partial sums)", e);
     own = true;
   } else if (workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 7)) {
     return fail(POLAR_B200_ERR_WORKSPACE, "fsum needs 8-byte aligned workspace of polar_b200_fsum_f32_workspace_bytes");
   }
-  sum_partials_kernel<<<grid, kThreads, 0, st>>>(in, partials, n, vec_ok);
-  int rc = check_launch("fsum_partials");
-  if (rc == POLAR_B200_OK) {
-    sum_finish_kernel<<<1, 32, 0, st>>>(partials, grid, out);
-    rc = check_launch("fsum");
-  }
-  if (own) cudaFreeAsync(partials, st);
+  int rc = launch("fsum_partials", sum_partials_kernel, grid, kThreads, 0, st, in, partials, n, vec_ok);
+  if (rc == POLAR_B200_OK) rc = launch("fsum", sum_finish_kernel, 1, 32, 0, st, partials, grid, out);
+  if (own) scratch_free(partials, st);
   return rc;
 }
 

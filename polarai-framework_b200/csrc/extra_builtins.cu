@@ -123,8 +123,8 @@ int polar_b200_fsoftmax(const float* in, float* out, uint64_t n, void* workspace
   double* total = static_cast<double*>(workspace);
   bool own = false;
   if (!total) {
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&total), sizeof(double), st);
-    if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaMallocAsync(softmax total)", e);
+    cudaError_t e = scratch_alloc(reinterpret_cast<void**>(&total), sizeof(double), st);
+    if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "scratch (softmax total)", e);
     own = true;
   } else if (workspace_bytes < sizeof(double) || (reinterpret_cast<uintptr_t>(workspace) & 7)) {
     return fail(POLAR_B200_ERR_WORKSPACE, "fsoftmax needs 8 bytes of 8-byte aligned workspace");
@@ -137,7 +137,7 @@ int polar_b200_fsoftmax(const float* in, float* out, uint64_t n, void* workspace
     softmax_div_kernel<<<blocks_for(n), kThreads, 0, st>>>(in, total, out, n);
     rc = check_launch("fsoftmax");
   }
-  if (own) cudaFreeAsync(total, st);
+  if (own) scratch_free(total, st);
   return rc;
 }
 
