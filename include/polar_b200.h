@@ -159,9 +159,9 @@ int polar_b200_fslice(const float* in, uint64_t first_dim, uint64_t inner, uint6
  * non-zero when the sum over k is cut into several work units whose partial
  * products are added afterwards in a fixed order: narrow results with a long k,
  * and tensor-core shapes with too few tiles to load every SM).
- * With workspace == NULL the call takes the scratch it needs from the
- * device's stream-ordered memory pool (cudaMallocAsync/cudaFreeAsync on
- * `stream`). */
+ * With workspace == NULL the call takes the scratch it needs from a
+ * stream-ordered memory pool of the library's own (see
+ * polar_b200_trim_scratch). */
 int polar_b200_fmatmul(int transLeft, int transRight, uint64_t m, uint64_t n,
                        uint64_t k, const float* left, const float* right,
                        float* out, void* workspace, uint64_t workspace_bytes,
@@ -480,6 +480,33 @@ int polar_b200_allreduce_fadd_multicast(void* const* buffers, void* multicast, u
  * fmatmul shapes).  Only shapes are read, not the data pointers. */
 uint64_t polar_b200_launch_workspace_bytes(const char* nativeKernelName,
                                            const polar_b200_arg* args, uint64_t argsCount);
+
+/* ---- builtin programs ------------------------------------------------------
+ * A list of builtin launches prepared once and run many times: what a compiled graph is.
+ * One run launches the operations in order on `stream`, exactly as polar_b200_launch_by_name
+ * would one by one (same checks, same statuses, every result tensor written with the same
+ * bits), but in fewer launches: consecutive elementwise builtins over the same element count
+ * share one, and from its third run on a program of several launches is replayed as a CUDA
+ * graph.  Names, argument lists and shapes are copied; the tensors and the workspace must
+ * stay allocated while the program exists.  A program may be run on any stream of its device, also
+ * one under capture, and from any thread; like the launches themselves, runs that overlap on the
+ * GPU share the tensors and the workspace.  polar_b200_program_steps: launch steps of one run. */
+typedef struct polar_b200_op {
+  const char* name;
+  const polar_b200_arg* args;
+  uint64_t argc;
+} polar_b200_op;
+
+int polar_b200_program_create(const polar_b200_op* ops, uint64_t count, void* workspace,
+                              uint64_t workspace_bytes, void** program);
+int polar_b200_program_run(void* program, void* stream);
+uint64_t polar_b200_program_steps(const void* program);
+void polar_b200_program_destroy(void* program);
+
+/* Scratch that a call takes because its caller hands in no workspace comes from a memory pool
+ * of the library's own, which keeps up to 256 MiB per device across synchronisations.  This
+ * gives back what is not in use beyond `keep_bytes` per device. */
+int polar_b200_trim_scratch(uint64_t keep_bytes);
 
 /* Number of kernels this library has launched since it was loaded (all
  * threads), for launch accounting in benchmarks. */

@@ -4,6 +4,7 @@
     python polarai-framework_b200/build.py --force    # ignore timestamps
 
 libpolar_b200.so    - the builtin kernels and their C ABI (include/polar_b200.h)
+polar_b200_torch.so - the builtins called with torch tensors (csrc/py), a CPython extension
 libpolar_rt_cuda.so - the PolarAI device-runtime plugin (initContext/closeContext)
                       built against the reference's runtime headers when the
                       reference tree is present (environment variable
@@ -23,7 +24,8 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-ccbin", "/usr/bin/g++"] + ARCH
 
-KERNEL_SOURCES = ["common.cu", "elementwise.cu", "extra_builtins.cu", "gemm_ffma.cu", "gemm_skinny.cu", "gemm_tc.cu", "peer_collective.cu", "dispatch.cu"]
+KERNEL_SOURCES = ["common.cu", "elementwise.cu", "extra_builtins.cu", "gemm_ffma.cu", "gemm_skinny.cu", "gemm_tc.cu", "peer_collective.cu", "dispatch.cu",
+                  "program.cu"]
 
 
 def _newer(src, dst, extra=()):
@@ -65,6 +67,27 @@ def build_kernels(force=False, verbose=False):
     lib = os.path.join(LIB, "libpolar_b200.so")
     if force or jobs or not os.path.exists(lib):
         _run([NVCC, "-shared", "-o", lib] + objs + ARCH + ["-ccbin", "/usr/bin/g++"])
+    return lib
+
+
+def build_binding(force=False):
+    """The CPython extension that calls the builtins with torch tensors."""
+    import sysconfig
+
+    import torch
+    src = os.path.join(CSRC, "py", "torch_binding.cpp")
+    lib = os.path.join(LIB, "polar_b200_torch.so")
+    if not (force or _newer(src, lib, (os.path.join(ROOT, "include", "polar_b200.h"),))):
+        return lib
+    tdir = os.path.dirname(torch.__file__)
+    inc = [sysconfig.get_paths()["include"], os.path.join(tdir, "include"),
+           os.path.join(tdir, "include", "torch", "csrc", "api", "include"), os.path.join(ROOT, "include"),
+           os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
+    _run(["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] +
+         [f for i in inc for f in ("-isystem", i)] +
+         ["-o", lib, src, "-L", LIB, "-lpolar_b200", "-L", os.path.join(tdir, "lib"), "-ltorch_python", "-ltorch",
+          "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
     return lib
 
 
@@ -226,7 +249,7 @@ def build_reference_host(force=False):
 
 
 def build_all(force=False, verbose=False):
-    libs = [build_kernels(force, verbose)]
+    libs = [build_kernels(force, verbose), build_binding(force)]
     rt = build_runtime(force)
     if rt:
         libs.append(rt)

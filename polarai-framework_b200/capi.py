@@ -29,6 +29,10 @@ class Arg(ctypes.Structure):
     _fields_ = [("is_tensor", _i), ("tensor", Tensor), ("scalar", _f), ("integer", ctypes.c_int64)]
 
 
+class Op(ctypes.Structure):
+    _fields_ = [("name", ctypes.c_char_p), ("args", ctypes.POINTER(Arg)), ("argc", _u64)]
+
+
 SIGNATURES = {
     "polar_b200_last_error": (ctypes.c_char_p, []),
     "polar_b200_version": (_i, []),
@@ -86,6 +90,11 @@ SIGNATURES = {
                                                  ctypes.c_uint32, _u64, _u64, _p, ctypes.c_uint32, _f, _f, _p]),
     "polar_b200_launch_by_name": (_i, [ctypes.c_char_p, ctypes.POINTER(Arg), _u64, _p, _u64, _p]),
     "polar_b200_launch_workspace_bytes": (_u64, [ctypes.c_char_p, ctypes.POINTER(Arg), _u64]),
+    "polar_b200_program_create": (_i, [ctypes.POINTER(Op), _u64, _p, _u64, ctypes.POINTER(_p)]),
+    "polar_b200_program_run": (_i, [_p, _p]),
+    "polar_b200_program_steps": (_u64, [_p]),
+    "polar_b200_program_destroy": (None, [_p]),
+    "polar_b200_trim_scratch": (_i, [_u64]),
     "polar_b200_launch_count": (_u64, []),
     "polar_b200_result_count": (_i, [ctypes.c_char_p]),
 }
@@ -121,6 +130,7 @@ class Library:
 
 
 _lib = None
+_binding = None
 
 
 def lib():
@@ -128,3 +138,21 @@ def lib():
     if _lib is None:
         _lib = Library()
     return _lib
+
+
+def binding():
+    """The CPython extension that calls the builtins with torch tensors (csrc/py/torch_binding.cpp)."""
+    global _binding
+    if _binding is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401 - its libraries must be loaded first
+        path = os.path.join(_HERE, "lib", "polar_b200_torch.so")
+        if not os.path.exists(path):
+            raise FileNotFoundError(f"{path} is not built; run `python polarai-framework_b200/build.py` (needs nvcc)")
+        loader = importlib.machinery.ExtensionFileLoader("polar_b200_torch", path)
+        spec = importlib.util.spec_from_file_location("polar_b200_torch", path, loader=loader)
+        _binding = importlib.util.module_from_spec(spec)
+        loader.exec_module(_binding)
+    return _binding

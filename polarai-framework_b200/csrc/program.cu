@@ -1,0 +1,464 @@
+// Builtin programs: a list of builtin launches, prepared once and run many times.
+//
+// What a small program costs is not its arithmetic but its launches: on B200 about 2.5 us of host time
+// each and 3 us of GPU time from one short kernel to the next.  Two things take them out:
+//
+//  - Consecutive elementwise builtins over the same element count become ONE launch (chain_kernel): each
+//    thread carries four elements through the whole chain.  Every tensor a builtin of the chain names as its
+//    result is still written, with the bits its own launch gives; what goes away is reading a
+//    tensor back that the same pass has just computed or read (the four-builtin chain of
+//    (a + b) * c / d -> sigmoid moves 32 instead of 44 bytes per element).
+//  - From its third run on, a program of several launches is replayed as a CUDA graph: one host call,
+//    and 1.5 us from kernel to kernel.  The first two runs are launched one by one, so that a program run
+//    once or twice never pays for the instantiation; a run under the caller's own stream capture is
+//    always launched one by one.
+#include <cstring>
+#include <mutex>
+#include <new>
+#include <string>
+#include <vector>
+
+#include "elementwise_ops.cuh"
+
+namespace polar_b200 {
+// dispatch.cu: while a thread captures a program, its forks take this stream set instead of the device's
+// shared one, which other threads may be using at the same time.
+bool use_capture_side_stream(bool on);
+
+namespace {
+
+constexpr int kChainThreads = 128;
+constexpr int kChainOps = 16;
+constexpr int kChainInputs = 8;
+constexpr uint8_t kPrevious = 0xff;   // operand = the result of the instruction before
+constexpr uint8_t kNoSlot = 0xff;
+
+enum Code : uint8_t { kFill, kCopy, kAdd, kMul, kDivide, kSigmoid, kLogLoss, kMulConcat, kRelu, kSigmoidGrad, kSigmoidLogLossGrad };
+
+struct ChainOp {
+  uint8_t code, a, b;      // operands: slot numbers (inputs first, then kept results), or kPrevious
+  uint8_t result;          // slot of the result, or kNoSlot
+  float s0, s1;            // fadd's scales, ffill's value
+  const float* scalar;     // fmulconcat's factor, in device memory
+  float* out;
+};
+struct ChainParams {
+  uint64_t n;
+  uint32_t inputs, ops;
+  const float* in[kChainInputs];
+  ChainOp op[kChainOps];
+};
+
+template <class Op>
+__device__ __forceinline__ float4 map4(Op op, float4 a, float4 b) {
+  return make_float4(op(a.x, b.x), op(a.y, b.y), op(a.z, b.z), op(a.w, b.w));
+}
+
+// A chain of elementwise builtins on one vector of four elements per thread.  HBM-bound for long vectors
+// (the interpreter's shared-memory traffic is 48 bytes per instruction and vector, a quarter of what
+// an SM can move in the time its share of HBM delivers the vector), one launch latency for short ones.
+// Values live in shared memory, [slot][thread]: a thread only ever touches its own column, so there
+// is no barrier, and consecutive lanes touch consecutive 16 bytes.
+// Measured, four-builtin chain: 2^20 elements 18.4 us as four launches, 3.6 us as one.
+__global__ void __launch_bounds__(kChainThreads) chain_kernel(const __grid_constant__ ChainParams p) {
+  extern __shared__ float4 slots[];
+  pdl_enter();
+  const uint64_t v = (uint64_t)blockIdx.x * kChainThreads + threadIdx.x;
+  const uint64_t e0 = v * 4;
+  if (e0 >= p.n) return;
+  const bool whole = e0 + 4 <= p.n;
+  const int left = whole ? 4 : (int)(p.n - e0);   // the last vector of an n that is no multiple of four
+  float4* mine = slots + threadIdx.x;
+  float4 first[kChainInputs];
+#pragma unroll
+  for (int i = 0; i < kChainInputs; ++i) {
+    if (i < (int)p.inputs) {
+      const float* src = p.in[i] + e0;
+      if (whole) {
+        first[i] = *reinterpret_cast<const float4*>(src);
+      } else {
+        first[i] = make_float4(src[0], left > 1 ? src[1] : 0.f, left > 2 ? src[2] : 0.f, 0.f);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kChainInputs; ++i)
+    if (i < (int)p.inputs) mine[i * kChainThreads] = first[i];
+  float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t i = 0; i < p.ops; ++i) {
+    const ChainOp& o = p.op[i];
+    const float4 a = o.a == kPrevious ? r : mine[o.a * kChainThreads];
+    const float4 b = o.b == kPrevious ? r : mine[o.b * kChainThreads];
+    switch (o.code) {   // the same for all threads
+      case kFill: r = make_float4(o.s0, o.s0, o.s0, o.s0); break;
+      case kCopy: r = a; break;
+      case kAdd: r = map4(ew::AddOp{o.s0, o.s1}, a, b); break;
+      case kMul: r = map4(ew::MulOp{}, a, b); break;
+      case kDivide: r = map4(ew::DivOp{}, a, b); break;
+      case kSigmoid: r = map4(ew::SigmoidOp<true>{}, a, a); break;
+      case kLogLoss: {
+        auto hard = [](float y) { return y == 0.0f || y == 1.0f; };
+        if (hard(b.x) && hard(b.y) && hard(b.z) && hard(b.w)) {
+          r = make_float4(ew::logloss_binary(a.x, b.x), ew::logloss_binary(a.y, b.y), ew::logloss_binary(a.z, b.z),
+                          ew::logloss_binary(a.w, b.w));
+        } else {
+          r = map4(ew::LogLossOp{}, a, b);
+        }
+        break;
+      }
+      case kMulConcat: r = map4(ew::ScaleByFirstOp{*o.scalar}, a, a); break;
+      case kRelu: r = map4(ew::ReluOp{}, a, a); break;
+      case kSigmoidGrad: r = map4(ew::SigmoidGradOp{}, a, b); break;
+      default: r = map4(ew::SigmoidLogLossGradOp{}, a, b); break;
+    }
+    if (o.result != kNoSlot) mine[o.result * kChainThreads] = r;
+    float* dst = o.out + e0;
+    if (whole) {
+      *reinterpret_cast<float4*>(dst) = r;
+    } else {
+      dst[0] = r.x;
+      if (left > 1) dst[1] = r.y;
+      if (left > 2) dst[2] = r.z;
+    }
+  }
+}
+
+// ---- host side
+
+struct Op {                    // one builtin, its argument list owned by the program
+  std::string name;
+  std::vector<polar_b200_arg> args;
+  std::vector<std::vector<uint64_t>> shapes;
+};
+struct Step {                  // one builtin, or a chain
+  int op = -1;
+  ChainParams chain;
+  size_t smem = 0;
+};
+struct Program {
+  std::vector<Op> ops;
+  std::vector<Step> steps;
+  const void* any_pointer = nullptr;
+  void* workspace = nullptr;
+  uint64_t workspace_bytes = 0;
+  std::mutex mu;
+  int runs = 0;
+  bool graph_failed = false;
+  cudaGraphExec_t graph = nullptr;
+  uint64_t graph_launches = 0;
+};
+
+uint64_t elements(const polar_b200_tensor& t) {
+  uint64_t n = 1;
+  for (uint64_t d = 0; d < t.dims; ++d) n *= t.shape[d];
+  return n;
+}
+
+// An elementwise builtin in the form the chain takes; false for anything else.
+struct Elementwise {
+  Code code;
+  uint64_t n;
+  const float* in[2] = {nullptr, nullptr};
+  const float* scalar = nullptr;
+  float s0 = 0.f, s1 = 0.f;
+  float* out;
+};
+bool elementwise(const Op& op, Elementwise* e) {
+  struct Form { const char* name; Code code; const char* args; };
+  static const Form forms[] = {
+      {"ffill", kFill, "fT"}, {"fcopy", kCopy, "TT"}, {"fadd", kAdd, "TfTfT"}, {"fmul", kMul, "TTT"}, {"fdivide", kDivide, "TTT"},
+      {"fsigmoid", kSigmoid, "TT"}, {"flogloss", kLogLoss, "TTT"}, {"fmulconcat", kMulConcat, "TTT"}, {"frelu", kRelu, "TT"},
+      {"fsigmoid_grad", kSigmoidGrad, "TTT"}, {"fsigmoid_logloss_grad", kSigmoidLogLossGrad, "TTT"}};
+  for (const Form& f : forms) {
+    if (op.name != f.name) continue;
+    if (op.args.size() != std::strlen(f.args)) return false;
+    const polar_b200_arg& result = op.args.back();
+    if (!result.is_tensor) return false;
+    e->code = f.code;
+    e->out = result.tensor.data;
+    e->n = elements(result.tensor);
+    if (e->n == 0 || e->n > (1ull << 40) || !e->out || !aligned16(e->out)) return false;
+    int tensors = 0, scalars = 0;
+    for (size_t i = 0; i + 1 < op.args.size(); ++i) {
+      const polar_b200_arg& a = op.args[i];
+      if ((f.args[i] == 'T') != (a.is_tensor != 0)) return false;
+      if (!a.is_tensor) {
+        (scalars++ == 0 ? e->s0 : e->s1) = a.scalar;
+      } else if (f.code == kMulConcat && tensors == 0 && !e->scalar) {
+        if (elements(a.tensor) < 1 || !a.tensor.data) return false;
+        e->scalar = a.tensor.data;
+      } else {
+        if (elements(a.tensor) != e->n || !a.tensor.data || !aligned16(a.tensor.data)) return false;
+        e->in[tensors++] = a.tensor.data;
+      }
+    }
+    return !(e->scalar && e->scalar >= e->out && e->scalar < e->out + e->n);
+  }
+  return false;
+}
+
+// Builds chains.  An instruction joins the open one when it covers the same number of elements and
+// nothing it touches overlaps what the chain touches other than as the same whole tensor: a thread
+// sees its own four elements only.
+class ChainBuilder {
+public:
+  bool add(const Elementwise& e) {
+    if (!ops_.empty() && (e.n != n_ || ops_.size() == kChainOps || !compatible(e))) return false;
+    size_t fresh = e.in[0] && find(e.in[0]) < 0;
+    fresh += e.in[1] && e.in[1] != e.in[0] && find(e.in[1]) < 0;
+    if (inputs_.size() + fresh > kChainInputs) return false;
+    n_ = e.n;
+    Entry t{e, {-1, -1}};
+    for (int i = 0; i < 2; ++i) {
+      if (!e.in[i]) continue;
+      int v = find(e.in[i]);
+      if (v < 0) {
+        inputs_.push_back(e.in[i]);
+        values_.push_back({e.in[i], false, (int)inputs_.size() - 1});
+        v = (int)values_.size() - 1;
+      }
+      t.operand[i] = v;
+    }
+    values_.push_back({e.out, true, (int)ops_.size()});
+    ops_.push_back(t);
+    return true;
+  }
+  size_t size() const { return ops_.size(); }
+  Step finish() {
+    Step s;
+    ChainParams& p = s.chain;
+    p.n = n_;
+    p.inputs = (uint32_t)inputs_.size();
+    p.ops = (uint32_t)ops_.size();
+    for (size_t i = 0; i < inputs_.size(); ++i) p.in[i] = inputs_[i];
+    // a result gets a slot when something later than the next instruction reads it
+    std::vector<int> slot_of(ops_.size(), -1);
+    size_t slots = inputs_.size();
+    for (size_t i = 0; i < ops_.size(); ++i)
+      for (int v : ops_[i].operand)
+        if (v >= 0 && values_[v].computed && values_[v].index + 1 != (int)i) slot_of[values_[v].index] = 0;
+    for (int& n : slot_of)
+      if (n == 0) n = (int)slots++;
+    for (size_t i = 0; i < ops_.size(); ++i) {
+      const Entry& t = ops_[i];
+      ChainOp& o = p.op[i];
+      o.code = t.e.code;
+      o.s0 = t.e.s0;
+      o.s1 = t.e.s1;
+      o.scalar = t.e.scalar;
+      o.out = t.e.out;
+      o.result = slot_of[i] < 0 ? kNoSlot : (uint8_t)slot_of[i];
+      auto operand = [&](int v) -> uint8_t {
+        if (v < 0) return kPrevious;                       // no such operand: any value will do
+        const Value& val = values_[v];
+        if (!val.computed) return (uint8_t)val.index;
+        return val.index + 1 == (int)i ? kPrevious : (uint8_t)slot_of[val.index];
+      };
+      o.a = operand(t.operand[0]);
+      o.b = t.operand[1] < 0 ? o.a : operand(t.operand[1]);
+    }
+    s.smem = slots * kChainThreads * sizeof(float4);
+    *this = ChainBuilder();
+    return s;
+  }
+
+private:
+  struct Entry { Elementwise e; int operand[2]; };
+  struct Value { const float* tensor; bool computed; int index; };   // index: input number, or instruction number
+  // The value the tensor holds at this point of the chain.
+  int find(const float* tensor) const {
+    for (int i = (int)values_.size() - 1; i >= 0; --i)
+      if (values_[i].tensor == tensor) return i;
+    return -1;
+  }
+  static bool overlap(const float* a, uint64_t na, const float* b, uint64_t nb) { return a < b + nb && b < a + na; }
+  bool compatible(const Elementwise& e) const {
+    auto partial = [&](const float* a, const float* b) { return a && b && a != b && overlap(a, n_, b, n_); };
+    for (const Value& v : values_) {
+      if (partial(e.in[0], v.tensor) || partial(e.in[1], v.tensor) || partial(e.out, v.tensor)) return false;
+      // fmulconcat's factor is read by every thread: nothing in the chain may write it
+      if (e.scalar && v.computed && overlap(e.scalar, 1, v.tensor, n_)) return false;
+    }
+    for (const Entry& t : ops_)
+      if (t.e.scalar && overlap(t.e.scalar, 1, e.out, n_)) return false;
+    return true;
+  }
+  uint64_t n_ = 0;
+  std::vector<const float*> inputs_;
+  std::vector<Value> values_;
+  std::vector<Entry> ops_;
+};
+
+void plan(Program* p) {
+  ChainBuilder chain;
+  int first = -1;                                          // the builtin a one-instruction chain stands for
+  auto flush = [&] {
+    if (chain.size() == 1) {
+      Step s;
+      s.op = first;
+      p->steps.push_back(s);
+      chain = ChainBuilder();
+    } else if (chain.size() > 1) {
+      p->steps.push_back(chain.finish());
+    }
+  };
+  for (size_t i = 0; i < p->ops.size(); ++i) {
+    Elementwise e;
+    const bool ok = elementwise(p->ops[i], &e);
+    if (!ok || !chain.add(e)) {
+      flush();
+      if (!ok || !chain.add(e)) {
+        Step s;
+        s.op = (int)i;
+        p->steps.push_back(s);
+        continue;
+      }
+    }
+    if (chain.size() == 1) first = (int)i;
+  }
+  flush();
+}
+
+int run_steps(Program* p, cudaStream_t stream) {
+  for (const Step& s : p->steps) {
+    int rc;
+    if (s.op >= 0) {
+      const Op& op = p->ops[s.op];
+      rc = polar_b200_launch_by_name(op.name.c_str(), op.args.data(), op.args.size(), p->workspace, p->workspace_bytes, stream);
+    } else {
+      const uint64_t vectors = (s.chain.n + 3) / 4, grid = (vectors + kChainThreads - 1) / kChainThreads;
+      if (grid > 0x7fffffffull) return fail(POLAR_B200_ERR_INVALID, "element count too large");
+      rc = launch("chain of elementwise builtins", chain_kernel, (unsigned)grid, kChainThreads, s.smem, stream, s.chain);
+    }
+    if (rc) return rc;
+  }
+  return POLAR_B200_OK;
+}
+
+// Captures one pass on a stream of the program's own and instantiates it.  Thread-local capture mode: other
+// threads may go on launching and allocating.
+bool make_graph(Program* p) {
+  static std::mutex one_at_a_time;                         // the capture side stream is one per device
+  std::lock_guard<std::mutex> guard(one_at_a_time);
+  cudaStream_t s = nullptr;
+  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  bool ok = false;
+  if (use_capture_side_stream(true) && cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    const int rc = run_steps(p, s);
+    cudaGraph_t g = nullptr;
+    const bool ended = cudaStreamEndCapture(s, &g) == cudaSuccess && g;
+    if (rc == POLAR_B200_OK && ended) {
+      ok = cudaGraphInstantiate(&p->graph, g, 0) == cudaSuccess;
+      size_t nodes = 0;
+      cudaGraphGetNodes(g, nullptr, &nodes);
+      std::vector<cudaGraphNode_t> list(nodes);
+      cudaGraphGetNodes(g, list.data(), &nodes);
+      p->graph_launches = 0;
+      for (cudaGraphNode_t n : list) {
+        cudaGraphNodeType type;
+        if (cudaGraphNodeGetType(n, &type) == cudaSuccess && type == cudaGraphNodeTypeKernel) p->graph_launches++;
+      }
+      count_launch(0 - p->graph_launches);                 // captured, not launched
+    }
+    if (g) cudaGraphDestroy(g);
+  }
+  use_capture_side_stream(false);
+  cudaGetLastError();
+  cudaStreamDestroy(s);
+  return ok;
+}
+
+}  // namespace
+}  // namespace polar_b200
+
+using namespace polar_b200;
+
+extern "C" {
+
+int polar_b200_program_create(const polar_b200_op* ops, uint64_t count, void* workspace, uint64_t workspace_bytes,
+                              void** program) {
+  clear_error();
+  if (!program || (count && !ops)) return fail(POLAR_B200_ERR_INVALID, "null program or operation list");
+  *program = nullptr;
+  Program* p = new (std::nothrow) Program;
+  if (!p) return fail(POLAR_B200_ERR_INVALID, "out of host memory");
+  for (uint64_t i = 0; i < count; ++i) {
+    const polar_b200_op& o = ops[i];
+    if (!o.name || (o.argc && !o.args)) {
+      delete p;
+      return fail(POLAR_B200_ERR_INVALID, "null kernel name or argument list");
+    }
+    Op op;
+    op.name = o.name;
+    op.args.assign(o.args, o.args + o.argc);
+    op.shapes.resize(o.argc);
+    for (uint64_t a = 0; a < o.argc; ++a) {
+      if (!o.args[a].is_tensor) continue;
+      const polar_b200_tensor& t = o.args[a].tensor;
+      if (t.dims && !t.shape) {
+        delete p;
+        return fail(POLAR_B200_ERR_INVALID, "tensor without a shape");
+      }
+      op.shapes[a].assign(t.shape, t.shape + t.dims);
+      if (!p->any_pointer) p->any_pointer = t.data;
+    }
+    p->ops.push_back(std::move(op));
+    Op& kept = p->ops.back();
+    for (uint64_t a = 0; a < o.argc; ++a)
+      if (kept.args[a].is_tensor) kept.args[a].tensor.shape = kept.shapes[a].data();
+  }
+  p->workspace = workspace;
+  p->workspace_bytes = workspace_bytes;
+  plan(p);
+  *program = p;
+  return POLAR_B200_OK;
+}
+
+int polar_b200_program_run(void* program, void* stream) {
+  clear_error();
+  Program* p = static_cast<Program*>(program);
+  if (!p) return fail(POLAR_B200_ERR_INVALID, "null program");
+  cudaStream_t st = as_stream(stream);
+  LaunchDeviceScope on(stream, p->any_pointer);
+  if (p->steps.size() > 1) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    // (a query on the legacy stream fails while some other stream is capturing: then launch one by one)
+    const bool eager = cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone;
+    if (eager) {
+      cudaGetLastError();
+    } else {
+      std::lock_guard<std::mutex> guard(p->mu);
+      if (p->runs < 2) {
+        ++p->runs;
+      } else if (!p->graph && !p->graph_failed) {
+        p->graph_failed = !make_graph(p);
+      }
+      if (p->graph) {
+        cudaError_t e = cudaGraphLaunch(p->graph, st);
+        if (e != cudaSuccess) {
+          cudaGetLastError();
+          return fail(POLAR_B200_ERR_CUDA, "cudaGraphLaunch", e);
+        }
+        count_launch(p->graph_launches);
+        return POLAR_B200_OK;
+      }
+    }
+  }
+  return run_steps(p, st);
+}
+
+uint64_t polar_b200_program_steps(const void* program) {
+  return program ? static_cast<const Program*>(program)->steps.size() : 0;
+}
+
+void polar_b200_program_destroy(void* program) {
+  Program* p = static_cast<Program*>(program);
+  if (!p) return;
+  if (p->graph) cudaGraphExecDestroy(p->graph);
+  delete p;
+}
+
+}  // extern "C"

@@ -4,11 +4,15 @@
 the benchmark times); `HostBuiltins` has the oracle's call signatures - numpy in,
 numpy out - and moves the data through the device, for the parity tests.
 torch is used for device memory and streams only.
+
+Each builtin first goes to the native binding (capi.binding), which checks its tensors
+and launches without the interpreter; what that declines - tensors it would reject, a failing
+call - runs the checked path below it, which raises.
 """
 import numpy as np
 import torch
 
-from .capi import lib
+from .capi import binding, lib
 
 
 def _ptr(t):
@@ -31,78 +35,92 @@ class DeviceBuiltins:
         if not torch.cuda.is_available():
             raise RuntimeError("no CUDA device: the PolarAI B200 builtins have no CPU path")
         self.lib = lib()
+        self._native = binding()
 
     def ffill(self, pattern, out):
-        _chk(out)
-        self.lib.call("polar_b200_ffill", float(pattern), _ptr(out), out.numel(), _stream(out))
+        if not self._native.ffill(pattern, out):
+            _chk(out)
+            self.lib.call("polar_b200_ffill", float(pattern), _ptr(out), out.numel(), _stream(out))
         return out
 
     def fcopy(self, a, out):
-        _chk(a, out)
-        self.lib.call("polar_b200_fcopy", _ptr(a), _ptr(out), out.numel(), _stream(out))
+        if not self._native.fcopy(a, out):
+            _chk(a, out)
+            self.lib.call("polar_b200_fcopy", _ptr(a), _ptr(out), out.numel(), _stream(out))
         return out
 
     def fadd(self, a, sa, b, sb, out):
-        _chk(a, b, out)
-        self.lib.call("polar_b200_fadd", _ptr(a), float(sa), _ptr(b), float(sb), _ptr(out), out.numel(),
-                      _stream(out))
+        if not self._native.fadd(a, sa, b, sb, out):
+            _chk(a, b, out)
+            self.lib.call("polar_b200_fadd", _ptr(a), float(sa), _ptr(b), float(sb), _ptr(out), out.numel(),
+                          _stream(out))
         return out
 
     def fmul(self, a, b, out):
-        _chk(a, b, out)
-        self.lib.call("polar_b200_fmul", _ptr(a), _ptr(b), _ptr(out), out.numel(), _stream(out))
+        if not self._native.fmul(a, b, out):
+            _chk(a, b, out)
+            self.lib.call("polar_b200_fmul", _ptr(a), _ptr(b), _ptr(out), out.numel(), _stream(out))
         return out
 
     def fdivide(self, a, b, out):
-        _chk(a, b, out)
-        self.lib.call("polar_b200_fdivide", _ptr(a), _ptr(b), _ptr(out), out.numel(), _stream(out))
+        if not self._native.fdivide(a, b, out):
+            _chk(a, b, out)
+            self.lib.call("polar_b200_fdivide", _ptr(a), _ptr(b), _ptr(out), out.numel(), _stream(out))
         return out
 
     def fsigmoid(self, a, out, clamp=True):
-        _chk(a, out)
-        name = "polar_b200_fsigmoid" if clamp else "polar_b200_fsigmoid_unclamped"
-        self.lib.call(name, _ptr(a), _ptr(out), out.numel(), _stream(out))
+        if not (self._native.fsigmoid if clamp else self._native.fsigmoid_unclamped)(a, out):
+            _chk(a, out)
+            name = "polar_b200_fsigmoid" if clamp else "polar_b200_fsigmoid_unclamped"
+            self.lib.call(name, _ptr(a), _ptr(out), out.numel(), _stream(out))
         return out
 
     def flogloss(self, predicted, ground_truth, out):
-        _chk(predicted, ground_truth, out)
-        self.lib.call("polar_b200_flogloss", _ptr(predicted), _ptr(ground_truth), _ptr(out), out.numel(),
-                      _stream(out))
+        if not self._native.flogloss(predicted, ground_truth, out):
+            _chk(predicted, ground_truth, out)
+            self.lib.call("polar_b200_flogloss", _ptr(predicted), _ptr(ground_truth), _ptr(out), out.numel(),
+                          _stream(out))
         return out
 
     def fmulconcat(self, gradient, local, out):
-        _chk(gradient, local, out)
-        self.lib.call("polar_b200_fmulconcat", _ptr(gradient), _ptr(local), _ptr(out), out.numel(), _stream(out))
+        if not self._native.fmulconcat(gradient, local, out):
+            _chk(gradient, local, out)
+            self.lib.call("polar_b200_fmulconcat", _ptr(gradient), _ptr(local), _ptr(out), out.numel(), _stream(out))
         return out
 
     def frelu(self, a, out):
-        _chk(a, out)
-        self.lib.call("polar_b200_frelu", _ptr(a), _ptr(out), out.numel(), _stream(out))
+        if not self._native.frelu(a, out):
+            _chk(a, out)
+            self.lib.call("polar_b200_frelu", _ptr(a), _ptr(out), out.numel(), _stream(out))
         return out
 
     def fsoftmax(self, a, out):
-        _chk(a, out)
-        self.lib.call("polar_b200_fsoftmax", _ptr(a), _ptr(out), out.numel(), None, 0, _stream(out))
+        if not self._native.fsoftmax(a, out):
+            _chk(a, out)
+            self.lib.call("polar_b200_fsoftmax", _ptr(a), _ptr(out), out.numel(), None, 0, _stream(out))
         return out
 
     def fpool(self, a, window, stride, out):
-        _chk(a, out)
-        h, w = a.shape
-        self.lib.call("polar_b200_fpool", _ptr(a), h, w, window[0], window[1], stride[0], stride[1], _ptr(out),
-                      _stream(out))
+        if not self._native.fpool(a, window[0], window[1], stride[0], stride[1], out):
+            _chk(a, out)
+            h, w = a.shape
+            self.lib.call("polar_b200_fpool", _ptr(a), h, w, window[0], window[1], stride[0], stride[1], _ptr(out),
+                          _stream(out))
         return out
 
     def fconv2d(self, a, kernel, out):
-        _chk(a, kernel, out)
-        h, w = a.shape
-        kh, kw = kernel.shape
-        self.lib.call("polar_b200_fconv2d", _ptr(a), h, w, _ptr(kernel), kh, kw, _ptr(out), _stream(out))
+        if not self._native.fconv2d(a, kernel, out):
+            _chk(a, kernel, out)
+            h, w = a.shape
+            kh, kw = kernel.shape
+            self.lib.call("polar_b200_fconv2d", _ptr(a), h, w, _ptr(kernel), kh, kw, _ptr(out), _stream(out))
         return out
 
     def ftranspose(self, a, out):
-        _chk(a, out)
-        rows, cols = a.shape
-        self.lib.call("polar_b200_ftranspose", _ptr(a), rows, cols, _ptr(out), _stream(out))
+        if not self._native.ftranspose(a, out):
+            _chk(a, out)
+            rows, cols = a.shape
+            self.lib.call("polar_b200_ftranspose", _ptr(a), rows, cols, _ptr(out), _stream(out))
         return out
 
     def fslice(self, a, index, out):
@@ -117,12 +135,13 @@ class DeviceBuiltins:
         return acc
 
     def fmatmul(self, tl, tr, left, right, out):
-        _chk(left, right, out)
-        m, n, k = matmul_dims(tl, tr, left.shape, right.shape)
-        if tuple(out.shape) != (m, n):
-            raise ValueError(f"out must be [{m},{n}]")
-        self.lib.call("polar_b200_fmatmul", int(tl), int(tr), m, n, k, _ptr(left), _ptr(right), _ptr(out),
-                      None, 0, _stream(out))
+        if not self._native.fmatmul(tl, tr, left, right, out):
+            _chk(left, right, out)
+            m, n, k = matmul_dims(tl, tr, left.shape, right.shape)
+            if tuple(out.shape) != (m, n):
+                raise ValueError(f"out must be [{m},{n}]")
+            self.lib.call("polar_b200_fmatmul", int(tl), int(tr), m, n, k, _ptr(left), _ptr(right), _ptr(out),
+                          None, 0, _stream(out))
         return out
 
     def fmatmul_ffma(self, tl, tr, left, right, out):

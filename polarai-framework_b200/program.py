@@ -20,7 +20,7 @@ from dataclasses import dataclass, field
 
 import torch
 
-from .capi import Arg, lib
+from .capi import Arg, Tensor, binding, lib
 
 
 @dataclass
@@ -338,9 +338,11 @@ def overlap_gradient_exchange(program, tile_rows=256):
 
 class DeviceExecutor:
     """Runs a Program on one GPU: one device tensor per program tensor, every op
-    through polar_b200_launch_by_name on torch's current stream.  Argument
-    structs are built once, so replaying the program costs one ctypes call per
-    launch.  `allreduce` is a callable taking a tensor (torch.distributed over
+    on torch's current stream.  The builtins between two exchanges are one native
+    program (polar_b200_program_create): a run is one call for all of them, consecutive
+    elementwise builtins share a launch, and a program that is run again and again is
+    replayed as a CUDA graph; every tensor still gets the bits that launching the builtins
+    one by one gives it.  `allreduce` is a callable taking a tensor (torch.distributed over
     NCCL in the data-parallel runs; None = single rank, no-op).  A program with an
     ALLREDUCE_FADD op needs `peers`, a PeerGradients built for program.exchanged():
     those gradients then live in its peer buffer."""
@@ -360,6 +362,11 @@ class DeviceExecutor:
         self.t = {n: (peers.tensors[n] if n in exchanged else torch.empty(s, dtype=torch.float32, device=self.device))
                   for n, s in program.tensors.items()}
         self._keep = []
+        described = {}
+        for n, tt in self.t.items():
+            shp = (ctypes.c_uint64 * tt.dim())(*tt.shape)
+            self._keep.append(shp)
+            described[n] = Tensor(tt.data_ptr(), tt.dim(), shp)
         self._compiled = []
         fn = self.lib.cdll.polar_b200_launch_by_name
         for kernel, args in program.ops:
@@ -377,19 +384,12 @@ class DeviceExecutor:
                                                       float(args[1])), 0))
                 continue
             arr = (Arg * len(args))()
-            for i, a in enumerate(args):
+            for x, a in zip(arr, args):
                 if isinstance(a, str):
-                    tt = self.t[a]
-                    shp = (ctypes.c_uint64 * tt.dim())(*tt.shape)
-                    self._keep.append(shp)
-                    arr[i].is_tensor = 1
-                    arr[i].tensor.data = tt.data_ptr()
-                    arr[i].tensor.dims = tt.dim()
-                    arr[i].tensor.shape = shp
+                    x.is_tensor = 1
+                    x.tensor = described[a]
                 else:
-                    arr[i].is_tensor = 0
-                    arr[i].scalar = float(a)
-            self._keep.append(arr)
+                    x.scalar = float(a)
             self._compiled.append((kernel.encode(), arr, len(args)))
         self._fn = fn
         # an exchange marked "overlapped" runs on a second stream, forked from the launch stream where
@@ -399,11 +399,42 @@ class DeviceExecutor:
             self._side = torch.cuda.Stream(self.device)
             self._fork, self._join = torch.cuda.Event(), torch.cuda.Event()
         # one scratch buffer, sized for the most demanding launch of the program
-        wsb = self.lib.cdll.polar_b200_launch_workspace_bytes
-        need = max([0] + [int(wsb(k, arr, n)) for k, arr, n in self._compiled if isinstance(k, bytes)])
+        native = binding()
+        need = native.workspace_bytes([(k, ctypes.addressof(arr), n) for k, arr, n in self._compiled
+                                       if isinstance(k, bytes)])
         self.workspace = torch.empty(max(need, 16), dtype=torch.uint8, device=self.device)
         self._ws_ptr, self._ws_bytes = self.workspace.data_ptr(), need
+        self._index = self.device.index if self.device.index is not None else torch.cuda.current_device()
+        self._run_native = native.run_program
+        self._segments = self._build_segments(native)
+        # the common case, nothing but builtins: run() is one native call
+        self._only = self._segments[0][1] if len(self._segments) == 1 and self._segments[0][0] == "builtins" else None
         self.fill_constants()
+
+    def _build_segments(self, native):
+        """The program as a list of ("builtins", native handle) and the exchange ops between them."""
+        segments, ops = [], []
+
+        def flush():
+            if ops:
+                status, handle = native.create_program(ops, self._ws_ptr, self._ws_bytes)
+                self.lib.check(status)
+                segments.append(("builtins", handle))
+                ops.clear()
+
+        for kernel, arr, n in self._compiled:
+            if isinstance(kernel, bytes):
+                ops.append((kernel, ctypes.addressof(arr), n))
+            elif kernel is not None or self.allreduce is not None:
+                flush()
+                segments.append((kernel, arr))
+        flush()
+        return segments
+
+    def __del__(self):
+        for kind, what in getattr(self, "_segments", ()):
+            if kind == "builtins":
+                self.lib.cdll.polar_b200_program_destroy(what)
 
     def fill_constants(self):
         s = torch.cuda.current_stream(self.device).cuda_stream
@@ -415,19 +446,23 @@ class DeviceExecutor:
             self.t[name].copy_(a if isinstance(a, torch.Tensor) else torch.from_numpy(a))
 
     def run(self):
+        if self._only is not None:
+            rc = self._run_native(self._only, self._index)
+            if rc:
+                self.lib.check(rc)
+            return
         main = torch.cuda.current_stream(self.device)
         s = main.cuda_stream
         forked = False
-        for kernel, arr, n in self._compiled:
-            if kernel is None:
-                if self.allreduce is not None:
-                    self.allreduce(self.t[arr])
-                continue
-            if kernel == "peers":
-                self.peers.launch(arr[0], arr[1], arr[2], s)
-                continue
-            if kernel == "peers_part":
-                seg, first, count, channel, overlapped, sw, sg = arr
+        for kind, what in self._segments:
+            if kind == "builtins":
+                self.lib.check(self._run_native(what, self._index))
+            elif kind is None:
+                self.allreduce(self.t[what])
+            elif kind == "peers":
+                self.peers.launch(what[0], what[1], what[2], s)
+            else:
+                seg, first, count, channel, overlapped, sw, sg = what
                 if overlapped:
                     self._fork.record(main)
                     self._side.wait_event(self._fork)
@@ -435,10 +470,6 @@ class DeviceExecutor:
                     forked = True
                 else:
                     self.peers.launch_range(channel, first, count, seg, sw, sg, s)
-                continue
-            rc = self._fn(kernel, arr, n, self._ws_ptr, self._ws_bytes, s)
-            if rc != 0:
-                self.lib.check(rc)
         if forked:
             self._join.record(self._side)
             main.wait_event(self._join)
