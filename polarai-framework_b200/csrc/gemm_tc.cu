@@ -149,7 +149,7 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_gen + C::kTileBytes + 8 * (3 * S + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const uint32_t num_kb = (uint32_t)((p.k + BK - 1) / BK);
   // Work comes in pieces (PieceWalk): a (tile, split) unit with a fixed share of the k slabs,
@@ -161,12 +161,12 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(full_raw(s), 1);
-      mbar_init(full_lo(s), kSplitWarps * 32);
+      mbar_init(full_lo(s), kSplitWarps);
       mbar_init(empty(s), 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(acc_full(a), 1);
-      mbar_init(acc_empty(a), (kEpilogueWarps + (MT == 2 ? kSplitWarps : 0)) * 32);
+      mbar_init(acc_empty(a), kEpilogueWarps + (MT == 2 ? kSplitWarps : 0));
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -178,7 +178,7 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);   // (known to be uniform)
 
   // Drains row sub-tiles [h0, h1) of the finished piece in accumulator buffer `as` for lane
   // quarter q (a warp may only touch tensor-memory lanes [32*(warp%4), +32)) and one half of
@@ -268,8 +268,10 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      uint32_t it = 0;   // k slabs issued so far, over all tiles of this CTA
+    const bool leader = elect_one();
+    {
+      int s = 0;
+      uint32_t ph = 1;
       bool ok = true;
       PieceWalk walk = make_walk();
       Piece pc;
@@ -279,45 +281,47 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         // a column half of a tile: half of the B slab, at the start of the stage's B area
         const int bn_now = pc.half ? BN / 2 : BN;
         if (pc.half == 2) n0 += BN / 2;
-        for (uint32_t kb = pc.kb0, kb_end = pc.kb1; kb < kb_end; ++kb, ++it) {
-          const int s = it % S;
-          const uint32_t ph = (it / S) & 1u;
-          if (!mbar_wait(empty(s), ph ^ 1u, abort_flag, p.status, 101, p.wait_ns)) { ok = false; break; }
+        for (uint32_t kb = pc.kb0, kb_end = pc.kb1; kb < kb_end; ++kb) {
+          if (!mbar_wait(empty(s), ph, abort_flag, p.status, 101, p.wait_ns)) { ok = false; break; }
           const uint32_t stage = smem_base + s * C::kStageBytes;
-          mbar_expect_tx(full_raw(s), C::kABytes + (pc.half ? C::kBBytes / 2 : C::kBBytes));
-          const int k0 = (int)(kb * BK);
-          // The TMA unit takes 50-100 ns per instruction whatever its size, so a slab comes in as few
-          // boxes as possible: an MN-major slab, 32-element chunks of BK rows each, in one or two 3-D
-          // boxes of 4 or 8 chunks.  (As one 2-D box per chunk - 16 instructions for a 256 x 256 x 16
-          // slab of a t_f product, 0.85 us - TMA was slower than the slab's three products, 0.8 us:
-          // measured 5.7 TB/s in 2 KB boxes, 17 TB/s in 16 KB ones.)  A contiguous extent that is no
-          // multiple of 32 still takes the 2-D boxes, whose reads TMA cuts off at the extent.
-          if (!p.a_mn_major) {
-            tma_load_2d(stage, &map_a, full_raw(s), k0, m0);           // box {BK k, kTileM m}
-          } else if (p.a_chunked) {
-            tma_load_3d(stage, &map_a, full_raw(s), 0, k0, m0 / 32);  // box {32 m, BK k, kTileM / 32}
-          } else {
-            for (int c = 0; c < kTileM / 32; ++c)                      // boxes {32 m, BK k}
-              tma_load_2d(stage + c * C::kBoxBytes, &map_a, full_raw(s), m0 + 32 * c, k0);
+          if (leader) {
+            mbar_expect_tx(full_raw(s), C::kABytes + (pc.half ? C::kBBytes / 2 : C::kBBytes));
+            const int k0 = (int)(kb * BK);
+            // The TMA unit takes 50-100 ns per instruction whatever its size, so a slab comes in as few
+            // boxes as possible: an MN-major slab, 32-element chunks of BK rows each, in one or two 3-D
+            // boxes of 4 or 8 chunks.  (As one 2-D box per chunk - 16 instructions for a 256 x 256 x 16
+            // slab of a t_f product, 0.85 us - TMA was slower than the slab's three products, 0.8 us:
+            // measured 5.7 TB/s in 2 KB boxes, 17 TB/s in 16 KB ones.)  A contiguous extent that is no
+            // multiple of 32 still takes the 2-D boxes, whose reads TMA cuts off at the extent.
+            if (!p.a_mn_major) {
+              tma_load_2d(stage, &map_a, full_raw(s), k0, m0);           // box {BK k, kTileM m}
+            } else if (p.a_chunked) {
+              tma_load_3d(stage, &map_a, full_raw(s), 0, k0, m0 / 32);  // box {32 m, BK k, kTileM / 32}
+            } else {
+              for (int c = 0; c < kTileM / 32; ++c)                      // boxes {32 m, BK k}
+                tma_load_2d(stage + c * C::kBoxBytes, &map_a, full_raw(s), m0 + 32 * c, k0);
+            }
+            const uint32_t bdst = stage + C::kABytes;
+            if (!p.b_mn_major) {
+              for (int c = 0; c < bn_now / C::kBBoxRows; ++c)            // boxes {BK k, 128 n}
+                tma_load_2d(bdst + c * (C::kBBoxRows * BK * 4), &map_b, full_raw(s), k0, n0 + C::kBBoxRows * c);
+            } else if (p.b_chunked) {
+              for (int c = 0; c < bn_now / C::kBBoxRows; ++c)            // boxes {32 n, BK k, 4}
+                tma_load_3d(bdst + c * (C::kBBoxRows * BK * 4), &map_b, full_raw(s), 0, k0,
+                            (n0 + C::kBBoxRows * c) / 32);
+            } else {
+              for (int c = 0; c < bn_now / 32; ++c)                      // boxes {32 n, BK k}
+                tma_load_2d(bdst + c * C::kBoxBytes, &map_b, full_raw(s), n0 + 32 * c, k0);
+            }
           }
-          const uint32_t bdst = stage + C::kABytes;
-          if (!p.b_mn_major) {
-            for (int c = 0; c < bn_now / C::kBBoxRows; ++c)            // boxes {BK k, 128 n}
-              tma_load_2d(bdst + c * (C::kBBoxRows * BK * 4), &map_b, full_raw(s), k0, n0 + C::kBBoxRows * c);
-          } else if (p.b_chunked) {
-            for (int c = 0; c < bn_now / C::kBBoxRows; ++c)            // boxes {32 n, BK k, 4}
-              tma_load_3d(bdst + c * (C::kBBoxRows * BK * 4), &map_b, full_raw(s), 0, k0,
-                          (n0 + C::kBBoxRows * c) / 32);
-          } else {
-            for (int c = 0; c < bn_now / 32; ++c)                      // boxes {32 n, BK k}
-              tma_load_2d(bdst + c * C::kBoxBytes, &map_b, full_raw(s), n0 + 32 * c, k0);
-          }
+          if (++s == S) s = 0, ph ^= 1;
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    const bool leader = elect_one();
+    {
       const uint32_t idesc_whole = make_idesc(BM, BN, p.a_mn_major, p.b_mn_major);
       const uint32_t idesc_half = make_idesc(BM, BN / 2, p.a_mn_major, p.b_mn_major);
       // K-major: rows of BK floats (128 or 64 bytes, swizzled over that span:
@@ -328,11 +332,15 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       // 32-element chunks of m/n one TMA box apart (LBO); a k step of 8 = +1024 B.
       constexpr uint32_t kRowGroup = 8u * BK * 4u;
       constexpr uint32_t kKMajorLayout = (BK == 32) ? 2u : 4u;
-      const uint32_t a_lbo = p.a_mn_major ? C::kBoxBytes : 16u, a_step = p.a_mn_major ? 1024u : 32u;
-      const uint32_t b_lbo = p.b_mn_major ? C::kBoxBytes : 16u, b_step = p.b_mn_major ? 1024u : 32u;
-      const uint32_t a_sbo = p.a_mn_major ? 512u : kRowGroup, a_lt = p.a_mn_major ? 1u : kKMajorLayout;
-      const uint32_t b_sbo = p.b_mn_major ? 512u : kRowGroup, b_lt = p.b_mn_major ? 1u : kKMajorLayout;
-      uint32_t it = 0, tile_iter = 0;
+      const Operand a_op = make_desc(0, p.a_mn_major ? C::kBoxBytes : 16u, p.a_mn_major ? 512u : kRowGroup,
+                                     p.a_mn_major ? 1u : kKMajorLayout);
+      const Operand b_op = make_desc(0, p.b_mn_major ? C::kBoxBytes : 16u, p.b_mn_major ? 512u : kRowGroup,
+                                     p.b_mn_major ? 1u : kKMajorLayout);
+      const uint32_t a_step = (p.a_mn_major ? 1024u : 32u) >> 4, b_step = (p.b_mn_major ? 1024u : 32u) >> 4;
+      constexpr uint32_t kSub = C::kASubBytes >> 4;
+      int s = 0;
+      uint32_t ph = 0;
+      uint32_t tile_iter = 0;
       bool ok = true;
       PieceWalk walk = make_walk();
       Piece pc;
@@ -345,97 +353,93 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         if (!ok) break;
         tc_fence_after();
         const uint32_t idesc = pc.half ? idesc_half : idesc_whole;   // a column half: 128-column MMAs
-        const uint32_t kb_first = pc.kb0;
-        for (uint32_t kb = kb_first, kb_end = pc.kb1; kb < kb_end; ++kb, ++it) {
-          const int s = it % S;
-          const uint32_t ph = (it / S) & 1u;
+        uint32_t accumulate = 0;
+        for (uint32_t kb = pc.kb0, kb_end = pc.kb1; kb < kb_end; ++kb, accumulate = 1) {
           ok = mbar_wait(full_raw(s), ph, abort_flag, p.status, 102, p.wait_ns);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t a_hi = smem_base + s * C::kStageBytes;
-          const uint32_t b_hi = a_hi + C::kABytes;
-          const uint32_t a_lo = a_hi + C::kRawBytes;
-          const uint32_t b_lo = b_hi + C::kRawBytes;
+          const uint32_t a_hi = ((smem_base & 0x3FFFFu) + s * C::kStageBytes) >> 4, b_hi = a_hi + (C::kABytes >> 4);
+          const uint32_t a_lo = a_hi + (C::kRawBytes >> 4), b_lo = b_hi + (C::kRawBytes >> 4);
           // hi*hi needs only what TMA delivered: issue it while the split warps work
+          if (leader) {
 #pragma unroll
-          for (int kk = 0; kk < BK / 8; ++kk) {
-            const uint64_t db_hi = make_desc(b_hi + kk * b_step, b_lbo, b_sbo, b_lt);
+            for (int kk = 0; kk < BK / 8; ++kk)
 #pragma unroll
-            for (int h = 0; h < MT; ++h) {
-              const uint64_t da_hi = make_desc(a_hi + h * C::kASubBytes + kk * a_step, a_lbo, a_sbo, a_lt);
-              tc_mma_tf32(tmem_base + acc_col(as, h), da_hi, db_hi, idesc,
-                          ((kb - kb_first) | (uint32_t)kk) ? 1u : 0u);
-            }
+              for (int h = 0; h < MT; ++h)
+                tc_mma_tf32(tmem_base + acc_col(as, h), a_op, a_hi + h * kSub + kk * a_step, b_op, b_hi + kk * b_step, idesc,
+                            kk ? 1u : accumulate);
           }
           if (p.passes == 3) {
             ok = mbar_wait(full_lo(s), ph, abort_flag, p.status, 103, p.wait_ns);
             if (!ok) break;
             tc_fence_after();
+            if (leader) {
 #pragma unroll
-            for (int kk = 0; kk < BK / 8; ++kk) {
-              const uint64_t db_hi = make_desc(b_hi + kk * b_step, b_lbo, b_sbo, b_lt);
-              const uint64_t db_lo = make_desc(b_lo + kk * b_step, b_lbo, b_sbo, b_lt);
+              for (int kk = 0; kk < BK / 8; ++kk)
 #pragma unroll
-              for (int h = 0; h < MT; ++h) {
-                const uint32_t sub = h * C::kASubBytes + kk * a_step;
-                const uint64_t da_hi = make_desc(a_hi + sub, a_lbo, a_sbo, a_lt);
-                const uint64_t da_lo = make_desc(a_lo + sub, a_lbo, a_sbo, a_lt);
-                tc_mma_tf32(tmem_base + acc_col(as, h), da_lo, db_hi, idesc, 1u);
-                tc_mma_tf32(tmem_base + acc_col(as, h), da_hi, db_lo, idesc, 1u);
-              }
+                for (int h = 0; h < MT; ++h) {
+                  tc_mma_tf32(tmem_base + acc_col(as, h), a_op, a_lo + h * kSub + kk * a_step, b_op, b_hi + kk * b_step, idesc, 1u);
+                  tc_mma_tf32(tmem_base + acc_col(as, h), a_op, a_hi + h * kSub + kk * a_step, b_op, b_lo + kk * b_step, idesc, 1u);
+                }
             }
           }
-          if (p.passes == 13) {
+          if (p.passes == 13 && leader) {
             // diagnostic: the issue rate of three products per slab with no split
             // pass at all (the result is 3 x the plain TF32 product)
 #pragma unroll
-            for (int kk = 0; kk < BK / 8; ++kk) {
-              const uint64_t db_hi = make_desc(b_hi + kk * b_step, b_lbo, b_sbo, b_lt);
+            for (int kk = 0; kk < BK / 8; ++kk)
 #pragma unroll
-              for (int h = 0; h < MT; ++h) {
-                const uint64_t da_hi = make_desc(a_hi + h * C::kASubBytes + kk * a_step, a_lbo, a_sbo, a_lt);
-                tc_mma_tf32(tmem_base + acc_col(as, h), da_hi, db_hi, idesc, 1u);
-                tc_mma_tf32(tmem_base + acc_col(as, h), da_hi, db_hi, idesc, 1u);
-              }
-            }
+              for (int h = 0; h < MT; ++h)
+                for (int r = 0; r < 2; ++r)
+                  tc_mma_tf32(tmem_base + acc_col(as, h), a_op, a_hi + h * kSub + kk * a_step, b_op, b_hi + kk * b_step, idesc, 1u);
           }
-          tc_commit(empty(s));   // frees the stage once these MMAs have read it
+          if (leader) tc_commit(empty(s));   // frees the stage once these MMAs have read it
+          if (++s == S) s = 0, ph ^= 1;
         }
-        if (ok) tc_commit(acc_full(as));
+        if (ok && leader) tc_commit(acc_full(as));
       }
     }
   } else if (warp < 2 + kSplitWarps) {
     // ---------------- split warps ----------------
     const int tid = threadIdx.x - 64;  // 0..255
     if (p.passes == 3 || MT == 2) {
-      uint32_t it = 0, tile_iter = 0;
+      int s = 0;
+      uint32_t ph = 0, tile_iter = 0;
       bool ok = true;
       PieceWalk walk = make_walk();
       Piece pc;
       for (; ok && walk.next(pc); ++tile_iter) {
-        for (uint32_t kb = pc.kb0, kb_end = pc.kb1; p.passes == 3 && kb < kb_end; ++kb, ++it) {
-          const int s = it % S;
-          const uint32_t ph = (it / S) & 1u;
+        for (uint32_t kb = pc.kb0, kb_end = pc.kb1; p.passes == 3 && kb < kb_end; ++kb) {
           if (!mbar_wait(full_raw(s), ph, abort_flag, p.status, 104, p.wait_ns)) { ok = false; break; }
           float4* raw = reinterpret_cast<float4*>(smem_gen + s * C::kStageBytes);
           float4* lo = reinterpret_cast<float4*>(smem_gen + s * C::kStageBytes + C::kRawBytes);
           constexpr int kVecs = C::kRawBytes / 16;
           static_assert(kVecs % (kSplitWarps * 32) == 0, "slab must divide over the split warps");
+          // all loads before the first store: the compiler cannot tell that the two never meet, and would
+          // make one latency of each vector
+          constexpr int kMine = kVecs / (kSplitWarps * 32), kHalf = kMine > 4 ? kMine / 2 : kMine;
+          static_assert(kMine % kHalf == 0, "split in equal batches");
+          for (int i0 = 0; i0 < kMine; i0 += kHalf) {
+            float4 v[kHalf];
 #pragma unroll
-          for (int i = 0; i < kVecs / (kSplitWarps * 32); ++i) {
-            const int e = tid + i * kSplitWarps * 32;
-            float4 v = raw[e];
-            float4 h;
-            h.x = __uint_as_float(__float_as_uint(v.x) & 0xFFFFE000u);
-            h.y = __uint_as_float(__float_as_uint(v.y) & 0xFFFFE000u);
-            h.z = __uint_as_float(__float_as_uint(v.z) & 0xFFFFE000u);
-            h.w = __uint_as_float(__float_as_uint(v.w) & 0xFFFFE000u);
-            float4 l = {v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w};
-            lo[e] = l;
-            if (p.write_hi == 1) raw[e] = h;
+            for (int i = 0; i < kHalf; ++i) v[i] = raw[tid + (i0 + i) * kSplitWarps * 32];
+#pragma unroll
+            for (int i = 0; i < kHalf; ++i) {
+              const int e = tid + (i0 + i) * kSplitWarps * 32;
+              float4 h;
+              h.x = __uint_as_float(__float_as_uint(v[i].x) & 0xFFFFE000u);
+              h.y = __uint_as_float(__float_as_uint(v[i].y) & 0xFFFFE000u);
+              h.z = __uint_as_float(__float_as_uint(v[i].z) & 0xFFFFE000u);
+              h.w = __uint_as_float(__float_as_uint(v[i].w) & 0xFFFFE000u);
+              lo[e] = make_float4(v[i].x - h.x, v[i].y - h.y, v[i].z - h.z, v[i].w - h.w);
+              if (p.write_hi == 1) raw[e] = h;
+            }
           }
           fence_async_smem();
-          mbar_arrive(full_lo(s));
+          // one arrival per warp
+          __syncwarp();
+          if (lane == 0) mbar_arrive(full_lo(s));
+          if (++s == S) s = 0, ph ^= 1;
         }
         if (MT == 2 && ok) {
           // 256-row tiles: nothing is left to split until this tile is drained, so these
@@ -444,7 +448,8 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           tc_fence_after();
           drain(pc, 0, 1, 2, warp & 3, (warp - 2) >> 2);
           tc_fence_before();
-          mbar_arrive(acc_empty(0));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty(0));
         }
       }
     }
@@ -465,7 +470,8 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       tc_fence_after();
       drain(pc, as, 0, 1, q, half);
       tc_fence_before();
-      mbar_arrive(acc_empty(as));   // this accumulator may be overwritten
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty(as));   // this accumulator may be overwritten
     }
   }
 
@@ -508,7 +514,7 @@ static EncodeTiledFn get_encode() {
 // `pitch` (floats between consecutive outer rows; 0 = inner) lets a map cover the first
 // `inner` columns of a wider stored matrix.
 int make_map(CUtensorMap* map, const float* base, uint64_t inner, uint64_t outer,
-                    uint32_t box_inner, uint32_t box_outer, bool mn_major, int bk, uint64_t pitch = 0) {
+                    uint32_t box_inner, uint32_t box_outer, bool mn_major, int bk, uint64_t pitch) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return fail(POLAR_B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
   cuuint64_t dims[2] = {inner, outer};
@@ -698,9 +704,9 @@ static int launch_cfg(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const 
                    : make_map(&map_a, left, m, k, 32, BK, true, BK, left_pitch);
   if (rc) return rc;
   // right: stored [n,k] when transposed (K-major: inner k, box {BK, 128}) or [k,n] (MN-major)
-  rc = tr ? make_map(&map_b, right, k, n, BK, C::kBBoxRows, false, BK)
+  rc = tr ? make_map(&map_b, right, k, n, BK, C::kBBoxRows, false, BK, 0)
        : b_chunked ? make_map_chunks(&map_b, right, n / 32, k, BK, C::kBBoxRows / 32, n)
-                   : make_map(&map_b, right, n, k, 32, BK, true, BK);
+                   : make_map(&map_b, right, n, k, 32, BK, true, BK, 0);
   if (rc) return rc;
   Params p;
   p.m = m; p.n = n; p.k = k; p.out = out;

@@ -27,12 +27,23 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(bar), "r"(parity)
+      : "r"(bar), "r"(parity), "r"(10000u)   // the hardware may park the warp for up to 10 us: a polling warp takes issue slots
       : "memory");
   return ok != 0;
+}
+
+// The warp's number as a value the compiler knows to be the same for all lanes, and one lane of the warp.  A role that
+// issues tcgen05 or TMA instructions runs its loop on the WHOLE warp and only the instructions themselves on
+// one lane: their operands then live in uniform registers.  In a loop of a single lane every operand had to be moved
+// there first, 51 clocks per tcgen05.mma and 465 per loop pass - the tensor core needs 64 to 128 for the instruction.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
 }
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -44,16 +55,18 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // Bounded wait: gives up after `limit_ns` nanoseconds of polling (the host's setting, two
 // seconds unless changed with polar_b200_set_wait_limit_ns), records `code` in the device's
 // status word (the first code wins) and raises the CTA's abort flag.  Returns false when the
-// CTA is aborting.  The clock is read once per 256 polls.
+// CTA is aborting.  The clock is first read after 64 polls, and once per 64 from then on: reading
+// %globaltimer on every wait that was not satisfied at once cost more than most of the waits.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code, unsigned long long limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long start = global_ns();
+  unsigned long long start = 0;
   for (uint32_t it = 1;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 255u) == 0) {
+    if ((it & 63u) == 0) {
       if (*abort_flag) return false;
-      if (global_ns() - start > limit_ns) {
+      const unsigned long long now = global_ns();
+      if (start == 0) start = now;
+      if (now - start > limit_ns) {
         *abort_flag = 1;
         atomicCAS(status, 0, code);
         return false;
@@ -100,15 +113,6 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
 }
-__device__ __forceinline__ void tc_mma_tf32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                            uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // 32 lanes x 32 consecutive fp32 columns: thread t gets row (lane base + t).
 // One 256-bit store (sm_100): eight consecutive floats, 32-byte aligned.
 __device__ __forceinline__ void st_global_v8(float* dst, const uint32_t* r) {
@@ -127,6 +131,17 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t* r) {
         "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
         "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
         "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+// The same for 16 columns.
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
 }
@@ -153,6 +168,26 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
   return d;
 }
 
+// An operand of tcgen05.mma: make_desc(0, ...), to which an instruction adds its address (the low 18 bits of the
+// shared address, in 16-byte units): the
+// fields above the address do not change from one instruction to the next, so an operand costs its issuing thread one addition.  (Built from
+// scratch, the 12 to 24 descriptors of a slab took the one issuing thread longer than the tensor core took
+// for their products.)
+struct Operand {
+  uint32_t lo, hi;
+  __device__ __forceinline__ Operand(uint64_t desc) : lo((uint32_t)desc), hi((uint32_t)(desc >> 32)) {}
+};
+__device__ __forceinline__ void tc_mma_tf32(uint32_t d_tmem, Operand a, uint32_t a_units, Operand b, uint32_t b_units,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %2};\n\t"
+      "mov.b64 db, {%3, %4};\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %5, p;\n\t}"
+      ::"r"(d_tmem), "r"(a.lo + a_units), "r"(a.hi), "r"(b.lo + b_units), "r"(b.hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // Instruction descriptor for kind::tf32: fp32 accumulate (bits 4-5 = 1), A and B
 // formats TF32 (2 at bits 7-9 and 10-12), major bits 15/16 (1 = MN-major), N/8 at
 // bits 17-22, M/16 at bits 24-28.
