@@ -219,8 +219,8 @@ int polar_b200_fmatmul_tn_small_n_static(int transRight, uint64_t m, uint64_t n,
 uint64_t polar_b200_static_scratch_bytes(void);
 
 /* The same product on the CUDA cores: one FFMA per term, k ascending per
- * output within a thread.  Kept only as a device-side cross-check of the
- * tensor-core path; no dispatch reaches it unless a caller asks for it. */
+ * output within a thread.  The device-side cross-check of the tensor-core paths; the
+ * dispatch takes it for the smallest products only. */
 int polar_b200_fmatmul_ffma(int transLeft, int transRight, uint64_t m,
                             uint64_t n, uint64_t k, const float* left,
                             const float* right, float* out, void* stream);
@@ -236,7 +236,9 @@ int polar_b200_fmatmul_ffma(int transLeft, int transRight, uint64_t m,
  * units the k range of each tile is cut into (1 = none, 0 = the automatic choice,
  * -1 = stream mode: the CTAs take equal shares of all k slabs of all tiles and a tile
  * may be finished by the next CTA - 128 x 256 tiles only; scratch for the partial
- * products comes from the stream-ordered pool).  Fails with
+ * products comes from the stream-ordered pool).  tile_n 2032, 2064 or 2128: one 128 x 32/64/128
+ * tile per cluster of `splits` = 1, 2, 4 or 8 CTAs (+ 1000: exchanged roles; write_hi == 1: the rounded split
+ * with short sums), for operands of any alignment.  Fails with
  * POLAR_B200_ERR_UNSUPPORTED when the operands cannot be described to TMA
  * (bases not 16-byte aligned, or a contiguous extent that is not a multiple of
  * 4 floats). */
@@ -269,8 +271,10 @@ void polar_b200_set_wait_limit_ns(uint64_t ns);
 uint64_t polar_b200_wait_limit_ns(void);
 
 /* Which matmul path polar_b200_fmatmul would take for these sizes:
- * 0 = tcgen05 tensor-core tiles, 1 = skinny (bandwidth-bound CUDA-core) path,
- * 2 = FFMA tiles. */
+ * 0 = tcgen05 tensor-core tiles on the operands as they are stored, 1 = skinny
+ * (bandwidth-bound CUDA-core) path, 2 = operands TMA cannot address as they are stored, or less
+ * than a tile: clusters of tensor-core CTAs, on padded copies where needed (scratch), with the
+ * accuracy of FFMA sums - or, for the smallest, FFMA tiles. */
 int polar_b200_fmatmul_path(int transLeft, int transRight, uint64_t m,
                             uint64_t n, uint64_t k);
 
@@ -281,7 +285,9 @@ int polar_b200_fmatmul_path(int transLeft, int transRight, uint64_t m,
  * writes one 128-byte line of a result row (taken for sums of a few hundred to a few thousand
  * terms, where the epilogue is a visible share of a tile's time) - and *splits = work units per
  * tile (1 = whole tiles, 0 = stream mode, >1 = fixed cuts of k).  For a t_f product with rows
- * just past a tile boundary the answer describes the whole-tile part.  Any pointer may be NULL. */
+ * just past a tile boundary the answer describes the whole-tile part.  Products too small to fill
+ * the chip with such tiles run one 128-row tile per cluster of CTAs: *tile_rows = 128 and *splits =
+ * CTAs per cluster, which add their parts through distributed shared memory.  Any pointer may be NULL. */
 void polar_b200_fmatmul_tc_plan(int transLeft, int transRight, uint64_t m, uint64_t n, uint64_t k,
                                 int* tile_rows, int* exchanged, int* splits);
 

@@ -16,6 +16,9 @@ bool tc_tail_in_halves(uint64_t tiles, uint64_t grid);
 uint64_t tc_workspace_bytes(uint64_t m, uint64_t n, uint64_t k, uint32_t splits, int mt = 1);
 bool tc_shape_ok(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                  const float* right);
+uint64_t mid_workspace_bytes(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right);
+int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right, float* out, int bn,
+               int cluster, int round, int swap, int epilogue, float* ws, cudaStream_t stream);
 int skinny_kind(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                 const float* right, const float* out);
 uint64_t skinny_workspace_bytes(int kind, uint64_t m, uint64_t n, uint64_t k);
@@ -184,6 +187,72 @@ bool use_capture_side_stream(bool on) {
 
 namespace {
 
+// ---- the cluster kernel (gemm_tc_mid.cu) --------------------------------------------------------------
+// One 128 x bn tile per cluster of CTAs.  Times in microseconds, fitted to measurements on B200 between
+// 128 x 64 x 64 and 2048^3 (within 15 % there): a slab of 32 k costs a CTA 0.43 / 0.48 / 0.60 us with tiles of 32 / 64 / 128
+// columns (0.62 / 0.70 / 0.98 with the rounded split), set-up, pipeline fill and the store of the tile 4 to 5.5 us,
+// the exchange between the CTAs of a cluster 1 us.
+struct MidChoice {
+  int bn = 0, cluster = 1, swap = 0;
+  double us = 1e30;
+};
+
+MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool round) {
+  MidChoice best;
+  const uint64_t sms = (uint64_t)sm_count(), slabs = (k + 31) / 32;
+  for (int swap = 0; swap < 2; ++swap) {
+    const uint64_t rows = swap ? n : m, cols = swap ? m : n;
+    for (int i = 0; i < 3; ++i) {
+      const int bn = 32 << i;
+      static const double slab_us[2][3] = {{0.43, 0.48, 0.60}, {0.62, 0.70, 0.98}};
+      const uint64_t tiles = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
+      for (int cl = 1; cl <= 8 && (uint64_t)cl <= slabs; cl *= 2) {
+        // clusters of 4 and 8 leave SMs of a GPC unused
+        const uint64_t at_once = cl <= 2 ? sms : cl == 4 ? sms / 37 * 34 : sms / 37 * 32;
+        const uint64_t waves = (tiles * cl + at_once - 1) / at_once;
+        const double one = (double)((slabs + cl - 1) / cl) * slab_us[round][i] + (bn == 128 ? 5.5 : 4.0) + (cl > 1 ? 1.0 : 0.0);
+        const double us = (double)waves * one;
+        if (us < best.us - 0.01) best = MidChoice{bn, cl, swap, us};
+      }
+    }
+  }
+  return best;
+}
+
+// What the 256-column tiles of gemm_tc.cu take, on the same scale (same measurements): a slab of 16 k of a
+// 256 x 256 tile 0.85 us, of a 128 x 256 tile 0.55, and 10 (6) us around them per tile; cuts of k move the partial
+// products through memory and a second kernel.
+double tc_estimate_us(uint64_t m, uint64_t n, uint64_t k, const TcChoice& c) {
+  const uint64_t rows = c.swap ? n : m, cols = c.swap ? m : n, sms = (uint64_t)sm_count(), slabs = (k + 15) / 16;
+  const uint64_t tiles = ((rows + 128 * c.mt - 1) / (128 * c.mt)) * ((cols + 255) / 256);
+  const double slab = c.mt == 2 ? 0.85 : 0.55, around = c.mt == 2 ? 10.0 : 6.0;
+  const double mb = (double)m * (double)n * 4e-6;
+  if (c.splits == 0) return (double)(tiles * slabs) / (double)sms * slab + around + 8.0 + mb / 2.0;
+  const uint64_t units = tiles * c.splits;
+  const double waves = (double)((units + sms - 1) / sms);
+  return waves * ((double)((slabs + c.splits - 1) / c.splits) * slab + around) + (c.splits > 1 ? 3.0 + c.splits * mb / 2.0 : 0.0);
+}
+
+// Operands that TMA addresses as they are stored: the cluster kernel where it is the faster of the two.
+MidChoice mid_for_tc(uint64_t m, uint64_t n, uint64_t k, bool may_swap) {
+  MidChoice c = mid_choose(m, n, k, false);
+  if (c.us >= tc_estimate_us(m, n, k, tc_choose(m, n, k, may_swap))) c.bn = 0;
+  return c;
+}
+
+// The rest - operands with an unaligned base or row pitch, which the cluster kernel takes as padded copies, and
+// products below a tile of gemm_tc.cu.  They had the FFMA kernel's round-to-nearest sums, so they get the rounded
+// split with short sums in tensor memory: 1.3e-7 to 1.6e-7 of the result's norm against float64 where FFMA
+// has 1.8e-7 (k = 98) to 8e-7 (k = 2048).  FFMA tiles (64 x 64, about two CTAs per SM at a time, 0.15 us per term) keep
+// what is over before a padded copy and a pipeline have started.
+MidChoice mid_for_rest(uint64_t m, uint64_t n, uint64_t k, uint64_t pad_bytes) {
+  MidChoice c = mid_choose(m, n, k, true);
+  const double ffma_waves = (double)(((m + 63) / 64) * ((n + 63) / 64)) / (2.0 * sm_count());
+  const double ffma = 3.0 + 0.15 * (double)k * (ffma_waves > 1.0 ? ffma_waves : 1.0);
+  if (c.us + (pad_bytes ? 2.0 + (double)pad_bytes * 2.0 / 4e6 : 0.0) >= ffma) c.bn = 0;
+  return c;
+}
+
 int check_mm(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
              const float* right, float* out) {
   if ((tl != 0 && tl != 1) || (tr != 0 && tr != 1))
@@ -211,6 +280,7 @@ static uint64_t workspace_need(int tl, int tr, uint64_t m, uint64_t n, uint64_t 
   if (kind) return skinny_workspace_bytes(kind, m, n, k);
   if (choose_path(tl, tr, m, n, k, al, al, al) == kPathTc) {
     const uint64_t rem = ragged_rows(tl, tr, m, n, k, al, fused == 1 ? 1 : 0);
+    if (rem == 0 && !pitched && mid_for_tc(m, n, k, true).bn) return 0;
     const uint64_t mm = m - rem;
     const TcChoice c = tc_choose(mm, n, k, rem == 0 && !pitched);
     uint64_t need = c.swap ? tc_workspace_bytes(n, mm, k, c.splits, c.mt) : tc_workspace_bytes(mm, n, k, c.splits, c.mt);
@@ -218,7 +288,9 @@ static uint64_t workspace_need(int tl, int tr, uint64_t m, uint64_t n, uint64_t 
     if (rem) need = align256(need) + ragged_rows_workspace_bytes(rem, n, k);
     return need;
   }
-  return 0;
+  if (m == 0 || n == 0 || k == 0) return 0;
+  const uint64_t pad = mid_workspace_bytes(tl, tr, m, n, k, al, al);
+  return mid_for_rest(m, n, k, pad).bn ? pad : 0;
 }
 
 uint64_t polar_b200_fmatmul_workspace_bytes(int tl, int tr, uint64_t m, uint64_t n, uint64_t k) {
@@ -260,6 +332,13 @@ void polar_b200_fmatmul_tc_plan(int tl, int tr, uint64_t m, uint64_t n, uint64_t
                                 int* splits) {
   const float* al = reinterpret_cast<const float*>(256);
   const uint64_t rem = ragged_rows(tl, tr, m, n, k, al, 0);
+  const MidChoice mid = rem == 0 ? mid_for_tc(m, n, k, true) : MidChoice{};
+  if (mid.bn) {
+    if (tile_rows) *tile_rows = 128;
+    if (exchanged) *exchanged = mid.swap;
+    if (splits) *splits = mid.cluster;
+    return;
+  }
   const TcChoice c = tc_choose(m - rem, n, k, rem == 0);
   if (tile_rows) *tile_rows = 128 * c.mt;
   if (exchanged) *exchanged = c.swap;
@@ -277,6 +356,12 @@ static int tc_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const flo
   const uint64_t lp = pitch ? pitch : m;
   const uint64_t rem = ragged_rows(tl, tr, m, n, k, right, fused);
   if (rem == 0) {
+    if (pitch == 0) {
+      const MidChoice mid = mid_for_tc(m, n, k, true);
+      if (mid.bn)
+        return launch_mid(tl, tr, m, n, k, left, right, out, mid.bn, mid.cluster, 0, mid.swap, fused == 1 ? 1 : 0, nullptr,
+                          as_stream(stream));
+    }
     const TcChoice c = tc_choose(m, n, k, pitch == 0);
     return run_tc(tl, tr, m, n, k, left, right, out, 256, 16, 3, 0, c.splits, workspace,
                   workspace_bytes, as_stream(stream), fused == 1 ? 1 : 0, pitch, c.mt, c.swap);
@@ -348,6 +433,32 @@ static int fmatmul_impl(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, cons
                       : polar_b200_fsigmoid_grad(out, sig, out, m * n, stream);
   }
   const int path = choose_path(tl, tr, m, n, k, left, right, out);
+  if (path == kPathFfma && fused != 2) {
+    const uint64_t pad = mid_workspace_bytes(tl, tr, m, n, k, left, right);
+    const MidChoice mid = mid_for_rest(m, n, k, pad);
+    if (mid.bn) {
+      // What the workspace query promised is for aligned base pointers; other pointers may need more copies than that,
+      // for which the library's own scratch steps in.
+      const float* al = reinterpret_cast<const float*>(256);
+      if (workspace && pad && (workspace_bytes < mid_workspace_bytes(tl, tr, m, n, k, al, al) || (reinterpret_cast<uintptr_t>(workspace) & 15)))
+        return fail(POLAR_B200_ERR_WORKSPACE, "workspace too small or not 16-byte aligned");
+      void *ws = workspace, *own = nullptr;
+      if (pad && (!workspace || workspace_bytes < pad)) {
+        // (no memory for the copies: the FFMA kernel below needs none)
+        if (scratch_alloc(&own, pad, as_stream(stream)) != cudaSuccess) cudaGetLastError();
+        ws = own;
+      }
+      if (!pad || ws) {
+        rc = launch_mid(tl, tr, m, n, k, left, right, out, mid.bn, mid.cluster, 1, mid.swap, fused == 1 ? 1 : 0,
+                        static_cast<float*>(ws), as_stream(stream));
+        if (own) {
+          cudaError_t e = scratch_free(own, as_stream(stream));
+          if (!rc && e != cudaSuccess) rc = fail(POLAR_B200_ERR_CUDA, "returning scratch", e);
+        }
+        return rc;
+      }
+    }
+  }
   const int kind0 = path == kPathSkinny ? skinny_kind(tl, tr, m, n, k, left, right, out) : 0;
   const bool fused_in_kernel = (fused == 1 && (path == kPathTc || kind0 == 1)) || (fused == 2 && kind0 == 3);
   if (fused != 0 && !fused_in_kernel) {
@@ -493,6 +604,21 @@ int polar_b200_fmatmul_tc(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, co
   int rc = check_mm(tl, tr, m, n, k, left, right, out);
   if (rc) return rc;
   if (m == 0 || n == 0 || k == 0) return fail(POLAR_B200_ERR_UNSUPPORTED, "empty matrix");
+  if (tile_n >= 2000) {
+    // one 128 x (tile_n - 2000) tile per cluster of `splits` CTAs; + 1000: the operands exchange roles
+    const int swap = tile_n >= 3000;
+    const uint64_t need = mid_workspace_bytes(tl, tr, m, n, k, left, right);
+    LaunchDeviceScope on(stream, out);
+    void* ws = nullptr;
+    if (need) {
+      cudaError_t e = scratch_alloc(&ws, need, as_stream(stream));
+      if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "scratch (padded operands)", e);
+    }
+    rc = launch_mid(tl, tr, m, n, k, left, right, out, tile_n - (swap ? 3000 : 2000), splits, write_hi == 1, swap, 0,
+                    static_cast<float*>(ws), as_stream(stream));
+    if (ws) scratch_free(ws, as_stream(stream));
+    return rc;
+  }
   // tile_n + 1000: the operands exchange roles (the transposed product is computed and stored
   // transposed; whole tiles or fixed k cuts only)
   const int swap_ab = tile_n >= 1000 ? 1 : 0;

@@ -1,0 +1,551 @@
+// fmatmul on the tensor cores for products that are too small, or too oddly shaped, to fill the chip with the
+// 256-column tiles of gemm_tc.cu: one output tile of 128 x BN per cluster of CTAs, the k range divided over the
+// CTAs of the cluster, the partial tiles added through distributed shared memory.
+//
+// Why it exists.  1024^3 is 16 tiles of 256 x 256 or 32 of 128 x 256: cut along k they fill 64 of 148 SMs, and
+// the partial products travel through global memory and a second kernel.  Here it is 64 tiles of
+// 128 x 128 in clusters of two.  An operand whose rows TMA cannot address (a row pitch that is no multiple of 16
+// bytes) is first copied to scratch with a padded pitch (pad_kernel); those shapes had only
+// the FFMA kernel, at 15 TFLOP/s.
+//
+// One CTA:
+//   warp 0      TMA producer: 32-float k slabs of A (128 rows) and B (BN rows), two instructions per slab;
+//   warp 1      tcgen05.mma issuer: per slab and 8 k the three products of the TF32 split;
+//   warps 2-9   split warps: x -> hi + lo in shared memory.  With ROUND, hi is x rounded to the nearest TF32
+//               (written back over x) and lo = x - hi is at most half as long and of either sign, so that what
+//               the split drops (lo.lo, the bits of lo past TF32) is four times smaller and unbiased;
+//   warps 10-17 accumulator warps: every `chunk` slabs they read the tensor-memory accumulator and add it to
+//               registers in round-to-nearest.  The tensor core's own accumulator rounds toward zero, an error that
+//               grows with the length of the sum (8e-9 of the result per term for zero-mean operands);
+//               chunks keep it at that of a short sum.
+// At the end the tile goes to shared memory in the layout of the result's rows; the cluster's CTAs each
+// add one share of it over all CTAs in rank order (the same bits run to run) and store whole lines.
+//
+// Orientation: rows of a tile are tensor-memory lanes, 128 of them; with `out_t` the kernel was given the
+// operands in exchanged roles, and the tile's rows are columns of the result (results of few rows).
+//
+// Waits are bounded as in gemm_tc.cu; codes 111 ... 117.
+#include <cuda.h>
+
+#include <mutex>
+
+#include "common.cuh"
+#include "tc_ptx.cuh"
+
+namespace polar_b200 {
+namespace tc {
+int make_map(CUtensorMap* map, const float* base, uint64_t inner, uint64_t outer, uint32_t box_inner, uint32_t box_outer,
+             bool mn_major, int bk, uint64_t pitch);
+int make_map_chunks(CUtensorMap* map, const float* base, uint64_t chunks, uint64_t outer, uint32_t box_outer,
+                    uint32_t box_chunks, uint64_t pitch);
+}  // namespace tc
+
+namespace mid {
+using namespace tc;
+
+constexpr int BM = 128, BK = 32;
+constexpr int kSplitWarps = 8, kAccWarps = 8;
+constexpr int kThreads = 32 * (2 + kSplitWarps + kAccWarps);
+constexpr uint32_t kBox = 32 * BK * 4;                      // one MN-major chunk of a slab: 32 elements x BK rows
+
+// Shared memory is a ring of raw slabs and a shorter ring of lo parts.  A raw slab is held from the TMA
+// request to the end of its products (about 2 us: L2 latency, split, products), a lo part only from the
+// split on, so the raw ring is what has to be deep: at 128 x 128 x 32 a slab's products take 0.4 us.
+template <int BN> struct Cfg {
+  static constexpr uint32_t kABytes = BM * BK * 4, kBBytes = BN * BK * 4, kRawBytes = kABytes + kBBytes;
+  static constexpr int kRaw = BN == 128 ? 5 : BN == 64 ? 6 : 7, kLo = BN == 128 ? 2 : BN == 64 ? 3 : 4;
+  static constexpr uint32_t kLoBase = kRaw * kRawBytes;
+  static constexpr uint32_t kTileBytes = (kRaw + kLo) * kRawBytes;
+  static constexpr uint32_t kSmemBytes = kTileBytes + 1024 + 256;
+  static_assert(kSmemBytes <= 227 * 1024, "rings must fit shared memory");
+  static_assert(BM * (BN + 4) * 4 <= (int)kTileBytes && BN * (BM + 4) * 4 <= (int)kTileBytes, "the tile must fit the rings");
+};
+
+struct Params {
+  uint64_t m, n;            // of the product as the kernel sees it (rows = lanes)
+  float* out;
+  uint64_t pitch;           // floats per row of the result
+  uint32_t tiles_m, slabs, cluster, chunk;
+  int a_mn, b_mn;           // operand stored with m (n) contiguous
+  int a_whole, b_whole;     // whole 32-element chunks of that extent: tiles inside them come in one 3-D box
+  int out_t, epilogue, vec_out;
+  int* status;
+  unsigned long long wait_ns;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float4 ld_shared_v4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr, uint32_t rank) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+  return v;
+}
+
+// A CTA's share of the finished tile: the parts of all CTAs of the cluster, added in rank order, to the result.
+// Eight 128-bit reads of (distributed) shared memory are in flight per thread before the first is used.
+template <int BN, int CL>
+__device__ __forceinline__ void store_share(const Params& p, uint32_t base, uint32_t rank, int m0, int n0) {
+  constexpr int kVecs = BM * BN / 4, kShare = kVecs / CL, kBatch = 8 / CL;
+  const int shift = p.out_t ? 5 : (BN == 128 ? 5 : BN == 64 ? 4 : 3);       // log2 of the vectors in a row of the result
+  const int width = 4 << shift;
+  const uint64_t out_rows = p.out_t ? p.n : p.m, out_cols = p.out_t ? p.m : p.n;
+  const uint64_t r0 = (uint64_t)(p.out_t ? n0 : m0), c0 = (uint64_t)(p.out_t ? m0 : n0);
+  for (int first = 0; first < kShare; first += kBatch * kThreads) {
+    float4 part[kBatch][CL];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int w = first + u * kThreads + (int)threadIdx.x, v = (int)rank * kShare + w;
+      if (w >= kShare) continue;
+      const uint32_t at = base + (uint32_t)((v >> shift) * (width + 4) + (v & ((1 << shift) - 1)) * 4) * 4u;
+#pragma unroll
+      for (int k = 0; k < CL; ++k) part[u][k] = CL == 1 ? ld_shared_v4(at) : ld_cluster_v4(at, (uint32_t)k);
+    }
+    if (CL > 1 && first + kBatch * kThreads >= kShare) cluster_arrive();     // nothing of another CTA is read after this
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int w = first + u * kThreads + (int)threadIdx.x, v = (int)rank * kShare + w;
+      if (w >= kShare) continue;
+      const uint64_t r = r0 + (uint64_t)(v >> shift), c = c0 + (uint64_t)(v & ((1 << shift) - 1)) * 4;
+      if (r >= out_rows || c >= out_cols) continue;
+      float4 y = part[u][0];
+#pragma unroll
+      for (int k = 1; k < CL; ++k) y.x += part[u][k].x, y.y += part[u][k].y, y.z += part[u][k].z, y.w += part[u][k].w;
+      if (p.epilogue == 1) y = make_float4(sigmoid_clamped(y.x), sigmoid_clamped(y.y), sigmoid_clamped(y.z), sigmoid_clamped(y.w));
+      float* dst = p.out + r * p.pitch + c;
+      if (p.vec_out && c + 4 <= out_cols) {
+        *reinterpret_cast<float4*>(dst) = y;
+      } else {
+        dst[0] = y.x;
+        if (c + 1 < out_cols) dst[1] = y.y;
+        if (c + 2 < out_cols) dst[2] = y.z;
+        if (c + 3 < out_cols) dst[3] = y.w;
+      }
+    }
+  }
+}
+
+template <int BN, bool ROUND>
+__global__ void __launch_bounds__(kThreads, 1)
+fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                   const __grid_constant__ CUtensorMap map_a3, const __grid_constant__ CUtensorMap map_b3,
+                   const Params p) {
+  using C = Cfg<BN>;
+  // accumulators: with ROUND the cross products get one of their own (see above)
+  constexpr int kKinds = ROUND ? 2 : 1, kAccs = 4 / kKinds;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
+  const uint32_t bars = base + C::kTileBytes;
+  auto full_raw = [&](int s) { return bars + 8u * s; };
+  auto empty = [&](int s) { return bars + 8u * (C::kRaw + s); };
+  auto full_lo = [&](int s) { return bars + 8u * (2 * C::kRaw + s); };
+  constexpr int kRings = 2 * C::kRaw + C::kLo;
+  auto acc_full = [&](int a) { return bars + 8u * (kRings + a); };
+  auto acc_empty = [&](int a) { return bars + 8u * (kRings + kAccs + a); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + C::kTileBytes + 8 * (kRings + 2 * kAccs));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  static_assert(8 * (kRings + 2 * kAccs) + 8 <= 256, "barrier block");
+
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
+  const uint32_t rank = p.cluster > 1 ? cluster_rank() : 0u;
+  const uint32_t tile = blockIdx.x / p.cluster;
+  const int m0 = (int)((tile % p.tiles_m) * BM), n0 = (int)((tile / p.tiles_m) * BN);
+  const uint32_t kb0 = (uint32_t)((uint64_t)rank * p.slabs / p.cluster);
+  const uint32_t kb1 = (uint32_t)((uint64_t)(rank + 1) * p.slabs / p.cluster);
+  const uint32_t mine = kb1 - kb0, chunks = (mine + p.chunk - 1) / p.chunk;
+
+  constexpr int kBars = kRings + 2 * kAccs;
+  static_assert(kBars <= 32, "one lane initialises one barrier");
+  if (warp == 0) {
+    if (lane < kBars) {
+      const bool by_warps = (lane >= 2 * C::kRaw && lane < kRings) || lane >= kRings + kAccs;   // full_lo, acc_empty
+      mbar_init(bars + 8u * lane, by_warps ? (uint32_t)kSplitWarps : 1u);
+    }
+    if (lane == 0) *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  static_assert(kSplitWarps == kAccWarps, "by_warps");
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), 4 * BN);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);   // (known to be uniform)
+  pdl_enter();              // the set-up above overlaps the kernel before; operands and result are touched from here on
+
+  if (warp == 0) {
+    const bool leader = elect_one();
+    {
+      uint32_t s = 0, ph = 1;
+      for (uint32_t it = 0; it < mine; ++it) {
+        if (!mbar_wait(empty(s), ph, abort_flag, p.status, 111, p.wait_ns)) break;
+        if (leader) {
+          const uint32_t a = base + s * C::kRawBytes, b = a + C::kABytes;
+          mbar_expect_tx(full_raw(s), C::kRawBytes);
+          const int k0 = (int)((kb0 + it) * BK);
+          if (!p.a_mn) {
+            tma_load_2d(a, &map_a, full_raw(s), k0, m0);
+          } else if (m0 + BM <= 32 * p.a_whole) {
+            tma_load_3d(a, &map_a3, full_raw(s), 0, k0, m0 / 32);
+          } else {
+            for (int c = 0; c < BM / 32; ++c) tma_load_2d(a + c * kBox, &map_a, full_raw(s), m0 + 32 * c, k0);
+          }
+          if (!p.b_mn) {
+            tma_load_2d(b, &map_b, full_raw(s), k0, n0);
+          } else if (n0 + BN <= 32 * p.b_whole) {
+            tma_load_3d(b, &map_b3, full_raw(s), 0, k0, n0 / 32);
+          } else {
+            for (int c = 0; c < BN / 32; ++c) tma_load_2d(b + c * kBox, &map_b, full_raw(s), n0 + 32 * c, k0);
+          }
+        }
+        if (++s == C::kRaw) s = 0, ph ^= 1;
+      }
+    }
+  } else if (warp == 1) {
+    const bool leader = elect_one();
+    {
+      const uint32_t idesc = make_idesc(BM, BN, p.a_mn, p.b_mn);
+      // K-major: 128-byte rows in the 128-byte swizzle (layout 2), 8-row groups 1 KB apart, 8 k = 32 bytes
+      // inside the row.  MN-major: chunks of 32 elements x BK rows (layout 1), chunks kBox apart, 8 k = 1 KB.
+      const Operand a_op = make_desc(0, p.a_mn ? kBox : 16u, p.a_mn ? 512u : 1024u, p.a_mn ? 1u : 2u);
+      const Operand b_op = make_desc(0, p.b_mn ? kBox : 16u, p.b_mn ? 512u : 1024u, p.b_mn ? 1u : 2u);
+      const uint32_t a_step = (p.a_mn ? 1024u : 32u) >> 4, b_step = (p.b_mn ? 1024u : 32u) >> 4;
+      // (in a cluster the upper bits of a shared address hold the CTA's rank; a descriptor has no room for them)
+      const uint32_t ring = (base & 0x3FFFFu) >> 4;
+      uint32_t it = 0, s = 0, s_ph = 0, l = 0, l_ph = 0;    // slab; its place and phase in either ring
+      bool ok = true;
+      for (uint32_t c = 0; ok && c < chunks; ++c) {
+        const int acc = c % kAccs;
+        ok = mbar_wait(acc_empty(acc), ((c / kAccs) & 1u) ^ 1u, abort_flag, p.status, 115, p.wait_ns);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = tmem + acc * kKinds * BN, cross = d + (kKinds - 1) * BN;
+        const uint32_t last = it + p.chunk < mine ? it + p.chunk : mine;
+        for (uint32_t accumulate = 0; it < last; ++it, accumulate = 1) {
+          const uint32_t a_hi = ring + ((s * C::kRawBytes) >> 4), b_hi = a_hi + (C::kABytes >> 4);
+          const uint32_t a_lo = ring + ((C::kLoBase + l * C::kRawBytes) >> 4), b_lo = a_lo + (C::kABytes >> 4);
+          auto high_products = [&] {
+#pragma unroll
+            for (int kk = 0; kk < BK / 8; ++kk)
+              tc_mma_tf32(d, a_op, a_hi + kk * a_step, b_op, b_hi + kk * b_step, idesc, kk ? 1u : accumulate);
+          };
+          if (!ROUND) {                                     // the raw words are the hi parts: no need to wait for the split
+            ok = mbar_wait(full_raw(s), s_ph, abort_flag, p.status, 112, p.wait_ns);
+            if (!ok) break;
+            tc_fence_after();
+            if (leader) high_products();
+          }
+          ok = mbar_wait(full_lo(l), l_ph, abort_flag, p.status, 113, p.wait_ns);
+          if (!ok) break;
+          tc_fence_after();
+          if (leader) {
+            if (ROUND) high_products();
+#pragma unroll
+            for (int kk = 0; kk < BK / 8; ++kk) {
+              tc_mma_tf32(cross, a_op, a_lo + kk * a_step, b_op, b_hi + kk * b_step, idesc, (!ROUND || kk) ? 1u : accumulate);
+              tc_mma_tf32(cross, a_op, a_hi + kk * a_step, b_op, b_lo + kk * b_step, idesc, 1u);
+            }
+            tc_commit(empty(s));
+          }
+          if (++s == C::kRaw) s = 0, s_ph ^= 1;
+          if (++l == C::kLo) l = 0, l_ph ^= 1;
+        }
+        if (ok && leader) tc_commit(acc_full(acc));
+      }
+    }
+  } else if (warp < 2 + kSplitWarps) {
+    const int tid = threadIdx.x - 64;
+    uint32_t s = 0, ph = 0, l = 0, prev = 0, prev_ph = 0;   // prev: the slab that used this place of the lo ring before
+    for (uint32_t it = 0; it < mine; ++it) {
+      if (it >= (uint32_t)C::kLo) {
+        if (!mbar_wait(empty(prev), prev_ph, abort_flag, p.status, 117, p.wait_ns)) break;
+        if (++prev == C::kRaw) prev = 0, prev_ph ^= 1;
+      }
+      if (!mbar_wait(full_raw(s), ph, abort_flag, p.status, 114, p.wait_ns)) break;
+      float4* raw = reinterpret_cast<float4*>(gen + s * C::kRawBytes);
+      float4* lo = reinterpret_cast<float4*>(gen + C::kLoBase + l * C::kRawBytes);
+      constexpr int kVecs = C::kRawBytes / 16;
+      static_assert(kVecs % (kSplitWarps * 32) == 0, "slab must divide over the split warps");
+      auto high = [](float x) {
+        uint32_t u = __float_as_uint(x);
+        if (ROUND) asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
+        return __uint_as_float(u & 0xFFFFE000u);
+      };
+      // all loads before the first store: the compiler cannot tell that the two never meet, and would
+      // make one latency of each vector
+      constexpr int kMine = kVecs / (kSplitWarps * 32);
+      float4 v[kMine];
+#pragma unroll
+      for (int i = 0; i < kMine; ++i) v[i] = raw[tid + i * kSplitWarps * 32];
+#pragma unroll
+      for (int i = 0; i < kMine; ++i) {
+        const int e = tid + i * kSplitWarps * 32;
+        const float4 h = {high(v[i].x), high(v[i].y), high(v[i].z), high(v[i].w)};
+        lo[e] = make_float4(v[i].x - h.x, v[i].y - h.y, v[i].z - h.z, v[i].w - h.w);
+        if (ROUND) raw[e] = h;
+      }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full_lo(l));               // one arrival per warp
+      if (++s == C::kRaw) s = 0, ph ^= 1;
+      if (++l == C::kLo) l = 0;
+    }
+  } else {
+    // four consecutive warps cover the 128 lanes, the two warps of a lane quarter half of the columns each
+    const int q = warp & 3, half = (warp - (2 + kSplitWarps)) >> 2;
+    constexpr int kCols = BN / 2;
+    constexpr int kPart = 16;                               // columns read at a time: what the register budget allows
+    float acc[kCols];
+#pragma unroll
+    for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
+    bool ok = true;
+    for (uint32_t c = 0; c < chunks; ++c) {
+      const int a = c % kAccs;
+      ok = mbar_wait(acc_full(a), (c / kAccs) & 1u, abort_flag, p.status, 116, p.wait_ns);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int j0 = 0; j0 < kCols; j0 += kPart) {
+        uint32_t r[kPart];
+        const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * kKinds * BN + half * kCols + j0);
+        tmem_ld_32x16(at, r);
+        tmem_ld_wait();
+        if (ROUND) {
+          uint32_t x[kPart];
+          tmem_ld_32x16(at + BN, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < kPart; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(x[j]));
+        }
+#pragma unroll
+        for (int j = 0; j < kPart; ++j) acc[j0 + j] += __uint_as_float(r[j]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty(a));
+    }
+    // all products of this CTA are done and every stage has been read: the tile takes their place, in rows of the result
+    if (ok) {
+      float* t = reinterpret_cast<float*>(gen);
+      const int row = q * 32 + lane;
+      if (p.out_t) {
+#pragma unroll
+        for (int j = 0; j < kCols; ++j) t[(half * kCols + j) * (BM + 4) + row] = acc[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < kCols; j += 4)
+          *reinterpret_cast<float4*>(t + row * (BN + 4) + half * kCols + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+      }
+    }
+  }
+
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (p.cluster > 1) {
+    cluster_arrive();
+    cluster_wait();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    if (*abort_flag) {     // let copies and MMAs in flight finish before the tensor memory goes away
+      const long long t0 = clock64();
+      while (clock64() - t0 < 2000000ll) { }
+    }
+    tmem_dealloc(tmem, 4 * BN);
+  }
+  switch (p.cluster) {
+    case 1: store_share<BN, 1>(p, base, 0, m0, n0); break;
+    case 2: store_share<BN, 2>(p, base, rank, m0, n0); break;
+    case 4: store_share<BN, 4>(p, base, rank, m0, n0); break;
+    default: store_share<BN, 8>(p, base, rank, m0, n0);
+  }
+  if (p.cluster > 1) cluster_wait();   // nobody leaves while another CTA may still read its part
+}
+
+// Copies up to two matrices to scratch with their rows padded to `pitch` floats (a multiple of 32; the
+// padding is zero), four floats of the copy per thread.  Bound by memory: 8 bytes per element, 4-byte loads because
+// the rows start anywhere.
+struct Padded {
+  const float* src;
+  float* dst;
+  uint64_t rows, cols, pitch;
+  uint64_t vecs() const { return rows * (pitch / 4); }
+};
+__global__ void __launch_bounds__(256) pad_kernel(const Padded a, const Padded b, uint64_t vecs_a, uint64_t vecs) {
+  pdl_enter();
+  uint64_t v = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+  if (v >= vecs) return;
+  const bool second = v >= vecs_a;
+  if (second) v -= vecs_a;
+  const float* src = second ? b.src : a.src;
+  float* dst = second ? b.dst : a.dst;
+  const uint32_t cols = (uint32_t)(second ? b.cols : a.cols), per_row = (uint32_t)((second ? b.pitch : a.pitch) / 4);
+  const uint64_t r = v / per_row;
+  const uint32_t c = (uint32_t)(v - r * per_row) * 4;
+  const float* s = src + r * cols + c;
+  float4 x;
+  x.x = c < cols ? s[0] : 0.f;
+  x.y = c + 1 < cols ? s[1] : 0.f;
+  x.z = c + 2 < cols ? s[2] : 0.f;
+  x.w = c + 3 < cols ? s[3] : 0.f;
+  *reinterpret_cast<float4*>(dst + v * 4) = x;
+}
+
+// An operand as it is stored: rows of `cols` contiguous floats, `pitch` floats apart.
+struct Stored {
+  const float* p;
+  uint64_t rows, cols, pitch;
+  bool padded;                                              // columns up to the pitch are there, and zero
+};
+
+template <int BN, bool ROUND>
+int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Params p, uint64_t k, cudaStream_t stream) {
+  using C = Cfg<BN>;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  static std::mutex mu;
+  static bool attr_done[64] = {false};
+  {
+    std::lock_guard<std::mutex> guard(mu);
+    if (dev >= 0 && dev < 64 && !attr_done[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(fmatmul_mid_kernel<BN, ROUND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
+      if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFuncSetAttribute(smem)", e);
+      attr_done[dev] = true;
+    }
+  }
+  // The extents are the true ones wherever TMA has to cut a box off; a padded MN-major operand offers whole chunks.
+  CUtensorMap maps[2], maps3[2];
+  const Stored* op[2] = {&left, &right};
+  const bool mn[2] = {a_mn, b_mn};
+  const uint32_t tile_rows[2] = {(uint32_t)BM, (uint32_t)BN};
+  const uint64_t extent[2] = {p.m, p.n};
+  int whole[2] = {0, 0};
+  for (int i = 0; i < 2; ++i) {
+    const Stored& o = *op[i];
+    int rc = POLAR_B200_OK;
+    if (!mn[i]) {
+      rc = make_map(&maps[i], o.p, k, extent[i], BK, tile_rows[i], false, BK, o.pitch);
+      maps3[i] = maps[i];
+    } else {
+      const uint64_t cols = o.padded ? o.pitch : o.cols;
+      whole[i] = (int)(cols / 32);
+      const bool boxes_2d = (extent[i] + tile_rows[i] - 1) / tile_rows[i] * tile_rows[i] > 32ull * whole[i];
+      if (whole[i]) rc = make_map_chunks(&maps3[i], o.p, whole[i], k, BK, tile_rows[i] / 32, o.pitch);
+      if (!rc && (boxes_2d || !whole[i])) rc = make_map(&maps[i], o.p, cols, k, 32, BK, true, BK, o.pitch);
+      else maps[i] = maps3[i];
+      if (!whole[i]) maps3[i] = maps[i];
+    }
+    if (rc) return rc;
+  }
+  p.a_mn = a_mn;
+  p.b_mn = b_mn;
+  p.a_whole = whole[0];
+  p.b_whole = whole[1];
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(p.tiles_m * (uint32_t)((p.n + BN - 1) / BN) * p.cluster);
+  c.blockDim = dim3(kThreads);
+  c.dynamicSmemBytes = C::kSmemBytes;
+  c.stream = stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = p.cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  c.attrs = at;
+  c.numAttrs = p.cluster > 1 ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&c, fmatmul_mid_kernel<BN, ROUND>, maps[0], maps[1], maps3[0], maps3[1], p);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(POLAR_B200_ERR_CUDA, "fmatmul_mid", e);
+  }
+  count_launch();
+  return POLAR_B200_OK;
+}
+
+}  // namespace mid
+
+namespace {
+uint64_t pad32(uint64_t v) { return (v + 31) & ~31ull; }
+bool addressable(const float* p, uint64_t cols) { return aligned16(p) && (cols & 3) == 0; }
+}  // namespace
+
+// Scratch for operands that TMA cannot address as they are (0: none).
+uint64_t mid_workspace_bytes(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right) {
+  const uint64_t lc = tl ? m : k, lr = tl ? k : m, rc = tr ? k : n, rr = tr ? n : k;
+  uint64_t floats = 0;
+  if (!addressable(left, lc)) floats += lr * pad32(lc);
+  if (!addressable(right, rc)) floats += rr * pad32(rc);
+  return floats * sizeof(float);
+}
+
+// out[m,n] = L'.R' with tiles of 128 x bn, `cluster` CTAs per tile.  swap: the operands exchange roles, the tile's
+// rows are columns of the result.  ws: mid_workspace_bytes.
+int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right, float* out, int bn,
+               int cluster, int round, int swap, int epilogue, float* ws, cudaStream_t stream) {
+  using namespace mid;
+  Stored l{left, tl ? k : m, tl ? m : k, tl ? m : k, false}, r{right, tr ? n : k, tr ? k : n, tr ? k : n, false};
+  Padded copies[2] = {};
+  int count = 0;
+  for (Stored* s : {&l, &r}) {
+    if (addressable(s->p, s->cols)) continue;
+    const uint64_t pitch = pad32(s->cols);
+    copies[count++] = Padded{s->p, ws, s->rows, s->cols, pitch};
+    s->p = ws;
+    s->pitch = pitch;
+    s->padded = true;
+    ws += s->rows * pitch;
+  }
+  if (count) {
+    const uint64_t va = copies[0].vecs(), v = va + (count > 1 ? copies[1].vecs() : 0);
+    if ((v + 255) / 256 > 0x7fffffffull) return fail(POLAR_B200_ERR_UNSUPPORTED, "operand too large");
+    int rc = launch("fmatmul_pad", pad_kernel, (unsigned)((v + 255) / 256), 256, 0, stream, copies[0], copies[1], va, v);
+    if (rc) return rc;
+  }
+  int rc = POLAR_B200_OK;
+  Params p = {};
+  p.status = device_status_word(&rc);
+  if (!p.status) return rc;
+  p.wait_ns = wait_limit_ns(2000000000ull);
+  p.out = out;
+  p.pitch = n;
+  p.vec_out = (n & 3) == 0 && aligned16(out);
+  p.out_t = swap;
+  p.epilogue = epilogue;
+  p.m = swap ? n : m;
+  p.n = swap ? m : n;
+  p.tiles_m = (uint32_t)((p.m + BM - 1) / BM);
+  p.slabs = (uint32_t)((k + BK - 1) / BK);
+  p.cluster = (uint32_t)cluster;
+  // sums of this many terms in tensor memory, the rest in registers
+  p.chunk = round ? 1 : 8;
+  if ((cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) || p.slabs < p.cluster) return fail(POLAR_B200_ERR_UNSUPPORTED, "fewer slabs than CTAs in a cluster");
+  if ((uint64_t)p.tiles_m * ((p.n + bn - 1) / bn) * p.cluster > 0x7fffffffull) return fail(POLAR_B200_ERR_UNSUPPORTED, "too many tiles");
+  // exchanged: right' plays the row operand - stored [k, n] is "row extent contiguous" - and left the column operand
+  const Stored &a = swap ? r : l, &b = swap ? l : r;
+  const bool a_mn = swap ? !tr : tl, b_mn = swap ? tl : !tr;
+#define POLAR_MID(BN)   case BN: return round ? launch_cfg<BN, true>(a, b, a_mn, b_mn, p, k, stream) : launch_cfg<BN, false>(a, b, a_mn, b_mn, p, k, stream);
+  switch (bn) {
+    POLAR_MID(32) POLAR_MID(64) POLAR_MID(128)
+  }
+#undef POLAR_MID
+  return fail(POLAR_B200_ERR_INVALID, "tile width must be 32, 64 or 128");
+}
+
+}  // namespace polar_b200
