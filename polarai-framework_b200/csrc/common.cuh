@@ -118,19 +118,23 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// `cluster`: CTAs per cluster along y (1: no clusters).
 template <typename... P, typename... A>
-int launch(const char* what, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
-           A... args) {
+int launch_clusters(const char* what, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+                    unsigned cluster, A... args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
   c.blockDim = dim3(threads);
   c.dynamicSmemBytes = smem;
   c.stream = stream;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  c.attrs = &at;
-  c.numAttrs = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = at[1].val.clusterDim.z = 1;
+  at[1].val.clusterDim.y = cluster;
+  c.attrs = at;
+  c.numAttrs = cluster > 1 ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -138,6 +142,27 @@ int launch(const char* what, void (*kernel)(P...), dim3 grid, unsigned threads, 
   }
   count_launch();
   return POLAR_B200_OK;
+}
+template <typename... P, typename... A>
+int launch(const char* what, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+           A... args) {
+  return launch_clusters(what, kernel, grid, threads, smem, stream, 1, args...);
+}
+
+// ---- clusters: the CTA's rank, the two halves of the cluster barrier, a read of another CTA's shared memory
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
+  uint32_t remote;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+  return v;
 }
 
 // fsigmoid's arithmetic, shared by the elementwise builtin and the fused matmul

@@ -54,63 +54,108 @@ __device__ __forceinline__ void store_row_sums(const float (&acc)[ROWS_PER_WARP]
   }
 }
 
-template <int NP>
+// Few rows (below kResidentRows), or rows TMA-like loads cannot take as vectors: a CTA computes 4 * RW rows, two warps per
+// row group, over one share of k; the CTAs of a cluster hold the shares of the same rows and add them through
+// distributed shared memory in rank order.  Bound by latency: what counts is that every SM has a CTA, so the host cuts k
+// into up to 8 shares and takes one row per warp until there are enough of them.  (The form with 32 rows
+// per CTA had one CTA for 16 rows: 16 x 10 x 4096 61 us, here 4.)
+constexpr uint64_t kResidentRows = 4096;
+template <int NP, int RW, bool VEC>
 __global__ void __launch_bounds__(kThreads)
-small_n_kmajor_kernel(const float* __restrict__ left, const float* __restrict__ right,
-                      float* __restrict__ out, uint64_t m, uint64_t n, uint64_t k, uint64_t rsk,
-                      uint64_t rsj, int act) {
-  extern __shared__ float bs[];   // [NP][KT_PAD], k contiguous
+small_n_rows_kernel(const float* __restrict__ left, const float* __restrict__ right, float* __restrict__ out, uint64_t m,
+                    uint64_t n, uint64_t k, uint64_t rsk, uint64_t rsj, int act, uint32_t shares) {
+  extern __shared__ float bs[];            // [NP][KT_PAD], k contiguous
+  __shared__ float part[2][4 * RW][NP];    // the two k halves of this CTA
+  __shared__ float mine[4 * RW][NP];       // its share of the sums
+  pdl_enter();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t rows_per_cta = (kThreads / 32) * ROWS_PER_WARP;
-  const uint64_t row0 = (uint64_t)blockIdx.x * rows_per_cta + (uint64_t)warp * ROWS_PER_WARP;
-  float acc[ROWS_PER_WARP][NP];
+  const int group = warp & 3, half = warp >> 2;
+  const uint64_t row0 = (uint64_t)blockIdx.x * (4 * RW) + (uint64_t)group * RW;
+  // shares are whole vectors of 4
+  const uint64_t per = ((k + shares - 1) / shares + 3) & ~3ull;
+  const uint64_t kbeg = (uint64_t)blockIdx.y * per, kend = kbeg + per < k ? kbeg + per : k;
+  float acc[RW][NP];
 #pragma unroll
-  for (int r = 0; r < ROWS_PER_WARP; ++r)
+  for (int r = 0; r < RW; ++r)
 #pragma unroll
     for (int j = 0; j < NP; ++j) acc[r][j] = 0.f;
-
-  for (uint64_t k0 = 0; k0 < k; k0 += KT) {
-    const int kt = (int)((k - k0 < KT) ? (k - k0) : KT);
+  for (uint64_t k0 = kbeg; k0 < kend; k0 += KT) {
+    const int kt = (int)((kend - k0 < KT) ? (kend - k0) : KT);
     __syncthreads();
-    for (int e = threadIdx.x; e < NP * KT; e += kThreads) {
-      int j = e % NP, kk = e / NP;
-      float v = 0.f;
-      if (kk < kt && (uint64_t)j < n) v = right[(k0 + kk) * rsk + (uint64_t)j * rsj];
-      bs[j * KT_PAD + kk] = v;
+    // in the order the operand is stored in, so that the reads are whole lines
+    const bool by_k = rsk == 1;
+    for (int e = threadIdx.x; e < kt * (int)n; e += kThreads) {
+      const int j = by_k ? e / kt : e % (int)n, kk = by_k ? e % kt : e / (int)n;
+      bs[j * KT_PAD + kk] = right[(k0 + kk) * rsk + (uint64_t)j * rsj];
     }
     __syncthreads();
-    for (int kk = lane * 4; kk < kt; kk += 128) {   // k is a multiple of 4: no ragged vector
-      float4 a[ROWS_PER_WARP];
+    if (VEC) {
+      for (int kk = (half * 32 + lane) * 4; kk < kt; kk += 256) {
+        float4 a[RW];
 #pragma unroll
-      for (int r = 0; r < ROWS_PER_WARP; ++r) {
-        uint64_t row = row0 + r;
-        a[r] = row < m ? __ldcs(reinterpret_cast<const float4*>(left + row * k + k0 + kk))
-                       : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < RW; ++r)
+          a[r] = row0 + r < m ? *reinterpret_cast<const float4*>(left + (row0 + r) * k + k0 + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+          if (j >= (int)n) continue;
+          const float4 b = *reinterpret_cast<const float4*>(&bs[j * KT_PAD + kk]);
+#pragma unroll
+          for (int r = 0; r < RW; ++r) {
+            acc[r][j] = fmaf(a[r].x, b.x, acc[r][j]);
+            acc[r][j] = fmaf(a[r].y, b.y, acc[r][j]);
+            acc[r][j] = fmaf(a[r].z, b.z, acc[r][j]);
+            acc[r][j] = fmaf(a[r].w, b.w, acc[r][j]);
+          }
+        }
       }
+    } else {
+#pragma unroll 4
+      for (int kk = half * 32 + lane; kk < kt; kk += 64) {
+        float a[RW];
 #pragma unroll
-      for (int j = 0; j < NP; ++j) {
-        float4 b = *reinterpret_cast<const float4*>(&bs[j * KT_PAD + kk]);
+        for (int r = 0; r < RW; ++r) a[r] = row0 + r < m ? left[(row0 + r) * k + k0 + kk] : 0.f;
 #pragma unroll
-        for (int r = 0; r < ROWS_PER_WARP; ++r) {
-          acc[r][j] = fmaf(a[r].x, b.x, acc[r][j]);
-          acc[r][j] = fmaf(a[r].y, b.y, acc[r][j]);
-          acc[r][j] = fmaf(a[r].z, b.z, acc[r][j]);
-          acc[r][j] = fmaf(a[r].w, b.w, acc[r][j]);
+        for (int j = 0; j < NP; ++j) {
+          if (j >= (int)n) continue;
+          const float b = bs[j * KT_PAD + kk];
+#pragma unroll
+          for (int r = 0; r < RW; ++r) acc[r][j] = fmaf(a[r], b, acc[r][j]);
         }
       }
     }
   }
 #pragma unroll
-  for (int r = 0; r < ROWS_PER_WARP; ++r) {
+  for (int r = 0; r < RW; ++r)
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
       float v = acc[r][j];
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      acc[r][j] = v;
+      if (lane == 0) part[half][group * RW + r][j] = v;
     }
+  __syncthreads();
+  const int e = threadIdx.x, r = e / NP, j = e % NP;       // 4 * RW * NP <= 256 sums, one per thread
+  const bool live = r < 4 * RW;
+  float v = live ? part[0][r][j] + part[1][r][j] : 0.f;
+  if (shares > 1) {
+    if (live) mine[r][j] = v;
+    cluster_arrive();
+    cluster_wait();
+    if (live && cluster_rank() == 0) {
+      float other[8];
+#pragma unroll
+      for (uint32_t c = 1; c < 8; ++c)
+        if (c < shares) other[c] = ld_cluster(&mine[r][j], c);
+#pragma unroll
+      for (uint32_t c = 1; c < 8; ++c)
+        if (c < shares) v += other[c];
+    }
+    cluster_arrive();                      // nobody leaves while the first CTA may still read its sums
+    cluster_wait();
+    if (cluster_rank() != 0) return;
   }
-  store_row_sums<NP>(acc, out, row0, m, n, lane, act);
+  const uint64_t row = (uint64_t)blockIdx.x * (4 * RW) + (uint64_t)r;
+  if (live && row < m && j < (int)n) out[row * n + j] = act ? sigmoid_clamped(v) : v;
 }
 
 // ---------------------------------------------------------------- small n, K-major left, R resident
@@ -127,6 +172,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
 small_n_kmajor_resident_kernel(const float* __restrict__ left, const float* __restrict__ right,
                                float* __restrict__ out, uint64_t m, uint64_t n, uint64_t k, uint64_t rsk,
                                uint64_t rsj, int act) {
+  pdl_enter();
   extern __shared__ float bs[];   // [NP][k + 4], k contiguous
   const uint32_t kpad = (uint32_t)k + 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -209,6 +255,7 @@ small_n_kmajor_resident_kernel(const float* __restrict__ left, const float* __re
 // ---------------------------------------------------------------- small n, MN-major left (split k)
 
 constexpr int KS = 128;   // rows of R staged per pass
+constexpr uint64_t kClusterRows = 1024;   // sums of at most this many terms are cut over the CTAs of one cluster
 
 // Two fused multiply-adds in one instruction (sm_100: fma.rn.f32x2 on register pairs), each
 // an IEEE fma like fmaf: (c.lo, c.hi) = (a.lo, a.hi) * (b.lo, b.hi) + (c.lo, c.hi).
@@ -227,75 +274,116 @@ __device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& 
 // The kernel issues one instruction per two multiply-adds and reads each value of the staged
 // operand as a ready-made (b, b) pair: at 16 columns the plain form needs every issue slot of
 // the SM to keep up with HBM (64 FMA + 16 shared-memory loads per 16 bytes streamed).
-template <int NP>
+// VEC: the thread's four rows are neighbours, one 128-bit load per k; otherwise (rows of `left` that start anywhere) they
+// are kThreads apart, four coalesced 32-bit loads.
+// `shares` > 1: the splits are the CTAs of a cluster, which add their sums through distributed shared memory (ascending
+// split index, the order of reduce_splits_kernel: the same bits) and store the result; one launch and no scratch for
+// products of few k, where a second launch costs as much as the first.
+template <int NP, bool VEC>
 __global__ void __launch_bounds__(kThreads, 2)
 small_n_mnmajor_kernel(const float* __restrict__ left, const float* __restrict__ right,
                        float* __restrict__ partial, uint64_t m, uint64_t n, uint64_t k, uint64_t rsk,
-                       uint64_t rsj, uint64_t k_per_split) {
-  __shared__ __align__(8) float2 bs[KS][NP];   // every value twice: one 64-bit load yields the pair
-  const uint64_t m0 = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
+                       uint64_t rsj, uint64_t k_per_split, uint32_t shares) {
+  __shared__ __align__(16) float2 bs[KS][NP];   // every value twice: one 64-bit load yields the pair
+  extern __shared__ float tile[];               // with shares: this CTA's sums, [1024 rows][n]
+  pdl_enter();
+  const uint64_t block = (uint64_t)blockIdx.x * kThreads * 4;
+  const uint64_t m0 = VEC ? block + threadIdx.x * 4 : block + threadIdx.x;
+  const uint64_t step = VEC ? 1 : kThreads;     // between the thread's rows
   const uint64_t kbeg = (uint64_t)blockIdx.y * k_per_split;
   const uint64_t kend = (kbeg + k_per_split < k) ? kbeg + k_per_split : k;
   unsigned long long acc01[NP], acc23[NP];      // rows (0,1) and (2,3) of the thread's four
 #pragma unroll
   for (int j = 0; j < NP; ++j) acc01[j] = acc23[j] = 0ull;
-  const bool live = m0 < m;   // m is a multiple of 4
+  const bool live = m0 < m;   // VEC: m is a multiple of 4
+  auto load = [&](uint64_t kk) {
+    const float* src = left + kk * m + m0;
+    if (VEC) return __ldcs(reinterpret_cast<const float4*>(src));
+    return make_float4(__ldcs(src), m0 + kThreads < m ? __ldcs(src + kThreads) : 0.f,
+                       m0 + 2 * kThreads < m ? __ldcs(src + 2 * kThreads) : 0.f,
+                       m0 + 3 * kThreads < m ? __ldcs(src + 3 * kThreads) : 0.f);
+  };
+  auto multiply = [&](const float4& a, int kk) {
+    const unsigned long long a01 = pack2(a.x, a.y), a23 = pack2(a.z, a.w);
+#pragma unroll
+    for (int j = 0; j + 1 < NP; j += 2) {
+      // two pairs per 128-bit load
+      const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(&bs[kk][j]);
+      ffma2(acc01[j], a01, bb.x);
+      ffma2(acc23[j], a23, bb.x);
+      ffma2(acc01[j + 1], a01, bb.y);
+      ffma2(acc23[j + 1], a23, bb.y);
+    }
+    if (NP & 1) {
+      const unsigned long long bb = *reinterpret_cast<const unsigned long long*>(&bs[kk][NP - 1]);
+      ffma2(acc01[NP - 1], a01, bb);
+      ffma2(acc23[NP - 1], a23, bb);
+    }
+  };
   for (uint64_t k0 = kbeg; k0 < kend; k0 += KS) {
     const int ks = (int)((kend - k0 < KS) ? (kend - k0) : KS);
     __syncthreads();
-    for (int e = threadIdx.x; e < KS * NP; e += kThreads) {
+    for (int e = threadIdx.x; e < ks * NP; e += kThreads) {
       int j = e % NP, kk = e / NP;
-      float v = 0.f;
-      if (kk < ks && (uint64_t)j < n) v = right[(k0 + kk) * rsk + (uint64_t)j * rsj];
+      const float v = (uint64_t)j < n ? right[(k0 + kk) * rsk + (uint64_t)j * rsj] : 0.f;
       bs[kk][j] = make_float2(v, v);
     }
     __syncthreads();
     if (live) {
       int kk = 0;
       // eight 128-bit loads in flight per thread: two CTAs of 256 threads per SM then keep
-      // 64 KB outstanding, what HBM latency x bandwidth asks of one SM
-      for (; kk + 8 <= ks; kk += 8) {
-        float4 a[8];
+      // 64 KB outstanding, what HBM latency x bandwidth asks of one SM; sixteen where the sums leave registers for it
+      constexpr int kBatch = NP <= 4 ? 16 : 8;
+      for (; kk + kBatch <= ks; kk += kBatch) {
+        float4 a[kBatch];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          a[u] = __ldcs(reinterpret_cast<const float4*>(left + (k0 + kk + u) * m + m0));
+        for (int u = 0; u < kBatch; ++u) a[u] = load(k0 + kk + u);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const unsigned long long a01 = pack2(a[u].x, a[u].y), a23 = pack2(a[u].z, a[u].w);
-#pragma unroll
-          for (int j = 0; j < NP; ++j) {
-            const unsigned long long bb = *reinterpret_cast<const unsigned long long*>(&bs[kk + u][j]);
-            ffma2(acc01[j], a01, bb);
-            ffma2(acc23[j], a23, bb);
-          }
-        }
+        for (int u = 0; u < kBatch; ++u) multiply(a[u], kk + u);
       }
-      for (; kk < ks; ++kk) {
-        const float4 a = __ldcs(reinterpret_cast<const float4*>(left + (k0 + kk) * m + m0));
-        const unsigned long long a01 = pack2(a.x, a.y), a23 = pack2(a.z, a.w);
-#pragma unroll
-        for (int j = 0; j < NP; ++j) {
-          const unsigned long long bb = *reinterpret_cast<const unsigned long long*>(&bs[kk][j]);
-          ffma2(acc01[j], a01, bb);
-          ffma2(acc23[j], a23, bb);
-        }
-      }
+      for (; kk < ks; ++kk) multiply(load(k0 + kk), kk);
     }
   }
-  if (live) {
-    float* dst = partial + ((uint64_t)blockIdx.y * m + m0) * n;
+  float v[4][NP];
 #pragma unroll
-    for (int j = 0; j < NP; ++j) {
-      float r0, r1, r2, r3;
-      unpack2(acc01[j], r0, r1);
-      unpack2(acc23[j], r2, r3);
-      if ((uint64_t)j < n) {
-        dst[j] = r0;
-        dst[n + j] = r1;
-        dst[2 * n + j] = r2;
-        dst[3 * n + j] = r3;
-      }
+  for (int j = 0; j < NP; ++j) {
+    unpack2(acc01[j], v[0][j], v[1][j]);
+    unpack2(acc23[j], v[2][j], v[3][j]);
+  }
+  if (shares > 1) {
+    const uint32_t at = VEC ? threadIdx.x * 4 : threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < NP; ++j)
+        if ((uint64_t)j < n) tile[(at + i * (uint32_t)step) * (uint32_t)n + j] = v[i][j];
+    cluster_arrive();
+    cluster_wait();
+    const uint64_t rows = m - block < 4 * kThreads ? m - block : 4 * kThreads;
+    const uint32_t total = (uint32_t)(rows * n), rank = cluster_rank();
+    const uint32_t per = (total + shares - 1) / shares, end = (rank + 1) * per < total ? (rank + 1) * per : total;
+    for (uint32_t e = rank * per + threadIdx.x; e < end; e += kThreads) {
+      float part[8], s = 0.f;
+#pragma unroll
+      for (uint32_t c = 0; c < 8; ++c)
+        if (c < shares) part[c] = ld_cluster(&tile[e], c);
+#pragma unroll
+      for (uint32_t c = 0; c < 8; ++c)
+        if (c < shares) s += part[c];
+      partial[block * n + e] = s;          // the result itself
     }
+    cluster_arrive();                      // nobody leaves while another CTA may still read its sums
+    cluster_wait();
+    return;
+  }
+  float* dst = partial + (uint64_t)blockIdx.y * m * n;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint64_t row = m0 + i * step;
+    if (row >= m) continue;
+#pragma unroll
+    for (int j = 0; j < NP; ++j)
+      if ((uint64_t)j < n) dst[row * n + j] = v[i][j];
   }
 }
 
@@ -320,6 +408,7 @@ __device__ __forceinline__ float sum_splits(const float* __restrict__ partial, u
 __global__ void __launch_bounds__(kThreads)
 reduce_splits_kernel(const float* __restrict__ partial, float* __restrict__ out, uint64_t elems,
                      uint32_t splits) {
+  pdl_enter();
   const uint64_t stride = (uint64_t)gridDim.x * kThreads;
   for (uint64_t e = (uint64_t)blockIdx.x * kThreads + threadIdx.x; e < elems; e += stride)
     out[e] = sum_splits(partial, elems, e, splits);
@@ -331,6 +420,7 @@ reduce_splits_kernel(const float* __restrict__ partial, float* __restrict__ out,
 __global__ void __launch_bounds__(kThreads)
 reduce_splits_transposed_kernel(const float* __restrict__ partial, float* __restrict__ out, uint64_t m,
                                 uint64_t n, uint32_t splits) {
+  pdl_enter();
   const uint64_t elems = m * n, stride = (uint64_t)gridDim.x * kThreads;
   for (uint64_t e = (uint64_t)blockIdx.x * kThreads + threadIdx.x; e < elems; e += stride) {
     out[(e % n) * m + e / n] = sum_splits(partial, elems, e, splits);
@@ -348,6 +438,7 @@ small_k_kernel(const float* __restrict__ left, const float* __restrict__ right, 
                uint64_t m, uint64_t n, uint64_t k, uint64_t lsi, uint64_t lsk, uint64_t rsk,
                uint64_t rsj, int vec_store, const float* __restrict__ sig) {
   __shared__ float as[RK][KP];
+  pdl_enter();
   const uint64_t j0 = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
   // Each thread's four columns of the small operand stay in registers while the CTA walks
   // over row blocks (gridDim.y CTAs share the rows of one column block).
@@ -442,7 +533,8 @@ __global__ void __launch_bounds__(kThreads, NP > 10 ? 1 : 2)
 dense_grad_kernel(const float* __restrict__ H, const float* __restrict__ dz, const float* __restrict__ W,
                   float* __restrict__ din, float* __restrict__ partial, uint64_t rows, uint64_t kh, uint64_t n,
                   uint64_t rows_per_split) {
-  __shared__ __align__(8) float2 bs[KS][NP];   // dZ rows, every value twice: one 64-bit load yields the pair
+  pdl_enter();
+  __shared__ __align__(16) float2 bs[KS][NP];   // dZ rows, every value twice: one 64-bit load yields the pair
   const uint64_t m0 = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
   const uint64_t rbeg = (uint64_t)blockIdx.y * rows_per_split;
   const uint64_t rend = (rbeg + rows_per_split < rows) ? rbeg + rows_per_split : rows;
@@ -482,14 +574,19 @@ dense_grad_kernel(const float* __restrict__ H, const float* __restrict__ dz, con
         if (rr + u >= rs) continue;
         const unsigned long long h01 = pack2(h[u].x, h[u].y), h23 = pack2(h[u].z, h[u].w);
         unsigned long long c01 = 0ull, c23 = 0ull;   // (dZ . W^T) for the four columns
-#pragma unroll
-        for (int j = 0; j < NP; ++j) {
-          const unsigned long long dd = *reinterpret_cast<const unsigned long long*>(&bs[rr + u][j]);
+        auto term = [&](unsigned long long dd, int j) {
           ffma2(c01, dd, w01[j]);
           ffma2(c23, dd, w23[j]);
           ffma2(acc01[j], h01, dd);
           ffma2(acc23[j], h23, dd);
+        };
+#pragma unroll
+        for (int j = 0; j + 1 < NP; j += 2) {              // two pairs per 128-bit load
+          const ulonglong2 dd = *reinterpret_cast<const ulonglong2*>(&bs[rr + u][j]);
+          term(dd.x, j);
+          term(dd.y, j + 1);
         }
+        if (NP & 1) term(*reinterpret_cast<const unsigned long long*>(&bs[rr + u][NP - 1]), NP - 1);
         float c0, c1, c2, c3;
         unpack2(c01, c0, c1);
         unpack2(c23, c2, c3);
@@ -520,15 +617,26 @@ dense_grad_kernel(const float* __restrict__ H, const float* __restrict__ dz, con
 
 inline int round_np(uint64_t n) { return n <= 1 ? 1 : n <= 2 ? 2 : n <= 4 ? 4 : n <= 8 ? 8 : n <= 10 ? 10 : 16; }
 
+// Into how many parts the k range of a small-n product with M-contiguous left is cut: about two CTAs per SM, parts of at
+// least KS rows - or of 16, as long as parts of KS rows leave SMs without a CTA.
 uint32_t splits_for(uint64_t m, uint64_t k) {
-  uint64_t m_blocks = (m / 4 + kThreads - 1) / kThreads;
+  uint64_t m_blocks = (m + 4 * kThreads - 1) / (4 * kThreads);
+  if (m_blocks < 1) m_blocks = 1;
   uint64_t want = ((uint64_t)sm_count() * 2 + m_blocks - 1) / m_blocks;   // about two CTAs per SM
   uint64_t max_by_k = (k + KS - 1) / KS;
+  if (max_by_k * m_blocks < (uint64_t)sm_count()) {
+    const uint64_t fine = (k + 15) / 16, enough = ((uint64_t)sm_count() + m_blocks - 1) / m_blocks;
+    max_by_k = fine < enough ? fine : enough;
+    // few enough rows for one cluster: its sums need no second launch
+    if (k <= kClusterRows) max_by_k = max_by_k < 8 ? max_by_k : 8;
+  }
   uint64_t s = want < max_by_k ? want : max_by_k;
   if (s < 1) s = 1;
   if (s > 4096) s = 4096;
   return (uint32_t)s;
 }
+// Whether the parts run as one cluster that adds them itself.
+bool sum_in_cluster(uint64_t k, uint64_t n, uint32_t splits) { return splits > 1 && splits <= 8 && n <= 10 && k <= kClusterRows; }
 
 template <int NP>
 int launch_small_n_k(const float* l, const float* r, float* out, uint64_t m, uint64_t n, uint64_t k,
@@ -536,7 +644,7 @@ int launch_small_n_k(const float* l, const float* r, float* out, uint64_t m, uin
   // whole small operand resident in shared memory when it fits (and there are rows
   // enough to keep every SM busy); otherwise k slabs
   const size_t resident = (size_t)NP * (k + 4) * sizeof(float);
-  if (resident <= 200 * 1024 && m >= 4096) {
+  if (resident <= 200 * 1024 && m >= kResidentRows && (k & 3) == 0 && aligned16(l)) {
     static bool res_attr[64] = {false};
     int d = 0;
     cudaGetDevice(&d);
@@ -546,42 +654,53 @@ int launch_small_n_k(const float* l, const float* r, float* out, uint64_t m, uin
       if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFuncSetAttribute(small_n resident)", e);
       res_attr[d] = true;
     }
-    small_n_kmajor_resident_kernel<NP><<<(unsigned)sm_count(), kResidentThreads, resident, st>>>(
-        l, r, out, m, n, k, rsk, rsj, act);
-    return check_launch("fmatmul_small_n_resident");
+    return launch("fmatmul_small_n_resident", small_n_kmajor_resident_kernel<NP>, (unsigned)sm_count(), kResidentThreads,
+                  resident, st, l, r, out, m, n, k, rsk, rsj, act);
   }
+  // one row per warp until every SM has a CTA, then up to four; k in up to 8 shares of at least 128 while SMs are free
+  const uint64_t sms = (uint64_t)sm_count();
+  const int rw = m >= 16 * sms ? 4 : m >= 8 * sms ? 2 : 1;
+  const uint64_t groups = (m + 4 * rw - 1) / (4 * rw);
+  uint32_t shares = 1;
+  while (shares < 8 && groups * shares * 2 <= 2 * sms && k / (shares * 2) >= 128) shares *= 2;
+  if (groups > 0x7fffffffull) return fail(POLAR_B200_ERR_UNSUPPORTED, "too many rows");
   const size_t smem = (size_t)NP * KT_PAD * sizeof(float);
-  static bool attr_done[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (smem > 48 * 1024 && dev >= 0 && dev < 64 && !attr_done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(small_n_kmajor_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const bool vec = (k & 3) == 0 && aligned16(l);
+  auto go = [&](auto kernel) {
+    cudaError_t e = smem > 48 * 1024 - 4096 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
     if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFuncSetAttribute(small_n)", e);
-    attr_done[dev] = true;
-  }
-  uint64_t rows_per_cta = (kThreads / 32) * ROWS_PER_WARP;
-  uint64_t grid = (m + rows_per_cta - 1) / rows_per_cta;
-  if (grid > 0x7fffffffull) return fail(POLAR_B200_ERR_UNSUPPORTED, "too many rows");
-  small_n_kmajor_kernel<NP><<<(unsigned)grid, kThreads, smem, st>>>(l, r, out, m, n, k, rsk, rsj, act);
-  return check_launch("fmatmul_small_n");
+    return launch_clusters("fmatmul_small_n", kernel, dim3((unsigned)groups, shares), kThreads, smem, st, shares, l, r, out, m, n, k,
+                           rsk, rsj, act, shares);
+  };
+  if (vec) return rw == 4 ? go(small_n_rows_kernel<NP, 4, true>) : rw == 2 ? go(small_n_rows_kernel<NP, 2, true>) : go(small_n_rows_kernel<NP, 1, true>);
+  return rw == 4 ? go(small_n_rows_kernel<NP, 4, false>) : rw == 2 ? go(small_n_rows_kernel<NP, 2, false>) : go(small_n_rows_kernel<NP, 1, false>);
+}
+
+int launch_reduce(const float* ws, float* out, uint64_t elems, uint32_t splits, cudaStream_t st) {
+  const uint64_t g = (elems + kThreads - 1) / kThreads, cap = (uint64_t)sm_count() * 4;
+  return launch("fmatmul_reduce_splits", reduce_splits_kernel, (unsigned)(g < cap ? g : cap), kThreads, 0, st, ws, out, elems, splits);
 }
 
 template <int NP>
 int launch_small_n_mn(const float* l, const float* r, float* out, float* ws, uint32_t splits, uint64_t m,
                       uint64_t n, uint64_t k, uint64_t rsk, uint64_t rsj, cudaStream_t st) {
-  uint64_t m_blocks = (m / 4 + kThreads - 1) / kThreads;
+  uint64_t m_blocks = (m + 4 * kThreads - 1) / (4 * kThreads);
   uint64_t k_per_split = (k + splits - 1) / splits;
   k_per_split = (k_per_split + 3) & ~3ull;
+  if (m_blocks < 1) m_blocks = 1;
   dim3 grid((unsigned)m_blocks, splits);
-  float* dst = splits > 1 ? ws : out;
-  small_n_mnmajor_kernel<NP><<<grid, kThreads, 0, st>>>(l, r, dst, m, n, k, rsk, rsj, k_per_split);
-  int rc = check_launch("fmatmul_small_n_split");
-  if (rc || splits == 1) return rc;
-  uint64_t elems = m * n;
-  uint64_t g = (elems + kThreads - 1) / kThreads;
-  uint64_t cap = (uint64_t)sm_count() * 4;
-  reduce_splits_kernel<<<(unsigned)(g < cap ? g : cap), kThreads, 0, st>>>(ws, out, elems, splits);
-  return check_launch("fmatmul_reduce_splits");
+  const bool in_cluster = sum_in_cluster(k, n, splits), vec = (m & 3) == 0 && aligned16(l);
+  float* dst = splits > 1 && !in_cluster ? ws : out;
+  const size_t smem = in_cluster ? (size_t)4 * kThreads * n * sizeof(float) : 0;
+  auto go = [&](auto kernel) {
+    cudaError_t e = smem + KS * NP * sizeof(float2) > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+    if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFuncSetAttribute(small_n split)", e);
+    return launch_clusters("fmatmul_small_n_split", kernel, grid, kThreads, smem, st, in_cluster ? splits : 1, l, r, dst, m, n, k, rsk,
+                           rsj, k_per_split, in_cluster ? splits : 1);
+  };
+  int rc = vec ? go(small_n_mnmajor_kernel<NP, true>) : go(small_n_mnmajor_kernel<NP, false>);
+  if (rc || splits == 1 || in_cluster) return rc;
+  return launch_reduce(ws, out, m * n, splits, st);
 }
 
 template <int NP>
@@ -593,14 +712,9 @@ int launch_dense_grad_np(const float* H, const float* dz, const float* W, float*
   rows_per_split = (rows_per_split + 3) & ~3ull;
   dim3 grid((unsigned)m_blocks, splits);
   float* dst = splits > 1 ? ws : dw;
-  dense_grad_kernel<NP><<<grid, kThreads, 0, st>>>(H, dz, W, din, dst, rows, kh, n, rows_per_split);
-  int rc = check_launch("fdense_grad");
+  int rc = launch("fdense_grad", dense_grad_kernel<NP>, grid, kThreads, 0, st, H, dz, W, din, dst, rows, kh, n, rows_per_split);
   if (rc || splits == 1) return rc;
-  uint64_t elems = kh * n;
-  uint64_t g = (elems + kThreads - 1) / kThreads;
-  uint64_t cap = (uint64_t)sm_count() * 4;
-  reduce_splits_kernel<<<(unsigned)(g < cap ? g : cap), kThreads, 0, st>>>(ws, dw, elems, splits);
-  return check_launch("fdense_grad_reduce");
+  return launch_reduce(ws, dw, kh * n, splits, st);
 }
 
 }  // namespace skinny
@@ -620,20 +734,19 @@ int launch_ragged_rows(const float* left_tail, uint64_t left_pitch, const float*
   uint64_t k_per_split = (k + splits - 1) / splits;
   k_per_split = (k_per_split + 3) & ~3ull;
   dim3 grid((unsigned)m_blocks, splits);
-  const int np = round_np(rem);
-  switch (np) {
+  int rc;
+  switch (round_np(rem)) {
 #define POLAR_RAGGED(NP) \
-  case NP: small_n_mnmajor_kernel<NP><<<grid, kThreads, 0, st>>>(right, left_tail, ws, n, rem, k, left_pitch, 1, k_per_split); break;
+  case NP: rc = launch("fmatmul_ragged_rows", small_n_mnmajor_kernel<NP, true>, grid, kThreads, 0, st, right, left_tail, ws, n, rem, k, left_pitch, (uint64_t)1, k_per_split, 1u); break;
     POLAR_RAGGED(1) POLAR_RAGGED(2) POLAR_RAGGED(4) POLAR_RAGGED(8) POLAR_RAGGED(10) POLAR_RAGGED(16)
 #undef POLAR_RAGGED
     default: return fail(POLAR_B200_ERR_UNSUPPORTED, "ragged rows: more than 16");
   }
-  int rc = check_launch("fmatmul_ragged_rows");
   if (rc) return rc;
   uint64_t g = (n * rem + kThreads - 1) / kThreads;
   uint64_t cap = (uint64_t)sm_count() * 4;
-  reduce_splits_transposed_kernel<<<(unsigned)(g < cap ? g : cap), kThreads, 0, st>>>(ws, out_tail, n, rem, splits);
-  return check_launch("fmatmul_ragged_rows_reduce");
+  return launch("fmatmul_ragged_rows_reduce", reduce_splits_transposed_kernel, (unsigned)(g < cap ? g : cap), kThreads, 0, st, ws,
+                out_tail, n, rem, splits);
 }
 
 // Which skinny kernel, if any, serves this shape: 1 = small n with K-major left,
@@ -642,8 +755,9 @@ int skinny_kind(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float*
                 const float* right, const float* out) {
   (void)tr; (void)right;
   if (n <= 16 && k >= 32) {
-    if (!tl && (k & 3) == 0 && aligned16(left)) return 1;
-    if (tl && (m & 3) == 0 && aligned16(left)) return 2;
+    // many unaligned rows stay off: their 32-bit loads would be bound by the re-reads of the small operand
+    if (!tl && (((k & 3) == 0 && aligned16(left)) || m < skinny::kResidentRows)) return 1;
+    if (tl) return 2;
   }
   if (k <= 16 && n >= 32) return 3;
   (void)out;
@@ -653,6 +767,7 @@ int skinny_kind(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float*
 uint64_t skinny_workspace_bytes(int kind, uint64_t m, uint64_t n, uint64_t k) {
   if (kind != 2) return 0;
   uint32_t s = skinny::splits_for(m, k);
+  if (skinny::sum_in_cluster(k, n, s)) return 0;
   return s > 1 ? (uint64_t)s * m * n * sizeof(float) : 0;
 }
 
@@ -682,8 +797,8 @@ int launch_skinny(int kind, int tl, int tr, uint64_t m, uint64_t n, uint64_t k, 
   }
   // small k
   const uint64_t lsi = tl ? 1 : k, lsk = tl ? m : 1;
-  uint64_t gx = ((n + 3) / 4 + kThreads - 1) / kThreads, gy = (m + RK - 1) / RK;
-  // about three CTAs per SM in all; each takes an equal share of the rows
+  // about three CTAs per SM in all, each with an equal share of the rows (a multiple of four)
+  uint64_t gx = ((n + 3) / 4 + kThreads - 1) / kThreads, gy = (m + 3) / 4;
   const uint64_t gy_cap = ((uint64_t)sm_count() * 3 + gx - 1) / gx;
   if (gy > gy_cap) gy = gy_cap;
   if (gy > 65535) {
@@ -691,15 +806,11 @@ int launch_skinny(int kind, int tl, int tr, uint64_t m, uint64_t n, uint64_t k, 
   }
   dim3 grid((unsigned)gx, (unsigned)gy);
   int vec = ((n & 3) == 0) && aligned16(out) && (!sig || aligned16(sig));
-  if (k <= 4)
-    small_k_kernel<4><<<grid, kThreads, 0, st>>>(left, right, out, m, n, k, lsi, lsk, rsk, rsj, vec, sig);
-  else if (k <= 10)
-    small_k_kernel<10><<<grid, kThreads, 0, st>>>(left, right, out, m, n, k, lsi, lsk, rsk, rsj, vec, sig);
-  else
-    small_k_kernel<16><<<grid, kThreads, 0, st>>>(left, right, out, m, n, k, lsi, lsk, rsk, rsj, vec, sig);
-  return check_launch("fmatmul_small_k");
+  auto go = [&](auto kernel) {
+    return launch("fmatmul_small_k", kernel, grid, kThreads, 0, st, left, right, out, m, n, k, lsi, lsk, rsk, rsj, vec, sig);
+  };
+  return k <= 4 ? go(small_k_kernel<4>) : k <= 10 ? go(small_k_kernel<10>) : go(small_k_kernel<16>);
 }
-
 
 // Whether the one-pass dense-layer backward serves these sizes, i.e. whether the two separate
 // products would run on the small-n (left M-contiguous) and small-k kernels whose arithmetic it
@@ -708,7 +819,8 @@ bool dense_grad_ok(uint64_t rows, uint64_t kh, uint64_t n, const float* H, const
   return n >= 1 && n <= 16 && rows >= 32 && kh >= 32 && (kh & 3) == 0 && aligned16(H) && aligned16(din);
 }
 uint64_t dense_grad_workspace_bytes(uint64_t rows, uint64_t kh, uint64_t n) {
-  return skinny_workspace_bytes(2, kh, n, rows);
+  const uint32_t s = skinny::splits_for(kh, rows);
+  return s > 1 ? (uint64_t)s * kh * n * sizeof(float) : 0;
 }
 int launch_dense_grad(const float* H, const float* dz, const float* W, float* din, float* dw, float* ws,
                       uint64_t rows, uint64_t kh, uint64_t n, cudaStream_t st) {
