@@ -54,6 +54,35 @@ __device__ __forceinline__ void store_row_sums(const float (&acc)[ROWS_PER_WARP]
   }
 }
 
+// Puts kt x n elements of the small operand into shared memory as [n][pitch], k contiguous.  Read in the order they are
+// stored in - whole lines - and eight at a time: one element per trip was one memory latency per trip, 15 us for the
+// 4096 x 10 of the MLP's output layer.
+template <int THREADS>
+__device__ __forceinline__ void stage_small_operand(const float* __restrict__ right, float* bs, int kt, int n, int pitch,
+                                                    uint64_t rsk, uint64_t rsj) {
+  constexpr int kBatch = 8;
+  const bool by_k = rsk == 1;
+  const uint32_t inner = by_k ? kt : n, total = (uint32_t)kt * (uint32_t)n;
+  const uint32_t step_out = THREADS / inner, step_in = THREADS % inner;
+  uint32_t o = threadIdx.x / inner, i = threadIdx.x % inner;   // one division: later elements are THREADS further on
+  for (uint32_t e = threadIdx.x; e < total; e += kBatch * THREADS) {
+    float v[kBatch];
+    uint32_t at[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const uint32_t j = by_k ? o : i, kk = by_k ? i : o;
+      at[u] = j * pitch + kk;
+      v[u] = e + u * THREADS < total ? right[(uint64_t)kk * rsk + (uint64_t)j * rsj] : 0.f;
+      i += step_in;
+      o += step_out;
+      if (i >= inner) i -= inner, ++o;
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u)
+      if (e + u * THREADS < total) bs[at[u]] = v[u];
+  }
+}
+
 // Few rows (below kResidentRows), or rows TMA-like loads cannot take as vectors: a CTA computes 4 * RW rows, two warps per
 // row group, over one share of k; the CTAs of a cluster hold the shares of the same rows and add them through
 // distributed shared memory in rank order.  Bound by latency: what counts is that every SM has a CTA, so the host cuts k
@@ -82,12 +111,7 @@ small_n_rows_kernel(const float* __restrict__ left, const float* __restrict__ ri
   for (uint64_t k0 = kbeg; k0 < kend; k0 += KT) {
     const int kt = (int)((kend - k0 < KT) ? (kend - k0) : KT);
     __syncthreads();
-    // in the order the operand is stored in, so that the reads are whole lines
-    const bool by_k = rsk == 1;
-    for (int e = threadIdx.x; e < kt * (int)n; e += kThreads) {
-      const int j = by_k ? e / kt : e % (int)n, kk = by_k ? e % kt : e / (int)n;
-      bs[j * KT_PAD + kk] = right[(k0 + kk) * rsk + (uint64_t)j * rsj];
-    }
+    stage_small_operand<kThreads>(right + k0 * rsk, bs, kt, (int)n, KT_PAD, rsk, rsj);
     __syncthreads();
     if (VEC) {
       for (int kk = (half * 32 + lane) * 4; kk < kt; kk += 256) {
@@ -194,10 +218,10 @@ small_n_kmajor_resident_kernel(const float* __restrict__ left, const float* __re
     }
   };
   if (g < groups && (uint32_t)lane * 4 < (uint32_t)k) load_chunk(g, lane * 4);
-  for (uint64_t e = threadIdx.x; e < (uint64_t)NP * k; e += kResidentThreads) {
-    uint32_t j = (uint32_t)(e % NP), kk = (uint32_t)(e / NP);
-    bs[j * kpad + kk] = ((uint64_t)j < n) ? right[(uint64_t)kk * rsk + (uint64_t)j * rsj] : 0.f;
-  }
+  if (n < NP)
+    for (uint32_t e = threadIdx.x; e < (NP - (uint32_t)n) * (uint32_t)k; e += kResidentThreads)
+      bs[((uint32_t)n + e / (uint32_t)k) * kpad + e % (uint32_t)k] = 0.f;
+  stage_small_operand<kResidentThreads>(right, bs, (int)k, (int)n, (int)kpad, rsk, rsj);
   __syncthreads();
   for (; g < groups; g += warps_total) {
     const uint64_t row0 = g * ROWS_PER_WARP;
@@ -255,7 +279,7 @@ small_n_kmajor_resident_kernel(const float* __restrict__ left, const float* __re
 // ---------------------------------------------------------------- small n, MN-major left (split k)
 
 constexpr int KS = 128;   // rows of R staged per pass
-constexpr uint64_t kClusterRows = 1024;   // sums of at most this many terms are cut over the CTAs of one cluster
+constexpr uint64_t kClusterRows = 384;   // sums of at most this many terms are cut over the CTAs of one cluster
 
 // Two fused multiply-adds in one instruction (sm_100: fma.rn.f32x2 on register pairs), each
 // an IEEE fma like fmaf: (c.lo, c.hi) = (a.lo, a.hi) * (b.lo, b.hi) + (c.lo, c.hi).
@@ -388,11 +412,18 @@ small_n_mnmajor_kernel(const float* __restrict__ left, const float* __restrict__
 }
 
 // Sum of one element over the splits, ascending split index (a fixed order); the loads of
-// eight splits are issued together, the additions stay in order.
+// up to 32 splits are issued together, the additions stay in order.
 __device__ __forceinline__ float sum_splits(const float* __restrict__ partial, uint64_t elems, uint64_t e,
                                             uint32_t splits) {
   float s = 0.f;
   uint32_t sp = 0;
+  for (; sp + 32 <= splits; sp += 32) {
+    float v[32];
+#pragma unroll
+    for (int u = 0; u < 32; ++u) v[u] = __ldcg(partial + (uint64_t)(sp + u) * elems + e);
+#pragma unroll
+    for (int u = 0; u < 32; ++u) s += v[u];
+  }
   for (; sp + 8 <= splits; sp += 8) {
     float v[8];
 #pragma unroll
