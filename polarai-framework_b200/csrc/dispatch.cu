@@ -190,27 +190,27 @@ namespace {
 // ---- the cluster kernel (gemm_tc_mid.cu) --------------------------------------------------------------
 // One 128 x bn tile per cluster of CTAs.  Times in microseconds, fitted to measurements on B200 between
 // 128 x 64 x 64 and 2048^3 (within 15 % there): a slab of 32 k costs a CTA 0.43 / 0.48 / 0.60 us with tiles of 32 / 64 / 128
-// columns (0.62 / 0.70 / 0.98 with the rounded split), set-up, pipeline fill and the store of the tile 4 to 5.5 us,
+// columns (0.58 / 0.66 / 0.80 with the exact split), set-up, pipeline fill and the store of the tile 4 to 5.5 us,
 // the exchange between the CTAs of a cluster 1 us.
 struct MidChoice {
   int bn = 0, cluster = 1, swap = 0;
   double us = 1e30;
 };
 
-MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool round) {
+MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact) {
   MidChoice best;
   const uint64_t sms = (uint64_t)sm_count(), slabs = (k + 31) / 32;
   for (int swap = 0; swap < 2; ++swap) {
     const uint64_t rows = swap ? n : m, cols = swap ? m : n;
     for (int i = 0; i < 3; ++i) {
       const int bn = 32 << i;
-      static const double slab_us[2][3] = {{0.43, 0.48, 0.60}, {0.62, 0.70, 0.98}};
+      static const double slab_us[2][3] = {{0.43, 0.48, 0.60}, {0.58, 0.66, 0.80}};
       const uint64_t tiles = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
       for (int cl = 1; cl <= 8 && (uint64_t)cl <= slabs; cl *= 2) {
-        // clusters of 4 and 8 leave SMs of a GPC unused
-        const uint64_t at_once = cl <= 2 ? sms : cl == 4 ? sms / 37 * 34 : sms / 37 * 32;
+        // clusters of 4 and 8 leave SMs of a GPC unused: 33 and 15 of them run at a time on 148 SMs
+        const uint64_t at_once = cl <= 2 ? sms : cl == 4 ? sms * 132 / 148 : sms * 120 / 148;
         const uint64_t waves = (tiles * cl + at_once - 1) / at_once;
-        const double one = (double)((slabs + cl - 1) / cl) * slab_us[round][i] + (bn == 128 ? 5.5 : 4.0) + (cl > 1 ? 1.0 : 0.0);
+        const double one = (double)((slabs + cl - 1) / cl) * slab_us[exact][i] + (bn == 128 ? 5.5 : 4.0) + (cl > 1 ? 1.0 : 0.0);
         const double us = (double)waves * one;
         if (us < best.us - 0.01) best = MidChoice{bn, cl, swap, us};
       }
@@ -241,9 +241,9 @@ MidChoice mid_for_tc(uint64_t m, uint64_t n, uint64_t k, bool may_swap) {
 }
 
 // The rest - operands with an unaligned base or row pitch, which the cluster kernel takes as padded copies, and
-// products below a tile of gemm_tc.cu.  They had the FFMA kernel's round-to-nearest sums, so they get the rounded
-// split with short sums in tensor memory: 1.3e-7 to 1.6e-7 of the result's norm against float64 where FFMA
-// has 1.8e-7 (k = 98) to 8e-7 (k = 2048).  FFMA tiles (64 x 64, about two CTAs per SM at a time, 0.15 us per term) keep
+// products below a tile of gemm_tc.cu.  They had the FFMA kernel's round-to-nearest sums, so they get the exact
+// split with short sums in tensor memory: 1.3e-7 to 2.2e-7 of the result's norm against float64 where FFMA
+// has 1.8e-7 (k = 98) to 1.2e-6 (k = 4096).  FFMA tiles (64 x 64, about two CTAs per SM at a time, 0.15 us per term) keep
 // what is over before a padded copy and a pipeline have started.
 MidChoice mid_for_rest(uint64_t m, uint64_t n, uint64_t k, uint64_t pad_bytes) {
   MidChoice c = mid_choose(m, n, k, true);

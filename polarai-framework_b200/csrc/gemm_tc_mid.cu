@@ -11,9 +11,10 @@
 // One CTA:
 //   warp 0      TMA producer: 32-float k slabs of A (128 rows) and B (BN rows), two instructions per slab;
 //   warp 1      tcgen05.mma issuer: per slab and 8 k the three products of the TF32 split;
-//   warps 2-9   split warps: x -> hi + lo in shared memory.  With ROUND, hi is x rounded to the nearest TF32
-//               (written back over x) and lo = x - hi is at most half as long and of either sign, so that what
-//               the split drops (lo.lo, the bits of lo past TF32) is four times smaller and unbiased;
+//   warps 2-9   split warps: the lo parts, x - hi, of each landed slab (hi is what the tensor core sees of the raw word).
+//               With EXACT, lo is rounded to the nearest TF32 instead of cut off, lo.lo is computed too, and
+//               the products other than hi.hi get an accumulator of their own, where the tensor core's
+//               truncation hurts 1000 times less;
 //   warps 10-17 accumulator warps: every `chunk` slabs they read the tensor-memory accumulator and add it to
 //               registers in round-to-nearest.  The tensor core's own accumulator rounds toward zero, an error that
 //               grows with the length of the sum (8e-9 of the result per term for zero-mean operands);
@@ -130,14 +131,14 @@ __device__ __forceinline__ void store_share(const Params& p, uint32_t base, uint
   }
 }
 
-template <int BN, bool ROUND>
+template <int BN, bool EXACT>
 __global__ void __launch_bounds__(kThreads, 1)
 fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_a3, const __grid_constant__ CUtensorMap map_b3,
                    const Params p) {
   using C = Cfg<BN>;
-  // accumulators: with ROUND the cross products get one of their own (see above)
-  constexpr int kKinds = ROUND ? 2 : 1, kAccs = 4 / kKinds;
+  // accumulators: with EXACT the cross products get one of their own (see above)
+  constexpr int kKinds = EXACT ? 2 : 1, kAccs = 4 / kKinds;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -232,26 +233,24 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         for (uint32_t accumulate = 0; it < last; ++it, accumulate = 1) {
           const uint32_t a_hi = ring + ((s * C::kRawBytes) >> 4), b_hi = a_hi + (C::kABytes >> 4);
           const uint32_t a_lo = ring + ((C::kLoBase + l * C::kRawBytes) >> 4), b_lo = a_lo + (C::kABytes >> 4);
-          auto high_products = [&] {
+          // the raw words are the hi parts: no need to wait for the split
+          ok = mbar_wait(full_raw(s), s_ph, abort_flag, p.status, 112, p.wait_ns);
+          if (!ok) break;
+          tc_fence_after();
+          if (leader) {
 #pragma unroll
             for (int kk = 0; kk < BK / 8; ++kk)
               tc_mma_tf32(d, a_op, a_hi + kk * a_step, b_op, b_hi + kk * b_step, idesc, kk ? 1u : accumulate);
-          };
-          if (!ROUND) {                                     // the raw words are the hi parts: no need to wait for the split
-            ok = mbar_wait(full_raw(s), s_ph, abort_flag, p.status, 112, p.wait_ns);
-            if (!ok) break;
-            tc_fence_after();
-            if (leader) high_products();
           }
           ok = mbar_wait(full_lo(l), l_ph, abort_flag, p.status, 113, p.wait_ns);
           if (!ok) break;
           tc_fence_after();
           if (leader) {
-            if (ROUND) high_products();
 #pragma unroll
             for (int kk = 0; kk < BK / 8; ++kk) {
-              tc_mma_tf32(cross, a_op, a_lo + kk * a_step, b_op, b_hi + kk * b_step, idesc, (!ROUND || kk) ? 1u : accumulate);
+              tc_mma_tf32(cross, a_op, a_lo + kk * a_step, b_op, b_hi + kk * b_step, idesc, (!EXACT || kk) ? 1u : accumulate);
               tc_mma_tf32(cross, a_op, a_hi + kk * a_step, b_op, b_lo + kk * b_step, idesc, 1u);
+              if (EXACT) tc_mma_tf32(cross, a_op, a_lo + kk * a_step, b_op, b_lo + kk * b_step, idesc, 1u);
             }
             tc_commit(empty(s));
           }
@@ -274,10 +273,10 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       float4* lo = reinterpret_cast<float4*>(gen + C::kLoBase + l * C::kRawBytes);
       constexpr int kVecs = C::kRawBytes / 16;
       static_assert(kVecs % (kSplitWarps * 32) == 0, "slab must divide over the split warps");
-      auto high = [](float x) {
-        uint32_t u = __float_as_uint(x);
-        if (ROUND) asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
-        return __uint_as_float(u & 0xFFFFE000u);
+      auto low = [](float x) {
+        const float l = x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
+        // the tensor core ignores the low 13 bits: adding half of the last one it sees rounds to nearest
+        return EXACT ? __uint_as_float(__float_as_uint(l) + 0x1000u) : l;
       };
       // all loads before the first store: the compiler cannot tell that the two never meet, and would
       // make one latency of each vector
@@ -286,12 +285,8 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
       for (int i = 0; i < kMine; ++i) v[i] = raw[tid + i * kSplitWarps * 32];
 #pragma unroll
-      for (int i = 0; i < kMine; ++i) {
-        const int e = tid + i * kSplitWarps * 32;
-        const float4 h = {high(v[i].x), high(v[i].y), high(v[i].z), high(v[i].w)};
-        lo[e] = make_float4(v[i].x - h.x, v[i].y - h.y, v[i].z - h.z, v[i].w - h.w);
-        if (ROUND) raw[e] = h;
-      }
+      for (int i = 0; i < kMine; ++i)
+        lo[tid + i * kSplitWarps * 32] = make_float4(low(v[i].x), low(v[i].y), low(v[i].z), low(v[i].w));
       fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(full_lo(l));               // one arrival per warp
@@ -318,7 +313,7 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * kKinds * BN + half * kCols + j0);
         tmem_ld_32x16(at, r);
         tmem_ld_wait();
-        if (ROUND) {
+        if (EXACT) {
           uint32_t x[kPart];
           tmem_ld_32x16(at + BN, x);
           tmem_ld_wait();
@@ -407,7 +402,7 @@ struct Stored {
   bool padded;                                              // columns up to the pitch are there, and zero
 };
 
-template <int BN, bool ROUND>
+template <int BN, bool EXACT>
 int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Params p, uint64_t k, cudaStream_t stream) {
   using C = Cfg<BN>;
   int dev = 0;
@@ -417,7 +412,7 @@ int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Pa
   {
     std::lock_guard<std::mutex> guard(mu);
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(fmatmul_mid_kernel<BN, ROUND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
+      cudaError_t e = cudaFuncSetAttribute(fmatmul_mid_kernel<BN, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
       if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFuncSetAttribute(smem)", e);
       attr_done[dev] = true;
     }
@@ -463,7 +458,7 @@ int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Pa
   at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   c.attrs = at;
   c.numAttrs = p.cluster > 1 ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&c, fmatmul_mid_kernel<BN, ROUND>, maps[0], maps[1], maps3[0], maps3[1], p);
+  cudaError_t e = cudaLaunchKernelEx(&c, fmatmul_mid_kernel<BN, EXACT>, maps[0], maps[1], maps3[0], maps3[1], p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(POLAR_B200_ERR_CUDA, "fmatmul_mid", e);
@@ -491,7 +486,7 @@ uint64_t mid_workspace_bytes(int tl, int tr, uint64_t m, uint64_t n, uint64_t k,
 // out[m,n] = L'.R' with tiles of 128 x bn, `cluster` CTAs per tile.  swap: the operands exchange roles, the tile's
 // rows are columns of the result.  ws: mid_workspace_bytes.
 int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right, float* out, int bn,
-               int cluster, int round, int swap, int epilogue, float* ws, cudaStream_t stream) {
+               int cluster, int exact, int swap, int epilogue, float* ws, cudaStream_t stream) {
   using namespace mid;
   Stored l{left, tl ? k : m, tl ? m : k, tl ? m : k, false}, r{right, tr ? n : k, tr ? k : n, tr ? k : n, false};
   Padded copies[2] = {};
@@ -526,14 +521,14 @@ int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* 
   p.tiles_m = (uint32_t)((p.m + BM - 1) / BM);
   p.slabs = (uint32_t)((k + BK - 1) / BK);
   p.cluster = (uint32_t)cluster;
-  // sums of this many terms in tensor memory, the rest in registers
-  p.chunk = round ? 1 : 8;
+  // slabs of 32 terms summed in tensor memory, the rest in registers: EXACT is to stay below the error of FFMA sums
+  p.chunk = !exact ? 8 : k < 512 ? 1 : 2;
   if ((cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) || p.slabs < p.cluster) return fail(POLAR_B200_ERR_UNSUPPORTED, "fewer slabs than CTAs in a cluster");
   if ((uint64_t)p.tiles_m * ((p.n + bn - 1) / bn) * p.cluster > 0x7fffffffull) return fail(POLAR_B200_ERR_UNSUPPORTED, "too many tiles");
   // exchanged: right' plays the row operand - stored [k, n] is "row extent contiguous" - and left the column operand
   const Stored &a = swap ? r : l, &b = swap ? l : r;
   const bool a_mn = swap ? !tr : tl, b_mn = swap ? tl : !tr;
-#define POLAR_MID(BN)   case BN: return round ? launch_cfg<BN, true>(a, b, a_mn, b_mn, p, k, stream) : launch_cfg<BN, false>(a, b, a_mn, b_mn, p, k, stream);
+#define POLAR_MID(BN)   case BN: return exact ? launch_cfg<BN, true>(a, b, a_mn, b_mn, p, k, stream) : launch_cfg<BN, false>(a, b, a_mn, b_mn, p, k, stream);
   switch (bn) {
     POLAR_MID(32) POLAR_MID(64) POLAR_MID(128)
   }
