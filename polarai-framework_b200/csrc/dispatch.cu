@@ -18,7 +18,7 @@ bool tc_shape_ok(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float
                  const float* right);
 uint64_t mid_workspace_bytes(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right);
 int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right, float* out, int bn,
-               int cluster, int round, int swap, int epilogue, float* ws, cudaStream_t stream);
+               int cluster, uint64_t whole, int exact, int swap, int epilogue, float* ws, cudaStream_t stream);
 int skinny_kind(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                 const float* right, const float* out);
 uint64_t skinny_workspace_bytes(int kind, uint64_t m, uint64_t n, uint64_t k);
@@ -194,6 +194,7 @@ namespace {
 // the exchange between the CTAs of a cluster 1 us.
 struct MidChoice {
   int bn = 0, cluster = 1, swap = 0;
+  uint64_t whole = 0;
   double us = 1e30;
 };
 
@@ -212,7 +213,14 @@ MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact) {
         const uint64_t waves = (tiles * cl + at_once - 1) / at_once;
         const double one = (double)((slabs + cl - 1) / cl) * slab_us[exact][i] + (bn == 128 ? 5.5 : 4.0) + (cl > 1 ? 1.0 : 0.0);
         const double us = (double)waves * one;
-        if (us < best.us - 0.01) best = MidChoice{bn, cl, swap, us};
+        if (us < best.us - 0.01) best = MidChoice{bn, cl, swap, 0, us};
+        // one CTA per tile, except that a last wave of at most half the SMs has its tiles cut in two
+        const uint64_t full = tiles / sms * sms, rest = tiles - full;
+        if (cl == 1 && full && rest && 2 * rest <= sms && (full & 1) == 0 && slabs >= 2) {
+          const double tail = (double)((slabs + 1) / 2) * slab_us[exact][i] + (bn == 128 ? 6.5 : 5.0);
+          const double cut = (double)(full / sms) * one + tail;
+          if (cut < best.us - 0.01) best = MidChoice{bn, 2, swap, full, cut};
+        }
       }
     }
   }
@@ -359,7 +367,7 @@ static int tc_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const flo
     if (pitch == 0) {
       const MidChoice mid = mid_for_tc(m, n, k, true);
       if (mid.bn)
-        return launch_mid(tl, tr, m, n, k, left, right, out, mid.bn, mid.cluster, 0, mid.swap, fused == 1 ? 1 : 0, nullptr,
+        return launch_mid(tl, tr, m, n, k, left, right, out, mid.bn, mid.cluster, mid.whole, 0, mid.swap, fused == 1 ? 1 : 0, nullptr,
                           as_stream(stream));
     }
     const TcChoice c = tc_choose(m, n, k, pitch == 0);
@@ -449,7 +457,7 @@ static int fmatmul_impl(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, cons
         ws = own;
       }
       if (!pad || ws) {
-        rc = launch_mid(tl, tr, m, n, k, left, right, out, mid.bn, mid.cluster, 1, mid.swap, fused == 1 ? 1 : 0,
+        rc = launch_mid(tl, tr, m, n, k, left, right, out, mid.bn, mid.cluster, mid.whole, 1, mid.swap, fused == 1 ? 1 : 0,
                         static_cast<float*>(ws), as_stream(stream));
         if (own) {
           cudaError_t e = scratch_free(own, as_stream(stream));
@@ -614,7 +622,7 @@ int polar_b200_fmatmul_tc(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, co
       cudaError_t e = scratch_alloc(&ws, need, as_stream(stream));
       if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "scratch (padded operands)", e);
     }
-    rc = launch_mid(tl, tr, m, n, k, left, right, out, tile_n - (swap ? 3000 : 2000), splits, write_hi == 1, swap, 0,
+    rc = launch_mid(tl, tr, m, n, k, left, right, out, tile_n - (swap ? 3000 : 2000), splits, 0, write_hi == 1, swap, 0,
                     static_cast<float*>(ws), as_stream(stream));
     if (ws) scratch_free(ws, as_stream(stream));
     return rc;

@@ -67,6 +67,7 @@ struct Params {
   float* out;
   uint64_t pitch;           // floats per row of the result
   uint32_t tiles_m, slabs, cluster, chunk;
+  uint32_t whole;           // the first tiles, one CTA each whatever the cluster (even; see launch_mid)
   int a_mn, b_mn;           // operand stored with m (n) contiguous
   int a_whole, b_whole;     // whole 32-element chunks of that extent: tiles inside them come in one 3-D box
   int out_t, epilogue, vec_out;
@@ -154,11 +155,13 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   static_assert(8 * (kRings + 2 * kAccs) + 8 <= 256, "barrier block");
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  const uint32_t rank = p.cluster > 1 ? cluster_rank() : 0u;
-  const uint32_t tile = blockIdx.x / p.cluster;
+  const bool whole = blockIdx.x < p.whole;
+  const uint32_t cluster = whole ? 1u : p.cluster;         // CTAs that share this tile
+  const uint32_t rank = cluster > 1 ? cluster_rank() : 0u;
+  const uint32_t tile = whole ? blockIdx.x : p.whole + (blockIdx.x - p.whole) / cluster;
   const int m0 = (int)((tile % p.tiles_m) * BM), n0 = (int)((tile / p.tiles_m) * BN);
-  const uint32_t kb0 = (uint32_t)((uint64_t)rank * p.slabs / p.cluster);
-  const uint32_t kb1 = (uint32_t)((uint64_t)(rank + 1) * p.slabs / p.cluster);
+  const uint32_t kb0 = (uint32_t)((uint64_t)rank * p.slabs / cluster);
+  const uint32_t kb1 = (uint32_t)((uint64_t)(rank + 1) * p.slabs / cluster);
   const uint32_t mine = kb1 - kb0, chunks = (mine + p.chunk - 1) / p.chunk;
 
   constexpr int kBars = kRings + 2 * kAccs;
@@ -345,7 +348,7 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (p.cluster > 1) {
+  if (cluster > 1) {
     cluster_arrive();
     cluster_wait();
   }
@@ -357,13 +360,13 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
     tmem_dealloc(tmem, 4 * BN);
   }
-  switch (p.cluster) {
+  switch (cluster) {
     case 1: store_share<BN, 1>(p, base, 0, m0, n0); break;
     case 2: store_share<BN, 2>(p, base, rank, m0, n0); break;
     case 4: store_share<BN, 4>(p, base, rank, m0, n0); break;
     default: store_share<BN, 8>(p, base, rank, m0, n0);
   }
-  if (p.cluster > 1) cluster_wait();   // nobody leaves while another CTA may still read its part
+  if (cluster > 1) cluster_wait();   // nobody leaves while another CTA may still read its part
 }
 
 // Copies up to two matrices to scratch with their rows padded to `pitch` floats (a multiple of 32; the
@@ -446,7 +449,7 @@ int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Pa
   p.a_whole = whole[0];
   p.b_whole = whole[1];
   cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(p.tiles_m * (uint32_t)((p.n + BN - 1) / BN) * p.cluster);
+  c.gridDim = dim3(p.whole + (p.tiles_m * (uint32_t)((p.n + BN - 1) / BN) - p.whole) * p.cluster);
   c.blockDim = dim3(kThreads);
   c.dynamicSmemBytes = C::kSmemBytes;
   c.stream = stream;
@@ -483,10 +486,12 @@ uint64_t mid_workspace_bytes(int tl, int tr, uint64_t m, uint64_t n, uint64_t k,
   return floats * sizeof(float);
 }
 
-// out[m,n] = L'.R' with tiles of 128 x bn, `cluster` CTAs per tile.  swap: the operands exchange roles, the tile's
+// out[m,n] = L'.R' with tiles of 128 x bn, `cluster` CTAs per tile - all but the first `whole` tiles, which get one each:
+// where one CTA per tile leaves a last wave at most half full, cutting just its tiles in two shortens the wave by half
+// (192 tiles on 148 SMs: one wave and a half instead of two).  swap: the operands exchange roles, the tile's
 // rows are columns of the result.  ws: mid_workspace_bytes.
 int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right, float* out, int bn,
-               int cluster, int exact, int swap, int epilogue, float* ws, cudaStream_t stream) {
+               int cluster, uint64_t whole, int exact, int swap, int epilogue, float* ws, cudaStream_t stream) {
   using namespace mid;
   Stored l{left, tl ? k : m, tl ? m : k, tl ? m : k, false}, r{right, tr ? n : k, tr ? k : n, tr ? k : n, false};
   Padded copies[2] = {};
@@ -521,6 +526,7 @@ int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* 
   p.tiles_m = (uint32_t)((p.m + BM - 1) / BM);
   p.slabs = (uint32_t)((k + BK - 1) / BK);
   p.cluster = (uint32_t)cluster;
+  p.whole = (uint32_t)whole;
   // slabs of 32 terms summed in tensor memory, the rest in registers: EXACT is to stay below the error of FFMA sums
   p.chunk = !exact ? 8 : k < 512 ? 1 : 2;
   if ((cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) || p.slabs < p.cluster) return fail(POLAR_B200_ERR_UNSUPPORTED, "fewer slabs than CTAs in a cluster");

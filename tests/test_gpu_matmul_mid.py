@@ -53,7 +53,7 @@ def test_every_configuration(gpu, par_oracle, tl, tr, m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k", [(999, 514, 301), (301, 514, 999), (16, 4096, 784), (33, 17, 50), (5, 7, 31), (64, 48, 32),
-                                   (1024, 1024, 1024), (1000, 2001, 130), (258, 130, 4097), (1, 1, 1)])
+                                   (1024, 1024, 1024), (1000, 2001, 130), (2001, 1511, 70), (258, 130, 4097), (1, 1, 1)])
 @pytest.mark.parametrize("tl,tr", [(0, 0), (1, 0), (0, 1), (1, 1)])
 def test_dispatch_on_ragged_and_small_products(gpu, par_oracle, tl, tr, m, n, k):
     # through fmatmul, with the library's own scratch and with a caller workspace; unaligned base pointers; and the
