@@ -315,6 +315,9 @@ int polar_b200_fsigmoid(const float* in, float* out, uint64_t n, void* stream) {
 int polar_b200_fsigmoid_unclamped(const float* in, float* out, uint64_t n, void* stream) {
   return launch_ew<1>("fsigmoid_unclamped", SigmoidOp<false>{}, in, nullptr, out, n, stream);
 }
+int polar_b200_frelu(const float* in, float* out, uint64_t n, void* stream) {
+  return launch_ew<1>("frelu", ReluOp{}, in, nullptr, out, n, stream);
+}
 int polar_b200_flogloss(const float* predicted, const float* groundTruth, float* out, uint64_t n,
                         void* stream) {
   if (n >= 4 && predicted && groundTruth && out && n <= (1ull << 40) && aligned16(predicted) &&

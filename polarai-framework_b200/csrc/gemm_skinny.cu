@@ -31,6 +31,7 @@ constexpr int kThreads = 256;
 // ---------------------------------------------------------------- small n, K-major left
 
 constexpr int KT = 1024;          // k-slab staged in shared memory
+static_assert(KT % 256 == 0, "two warps of four floats per lane walk a slab");
 constexpr int KT_PAD = KT + 4;    // keeps float4 alignment, staggers banks between columns
 constexpr int ROWS_PER_WARP = 4;
 
@@ -108,6 +109,14 @@ small_n_rows_kernel(const float* __restrict__ left, const float* __restrict__ ri
   for (int r = 0; r < RW; ++r)
 #pragma unroll
     for (int j = 0; j < NP; ++j) acc[r][j] = 0.f;
+  float4 ahead[RW];                        // the next vectors of the thread's rows, asked for before they are needed
+  auto fetch = [&](uint64_t kk) {
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+      ahead[r] = (row0 + r < m && kk < kend) ? *reinterpret_cast<const float4*>(left + (row0 + r) * k + kk)
+                                             : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  if (VEC) fetch(kbeg + (half * 32 + lane) * 4);
   for (uint64_t k0 = kbeg; k0 < kend; k0 += KT) {
     const int kt = (int)((kend - k0 < KT) ? (kend - k0) : KT);
     __syncthreads();
@@ -117,8 +126,9 @@ small_n_rows_kernel(const float* __restrict__ left, const float* __restrict__ ri
       for (int kk = (half * 32 + lane) * 4; kk < kt; kk += 256) {
         float4 a[RW];
 #pragma unroll
-        for (int r = 0; r < RW; ++r)
-          a[r] = row0 + r < m ? *reinterpret_cast<const float4*>(left + (row0 + r) * k + k0 + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < RW; ++r) a[r] = ahead[r];
+        // (KT is a multiple of 256: the first vectors of the next slab follow the last of this one)
+        fetch(k0 + kk + 256);
 #pragma unroll
         for (int j = 0; j < NP; ++j) {
           if (j >= (int)n) continue;

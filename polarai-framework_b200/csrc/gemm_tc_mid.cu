@@ -171,7 +171,11 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const bool by_warps = (lane >= 2 * C::kRaw && lane < kRings) || lane >= kRings + kAccs;   // full_lo, acc_empty
       mbar_init(bars + 8u * lane, by_warps ? (uint32_t)kSplitWarps : 1u);
     }
-    if (lane == 0) *abort_flag = 0;
+    if (lane == 0) {
+      *abort_flag = 0;
+      prefetch_map(p.a_mn && m0 + BM <= 32 * p.a_whole ? &map_a3 : &map_a);
+      prefetch_map(p.b_mn && n0 + BN <= 32 * p.b_whole ? &map_b3 : &map_b);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   static_assert(kSplitWarps == kAccWarps, "by_warps");
