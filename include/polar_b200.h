@@ -492,7 +492,7 @@ uint64_t polar_b200_launch_workspace_bytes(const char* nativeKernelName,
  * One run launches the operations in order on `stream`, exactly as polar_b200_launch_by_name
  * would one by one (same checks, same statuses, every result tensor written with the same
  * bits), but in fewer launches: consecutive elementwise builtins over the same element count
- * share one, and from its third run on a program of several launches is replayed as a CUDA
+ * share one, and from its third run on a program of many short launches is replayed as a CUDA
  * graph.  Names, argument lists and shapes are copied; the tensors and the workspace must
  * stay allocated while the program exists.  A program may be run on any stream of its device, also
  * one under capture, and from any thread; like the launches themselves, runs that overlap on the

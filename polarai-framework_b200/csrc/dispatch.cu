@@ -18,7 +18,7 @@ bool tc_shape_ok(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float
                  const float* right);
 uint64_t mid_workspace_bytes(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right);
 int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right, float* out, int bn,
-               int cluster, uint64_t whole, int exact, int swap, int epilogue, float* ws, cudaStream_t stream);
+               int cluster, uint64_t whole, int exact, int swap, int epilogue, float* ws, cudaStream_t stream, uint64_t left_pitch = 0);
 int skinny_kind(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                 const float* right, const float* out);
 uint64_t skinny_workspace_bytes(int kind, uint64_t m, uint64_t n, uint64_t k);
@@ -404,8 +404,17 @@ static int tc_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const flo
   } else {
     cudaGetLastError();   // no side stream: one after the other on the caller's stream
   }
-  rc = launch_ragged_rows(left + mm, lp, right, out + mm * n, reinterpret_cast<float*>(ws + tc_need), rem, n, k,
-                          rag_stream);
+  // Up to k = 32768 the last rows run as columns of cluster tiles (exact split, exchanged operands: 45 us for 16 x 4096 x
+  // 8192 against 67 us for the CUDA-core kernel and its sum); longer sums stay with the kernel that comes closer
+  // to the bandwidth of its one pass over `right` (280 us at k = 65536 against 300).
+  if (k <= 32768) {
+    const uint64_t tiles = (n + 127) / 128;
+    const int cluster = tiles * 8 <= 120 ? 8 : tiles * 4 <= 132 ? 4 : tiles * 2 <= (uint64_t)sm_count() ? 2 : 1;
+    rc = launch_mid(1, 0, rem, n, k, left + mm, right, out + mm * n, 32, cluster, 0, 1, 1, 0, nullptr, rag_stream, lp);
+  } else {
+    rc = launch_ragged_rows(left + mm, lp, right, out + mm * n, reinterpret_cast<float*>(ws + tc_need), rem, n, k,
+                            rag_stream);
+  }
   int rc2 = run_tc(tl, tr, mm, n, k, left, right, out, 256, 16, 3, 0, c.splits,
                    tc_need ? ws : nullptr, tc_need, main_stream, 0, lp, mt);
   // join: whatever follows on the caller's stream waits for the side stream too (also when a

@@ -493,15 +493,16 @@ uint64_t mid_workspace_bytes(int tl, int tr, uint64_t m, uint64_t n, uint64_t k,
 // out[m,n] = L'.R' with tiles of 128 x bn, `cluster` CTAs per tile - all but the first `whole` tiles, which get one each:
 // where one CTA per tile leaves a last wave at most half full, cutting just its tiles in two shortens the wave by half
 // (192 tiles on 148 SMs: one wave and a half instead of two).  swap: the operands exchange roles, the tile's
-// rows are columns of the result.  ws: mid_workspace_bytes.
+// rows are columns of the result.  ws: mid_workspace_bytes.  left_pitch: floats between the stored rows of left (0: they
+// follow one another), a multiple of 4.
 int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left, const float* right, float* out, int bn,
-               int cluster, uint64_t whole, int exact, int swap, int epilogue, float* ws, cudaStream_t stream) {
+               int cluster, uint64_t whole, int exact, int swap, int epilogue, float* ws, cudaStream_t stream, uint64_t left_pitch) {
   using namespace mid;
-  Stored l{left, tl ? k : m, tl ? m : k, tl ? m : k, false}, r{right, tr ? n : k, tr ? k : n, tr ? k : n, false};
+  Stored l{left, tl ? k : m, tl ? m : k, left_pitch ? left_pitch : tl ? m : k, false}, r{right, tr ? n : k, tr ? k : n, tr ? k : n, false};
   Padded copies[2] = {};
   int count = 0;
   for (Stored* s : {&l, &r}) {
-    if (addressable(s->p, s->cols)) continue;
+    if (addressable(s->p, s->pitch)) continue;
     const uint64_t pitch = pad32(s->cols);
     copies[count++] = Padded{s->p, ws, s->rows, s->cols, pitch};
     s->p = ws;

@@ -8,8 +8,11 @@
 //    result is still written, with the bits its own launch gives; what goes away is reading a
 //    tensor back that the same pass has just computed or read (the four-builtin chain of
 //    (a + b) * c / d -> sigmoid moves 32 instead of 44 bytes per element).
-//  - From its third run on, a program of several launches is replayed as a CUDA graph: one host call,
-//    and 1.5 us from kernel to kernel.  The first two runs are launched one by one, so that a program run
+//  - From its third run on, a program of many short launches is replayed as a CUDA graph: one host call instead of 2 us
+//    of host time per launch.  Programs of up to three steps, and programs with tensors of two million elements or
+//    more, whose kernels outlast their launches, stay with launches: programmatic dependent launch overlaps them more
+//    closely in a stream than in a graph (inference on 16 rows, two launches: 17.3 us against 19.9; MLP step at batch
+//    8192 640 against 645; ragged MLP step 57 us of host time against 29 at the same 59 us in all).  The first two runs are launched one by one, so that a program run
 //    once or twice never pays for the instantiation; a run under the caller's own stream capture is
 //    always launched one by one.
 #include <cstring>
@@ -54,43 +57,43 @@ __device__ __forceinline__ float4 map4(Op op, float4 a, float4 b) {
   return make_float4(op(a.x, b.x), op(a.y, b.y), op(a.z, b.z), op(a.w, b.w));
 }
 
-// A chain of elementwise builtins on one vector of four elements per thread.  HBM-bound for long vectors
-// (the interpreter's shared-memory traffic is 48 bytes per instruction and vector, a quarter of what
-// an SM can move in the time its share of HBM delivers the vector), one launch latency for short ones.
+// A chain of elementwise builtins on one vector of four elements per thread.  HBM-bound for long vectors, one launch
+// latency for short ones.  (Two vectors per thread halve the decoding and are no faster anywhere: 8.2 us against 6.6 at
+// 2^20 elements, the same from 2^22 on.)
 // Values live in shared memory, [slot][thread]: a thread only ever touches its own column, so there
 // is no barrier, and consecutive lanes touch consecutive 16 bytes.
-// Measured, four-builtin chain: 2^20 elements 18.4 us as four launches, 3.6 us as one.
+// Measured, four-builtin chain, 32 bytes per element: 2^20 elements 18.4 us as four launches, 6.6 us as one;
+// 2^25 elements 158 us, 6.8 TB/s.
 __global__ void __launch_bounds__(kChainThreads) chain_kernel(const __grid_constant__ ChainParams p) {
   extern __shared__ float4 slots[];
   pdl_enter();
-  const uint64_t v = (uint64_t)blockIdx.x * kChainThreads + threadIdx.x;
-  const uint64_t e0 = v * 4;
+  const uint64_t e0 = ((uint64_t)blockIdx.x * kChainThreads + threadIdx.x) * 4;
   if (e0 >= p.n) return;
-  const bool whole = e0 + 4 <= p.n;
-  const int left = whole ? 4 : (int)(p.n - e0);   // the last vector of an n that is no multiple of four
+  const bool full = e0 + 4 <= p.n;
+  const int left = full ? 4 : (int)(p.n - e0);             // the last vector of an n that is no multiple of four
   float4* mine = slots + threadIdx.x;
-  float4 first[kChainInputs];
 #pragma unroll
-  for (int i = 0; i < kChainInputs; ++i) {
-    if (i < (int)p.inputs) {
-      const float* src = p.in[i] + e0;
-      if (whole) {
-        first[i] = *reinterpret_cast<const float4*>(src);
-      } else {
-        first[i] = make_float4(src[0], left > 1 ? src[1] : 0.f, left > 2 ? src[2] : 0.f, 0.f);
-      }
+  for (int first = 0; first < kChainInputs; first += 4) {  // four inputs' loads in flight at a time
+    if (first >= (int)p.inputs) break;
+    float4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (first + i >= (int)p.inputs) continue;
+      const float* src = p.in[first + i] + e0;
+      v[i] = full ? *reinterpret_cast<const float4*>(src)
+                  : make_float4(src[0], left > 1 ? src[1] : 0.f, left > 2 ? src[2] : 0.f, 0.f);
     }
-  }
 #pragma unroll
-  for (int i = 0; i < kChainInputs; ++i)
-    if (i < (int)p.inputs) mine[i * kChainThreads] = first[i];
+    for (int i = 0; i < 4; ++i)
+      if (first + i < (int)p.inputs) mine[(first + i) * kChainThreads] = v[i];
+  }
   float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
   for (uint32_t i = 0; i < p.ops; ++i) {
     const ChainOp& o = p.op[i];
     const float4 a = o.a == kPrevious ? r : mine[o.a * kChainThreads];
     const float4 b = o.b == kPrevious ? r : mine[o.b * kChainThreads];
     switch (o.code) {   // the same for all threads
-      case kFill: r = make_float4(o.s0, o.s0, o.s0, o.s0); break;
+      case kFill: r = map4(ew::FillOp{o.s0}, a, b); break;
       case kCopy: r = a; break;
       case kAdd: r = map4(ew::AddOp{o.s0, o.s1}, a, b); break;
       case kMul: r = map4(ew::MulOp{}, a, b); break;
@@ -98,12 +101,10 @@ __global__ void __launch_bounds__(kChainThreads) chain_kernel(const __grid_const
       case kSigmoid: r = map4(ew::SigmoidOp<true>{}, a, a); break;
       case kLogLoss: {
         auto hard = [](float y) { return y == 0.0f || y == 1.0f; };
-        if (hard(b.x) && hard(b.y) && hard(b.z) && hard(b.w)) {
-          r = make_float4(ew::logloss_binary(a.x, b.x), ew::logloss_binary(a.y, b.y), ew::logloss_binary(a.z, b.z),
-                          ew::logloss_binary(a.w, b.w));
-        } else {
-          r = map4(ew::LogLossOp{}, a, b);
-        }
+        r = hard(b.x) && hard(b.y) && hard(b.z) && hard(b.w)
+                ? make_float4(ew::logloss_binary(a.x, b.x), ew::logloss_binary(a.y, b.y), ew::logloss_binary(a.z, b.z),
+                              ew::logloss_binary(a.w, b.w))
+                : map4(ew::LogLossOp{}, a, b);
         break;
       }
       case kMulConcat: r = map4(ew::ScaleByFirstOp{*o.scalar}, a, a); break;
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(kChainThreads) chain_kernel(const __grid_const
     }
     if (o.result != kNoSlot) mine[o.result * kChainThreads] = r;
     float* dst = o.out + e0;
-    if (whole) {
+    if (full) {
       *reinterpret_cast<float4*>(dst) = r;
     } else {
       dst[0] = r.x;
@@ -143,6 +144,7 @@ struct Program {
   uint64_t workspace_bytes = 0;
   std::mutex mu;
   int runs = 0;
+  bool short_launches = true;   // worth a graph
   bool graph_failed = false;
   cudaGraphExec_t graph = nullptr;
   uint64_t graph_launches = 0;
@@ -404,6 +406,7 @@ int polar_b200_program_create(const polar_b200_op* ops, uint64_t count, void* wo
       }
       op.shapes[a].assign(t.shape, t.shape + t.dims);
       if (!p->any_pointer) p->any_pointer = t.data;
+      if (elements(t) >= 2000000) p->short_launches = false;
     }
     p->ops.push_back(std::move(op));
     Op& kept = p->ops.back();
@@ -423,7 +426,7 @@ int polar_b200_program_run(void* program, void* stream) {
   if (!p) return fail(POLAR_B200_ERR_INVALID, "null program");
   cudaStream_t st = as_stream(stream);
   LaunchDeviceScope on(stream, p->any_pointer);
-  if (p->steps.size() > 1) {
+  if (p->steps.size() > 3 && p->short_launches) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     // (a query on the legacy stream fails while some other stream is capturing: then launch one by one)
     const bool eager = cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone;
