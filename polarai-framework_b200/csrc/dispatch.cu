@@ -133,46 +133,75 @@ inline uint64_t align256(uint64_t b) { return (b + 255) & ~255ull; }
 //  swap: the operands exchange roles (launch_tc), which turns the epilogue's stores into whole
 //    128-byte lines: 2-4 % on sums of a few hundred to a few thousand terms, where the epilogue
 //    is a visible share of a tile; needs whole tiles or fixed k cuts, and no row pitch.
-//  splits: as tc_default_splits, for the orientation chosen.
-// The choice compares padded tile area x relative cost / wave efficiency of the candidates.
+//  splits: work units per tile (0: stream mode).
+// Sums of up to 2048 terms take the candidate of the least estimated time; long ones, where the clock under the power
+// cap decides more than waves and epilogues do, compare padded tile area x relative cost / wave efficiency with the
+// cuts of tc_default_splits.
 struct TcChoice {
   int mt;
   int swap;
   uint32_t splits;
 };
 
+// What a choice takes in microseconds, fitted to 1400 measurements on B200 (60 shapes of 256 ... 8192, k from 96 on;
+// 11 % standard deviation): a slab of 16 k of a 256 x 256 tile 0.92, of a 128 x 256 tile 0.59, around them per tile
+// 7.2 (5.0 with whole-line stores) and 2.6 (1.0), per launch 7.4.  Cuts of k move the partial products
+// through memory, 0.21 per MB and pass; stream mode pays for its slots by the slab (1.12, 0.67) and 34 (23) per launch.
+double tc_estimate_us(uint64_t m, uint64_t n, uint64_t k, const TcChoice& c) {
+  const uint64_t rows = c.swap ? n : m, cols = c.swap ? m : n, sms = (uint64_t)sm_count(), slabs = (k + 15) / 16;
+  const uint64_t tiles = ((rows + 128 * c.mt - 1) / (128 * c.mt)) * ((cols + 255) / 256);
+  if (c.splits == 0) return (double)(tiles * slabs) / (double)sms * (c.mt == 2 ? 1.12 : 0.67) + (c.mt == 2 ? 34.0 : 23.0);
+  const uint64_t units = tiles * c.splits;
+  double waves = (double)((units + sms - 1) / sms);
+  // a tail of at most half a wave of whole tiles runs as column halves, which last about 0.6 of a tile
+  if (c.splits == 1 && tc_tail_in_halves(tiles, sms)) waves -= 0.4;
+  const double slab = c.mt == 2 ? 0.92 : 0.59, around = c.mt == 2 ? (c.swap ? 5.0 : 7.2) : (c.swap ? 1.0 : 2.6);
+  const double sum = c.splits > 1 ? 0.21 * (c.splits + 1) * (double)m * (double)n * 4e-6 : 0.0;
+  return waves * ((double)((slabs + c.splits - 1) / c.splits) * slab + around) + 7.4 + sum;
+}
+
 TcChoice tc_choose(uint64_t m, uint64_t n, uint64_t k, bool may_swap) {
   const double sms = (double)sm_count();
   TcChoice best{1, 0, 1};
   double best_est = 0.0;
-  for (int swap = 0; swap <= (may_swap && k >= 256 && k <= 2048 ? 1 : 0); ++swap) {
-    const uint64_t rows_dim = swap ? n : m, cols_dim = swap ? m : n;
-    for (int mt = 1; mt <= 2; ++mt) {
-      if (mt == 2 && (rows_dim < 256 || k < 512)) continue;
-      const uint64_t rows = 128ull * mt;
-      const uint64_t tiles_m = (rows_dim + rows - 1) / rows, tiles_n = (cols_dim + 255) / 256, tiles = tiles_m * tiles_n;
-      uint32_t splits = tc_default_splits(rows_dim, cols_dim, k, mt);
-      if (swap && splits == 0) splits = 1;             // stream mode stores through slots: whole tiles instead
-      // with cuts of k the exchanged epilogue only writes partial products; measured better at
-      // 2048^3 (206-217 vs 193 TFLOP/s) and worse at 1024^3 (48 vs 58), where stream mode stays
-      if (swap && splits > 1 && rows_dim * cols_dim < (4ull << 20)) continue;
-      double eff = 1.0;
-      const uint64_t units = tiles * (splits ? splits : 1);
-      if (splits >= 1 && (double)units < 8 * sms) {    // whole waves of work units (stream mode balances itself)
-        double waves = (double)((units + (uint64_t)sms - 1) / (uint64_t)sms);
-        // a tail of at most half a wave of whole tiles runs as column halves, which last about 0.6 of a tile
-        if (splits == 1 && tc_tail_in_halves(tiles, (uint64_t)sms)) waves -= 0.4;
-        eff = (double)units / (waves * sms);
+  if (k <= 2048) {
+    for (int swap = 0; swap <= (may_swap ? 1 : 0); ++swap) {
+      const uint64_t rows = swap ? n : m, cols = swap ? m : n;
+      for (int mt = 1; mt <= 2; ++mt) {
+        if (mt == 2 && rows < 256) continue;
+        for (uint32_t splits = 0; splits <= 8; ++splits) {
+          if (splits == 0 && (swap || tc_workspace_bytes(rows, cols, k, 0, mt) == 0)) continue;
+          // a unit of eight slabs at least, partial products of 256 MiB at most
+          if (splits > 1 && (k < 128 * splits || splits * m * n > (64ull << 20))) break;
+          const TcChoice c{mt, swap, splits};
+          const double est = tc_estimate_us(m, n, k, c);
+          if (best_est == 0.0 || est < best_est) {
+            best_est = est;
+            best = c;
+          }
+        }
       }
-      // measured against the 128-row tile: 0.67-0.85 of its cost from k = 16384 up, 0.83-0.88 at
-      // k = 784 ... 8192 (256-bit or line-wide stores in the epilogue)
-      double cost = mt == 1 ? 1.0 : (k < 16384 ? 0.85 : 0.75);
-      if (swap) cost *= 0.97;
-      const double est = (double)(tiles_m * rows) * (double)(tiles_n * 256) * cost / eff;
-      if (best_est == 0.0 || est < best_est) {
-        best_est = est;
-        best = TcChoice{mt, swap, splits};
-      }
+    }
+    return best;
+  }
+  for (int mt = 1; mt <= 2; ++mt) {
+    if (mt == 2 && m < 256) continue;
+    const uint64_t rows = 128ull * mt;
+    const uint64_t tiles_m = (m + rows - 1) / rows, tiles_n = (n + 255) / 256, tiles = tiles_m * tiles_n;
+    const uint32_t splits = tc_default_splits(m, n, k, mt);
+    double eff = 1.0;
+    const uint64_t units = tiles * (splits ? splits : 1);
+    if (splits >= 1 && (double)units < 8 * sms) {      // whole waves of work units (stream mode balances itself)
+      double waves = (double)((units + (uint64_t)sms - 1) / (uint64_t)sms);
+      if (splits == 1 && tc_tail_in_halves(tiles, (uint64_t)sms)) waves -= 0.4;
+      eff = (double)units / (waves * sms);
+    }
+    // measured against the 128-row tile: 0.67-0.85 of its cost from k = 16384 up, 0.83-0.88 below
+    const double cost = mt == 1 ? 1.0 : (k < 16384 ? 0.85 : 0.75);
+    const double est = (double)(tiles_m * rows) * (double)(tiles_n * 256) * cost / eff;
+    if (best_est == 0.0 || est < best_est) {
+      best_est = est;
+      best = TcChoice{mt, 0, splits};
     }
   }
   return best;
@@ -189,9 +218,9 @@ namespace {
 
 // ---- the cluster kernel (gemm_tc_mid.cu) --------------------------------------------------------------
 // One 128 x bn tile per cluster of CTAs.  Times in microseconds, fitted to measurements on B200 between
-// 128 x 64 x 64 and 2048^3 (within 15 % there): a slab of 32 k costs a CTA 0.43 / 0.48 / 0.60 us with tiles of 32 / 64 / 128
-// columns (0.58 / 0.66 / 0.80 with the exact split), set-up, pipeline fill and the store of the tile 4 to 5.5 us,
-// the exchange between the CTAs of a cluster 1 us.
+// 128 x 64 x 64 and 2048^3 (within 15 % there): a slab of 32 k costs a CTA 0.36 / 0.43 / 0.56 us with tiles of 32 / 64 / 128
+// columns (0.42 / 0.50 / 0.63 with short sums in tensor memory: reading them competes with the products), set-up,
+// pipeline fill and the store of the tile 4 to 5 us, the exchange between the CTAs of a cluster 1.3 to 3.3 us.
 struct MidChoice {
   int bn = 0, cluster = 1, swap = 0;
   uint64_t whole = 0;
@@ -205,19 +234,21 @@ MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact) {
     const uint64_t rows = swap ? n : m, cols = swap ? m : n;
     for (int i = 0; i < 3; ++i) {
       const int bn = 32 << i;
-      static const double slab_us[2][3] = {{0.43, 0.48, 0.60}, {0.58, 0.66, 0.80}};
+      static const double slab_us[2][3] = {{0.36, 0.43, 0.56}, {0.42, 0.50, 0.63}};
       const uint64_t tiles = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
       for (int cl = 1; cl <= 8 && (uint64_t)cl <= slabs; cl *= 2) {
         // clusters of 4 and 8 leave SMs of a GPC unused: 33 and 15 of them run at a time on 148 SMs
         const uint64_t at_once = cl <= 2 ? sms : cl == 4 ? sms * 132 / 148 : sms * 120 / 148;
         const uint64_t waves = (tiles * cl + at_once - 1) / at_once;
-        const double one = (double)((slabs + cl - 1) / cl) * slab_us[exact][i] + (bn == 128 ? 5.5 : 4.0) + (cl > 1 ? 1.0 : 0.0);
+        const int log_cl = cl == 8 ? 3 : cl / 2;
+        const double exchange = cl == 1 ? 0.0 : bn == 128 ? 1.5 + 0.6 * log_cl : 1.1 + 0.2 * log_cl;
+        const double one = (double)((slabs + cl - 1) / cl) * slab_us[exact][i] + (bn == 128 ? 5.0 : 4.0) + exchange;
         const double us = (double)waves * one;
         if (us < best.us - 0.01) best = MidChoice{bn, cl, swap, 0, us};
         // one CTA per tile, except that a last wave of at most half the SMs has its tiles cut in two
         const uint64_t full = tiles / sms * sms, rest = tiles - full;
         if (cl == 1 && full && rest && 2 * rest <= sms && (full & 1) == 0 && slabs >= 2) {
-          const double tail = (double)((slabs + 1) / 2) * slab_us[exact][i] + (bn == 128 ? 6.5 : 5.0);
+          const double tail = (double)((slabs + 1) / 2) * slab_us[exact][i] + (bn == 128 ? 7.1 : 5.3);
           const double cut = (double)(full / sms) * one + tail;
           if (cut < best.us - 0.01) best = MidChoice{bn, 2, swap, full, cut};
         }
@@ -227,24 +258,10 @@ MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact) {
   return best;
 }
 
-// What the 256-column tiles of gemm_tc.cu take, on the same scale (same measurements): a slab of 16 k of a
-// 256 x 256 tile 0.85 us, of a 128 x 256 tile 0.55, and 10 (6) us around them per tile; cuts of k move the partial
-// products through memory and a second kernel.
-double tc_estimate_us(uint64_t m, uint64_t n, uint64_t k, const TcChoice& c) {
-  const uint64_t rows = c.swap ? n : m, cols = c.swap ? m : n, sms = (uint64_t)sm_count(), slabs = (k + 15) / 16;
-  const uint64_t tiles = ((rows + 128 * c.mt - 1) / (128 * c.mt)) * ((cols + 255) / 256);
-  const double slab = c.mt == 2 ? 0.85 : 0.55, around = c.mt == 2 ? 10.0 : 6.0;
-  const double mb = (double)m * (double)n * 4e-6;
-  if (c.splits == 0) return (double)(tiles * slabs) / (double)sms * slab + around + 8.0 + mb / 2.0;
-  const uint64_t units = tiles * c.splits;
-  const double waves = (double)((units + sms - 1) / sms);
-  return waves * ((double)((slabs + c.splits - 1) / c.splits) * slab + around) + (c.splits > 1 ? 3.0 + c.splits * mb / 2.0 : 0.0);
-}
-
 // Operands that TMA addresses as they are stored: the cluster kernel where it is the faster of the two.
 MidChoice mid_for_tc(uint64_t m, uint64_t n, uint64_t k, bool may_swap) {
   MidChoice c = mid_choose(m, n, k, false);
-  if (c.us >= tc_estimate_us(m, n, k, tc_choose(m, n, k, may_swap))) c.bn = 0;
+  if (1.05 * c.us >= tc_estimate_us(m, n, k, tc_choose(m, n, k, may_swap))) c.bn = 0;
   return c;
 }
 

@@ -10,15 +10,26 @@
 //
 // One CTA:
 //   warp 0      TMA producer: 32-float k slabs of A (128 rows) and B (BN rows), two instructions per slab;
-//   warp 1      tcgen05.mma issuer: per slab and 8 k the three products of the TF32 split;
-//   warps 2-9   split warps: the lo parts, x - hi, of each landed slab (hi is what the tensor core sees of the raw word).
-//               With EXACT, lo is rounded to the nearest TF32 instead of cut off, lo.lo is computed too, and
-//               the products other than hi.hi get an accumulator of their own, where the tensor core's
-//               truncation hurts 1000 times less;
+//   warps 2-9   split warps: of each landed slab, the hi and lo parts of A to tensor memory and the lo parts of B to
+//               shared memory beside the raw words, which are its hi parts (the tensor core ignores the low 13 bits);
+//   warp 1      tcgen05.mma issuer: per slab and 8 k the three products of the TF32 split, A from tensor memory;
 //   warps 10-17 accumulator warps: every `chunk` slabs they read the tensor-memory accumulator and add it to
 //               registers in round-to-nearest.  The tensor core's own accumulator rounds toward zero, an error that
 //               grows with the length of the sum (8e-9 of the result per term for zero-mean operands);
 //               chunks keep it at that of a short sum.
+//
+// What bounds it: shared memory, 128 bytes per clock.  An instruction of 128 x BN x 8 with both operands there reads
+// 4 KB + 32 BN bytes: 64 / 48 / 40 clocks for 128 / 64 / 32 columns, where the tensor core needs 64 / 32 / 16 - all of the
+// bandwidth before TMA has written a slab and the split has read it and written the lo parts.  With A in tensor memory
+// a 128 x 128 x 32 slab takes 1024 clocks of shared memory instead of 1536 (768 of the tensor core); measured 0.54 us a
+// slab, 0.41 with 64 columns and 0.34 with 32 (0.60, 0.48, 0.43 before).  2001 x 1511 x 999: 60 -> 50 us; 16 x 4096 x 784:
+// 8.8 -> 7.5 us.  What is left per tile, 4 to 5 us, is set-up, the first slab's way through the pipeline and the store; the
+// exchange in a cluster runs at the 15 bytes per clock an SM gets from another SM's shared memory (pushing the parts
+// there instead of reading them was slower: 17.4 against 15.9 us at 1024^3).
+//
+// The split: A's hi is rounded to the nearest TF32 (it is written anyway), B's is cut off; the dropped lo.lo is below
+// 2^-23 |a||b| and of either sign: 9e-8 of the norm for uniform operands, where four products with both cut off left 1.1e-7
+// and an FFMA sum has 1.0e-7 (32 terms) to 5.7e-7 (1000 terms).
 // At the end the tile goes to shared memory in the layout of the result's rows; the cluster's CTAs each
 // add one share of it over all CTAs in rank order (the same bits run to run) and store whole lines.
 //
@@ -49,15 +60,20 @@ constexpr int kSplitWarps = 8, kAccWarps = 8;
 constexpr int kThreads = 32 * (2 + kSplitWarps + kAccWarps);
 constexpr uint32_t kBox = 32 * BK * 4;                      // one MN-major chunk of a slab: 32 elements x BK rows
 
-// Shared memory is a ring of raw slabs and a shorter ring of lo parts.  A raw slab is held from the TMA
-// request to the end of its products (about 2 us: L2 latency, split, products), a lo part only from the
-// split on, so the raw ring is what has to be deep: at 128 x 128 x 32 a slab's products take 0.4 us.
+// Shared memory is a ring of raw slabs and a shorter ring of B's lo parts, in step with a ring of A's parts in tensor
+// memory.  A raw slab is held from the TMA request to the end of its products (about 2 us: L2 latency, split,
+// products), the parts only from the split on, so the raw ring is what has to be deep: at 128 x 128 x 32 a slab's
+// products take 0.4 us.
 template <int BN> struct Cfg {
   static constexpr uint32_t kABytes = BM * BK * 4, kBBytes = BN * BK * 4, kRawBytes = kABytes + kBBytes;
-  static constexpr int kRaw = BN == 128 ? 5 : BN == 64 ? 6 : 7, kLo = BN == 128 ? 2 : BN == 64 ? 3 : 4;
+  static constexpr int kRaw = BN == 128 ? 6 : BN == 64 ? 8 : 10, kLo = BN == 128 ? 2 : BN == 64 ? 4 : 6;
+  static_assert(kRaw % 2 == 0 && kLo % 2 == 0, "even slabs and odd slabs have split warps of their own");
   static constexpr uint32_t kLoBase = kRaw * kRawBytes;
-  static constexpr uint32_t kTileBytes = (kRaw + kLo) * kRawBytes;
+  static constexpr uint32_t kTileBytes = kLoBase + kLo * kBBytes;
   static constexpr uint32_t kSmemBytes = kTileBytes + 1024 + 256;
+  // tensor memory: two accumulators that take turns, A's parts
+  static constexpr uint32_t kABase = 2 * BN, kASlab = 2 * BK, kTmemCols = 512;
+  static_assert(kABase + kLo * kASlab <= kTmemCols, "tensor memory");
   static_assert(kSmemBytes <= 227 * 1024, "rings must fit shared memory");
   static_assert(BM * (BN + 4) * 4 <= (int)kTileBytes && BN * (BM + 4) * 4 <= (int)kTileBytes, "the tile must fit the rings");
 };
@@ -69,7 +85,7 @@ struct Params {
   uint32_t tiles_m, slabs, cluster, chunk;
   uint32_t whole;           // the first tiles, one CTA each whatever the cluster (even; see launch_mid)
   int a_mn, b_mn;           // operand stored with m (n) contiguous
-  int a_whole, b_whole;     // whole 32-element chunks of that extent: tiles inside them come in one 3-D box
+  int b_whole;              // whole 32-element chunks of B's extent: tiles inside them come in one 3-D box
   int out_t, epilogue, vec_out;
   int* status;
   unsigned long long wait_ns;
@@ -106,7 +122,7 @@ __device__ __forceinline__ void store_share(const Params& p, uint32_t base, uint
       if (w >= kShare) continue;
       const uint32_t at = base + (uint32_t)((v >> shift) * (width + 4) + (v & ((1 << shift) - 1)) * 4) * 4u;
 #pragma unroll
-      for (int k = 0; k < CL; ++k) part[u][k] = CL == 1 ? ld_shared_v4(at) : ld_cluster_v4(at, (uint32_t)k);
+      for (int k = 0; k < CL; ++k) part[u][k] = CL == 1 || (uint32_t)k == rank ? ld_shared_v4(at) : ld_cluster_v4(at, (uint32_t)k);
     }
     if (CL > 1 && first + kBatch * kThreads >= kShare) cluster_arrive();     // nothing of another CTA is read after this
 #pragma unroll
@@ -132,14 +148,12 @@ __device__ __forceinline__ void store_share(const Params& p, uint32_t base, uint
   }
 }
 
-template <int BN, bool EXACT>
+template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                   const __grid_constant__ CUtensorMap map_a3, const __grid_constant__ CUtensorMap map_b3,
-                   const Params p) {
+                   const __grid_constant__ CUtensorMap map_b3, const Params p) {
   using C = Cfg<BN>;
-  // accumulators: with EXACT the cross products get one of their own (see above)
-  constexpr int kKinds = EXACT ? 2 : 1, kAccs = 4 / kKinds;
+  constexpr int kAccs = 2;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -168,19 +182,18 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   static_assert(kBars <= 32, "one lane initialises one barrier");
   if (warp == 0) {
     if (lane < kBars) {
-      const bool by_warps = (lane >= 2 * C::kRaw && lane < kRings) || lane >= kRings + kAccs;   // full_lo, acc_empty
-      mbar_init(bars + 8u * lane, by_warps ? (uint32_t)kSplitWarps : 1u);
+      const bool is_lo = lane >= 2 * C::kRaw && lane < kRings, is_acc_empty = lane >= kRings + kAccs;
+      mbar_init(bars + 8u * lane, is_lo ? (uint32_t)kSplitWarps / 2 : is_acc_empty ? (uint32_t)kAccWarps : 1u);
     }
     if (lane == 0) {
       *abort_flag = 0;
-      prefetch_map(p.a_mn && m0 + BM <= 32 * p.a_whole ? &map_a3 : &map_a);
+      prefetch_map(&map_a);
       prefetch_map(p.b_mn && n0 + BN <= 32 * p.b_whole ? &map_b3 : &map_b);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  static_assert(kSplitWarps == kAccWarps, "by_warps");
   if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), 4 * BN);
+    tmem_alloc(smem_u32(tmem_slot), C::kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -199,13 +212,8 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           const uint32_t a = base + s * C::kRawBytes, b = a + C::kABytes;
           mbar_expect_tx(full_raw(s), C::kRawBytes);
           const int k0 = (int)((kb0 + it) * BK);
-          if (!p.a_mn) {
-            tma_load_2d(a, &map_a, full_raw(s), k0, m0);
-          } else if (m0 + BM <= 32 * p.a_whole) {
-            tma_load_3d(a, &map_a3, full_raw(s), 0, k0, m0 / 32);
-          } else {
-            for (int c = 0; c < BM / 32; ++c) tma_load_2d(a + c * kBox, &map_a, full_raw(s), m0 + 32 * c, k0);
-          }
+          if (p.a_mn) tma_load_2d(a, &map_a, full_raw(s), m0, k0);
+          else tma_load_2d(a, &map_a, full_raw(s), k0, m0);
           if (!p.b_mn) {
             tma_load_2d(b, &map_b, full_raw(s), k0, n0);
           } else if (n0 + BN <= 32 * p.b_whole) {
@@ -220,12 +228,11 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   } else if (warp == 1) {
     const bool leader = elect_one();
     {
-      const uint32_t idesc = make_idesc(BM, BN, p.a_mn, p.b_mn);
+      const uint32_t idesc = make_idesc(BM, BN, 0, p.b_mn);
       // K-major: 128-byte rows in the 128-byte swizzle (layout 2), 8-row groups 1 KB apart, 8 k = 32 bytes
       // inside the row.  MN-major: chunks of 32 elements x BK rows (layout 1), chunks kBox apart, 8 k = 1 KB.
-      const Operand a_op = make_desc(0, p.a_mn ? kBox : 16u, p.a_mn ? 512u : 1024u, p.a_mn ? 1u : 2u);
       const Operand b_op = make_desc(0, p.b_mn ? kBox : 16u, p.b_mn ? 512u : 1024u, p.b_mn ? 1u : 2u);
-      const uint32_t a_step = (p.a_mn ? 1024u : 32u) >> 4, b_step = (p.b_mn ? 1024u : 32u) >> 4;
+      const uint32_t b_step = (p.b_mn ? 1024u : 32u) >> 4;
       // (in a cluster the upper bits of a shared address hold the CTA's rank; a descriptor has no room for them)
       const uint32_t ring = (base & 0x3FFFFu) >> 4;
       uint32_t it = 0, s = 0, s_ph = 0, l = 0, l_ph = 0;    // slab; its place and phase in either ring
@@ -235,30 +242,24 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         ok = mbar_wait(acc_empty(acc), ((c / kAccs) & 1u) ^ 1u, abort_flag, p.status, 115, p.wait_ns);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t d = tmem + acc * kKinds * BN, cross = d + (kKinds - 1) * BN;
+        const uint32_t d = tmem + acc * BN;
         const uint32_t last = it + p.chunk < mine ? it + p.chunk : mine;
         for (uint32_t accumulate = 0; it < last; ++it, accumulate = 1) {
-          const uint32_t a_hi = ring + ((s * C::kRawBytes) >> 4), b_hi = a_hi + (C::kABytes >> 4);
-          const uint32_t a_lo = ring + ((C::kLoBase + l * C::kRawBytes) >> 4), b_lo = a_lo + (C::kABytes >> 4);
-          // the raw words are the hi parts: no need to wait for the split
-          ok = mbar_wait(full_raw(s), s_ph, abort_flag, p.status, 112, p.wait_ns);
+          const uint32_t b_hi = ring + ((s * C::kRawBytes + C::kABytes) >> 4), b_lo = ring + ((C::kLoBase + l * C::kBBytes) >> 4);
+          const uint32_t a_hi = tmem + C::kABase + l * C::kASlab, a_lo = a_hi + BK;
+          ok = mbar_wait(full_raw(s), s_ph, abort_flag, p.status, 112, p.wait_ns) &&
+               mbar_wait(full_lo(l), l_ph, abort_flag, p.status, 113, p.wait_ns);
           if (!ok) break;
           tc_fence_after();
           if (leader) {
-#pragma unroll
-            for (int kk = 0; kk < BK / 8; ++kk)
-              tc_mma_tf32(d, a_op, a_hi + kk * a_step, b_op, b_hi + kk * b_step, idesc, kk ? 1u : accumulate);
-          }
-          ok = mbar_wait(full_lo(l), l_ph, abort_flag, p.status, 113, p.wait_ns);
-          if (!ok) break;
-          tc_fence_after();
-          if (leader) {
+            // the small products first: what the accumulator cuts off is relative to what it holds
 #pragma unroll
             for (int kk = 0; kk < BK / 8; ++kk) {
-              tc_mma_tf32(cross, a_op, a_lo + kk * a_step, b_op, b_hi + kk * b_step, idesc, (!EXACT || kk) ? 1u : accumulate);
-              tc_mma_tf32(cross, a_op, a_hi + kk * a_step, b_op, b_lo + kk * b_step, idesc, 1u);
-              if (EXACT) tc_mma_tf32(cross, a_op, a_lo + kk * a_step, b_op, b_lo + kk * b_step, idesc, 1u);
+              tc_mma_tf32_ts(d, a_lo + 8 * kk, b_op, b_hi + kk * b_step, idesc, kk ? 1u : accumulate);
+              tc_mma_tf32_ts(d, a_hi + 8 * kk, b_op, b_lo + kk * b_step, idesc, 1u);
             }
+#pragma unroll
+            for (int kk = 0; kk < BK / 8; ++kk) tc_mma_tf32_ts(d, a_hi + 8 * kk, b_op, b_hi + kk * b_step, idesc, 1u);
             tc_commit(empty(s));
           }
           if (++s == C::kRaw) s = 0, s_ph ^= 1;
@@ -268,43 +269,76 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
   } else if (warp < 2 + kSplitWarps) {
-    const int tid = threadIdx.x - 64;
-    uint32_t s = 0, ph = 0, l = 0, prev = 0, prev_ph = 0;   // prev: the slab that used this place of the lo ring before
-    for (uint32_t it = 0; it < mine; ++it) {
-      if (it >= (uint32_t)C::kLo) {
-        if (!mbar_wait(empty(prev), prev_ph, abort_flag, p.status, 117, p.wait_ns)) break;
-        if (++prev == C::kRaw) prev = 0, prev_ph ^= 1;
-      }
+    // Four warps take the even slabs, four the odd ones: a slab costs a warp 700 clocks of latencies (barriers, loads,
+    // the wait for its stores) whatever its width, more than the products of a narrow tile.
+    // A: a thread takes one row, the row being the tensor-memory lane its warp may write (warp mod 4).
+    // B: vectors of the slab as they lie.
+    const int tid = (threadIdx.x - 64) & 127, row = (warp & 3) * 32 + lane;
+    constexpr int kVecs = C::kBBytes / 16 / 128 / 2;        // B's vectors of a thread, in two halves like A's 32 k
+    static_assert(kVecs * 2 * 128 * 16 == C::kBBytes, "slab must divide over the split warps");
+    uint32_t s = (warp - 2) >> 2, ph = 0, l = s, prev = s, prev_ph = 0;   // prev: the slab that used this place of the lo ring before
+    for (uint32_t it = s; it < mine; it += 2) {
       if (!mbar_wait(full_raw(s), ph, abort_flag, p.status, 114, p.wait_ns)) break;
-      float4* raw = reinterpret_cast<float4*>(gen + s * C::kRawBytes);
-      float4* lo = reinterpret_cast<float4*>(gen + C::kLoBase + l * C::kRawBytes);
-      constexpr int kVecs = C::kRawBytes / 16;
-      static_assert(kVecs % (kSplitWarps * 32) == 0, "slab must divide over the split warps");
-      auto low = [](float x) {
-        const float l = x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-        // the tensor core ignores the low 13 bits: adding half of the last one it sees rounds to nearest
-        return EXACT ? __uint_as_float(__float_as_uint(l) + 0x1000u) : l;
+      const uint8_t* slab = gen + s * C::kRawBytes;
+      const float4* raw = reinterpret_cast<const float4*>(slab + C::kABytes) + tid;
+      float4* lo = reinterpret_cast<float4*>(gen + C::kLoBase + l * C::kBBytes) + tid;
+      // the tensor core ignores the low 13 bits: adding half of the last one it sees rounds to nearest.  The bound keeps what
+      // would round to infinity finite.
+      auto nearest = [](float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); };
+      auto high = [&](float x) {
+        const float h = __uint_as_float(__float_as_uint(nearest(x)) & 0xFFFFE000u), top = __uint_as_float(0x7F7FE000u);
+        return fminf(fmaxf(h, -top), top);
       };
-      // all loads before the first store: the compiler cannot tell that the two never meet, and would
-      // make one latency of each vector
-      constexpr int kMine = kVecs / (kSplitWarps * 32);
-      float4 v[kMine];
+      auto low = [&](float x) { return nearest(x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u)); };
+      bool ok = true;
 #pragma unroll
-      for (int i = 0; i < kMine; ++i) v[i] = raw[tid + i * kSplitWarps * 32];
+      for (int half = 0; half < 2; ++half) {
+        // all loads before the first store: the compiler cannot tell that the two never meet, and would
+        // make one latency of each vector
+        float a[16];
+        float4 v[kVecs];
+        if (p.a_mn) {                                       // rows of 128 m, one per k
 #pragma unroll
-      for (int i = 0; i < kMine; ++i)
-        lo[tid + i * kSplitWarps * 32] = make_float4(low(v[i].x), low(v[i].y), low(v[i].z), low(v[i].w));
+          for (int j = 0; j < 16; ++j) a[j] = reinterpret_cast<const float*>(slab)[(half * 16 + j) * BM + row];
+        } else {                                            // rows of 32 k in the 128-byte swizzle: eight rows cover all banks
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4*>(a + 4 * j) = *reinterpret_cast<const float4*>(slab + row * 128 + (((half * 4 + j) ^ (row & 7)) << 4));
+        }
+#pragma unroll
+        for (int i = 0; i < kVecs; ++i) v[i] = raw[(half * kVecs + i) * 128];
+        if (half == 0 && it >= (uint32_t)C::kLo) {
+          ok = mbar_wait(empty(prev), prev_ph, abort_flag, p.status, 117, p.wait_ns);
+          if (!ok) break;
+          if ((prev += 2) >= (uint32_t)C::kRaw) prev -= C::kRaw, prev_ph ^= 1;
+          tc_fence_after();
+        }
+        const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::kABase + l * C::kASlab + half * 16;
+        uint32_t part[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) part[j] = __float_as_uint(high(a[j]));
+        tmem_st_32x16(at, part);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) part[j] = __float_as_uint(nearest(a[j] - __uint_as_float(part[j])));
+        tmem_st_32x16(at + BK, part);
+#pragma unroll
+        for (int i = 0; i < kVecs; ++i)
+          lo[(half * kVecs + i) * 128] = make_float4(low(v[i].x), low(v[i].y), low(v[i].z), low(v[i].w));
+      }
+      if (!ok) break;
       fence_async_smem();
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(full_lo(l));               // one arrival per warp
-      if (++s == C::kRaw) s = 0, ph ^= 1;
-      if (++l == C::kLo) l = 0;
+      if ((s += 2) >= (uint32_t)C::kRaw) s -= C::kRaw, ph ^= 1;
+      if ((l += 2) >= (uint32_t)C::kLo) l -= C::kLo;
     }
   } else {
     // four consecutive warps cover the 128 lanes, the two warps of a lane quarter half of the columns each
     const int q = warp & 3, half = (warp - (2 + kSplitWarps)) >> 2;
     constexpr int kCols = BN / 2;
-    constexpr int kPart = 16;                               // columns read at a time: what the register budget allows
+    constexpr int kPart = kCols == 32 ? 32 : 16;             // columns in flight: what the register budget allows
     float acc[kCols];
 #pragma unroll
     for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
@@ -314,19 +348,13 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       ok = mbar_wait(acc_full(a), (c / kAccs) & 1u, abort_flag, p.status, 116, p.wait_ns);
       if (!ok) break;
       tc_fence_after();
+      const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * BN + half * kCols);
 #pragma unroll
       for (int j0 = 0; j0 < kCols; j0 += kPart) {
         uint32_t r[kPart];
-        const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * kKinds * BN + half * kCols + j0);
-        tmem_ld_32x16(at, r);
-        tmem_ld_wait();
-        if (EXACT) {
-          uint32_t x[kPart];
-          tmem_ld_32x16(at + BN, x);
-          tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < kPart; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(x[j]));
-        }
+        for (int j = 0; j < kPart; j += 16) tmem_ld_32x16(at + j0 + j, r + j);
+        tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < kPart; ++j) acc[j0 + j] += __uint_as_float(r[j]);
       }
@@ -362,7 +390,7 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const long long t0 = clock64();
       while (clock64() - t0 < 2000000ll) { }
     }
-    tmem_dealloc(tmem, 4 * BN);
+    tmem_dealloc(tmem, C::kTmemCols);
   }
   switch (cluster) {
     case 1: store_share<BN, 1>(p, base, 0, m0, n0); break;
@@ -409,7 +437,7 @@ struct Stored {
   bool padded;                                              // columns up to the pitch are there, and zero
 };
 
-template <int BN, bool EXACT>
+template <int BN>
 int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Params p, uint64_t k, cudaStream_t stream) {
   using C = Cfg<BN>;
   int dev = 0;
@@ -419,39 +447,30 @@ int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Pa
   {
     std::lock_guard<std::mutex> guard(mu);
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(fmatmul_mid_kernel<BN, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
+      cudaError_t e = cudaFuncSetAttribute(fmatmul_mid_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
       if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFuncSetAttribute(smem)", e);
       attr_done[dev] = true;
     }
   }
   // The extents are the true ones wherever TMA has to cut a box off; a padded MN-major operand offers whole chunks.
-  CUtensorMap maps[2], maps3[2];
-  const Stored* op[2] = {&left, &right};
-  const bool mn[2] = {a_mn, b_mn};
-  const uint32_t tile_rows[2] = {(uint32_t)BM, (uint32_t)BN};
-  const uint64_t extent[2] = {p.m, p.n};
-  int whole[2] = {0, 0};
-  for (int i = 0; i < 2; ++i) {
-    const Stored& o = *op[i];
-    int rc = POLAR_B200_OK;
-    if (!mn[i]) {
-      rc = make_map(&maps[i], o.p, k, extent[i], BK, tile_rows[i], false, BK, o.pitch);
-      maps3[i] = maps[i];
-    } else {
-      const uint64_t cols = o.padded ? o.pitch : o.cols;
-      whole[i] = (int)(cols / 32);
-      const bool boxes_2d = (extent[i] + tile_rows[i] - 1) / tile_rows[i] * tile_rows[i] > 32ull * whole[i];
-      if (whole[i]) rc = make_map_chunks(&maps3[i], o.p, whole[i], k, BK, tile_rows[i] / 32, o.pitch);
-      if (!rc && (boxes_2d || !whole[i])) rc = make_map(&maps[i], o.p, cols, k, 32, BK, true, BK, o.pitch);
-      else maps[i] = maps3[i];
-      if (!whole[i]) maps3[i] = maps[i];
-    }
-    if (rc) return rc;
+  CUtensorMap map_a, map_b, map_b3;
+  int rc = a_mn ? make_map(&map_a, left.p, p.m, k, BM, BK, false, 0, left.pitch)       // (the split warps read it: no swizzle)
+                : make_map(&map_a, left.p, k, p.m, BK, BM, false, BK, left.pitch);
+  if (!rc && !b_mn) {
+    rc = make_map(&map_b, right.p, k, p.n, BK, BN, false, BK, right.pitch);
+    map_b3 = map_b;
+  } else if (!rc) {
+    const uint64_t cols = right.padded ? right.pitch : right.cols;
+    p.b_whole = (int)(cols / 32);
+    const bool boxes_2d = (p.n + BN - 1) / BN * BN > 32ull * p.b_whole;
+    if (p.b_whole) rc = make_map_chunks(&map_b3, right.p, p.b_whole, k, BK, BN / 32, right.pitch);
+    if (!rc && (boxes_2d || !p.b_whole)) rc = make_map(&map_b, right.p, cols, k, 32, BK, true, BK, right.pitch);
+    else map_b = map_b3;
+    if (!p.b_whole) map_b3 = map_b;
   }
+  if (rc) return rc;
   p.a_mn = a_mn;
   p.b_mn = b_mn;
-  p.a_whole = whole[0];
-  p.b_whole = whole[1];
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(p.whole + (p.tiles_m * (uint32_t)((p.n + BN - 1) / BN) - p.whole) * p.cluster);
   c.blockDim = dim3(kThreads);
@@ -465,7 +484,7 @@ int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Pa
   at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   c.attrs = at;
   c.numAttrs = p.cluster > 1 ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&c, fmatmul_mid_kernel<BN, EXACT>, maps[0], maps[1], maps3[0], maps3[1], p);
+  cudaError_t e = cudaLaunchKernelEx(&c, fmatmul_mid_kernel<BN>, map_a, map_b, map_b3, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(POLAR_B200_ERR_CUDA, "fmatmul_mid", e);
@@ -532,18 +551,18 @@ int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* 
   p.slabs = (uint32_t)((k + BK - 1) / BK);
   p.cluster = (uint32_t)cluster;
   p.whole = (uint32_t)whole;
-  // slabs of 32 terms summed in tensor memory, the rest in registers: EXACT is to stay below the error of FFMA sums
+  // slabs of 32 terms summed in tensor memory, the rest in registers: `exact` is to stay below the error of FFMA sums
   p.chunk = !exact ? 8 : k < 512 ? 1 : 2;
   if ((cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) || p.slabs < p.cluster) return fail(POLAR_B200_ERR_UNSUPPORTED, "fewer slabs than CTAs in a cluster");
   if ((uint64_t)p.tiles_m * ((p.n + bn - 1) / bn) * p.cluster > 0x7fffffffull) return fail(POLAR_B200_ERR_UNSUPPORTED, "too many tiles");
   // exchanged: right' plays the row operand - stored [k, n] is "row extent contiguous" - and left the column operand
   const Stored &a = swap ? r : l, &b = swap ? l : r;
   const bool a_mn = swap ? !tr : tl, b_mn = swap ? tl : !tr;
-#define POLAR_MID(BN)   case BN: return exact ? launch_cfg<BN, true>(a, b, a_mn, b_mn, p, k, stream) : launch_cfg<BN, false>(a, b, a_mn, b_mn, p, k, stream);
   switch (bn) {
-    POLAR_MID(32) POLAR_MID(64) POLAR_MID(128)
+    case 32: return launch_cfg<32>(a, b, a_mn, b_mn, p, k, stream);
+    case 64: return launch_cfg<64>(a, b, a_mn, b_mn, p, k, stream);
+    case 128: return launch_cfg<128>(a, b, a_mn, b_mn, p, k, stream);
   }
-#undef POLAR_MID
   return fail(POLAR_B200_ERR_INVALID, "tile width must be 32, 64 or 128");
 }
 
