@@ -237,8 +237,8 @@ int polar_b200_fmatmul_ffma(int transLeft, int transRight, uint64_t m,
  * -1 = stream mode: the CTAs take equal shares of all k slabs of all tiles and a tile
  * may be finished by the next CTA - 128 x 256 tiles only; scratch for the partial
  * products comes from the stream-ordered pool).  tile_n 2032, 2064 or 2128: one 128 x 32/64/128
- * tile per cluster of `splits` = 1, 2, 4 or 8 CTAs (+ 1000: exchanged roles; write_hi == 1: short sums in tensor memory,
- * with short sums), for operands of any alignment.  Fails with
+ * tile per cluster of `splits` = 1, 2, 4 or 8 CTAs (+ 1000: exchanged roles; write_hi == 1: short sums
+ * in tensor memory), for operands of any alignment.  Fails with
  * POLAR_B200_ERR_UNSUPPORTED when the operands cannot be described to TMA
  * (bases not 16-byte aligned, or a contiguous extent that is not a multiple of
  * 4 floats). */

@@ -10,7 +10,8 @@ int launch_ffma(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float*
 int launch_tc(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
               const float* right, float* out, int bn, int bk, int passes, int write_hi, float* ws,
               uint32_t splits, int epilogue, cudaStream_t stream, uint64_t left_pitch = 0, int mt = 1,
-              int swap_ab = 0);
+              int swap_ab = 0, uint32_t tail_rows = 0, float* tail = nullptr);
+uint64_t tc_tail_bytes(uint64_t m, uint64_t n, uint64_t k, uint32_t splits, uint64_t rows);
 uint32_t tc_default_splits(uint64_t m, uint64_t n, uint64_t k, int mt = 1);
 bool tc_tail_in_halves(uint64_t tiles, uint64_t grid);
 uint64_t tc_workspace_bytes(uint64_t m, uint64_t n, uint64_t k, uint32_t splits, int mt = 1);
@@ -80,7 +81,8 @@ int run_tc(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left
 
 // A t_f product whose row count is a few rows past a multiple of the 128-row tile would
 // spend a whole tile row of tensor-core work on them (784 rows: 7 tile rows for 6.1 of
-// work).  Those rows go to the bandwidth-bound kernel instead, which reads `right` once
+// work).  Where the whole tile rows run as 256 x 256 tiles with a summing pass, those tiles' split warps take the
+// rows along (gemm_tc.cu, TAIL).  Else the rows go to another kernel, which reads `right` once
 // more - on a second stream of the library's own, forked from and joined back into the
 // caller's stream, so that the pass runs WHILE the tensor-core kernel computes the whole
 // tile rows (the two write disjoint rows of the result and use disjoint halves of the
@@ -408,6 +410,17 @@ static int tc_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const flo
     cudaError_t e = scratch_alloc(&own, tc_need + rag_need, main_stream);
     if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "scratch (workspace)", e);
     ws = static_cast<char*>(own);
+  }
+  // the tiles' own kernel takes the last rows along where it can
+  const uint64_t tail = mt == 2 ? tc_tail_bytes(mm, n, k, c.splits, rem) : 0;
+  if (tail != 0 && tail <= rag_need) {
+    rc = launch_tc(tl, tr, mm, n, k, left, right, out, 256, 16, 3, 0, reinterpret_cast<float*>(ws), c.splits, 0, main_stream, lp,
+                   mt, 0, (uint32_t)rem, reinterpret_cast<float*>(ws + tc_need));
+    if (own) {
+      cudaError_t e = scratch_free(own, main_stream);
+      if (!rc && e != cudaSuccess) rc = fail(POLAR_B200_ERR_CUDA, "returning scratch", e);
+    }
+    return rc;
   }
   // fork: the side stream starts where the caller's stream is now (one fork/join at a time
   // per process: the side stream's two events are shared)

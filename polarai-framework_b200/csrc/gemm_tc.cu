@@ -109,10 +109,17 @@ struct Params {
   // The kernel was given the operands in exchanged roles (it computes the transposed product):
   // a tile's rows are columns of the result, whose row length is m.  See launch_tc.
   int out_t;
+  // Rows past the last whole tile of a t_f product, at most kTailRows (TAIL; see the split warps): their partial sums,
+  // [piece][kTailParts][kTailRows][BN] floats.
+  float* tail;
   // Whole-tile mode: tiles from this one on are computed as two column halves by two CTAs
   // (halves_from in tc_plan.hpp; kNoHalves = none).  256-column tiles only.
   uint32_t half_from;
 };
+
+constexpr int kTailRows = 16;     // the most rows past the last whole tile that the TAIL configuration takes along
+constexpr int kTailShare = 6;     // of them per row tile
+constexpr int kTailParts = 4;     // groups of split warps that each sum every fourth k
 
 // Tile raster: groups of kGroupM row tiles walk the column tiles together, so the
 // CTAs running at the same time share A row panels and B column panels in L2.
@@ -127,10 +134,10 @@ __device__ __forceinline__ void tile_coords(uint32_t t, uint32_t tiles_m, uint32
   *n0 = (int)((r / rows) * bn);
 }
 
-template <int BN, int BK, int MT>
+template <int BN, int BK, int MT, bool TAIL>
 __global__ void __launch_bounds__(kThreads, 1)
 fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const Params p) {
+                  const __grid_constant__ CUtensorMap map_tail, const Params p) {
   using C = Cfg<BN, BK, MT>;
   constexpr int kTileM = BM * MT;
   // accumulator columns of row sub-tile h of the tile held in buffer `as`
@@ -149,6 +156,8 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_gen + C::kTileBytes + 8 * (3 * S + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
+  constexpr uint32_t kTailStage = kTailRows * BK * 4;         // [BK k][kTailRows] floats of the left operand
+  const uint32_t tail_base = bar_base + 256;
   const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const uint32_t num_kb = (uint32_t)((p.k + BK - 1) / BK);
@@ -285,8 +294,9 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           if (!mbar_wait(empty(s), ph, abort_flag, p.status, 101, p.wait_ns)) { ok = false; break; }
           const uint32_t stage = smem_base + s * C::kStageBytes;
           if (leader) {
-            mbar_expect_tx(full_raw(s), C::kABytes + (pc.half ? C::kBBytes / 2 : C::kBBytes));
+            mbar_expect_tx(full_raw(s), C::kABytes + (pc.half ? C::kBBytes / 2 : C::kBBytes) + (TAIL ? kTailStage : 0));
             const int k0 = (int)(kb * BK);
+            if (TAIL) tma_load_2d(tail_base + s * kTailStage, &map_tail, full_raw(s), (int)p.m, k0);
             // The TMA unit takes 50-100 ns per instruction whatever its size, so a slab comes in as few
             // boxes as possible: an MN-major slab, 32-element chunks of BK rows each, in one or two 3-D
             // boxes of 4 or 8 chunks.  (As one 2-D box per chunk - 16 instructions for a 256 x 256 x 16
@@ -409,6 +419,38 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       PieceWalk walk = make_walk();
       Piece pc;
       for (; ok && walk.next(pc); ++tile_iter) {
+        // TAIL: a t_f product with a few rows past its last whole tile (784 = 3 * 256 + 16) needs those rows' products with
+        // every slab of B, which pass through these warps' registers anyway: each row tile's CTAs take kTailShare of the
+        // rows along, in FMA.  As a product of their own they cost a second pass over B (43 of 271 us at 784 x 4096 x
+        // 8192, 310 of 1880 at 784 x 4096 x 65536; this way 16 of 243 and 99 of 1675); a tile row
+        // of the tensor core would be a quarter empty.  A warp has 128 columns and every fourth k - its lanes share the
+        // row values, a broadcast: shared memory is what the kernel is short of - and a lane four columns.
+        // Sums of 128 terms are added up in memory.
+        const int tail_half = warp & 1, tail_k = (warp - 2) >> 1, tail_cg = lane & 7;
+        float acc[kTailShare][4];
+        int tail_row = 0;
+        float* tail_dst = nullptr;
+        bool tail_first = true;
+        if (TAIL) {
+          int m0, n0;
+          tile_coords(pc.tile, p.tiles_m, p.tiles_n, BN, &m0, &n0, kTileM);
+          tail_row = m0 / kTileM * kTailShare;
+          const uint32_t column = (uint32_t)(n0 / BN), piece = p.share ? walk.team + column : pc.slot * p.tiles_n + column;
+          tail_dst = p.tail + (((uint64_t)piece * kTailParts + tail_k) * kTailRows + tail_row) * BN + tail_half * 128 + lane * 4;
+#pragma unroll
+          for (int r = 0; r < kTailShare; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+        }
+        auto tail_flush = [&]() {
+#pragma unroll
+          for (int r = 0; r < kTailShare; ++r) {
+            if (tail_row + r < kTailRows) {
+              if (tail_first) *reinterpret_cast<float4*>(tail_dst + r * BN) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+              else red_global_add_v4(tail_dst + r * BN, acc[r]);
+            }
+            acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+          }
+          tail_first = false;
+        };
         for (uint32_t kb = pc.kb0, kb_end = pc.kb1; p.passes == 3 && kb < kb_end; ++kb) {
           if (!mbar_wait(full_raw(s), ph, abort_flag, p.status, 104, p.wait_ns)) { ok = false; break; }
           float4* raw = reinterpret_cast<float4*>(smem_gen + s * C::kStageBytes);
@@ -419,13 +461,20 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           // make one latency of each vector
           constexpr int kMine = kVecs / (kSplitWarps * 32), kHalf = kMine > 4 ? kMine / 2 : kMine;
           static_assert(kMine % kHalf == 0, "split in equal batches");
+          // vector i of the batch from i0; TAIL takes B's, chunks of BK rows of 32 columns with the 32-byte quarters of a row
+          // exchanged by (k mod 4), so that a lane's columns stay the same
+          auto at = [&](int i0, int i) {
+            if (TAIL && i0 != 0)
+              return (int)(C::kABytes / 16) + (tail_half * 4 + (lane >> 3)) * 8 * BK + (4 * i + tail_k) * 8 + (tail_cg ^ (tail_k << 1));
+            return tid + (i0 + i) * kSplitWarps * 32;
+          };
           for (int i0 = 0; i0 < kMine; i0 += kHalf) {
             float4 v[kHalf];
 #pragma unroll
-            for (int i = 0; i < kHalf; ++i) v[i] = raw[tid + (i0 + i) * kSplitWarps * 32];
+            for (int i = 0; i < kHalf; ++i) v[i] = raw[at(i0, i)];
 #pragma unroll
             for (int i = 0; i < kHalf; ++i) {
-              const int e = tid + (i0 + i) * kSplitWarps * 32;
+              const int e = at(i0, i);
               float4 h;
               h.x = __uint_as_float(__float_as_uint(v[i].x) & 0xFFFFE000u);
               h.y = __uint_as_float(__float_as_uint(v[i].y) & 0xFFFFE000u);
@@ -434,13 +483,28 @@ fmatmul_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
               lo[e] = make_float4(v[i].x - h.x, v[i].y - h.y, v[i].z - h.z, v[i].w - h.w);
               if (p.write_hi == 1) raw[e] = h;
             }
+            if (TAIL && i0 != 0 && tail_row < kTailRows) {
+              const float* x = reinterpret_cast<const float*>(smem_gen + C::kTileBytes + 256 + s * kTailStage) + tail_row;
+#pragma unroll
+              for (int i = 0; i < kHalf; ++i)
+#pragma unroll
+                for (int r = 0; r < kTailShare; r += 2) {
+                  const float2 w = *reinterpret_cast<const float2*>(x + (4 * i + tail_k) * kTailRows + r);
+                  acc[r][0] = fmaf(w.x, v[i].x, acc[r][0]), acc[r][1] = fmaf(w.x, v[i].y, acc[r][1]);
+                  acc[r][2] = fmaf(w.x, v[i].z, acc[r][2]), acc[r][3] = fmaf(w.x, v[i].w, acc[r][3]);
+                  acc[r + 1][0] = fmaf(w.y, v[i].x, acc[r + 1][0]), acc[r + 1][1] = fmaf(w.y, v[i].y, acc[r + 1][1]);
+                  acc[r + 1][2] = fmaf(w.y, v[i].z, acc[r + 1][2]), acc[r + 1][3] = fmaf(w.y, v[i].w, acc[r + 1][3]);
+                }
+            }
           }
           fence_async_smem();
           // one arrival per warp
           __syncwarp();
           if (lane == 0) mbar_arrive(full_lo(s));
           if (++s == S) s = 0, ph ^= 1;
+          if (TAIL && ((kb - pc.kb0) & 31u) == 31u) tail_flush();
         }
+        if (TAIL && ok) tail_flush();
         if (MT == 2 && ok) {
           // 256-row tiles: nothing is left to split until this tile is drained, so these
           // warps drain its lower sub-tile while the epilogue warps drain the upper one
@@ -558,11 +622,43 @@ bool shape_ok(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* l
   return m > 0 && n > 0 && k > 0;
 }
 
+// The rows past the last whole tile: vector v of [rows][n / 4], the kTailParts partial sums of each of its column's pieces -
+// the first one and then every `step`-th of `count` - in that order.
+struct TailSum {
+  const float* parts;        // nullptr: none
+  float* out;
+  uint32_t rows, first_block;   // of the launch
+};
+__device__ __forceinline__ void sum_tail(const TailSum& t, uint64_t n, uint64_t v, uint32_t first, uint32_t step, uint32_t count) {
+  const uint64_t row = v / (n / 4), col = (v % (n / 4)) * 4;
+  const float* src = t.parts + ((uint64_t)first * kTailParts * kTailRows + row) * 256 + (col & 255);
+  float4 s = {0.f, 0.f, 0.f, 0.f};
+  for (uint32_t i = 0; i < count; ++i, src += (uint64_t)step * kTailParts * kTailRows * 256) {
+    float4 x[kTailParts];
+#pragma unroll
+    for (int j = 0; j < kTailParts; ++j) x[j] = __ldcg(reinterpret_cast<const float4*>(src + j * kTailRows * 256));
+#pragma unroll
+    for (int j = 0; j < kTailParts; ++j) s.x += x[j].x, s.y += x[j].y, s.z += x[j].z, s.w += x[j].w;
+  }
+  float* o = t.out + row * n + col;
+  if ((reinterpret_cast<uintptr_t>(t.out) & 15) == 0) {
+    *reinterpret_cast<float4*>(o) = s;
+  } else {
+    o[0] = s.x; o[1] = s.y; o[2] = s.z; o[3] = s.w;
+  }
+}
+
 // out[e] = sum of the splits' partial products, ascending split index (fixed order).  The
 // partial products live in 16-byte aligned scratch; `out` is the caller's and may be only
 // 4-byte aligned, in which case the four sums are stored one by one.
 __global__ void __launch_bounds__(256) add_splits_kernel(const float4* __restrict__ partial, float* __restrict__ out,
-                                                         uint64_t nvec, uint32_t splits, int epilogue, int out_vec) {
+                                                         uint64_t nvec, uint32_t splits, int epilogue, int out_vec, const TailSum tail, uint64_t n) {
+  if (blockIdx.x >= tail.first_block) {
+    const uint64_t v = (uint64_t)(blockIdx.x - tail.first_block) * 256 + threadIdx.x;
+    const uint32_t tiles_n = (uint32_t)((n + 255) / 256);
+    if (v < tail.rows * (n / 4)) sum_tail(tail, n, v, (uint32_t)(v % (n / 4) / 64), tiles_n, splits);
+    return;
+  }
   const uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= nvec) return;
   float4 s = __ldcs(partial + i);
@@ -581,11 +677,14 @@ __global__ void __launch_bounds__(256) add_splits_kernel(const float4* __restric
   }
 }
 
+unsigned tail_blocks(const TailSum& t, uint64_t n) { return t.parts ? (unsigned)((t.rows * (n / 4) + 255) / 256) : 0u; }
+
 int launch_add_splits(const float* ws, float* out, uint64_t m, uint64_t n, uint32_t splits, int epilogue,
-                      cudaStream_t stream) {
+                      TailSum tail, cudaStream_t stream) {
   const uint64_t nvec = m * n / 4;
-  add_splits_kernel<<<(unsigned)((nvec + 255) / 256), 256, 0, stream>>>(reinterpret_cast<const float4*>(ws), out, nvec,
-                                                                       splits, epilogue, aligned16(out) ? 1 : 0);
+  tail.first_block = (unsigned)((nvec + 255) / 256);
+  add_splits_kernel<<<tail.first_block + tail_blocks(tail, n), 256, 0, stream>>>(
+      reinterpret_cast<const float4*>(ws), out, nvec, splits, epilogue, aligned16(out) ? 1 : 0, tail, n);
   return check_launch("fmatmul_add_splits");
 }
 
@@ -598,7 +697,16 @@ template <int BN, int MT>
 __global__ void __launch_bounds__(256) stream_reduce_kernel(const float* __restrict__ slots, float* __restrict__ out,
                                                             uint64_t m, uint64_t n, uint32_t tiles_m, uint32_t tiles_n,
                                                             uint32_t num_kb, uint32_t share, uint32_t teams,
-                                                            int epilogue) {
+                                                            int epilogue, const TailSum tail) {
+  if (blockIdx.x >= tail.first_block) {
+    const uint64_t v = (uint64_t)(blockIdx.x - tail.first_block) * 256 + threadIdx.x;
+    if (v >= tail.rows * (n / 4)) return;
+    const uint32_t column = (uint32_t)(v % (n / 4) / 64);
+    uint32_t first, last;
+    stream_teams_of_column(column, num_kb, share, &first, &last);
+    sum_tail(tail, n, v, first + column, 1, last - first + 1);
+    return;
+  }
   constexpr uint32_t kVecsPerTile = BM * MT * BN / 4;
   constexpr uint32_t kBlocksPerTile = kVecsPerTile / 256;
   const uint32_t tile = blockIdx.x / kBlocksPerTile;
@@ -678,18 +786,22 @@ static bool halves_enabled() {
   return on;
 }
 
-template <int BN, int BK, int MT = 1>
+template <int BN, int BK, int MT = 1, bool TAIL = false>
 static int launch_cfg(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                       const float* right, float* out, int passes, int write_hi, float* ws, uint32_t splits,
-                      int epilogue, cudaStream_t stream, uint64_t left_pitch, int out_t) {
+                      int epilogue, cudaStream_t stream, uint64_t left_pitch, int out_t, uint32_t tail_rows = 0,
+                      float* tail = nullptr) {
   using C = Cfg<BN, BK, MT>;
-  static_assert(C::kStages >= 2 && C::kSmemBytes <= 227 * 1024, "stage ring must fit shared memory");
+  static_assert(!TAIL || (BN == 256 && BK == 16 && MT == 2), "the rows past the tiles ride on 256 x 256 tiles");
+  // (a warp's last share may read two floats past its stage)
+  constexpr uint32_t kSmemBytes = C::kSmemBytes + (TAIL ? C::kStages * kTailRows * BK * 4 + 64 : 0);
+  static_assert(C::kStages >= 2 && kSmemBytes <= 227 * 1024, "stage ring must fit shared memory");
   int dev = 0;
   cudaGetDevice(&dev);
   static bool attr_done[64] = {false};
   if (dev >= 0 && dev < 64 && !attr_done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(fmatmul_tc_kernel<BN, BK, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(fmatmul_tc_kernel<BN, BK, MT, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kSmemBytes);
     if (e != cudaSuccess) return fail(POLAR_B200_ERR_CUDA, "cudaFuncSetAttribute(smem)", e);
     attr_done[dev] = true;
   }
@@ -708,7 +820,12 @@ static int launch_cfg(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const 
        : b_chunked ? make_map_chunks(&map_b, right, n / 32, k, BK, C::kBBoxRows / 32, n)
                    : make_map(&map_b, right, n, k, 32, BK, true, BK, 0);
   if (rc) return rc;
+  CUtensorMap map_tail = map_a;
+  if (TAIL) rc = make_map(&map_tail, left, m + tail_rows, k, kTailRows, BK, false, 0, left_pitch);
+  if (rc) return rc;
+  const TailSum tail_sum = {TAIL ? tail : nullptr, out + m * n, tail_rows, 0};
   Params p;
+  p.tail = tail;
   p.m = m; p.n = n; p.k = k; p.out = out;
   p.a_mn_major = tl ? 1 : 0;
   p.b_mn_major = tr ? 0 : 1;
@@ -737,15 +854,18 @@ static int launch_cfg(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const 
     p.share = plan.share;
     p.teams = plan.teams;
     p.slots = ws;
-    fmatmul_tc_kernel<BN, BK, MT><<<plan.grid, kThreads, C::kSmemBytes, stream>>>(map_a, map_b, p);
+    fmatmul_tc_kernel<BN, BK, MT, TAIL><<<plan.grid, kThreads, kSmemBytes, stream>>>(map_a, map_b, map_tail, p);
     rc = check_launch("fmatmul_tc");
     if (rc) return rc;
     constexpr uint32_t kBlocksPerTile = BM * MT * BN / 4 / 256;
-    stream_reduce_kernel<BN, MT><<<(unsigned)(tm * tn * kBlocksPerTile), 256, 0, stream>>>(
-        ws, out, m, n, p.tiles_m, p.tiles_n, (uint32_t)num_kb, plan.share, plan.teams, epilogue);
+    TailSum t = tail_sum;
+    t.first_block = (unsigned)(tm * tn * kBlocksPerTile);
+    stream_reduce_kernel<BN, MT><<<t.first_block + tail_blocks(t, n), 256, 0, stream>>>(
+        ws, out, m, n, p.tiles_m, p.tiles_n, (uint32_t)num_kb, plan.share, plan.teams, epilogue, t);
     return check_launch("fmatmul_stream_reduce");
   }
   if (splits < 1 || !ws || splits > num_kb) splits = 1;
+  if (TAIL && splits == 1) return fail(POLAR_B200_ERR_UNSUPPORTED, "rows past the tiles: cuts of k or stream mode only");
   p.splits = splits;
   p.partial = splits > 1 ? ws : nullptr;
   p.epilogue = splits > 1 ? 0 : epilogue;
@@ -753,10 +873,10 @@ static int launch_cfg(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const 
   if (units > 0x7fffffffull) return fail(POLAR_B200_ERR_UNSUPPORTED, "too many tiles");
   unsigned grid = (unsigned)(units < (uint64_t)sm_count() ? units : (uint64_t)sm_count());   // one CTA per SM
   if (splits == 1 && BN == 256 && halves_enabled()) p.half_from = halves_from(units, grid);
-  fmatmul_tc_kernel<BN, BK, MT><<<grid, kThreads, C::kSmemBytes, stream>>>(map_a, map_b, p);
+  fmatmul_tc_kernel<BN, BK, MT, TAIL><<<grid, kThreads, kSmemBytes, stream>>>(map_a, map_b, map_tail, p);
   rc = check_launch("fmatmul_tc");
   if (rc || splits == 1) return rc;
-  return launch_add_splits(ws, out, m, n, splits, epilogue, stream);
+  return launch_add_splits(ws, out, m, n, splits, epilogue, tail_sum, stream);
 }
 
 }  // namespace tc
@@ -769,7 +889,10 @@ static int launch_cfg(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const 
 // epilogue is a visible part of a tile's time, i.e. for short sums.
 int launch_tc(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
               const float* right, float* out, int bn, int bk, int passes, int write_hi, float* ws,
-              uint32_t splits, int epilogue, cudaStream_t stream, uint64_t left_pitch, int mt, int swap_ab) {
+              uint32_t splits, int epilogue, cudaStream_t stream, uint64_t left_pitch, int mt, int swap_ab, uint32_t tail_rows,
+              float* tail) {
+  if (tail_rows)
+    return tc::launch_cfg<256, 16, 2, true>(tl, tr, m, n, k, left, right, out, passes, write_hi, ws, splits, epilogue, stream, left_pitch, 0, tail_rows, tail);
   if (swap_ab) {
     // left' = right: stored [k,n] (tr = 0) is "stored [k,m']" (tl' = 1); right' = left: stored
     // [m,k] (tl = 0) is "stored [n',k]" (tr' = 1)
@@ -807,6 +930,20 @@ uint64_t tc_workspace_bytes(uint64_t m, uint64_t n, uint64_t k, uint32_t splits,
   const uint64_t rows = 128ull * mt;
   if (splits == 0) return tc::stream_plan((m + rows - 1) / rows, (n + 255) / 256, (k + 15) / 16, 256, mt, (uint64_t)sm_count()).bytes;
   return splits > 1 ? (uint64_t)splits * m * n * sizeof(float) : 0;
+}
+
+// Scratch for the `rows` rows past the last whole tile when the 256 x 256-tile kernel takes them along (t_f products, `left`
+// with a row pitch, m rows without them): 0 if it cannot, because each row tile takes only a few of them, or because
+// no second kernel adds up partial products.
+uint64_t tc_tail_bytes(uint64_t m, uint64_t n, uint64_t k, uint32_t splits, uint64_t rows) {
+  const uint64_t tiles_m = (m + 255) / 256, tiles_n = (n + 255) / 256;
+  if (rows == 0 || rows > tc::kTailRows || rows > tiles_m * tc::kTailShare || splits == 1) return 0;
+  uint64_t pieces = splits * tiles_n;
+  if (splits == 0) {
+    const tc::StreamPlan plan = tc::stream_plan(tiles_m, tiles_n, (k + 15) / 16, 256, 2, (uint64_t)sm_count());
+    pieces = plan.teams ? plan.teams + tiles_n : 0;
+  }
+  return pieces * tc::kTailParts * tc::kTailRows * 256 * sizeof(float);
 }
 
 bool tc_shape_ok(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,

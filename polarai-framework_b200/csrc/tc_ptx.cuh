@@ -124,6 +124,11 @@ __device__ __forceinline__ void st_global_v8(float* dst, const uint32_t* r) {
                : "memory");
 }
 
+// Adds four floats to memory, 16-byte aligned, without waiting for it.
+__device__ __forceinline__ void red_global_add_v4(float* dst, const float* v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
