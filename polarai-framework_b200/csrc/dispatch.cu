@@ -220,8 +220,8 @@ namespace {
 
 // ---- the cluster kernel (gemm_tc_mid.cu) --------------------------------------------------------------
 // One 128 x bn tile per cluster of CTAs.  Times in microseconds, fitted to measurements on B200 between
-// 128 x 64 x 64 and 2048^3 (within 15 % there): a slab of 32 k costs a CTA 0.36 / 0.43 / 0.56 us with tiles of 32 / 64 / 128
-// columns (0.42 / 0.50 / 0.63 with short sums in tensor memory: reading them competes with the products), set-up,
+// 128 x 64 x 64 and 2048^3 (within 15 % there): a slab of 32 k costs a CTA 0.29 / 0.36 / 0.56 us with tiles of 32 / 64 / 128
+// columns (0.40 / 0.42 / 0.63 with short sums in tensor memory: reading them competes with the products), set-up,
 // pipeline fill and the store of the tile 4 to 5 us, the exchange between the CTAs of a cluster 1.3 to 3.3 us.
 struct MidChoice {
   int bn = 0, cluster = 1, swap = 0;
@@ -236,7 +236,7 @@ MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact) {
     const uint64_t rows = swap ? n : m, cols = swap ? m : n;
     for (int i = 0; i < 3; ++i) {
       const int bn = 32 << i;
-      static const double slab_us[2][3] = {{0.36, 0.43, 0.56}, {0.42, 0.50, 0.63}};
+      static const double slab_us[2][3] = {{0.29, 0.36, 0.56}, {0.40, 0.42, 0.63}};
       const uint64_t tiles = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
       for (int cl = 1; cl <= 8 && (uint64_t)cl <= slabs; cl *= 2) {
         // clusters of 4 and 8 leave SMs of a GPC unused: 33 and 15 of them run at a time on 148 SMs

@@ -10,10 +10,10 @@
 //
 // One CTA:
 //   warp 0      TMA producer: 32-float k slabs of A (128 rows) and B (BN rows), two instructions per slab;
-//   warps 2-9   split warps: of each landed slab, the hi and lo parts of A to tensor memory and the lo parts of B to
+//   warps 2...   split warps, two or three groups of four: of each landed slab, the hi and lo parts of A to tensor memory and the lo parts of B to
 //               shared memory beside the raw words, which are its hi parts (the tensor core ignores the low 13 bits);
 //   warp 1      tcgen05.mma issuer: per slab and 8 k the three products of the TF32 split, A from tensor memory;
-//   warps 10-17 accumulator warps: every `chunk` slabs they read the tensor-memory accumulator and add it to
+//   the rest    accumulator warps, eight or four: every `chunk` slabs they read the tensor-memory accumulator and add it to
 //               registers in round-to-nearest.  The tensor core's own accumulator rounds toward zero, an error that
 //               grows with the length of the sum (8e-9 of the result per term for zero-mean operands);
 //               chunks keep it at that of a short sum.
@@ -21,8 +21,10 @@
 // What bounds it: shared memory, 128 bytes per clock.  An instruction of 128 x BN x 8 with both operands there reads
 // 4 KB + 32 BN bytes: 64 / 48 / 40 clocks for 128 / 64 / 32 columns, where the tensor core needs 64 / 32 / 16 - all of the
 // bandwidth before TMA has written a slab and the split has read it and written the lo parts.  With A in tensor memory
-// a 128 x 128 x 32 slab takes 1024 clocks of shared memory instead of 1536 (768 of the tensor core); measured 0.54 us a
-// slab, 0.41 with 64 columns and 0.34 with 32 (0.60, 0.48, 0.43 before).  2001 x 1511 x 999: 60 -> 50 us; 16 x 4096 x 784:
+// a 128 x 128 x 32 slab takes 1024 clocks of shared memory instead of 1536 (768 of the tensor core); measured 0.55 us a
+// slab.  Narrower tiles are bound by the latencies of their loops: each role asks for its next barrier before it works on the
+// current slab (a wait on a barrier long complete took 150 of the 700 clocks per slab), 0.34 us with 64 columns and 0.29
+// with 32 (0.60, 0.48, 0.43 us at first).  2001 x 1511 x 999: 60 -> 50 us; 16 x 4096 x 784:
 // 8.8 -> 7.5 us.  What is left per tile, 4 to 5 us, is set-up, the first slab's way through the pipeline and the store; the
 // exchange in a cluster runs at the 15 bytes per clock an SM gets from another SM's shared memory (pushing the parts
 // there instead of reading them was slower: 17.4 against 15.9 us at 1024^3).
@@ -56,8 +58,7 @@ namespace mid {
 using namespace tc;
 
 constexpr int BM = 128, BK = 32;
-constexpr int kSplitWarps = 8, kAccWarps = 8;
-constexpr int kThreads = 32 * (2 + kSplitWarps + kAccWarps);
+constexpr int kThreads = 32 * 18;
 constexpr uint32_t kBox = 32 * BK * 4;                      // one MN-major chunk of a slab: 32 elements x BK rows
 
 // Shared memory is a ring of raw slabs and a shorter ring of B's lo parts, in step with a ring of A's parts in tensor
@@ -65,14 +66,18 @@ constexpr uint32_t kBox = 32 * BK * 4;                      // one MN-major chun
 // products), the parts only from the split on, so the raw ring is what has to be deep: at 128 x 128 x 32 a slab's
 // products take 0.4 us.
 template <int BN> struct Cfg {
+  // Groups of four split warps that take the slabs in turn: a slab costs a warp 700 clocks of latencies (barriers, loads, the
+  // wait for its stores) whatever its width, more than the products of a narrow tile.
+  static constexpr int kGroups = BN == 32 ? 3 : 2, kSplitWarps = 4 * kGroups, kAccWarps = 16 - kSplitWarps;
   static constexpr uint32_t kABytes = BM * BK * 4, kBBytes = BN * BK * 4, kRawBytes = kABytes + kBBytes;
-  static constexpr int kRaw = BN == 128 ? 6 : BN == 64 ? 8 : 10, kLo = BN == 128 ? 2 : BN == 64 ? 4 : 6;
-  static_assert(kRaw % 2 == 0 && kLo % 2 == 0, "even slabs and odd slabs have split warps of their own");
+  static constexpr int kRaw = BN == 128 ? 6 : BN == 64 ? 8 : 9, kLo = BN == 128 ? 2 : BN == 64 ? 4 : 6;
+  static_assert(kRaw % kGroups == 0 && kLo % kGroups == 0, "a place of a ring belongs to one group");
   static constexpr uint32_t kLoBase = kRaw * kRawBytes;
   static constexpr uint32_t kTileBytes = kLoBase + kLo * kBBytes;
-  static constexpr uint32_t kSmemBytes = kTileBytes + 1024 + 256;
-  // tensor memory: two accumulators that take turns, A's parts
-  static constexpr uint32_t kABase = 2 * BN, kASlab = 2 * BK, kTmemCols = 512;
+  static constexpr uint32_t kBarBytes = 320, kSmemBytes = kTileBytes + 1024 + kBarBytes;
+  // tensor memory: accumulators that take turns, A's parts
+  static constexpr int kAccs = BN == 128 ? 2 : 4;
+  static constexpr uint32_t kABase = kAccs * BN, kASlab = 2 * BK, kTmemCols = 512;
   static_assert(kABase + kLo * kASlab <= kTmemCols, "tensor memory");
   static_assert(kSmemBytes <= 227 * 1024, "rings must fit shared memory");
   static_assert(BM * (BN + 4) * 4 <= (int)kTileBytes && BN * (BM + 4) * 4 <= (int)kTileBytes, "the tile must fit the rings");
@@ -153,7 +158,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_b3, const Params p) {
   using C = Cfg<BN>;
-  constexpr int kAccs = 2;
+  constexpr int kAccs = C::kAccs, kSplitWarps = C::kSplitWarps, kAccWarps = C::kAccWarps;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -166,7 +171,7 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   auto acc_empty = [&](int a) { return bars + 8u * (kRings + kAccs + a); };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + C::kTileBytes + 8 * (kRings + 2 * kAccs));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert(8 * (kRings + 2 * kAccs) + 8 <= 256, "barrier block");
+  static_assert(8 * (kRings + 2 * kAccs) + 8 <= (int)C::kBarBytes, "barrier block");
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const bool whole = blockIdx.x < p.whole;
@@ -183,7 +188,7 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   if (warp == 0) {
     if (lane < kBars) {
       const bool is_lo = lane >= 2 * C::kRaw && lane < kRings, is_acc_empty = lane >= kRings + kAccs;
-      mbar_init(bars + 8u * lane, is_lo ? (uint32_t)kSplitWarps / 2 : is_acc_empty ? (uint32_t)kAccWarps : 1u);
+      mbar_init(bars + 8u * lane, is_lo ? 4u : is_acc_empty ? (uint32_t)kAccWarps : 1u);
     }
     if (lane == 0) {
       *abort_flag = 0;
@@ -206,8 +211,11 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const bool leader = elect_one();
     {
       uint32_t s = 0, ph = 1;
+      bool free = true;
       for (uint32_t it = 0; it < mine; ++it) {
-        if (!mbar_wait(empty(s), ph, abort_flag, p.status, 111, p.wait_ns)) break;
+        if (!free && !mbar_wait(empty(s), ph, abort_flag, p.status, 111, p.wait_ns)) break;
+        const uint32_t s_next = s + 1 == C::kRaw ? 0 : s + 1, ph_next = s_next ? ph : ph ^ 1;
+        free = mbar_test(empty(s_next), ph_next);
         if (leader) {
           const uint32_t a = base + s * C::kRawBytes, b = a + C::kABytes;
           mbar_expect_tx(full_raw(s), C::kRawBytes);
@@ -222,7 +230,7 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             for (int c = 0; c < BN / 32; ++c) tma_load_2d(b + c * kBox, &map_b, full_raw(s), n0 + 32 * c, k0);
           }
         }
-        if (++s == C::kRaw) s = 0, ph ^= 1;
+        s = s_next, ph = ph_next;
       }
     }
   } else if (warp == 1) {
@@ -235,22 +243,25 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const uint32_t b_step = (p.b_mn ? 1024u : 32u) >> 4;
       // (in a cluster the upper bits of a shared address hold the CTA's rank; a descriptor has no room for them)
       const uint32_t ring = (base & 0x3FFFFu) >> 4;
-      uint32_t it = 0, s = 0, s_ph = 0, l = 0, l_ph = 0;    // slab; its place and phase in either ring
-      bool ok = true;
+      uint32_t it = 0, s = 0, l = 0, l_ph = 0;              // slab; its place in either ring
+      bool ok = true, split = false, drained = true;        // (the accumulators are empty at first)
       for (uint32_t c = 0; ok && c < chunks; ++c) {
         const int acc = c % kAccs;
-        ok = mbar_wait(acc_empty(acc), ((c / kAccs) & 1u) ^ 1u, abort_flag, p.status, 115, p.wait_ns);
+        ok = drained || mbar_wait(acc_empty(acc), ((c / kAccs) & 1u) ^ 1u, abort_flag, p.status, 115, p.wait_ns);
         if (!ok) break;
         tc_fence_after();
+        drained = mbar_test(acc_empty((c + 1) % kAccs), (((c + 1) / kAccs) & 1u) ^ 1u);
         const uint32_t d = tmem + acc * BN;
         const uint32_t last = it + p.chunk < mine ? it + p.chunk : mine;
         for (uint32_t accumulate = 0; it < last; ++it, accumulate = 1) {
           const uint32_t b_hi = ring + ((s * C::kRawBytes + C::kABytes) >> 4), b_lo = ring + ((C::kLoBase + l * C::kBBytes) >> 4);
           const uint32_t a_hi = tmem + C::kABase + l * C::kASlab, a_lo = a_hi + BK;
-          ok = mbar_wait(full_raw(s), s_ph, abort_flag, p.status, 112, p.wait_ns) &&
-               mbar_wait(full_lo(l), l_ph, abort_flag, p.status, 113, p.wait_ns);
+          // (the split warps have waited for the raw slab)
+          ok = split || mbar_wait(full_lo(l), l_ph, abort_flag, p.status, 113, p.wait_ns);
           if (!ok) break;
           tc_fence_after();
+          if (++l == C::kLo) l = 0, l_ph ^= 1;
+          split = mbar_test(full_lo(l), l_ph);
           if (leader) {
             // the small products first: what the accumulator cuts off is relative to what it holds
 #pragma unroll
@@ -262,23 +273,22 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             for (int kk = 0; kk < BK / 8; ++kk) tc_mma_tf32_ts(d, a_hi + 8 * kk, b_op, b_hi + kk * b_step, idesc, 1u);
             tc_commit(empty(s));
           }
-          if (++s == C::kRaw) s = 0, s_ph ^= 1;
-          if (++l == C::kLo) l = 0, l_ph ^= 1;
+          if (++s == C::kRaw) s = 0;
         }
         if (ok && leader) tc_commit(acc_full(acc));
       }
     }
   } else if (warp < 2 + kSplitWarps) {
-    // Four warps take the even slabs, four the odd ones: a slab costs a warp 700 clocks of latencies (barriers, loads,
-    // the wait for its stores) whatever its width, more than the products of a narrow tile.
     // A: a thread takes one row, the row being the tensor-memory lane its warp may write (warp mod 4).
     // B: vectors of the slab as they lie.
     const int tid = (threadIdx.x - 64) & 127, row = (warp & 3) * 32 + lane;
     constexpr int kVecs = C::kBBytes / 16 / 128 / 2;        // B's vectors of a thread, in two halves like A's 32 k
     static_assert(kVecs * 2 * 128 * 16 == C::kBBytes, "slab must divide over the split warps");
     uint32_t s = (warp - 2) >> 2, ph = 0, l = s, prev = s, prev_ph = 0;   // prev: the slab that used this place of the lo ring before
-    for (uint32_t it = s; it < mine; it += 2) {
-      if (!mbar_wait(full_raw(s), ph, abort_flag, p.status, 114, p.wait_ns)) break;
+    bool landed = false;
+    for (uint32_t it = s; it < mine; it += C::kGroups) {
+      const bool free = it < (uint32_t)C::kLo || mbar_test(empty(prev), prev_ph);
+      if (!landed && !mbar_wait(full_raw(s), ph, abort_flag, p.status, 114, p.wait_ns)) break;
       const uint8_t* slab = gen + s * C::kRawBytes;
       const float4* raw = reinterpret_cast<const float4*>(slab + C::kABytes) + tid;
       float4* lo = reinterpret_cast<float4*>(gen + C::kLoBase + l * C::kBBytes) + tid;
@@ -308,9 +318,9 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
         for (int i = 0; i < kVecs; ++i) v[i] = raw[(half * kVecs + i) * 128];
         if (half == 0 && it >= (uint32_t)C::kLo) {
-          ok = mbar_wait(empty(prev), prev_ph, abort_flag, p.status, 117, p.wait_ns);
+          ok = free || mbar_wait(empty(prev), prev_ph, abort_flag, p.status, 117, p.wait_ns);
           if (!ok) break;
-          if ((prev += 2) >= (uint32_t)C::kRaw) prev -= C::kRaw, prev_ph ^= 1;
+          if ((prev += C::kGroups) >= (uint32_t)C::kRaw) prev -= C::kRaw, prev_ph ^= 1;
           tc_fence_after();
         }
         const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::kABase + l * C::kASlab + half * 16;
@@ -326,18 +336,19 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           lo[(half * kVecs + i) * 128] = make_float4(low(v[i].x), low(v[i].y), low(v[i].z), low(v[i].w));
       }
       if (!ok) break;
+      if ((s += C::kGroups) >= (uint32_t)C::kRaw) s -= C::kRaw, ph ^= 1;
+      landed = mbar_test(full_raw(s), ph);
       fence_async_smem();
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(full_lo(l));               // one arrival per warp
-      if ((s += 2) >= (uint32_t)C::kRaw) s -= C::kRaw, ph ^= 1;
-      if ((l += 2) >= (uint32_t)C::kLo) l -= C::kLo;
+      if ((l += C::kGroups) >= (uint32_t)C::kLo) l -= C::kLo;
     }
   } else {
-    // four consecutive warps cover the 128 lanes, the two warps of a lane quarter half of the columns each
+    // four consecutive warps cover the 128 lanes; with eight, the two warps of a lane quarter take half of the columns each
     const int q = warp & 3, half = (warp - (2 + kSplitWarps)) >> 2;
-    constexpr int kCols = BN / 2;
+    constexpr int kCols = BN / (kAccWarps / 4);
     constexpr int kPart = kCols == 32 ? 32 : 16;             // columns in flight: what the register budget allows
     float acc[kCols];
 #pragma unroll
@@ -552,7 +563,7 @@ int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* 
   p.cluster = (uint32_t)cluster;
   p.whole = (uint32_t)whole;
   // slabs of 32 terms summed in tensor memory, the rest in registers: `exact` is to stay below the error of FFMA sums
-  p.chunk = !exact ? 8 : k < 512 ? 1 : 2;
+  p.chunk = !exact ? 8 : k < 512 || bn == 32 ? 1 : 2;
   if ((cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) || p.slabs < p.cluster) return fail(POLAR_B200_ERR_UNSUPPORTED, "fewer slabs than CTAs in a cluster");
   if ((uint64_t)p.tiles_m * ((p.n + bn - 1) / bn) * p.cluster > 0x7fffffffull) return fail(POLAR_B200_ERR_UNSUPPORTED, "too many tiles");
   // exchanged: right' plays the row operand - stored [k, n] is "row extent contiguous" - and left the column operand

@@ -35,6 +35,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Whether the phase is over, without waiting.  A wait on a barrier that is long complete still takes 150 clocks of latency; a
+// loop that asks for its next barrier before it starts on the current one hides them.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // The warp's number as a value the compiler knows to be the same for all lanes, and one lane of the warp.  A role that
 // issues tcgen05 or TMA instructions runs its loop on the WHOLE warp and only the instructions themselves on
 // one lane: their operands then live in uniform registers.  In a loop of a single lane every operand had to be moved
