@@ -22,6 +22,7 @@ int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* 
                int cluster, uint64_t whole, int exact, int swap, int epilogue, float* ws, cudaStream_t stream, uint64_t left_pitch = 0);
 int skinny_kind(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                 const float* right, const float* out);
+double small_n_estimate_us(uint64_t m, uint64_t n, uint64_t k);
 uint64_t skinny_workspace_bytes(int kind, uint64_t m, uint64_t n, uint64_t k);
 int launch_skinny(int kind, int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                   const float* right, float* out, float* ws, cudaStream_t st, const float* sig, int sigmoid_out = 0);
@@ -229,12 +230,12 @@ struct MidChoice {
   double us = 1e30;
 };
 
-MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact) {
+MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact, int orientations = 2, int widths = 3) {
   MidChoice best;
   const uint64_t sms = (uint64_t)sm_count(), slabs = (k + 31) / 32;
-  for (int swap = 0; swap < 2; ++swap) {
+  for (int swap = 0; swap < orientations; ++swap) {
     const uint64_t rows = swap ? n : m, cols = swap ? m : n;
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < widths; ++i) {
       const int bn = 32 << i;
       static const double slab_us[2][3] = {{0.29, 0.36, 0.56}, {0.40, 0.42, 0.63}};
       const uint64_t tiles = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
@@ -280,6 +281,19 @@ MidChoice mid_for_rest(uint64_t m, uint64_t n, uint64_t k, uint64_t pad_bytes) {
   return c;
 }
 
+// Up to 16 columns and a K-major left operand: tiles of 32 columns - half of them and more for nothing, but the row operand is
+// what takes the time, and the tensor core takes a slab of 128 rows in 0.4 us.  From a few hundred rows on the narrow
+// kernels are bound by the arithmetic and shared-memory reads of n columns per element (512 x 10 x 4096 25 against 13 us,
+// 2048 x 10 x 4096 47 against 19, 8192 x 16 x 4096 110 against 33); at the largest, and for n of 1 to 4, by memory, which they
+// read faster.  Sums of 32 in tensor memory and two levels of them in registers: as close to float64 as the narrow kernels.
+MidChoice mid_for_small_n(uint64_t m, uint64_t n, uint64_t k, uint64_t pad_bytes) {
+  MidChoice c = mid_choose(m, n, k, true, 1, 1);
+  // (with a wave or more of tiles the narrow kernel runs several groups of rows per warp, closer to the memory than estimated)
+  const double other = small_n_estimate_us(m, n, k) * (m > 128ull * sm_count() / 2 ? 0.9 : 1.0);
+  if (c.us + (pad_bytes ? 2.0 + (double)pad_bytes * 2.0 / 4e6 : 0.0) >= other) c.bn = 0;
+  return c;
+}
+
 int check_mm(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
              const float* right, float* out) {
   if ((tl != 0 && tl != 1) || (tr != 0 && tr != 1))
@@ -304,6 +318,10 @@ extern "C" {
 static uint64_t workspace_need(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, int fused, bool pitched = false) {
   const float* al = reinterpret_cast<const float*>(256);   // allocator buffers are 256-byte aligned
   int kind = skinny_kind(tl, tr, m, n, k, al, al, al);
+  if (kind == 1) {
+    const uint64_t pad = mid_workspace_bytes(tl, tr, m, n, k, al, al);
+    if (mid_for_small_n(m, n, k, pad).bn) return pad;
+  }
   if (kind) return skinny_workspace_bytes(kind, m, n, k);
   if (choose_path(tl, tr, m, n, k, al, al, al) == kPathTc) {
     const uint64_t rem = ragged_rows(tl, tr, m, n, k, al, fused == 1 ? 1 : 0);
@@ -480,9 +498,10 @@ static int fmatmul_impl(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, cons
                       : polar_b200_fsigmoid_grad(out, sig, out, m * n, stream);
   }
   const int path = choose_path(tl, tr, m, n, k, left, right, out);
-  if (path == kPathFfma && fused != 2) {
+  const int kind0 = path == kPathSkinny ? skinny_kind(tl, tr, m, n, k, left, right, out) : 0;
+  if ((path == kPathFfma || kind0 == 1) && fused != 2) {
     const uint64_t pad = mid_workspace_bytes(tl, tr, m, n, k, left, right);
-    const MidChoice mid = mid_for_rest(m, n, k, pad);
+    const MidChoice mid = kind0 == 1 ? mid_for_small_n(m, n, k, pad) : mid_for_rest(m, n, k, pad);
     if (mid.bn) {
       // What the workspace query promised is for aligned base pointers; other pointers may need more copies than that,
       // for which the library's own scratch steps in.
@@ -491,7 +510,7 @@ static int fmatmul_impl(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, cons
         return fail(POLAR_B200_ERR_WORKSPACE, "workspace too small or not 16-byte aligned");
       void *ws = workspace, *own = nullptr;
       if (pad && (!workspace || workspace_bytes < pad)) {
-        // (no memory for the copies: the FFMA kernel below needs none)
+        // (no memory for the copies: the kernels below need none)
         if (scratch_alloc(&own, pad, as_stream(stream)) != cudaSuccess) cudaGetLastError();
         ws = own;
       }
@@ -506,7 +525,6 @@ static int fmatmul_impl(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, cons
       }
     }
   }
-  const int kind0 = path == kPathSkinny ? skinny_kind(tl, tr, m, n, k, left, right, out) : 0;
   const bool fused_in_kernel = (fused == 1 && (path == kPathTc || kind0 == 1)) || (fused == 2 && kind0 == 3);
   if (fused != 0 && !fused_in_kernel) {
     rc = fmatmul_impl(tl, tr, m, n, k, left, right, out, workspace, workspace_bytes, stream, 0, nullptr);
@@ -518,7 +536,7 @@ static int fmatmul_impl(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, cons
     case kPathTc:
       return tc_path(tl, tr, m, n, k, left, right, out, workspace, workspace_bytes, stream, fused, 0);
     case kPathSkinny: {
-      const int kind = skinny_kind(tl, tr, m, n, k, left, right, out);
+      const int kind = kind0;
       const uint64_t need = skinny_workspace_bytes(kind, m, n, k);
       if (need == 0)
         return launch_skinny(kind, tl, tr, m, n, k, left, right, out, nullptr, as_stream(stream),

@@ -805,6 +805,22 @@ int skinny_kind(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float*
   return 0;
 }
 
+// What kind 1 (small n, K-major left) takes in microseconds, fitted to measurements on B200 (n = 1 ... 16, k = 128 ... 8192,
+// 64 ... 32768 rows; within a third).  Up to 1024 rows the row kernel is a chain of latencies, longer with n and k; the
+// resident kernel takes 64 rows per SM at a time; without room for the small operand every CTA reads it again per 32 rows.
+double small_n_estimate_us(uint64_t m, uint64_t n, uint64_t k) {
+  const uint64_t np = n <= 1 ? 1 : n <= 4 ? 4 : n <= 8 ? 8 : n <= 10 ? 10 : 16;
+  const double kd = (double)k, nd = (double)n, md = (double)m;
+  if (m >= skinny::kResidentRows && np * (k + 4) * sizeof(float) <= 200 * 1024) {
+    const uint64_t at_once = 64ull * (uint64_t)sm_count();
+    const double passes = (double)((m + at_once - 1) / at_once) * kd / 4096 * (n <= 10 ? 10.0 + 2.0 * nd : 3.6 * nd);
+    const double memory = md * kd * 4e-6 / 6.2;
+    return 4.0 + (passes > memory ? passes : memory);
+  }
+  const double latency = 6.3e-7 * kd * (nd + 3.5) * (m < 1024 ? md : 1024.0), work = 2e-7 * kd * (nd + 3.5) * md;
+  return 4.0 + (latency > work ? latency : work);
+}
+
 uint64_t skinny_workspace_bytes(int kind, uint64_t m, uint64_t n, uint64_t k) {
   if (kind != 2) return 0;
   uint32_t s = skinny::splits_for(m, k);

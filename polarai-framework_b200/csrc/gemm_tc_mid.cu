@@ -350,9 +350,15 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const int q = warp & 3, half = (warp - (2 + kSplitWarps)) >> 2;
     constexpr int kCols = BN / (kAccWarps / 4);
     constexpr int kPart = kCols == 32 ? 32 : 16;             // columns in flight: what the register budget allows
-    float acc[kCols];
+    // 32-column tiles have registers for a second level: sums of 16 chunks are added up separately
+    constexpr bool kTwoLevels = BN == 32;
+    float acc[kCols], sum[kTwoLevels ? kCols : 1];
 #pragma unroll
     for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
+    if (kTwoLevels) {
+#pragma unroll
+      for (int j = 0; j < kCols; ++j) sum[j] = 0.f;
+    }
     bool ok = true;
     for (uint32_t c = 0; c < chunks; ++c) {
       const int a = c % kAccs;
@@ -368,6 +374,11 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < kPart; ++j) acc[j0 + j] += __uint_as_float(r[j]);
+      }
+      if (kTwoLevels && ((c & 15u) == 15u || c + 1 == chunks)) {
+        const bool last = c + 1 == chunks;
+#pragma unroll
+        for (int j = 0; j < kCols; ++j) sum[j] += acc[j], acc[j] = last ? sum[j] : 0.f;
       }
       tc_fence_before();
       __syncwarp();
@@ -562,6 +573,7 @@ int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* 
   p.slabs = (uint32_t)((k + BK - 1) / BK);
   p.cluster = (uint32_t)cluster;
   p.whole = (uint32_t)whole;
+  // (32-column tiles replace the narrow kernels too, whose sums are better than FFMA tiles')
   // slabs of 32 terms summed in tensor memory, the rest in registers: `exact` is to stay below the error of FFMA sums
   p.chunk = !exact ? 8 : k < 512 || bn == 32 ? 1 : 2;
   if ((cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) || p.slabs < p.cluster) return fail(POLAR_B200_ERR_UNSUPPORTED, "fewer slabs than CTAs in a cluster");
