@@ -23,6 +23,7 @@ int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* 
 int skinny_kind(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                 const float* right, const float* out);
 double small_n_estimate_us(uint64_t m, uint64_t n, uint64_t k);
+double small_tn_estimate_us(uint64_t m, uint64_t n, uint64_t k);
 uint64_t skinny_workspace_bytes(int kind, uint64_t m, uint64_t n, uint64_t k);
 int launch_skinny(int kind, int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                   const float* right, float* out, float* ws, cudaStream_t st, const float* sig, int sigmoid_out = 0);
@@ -286,10 +287,13 @@ MidChoice mid_for_rest(uint64_t m, uint64_t n, uint64_t k, uint64_t pad_bytes) {
 // kernels are bound by the arithmetic and shared-memory reads of n columns per element (512 x 10 x 4096 25 against 13 us,
 // 2048 x 10 x 4096 47 against 19, 8192 x 16 x 4096 110 against 33); at the largest, and for n of 1 to 4, by memory, which they
 // read faster.  Sums of 32 in tensor memory and two levels of them in registers: as close to float64 as the narrow kernels.
-MidChoice mid_for_small_n(uint64_t m, uint64_t n, uint64_t k, uint64_t pad_bytes) {
+// kind 2, an MN-major left operand: only where its rows are no vectors, since fdense_grad gives the bits of the narrow kernel
+// wherever they are.
+MidChoice mid_for_small_n(int kind, uint64_t m, uint64_t n, uint64_t k, uint64_t pad_bytes) {
+  if (kind == 2 && ((m & 3) == 0 || k < 512)) return MidChoice{};
   MidChoice c = mid_choose(m, n, k, true, 1, 1);
   // (with a wave or more of tiles the narrow kernel runs several groups of rows per warp, closer to the memory than estimated)
-  const double other = small_n_estimate_us(m, n, k) * (m > 128ull * sm_count() / 2 ? 0.9 : 1.0);
+  const double other = kind == 2 ? small_tn_estimate_us(m, n, k) : small_n_estimate_us(m, n, k) * (m > 128ull * sm_count() / 2 ? 0.9 : 1.0);
   if (c.us + (pad_bytes ? 2.0 + (double)pad_bytes * 2.0 / 4e6 : 0.0) >= other) c.bn = 0;
   return c;
 }
@@ -318,9 +322,9 @@ extern "C" {
 static uint64_t workspace_need(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, int fused, bool pitched = false) {
   const float* al = reinterpret_cast<const float*>(256);   // allocator buffers are 256-byte aligned
   int kind = skinny_kind(tl, tr, m, n, k, al, al, al);
-  if (kind == 1) {
+  if (kind == 1 || kind == 2) {
     const uint64_t pad = mid_workspace_bytes(tl, tr, m, n, k, al, al);
-    if (mid_for_small_n(m, n, k, pad).bn) return pad;
+    if (mid_for_small_n(kind, m, n, k, pad).bn) return pad;
   }
   if (kind) return skinny_workspace_bytes(kind, m, n, k);
   if (choose_path(tl, tr, m, n, k, al, al, al) == kPathTc) {
@@ -499,9 +503,9 @@ static int fmatmul_impl(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, cons
   }
   const int path = choose_path(tl, tr, m, n, k, left, right, out);
   const int kind0 = path == kPathSkinny ? skinny_kind(tl, tr, m, n, k, left, right, out) : 0;
-  if ((path == kPathFfma || kind0 == 1) && fused != 2) {
+  if ((path == kPathFfma || kind0 == 1 || kind0 == 2) && fused != 2) {
     const uint64_t pad = mid_workspace_bytes(tl, tr, m, n, k, left, right);
-    const MidChoice mid = kind0 == 1 ? mid_for_small_n(m, n, k, pad) : mid_for_rest(m, n, k, pad);
+    const MidChoice mid = kind0 ? mid_for_small_n(kind0, m, n, k, pad) : mid_for_rest(m, n, k, pad);
     if (mid.bn) {
       // What the workspace query promised is for aligned base pointers; other pointers may need more copies than that,
       // for which the library's own scratch steps in.

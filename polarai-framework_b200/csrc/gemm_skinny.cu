@@ -821,6 +821,14 @@ double small_n_estimate_us(uint64_t m, uint64_t n, uint64_t k) {
   return 4.0 + (latency > work ? latency : work);
 }
 
+// The same for kind 2 (small n, MN-major left), its summing kernel included.
+double small_tn_estimate_us(uint64_t m, uint64_t n, uint64_t k) {
+  const double width = (double)(m < 1024 ? m : 1024) * (double)n;
+  double doublings = 0;
+  for (uint64_t v = k; v > 128; v >>= 1) doublings += 1;
+  return 3.5 + 4e-4 * width + (1.4 + 3.6e-4 * width) * doublings + 0.5 * (double)m * (double)k * 4e-6 / 6.2;
+}
+
 uint64_t skinny_workspace_bytes(int kind, uint64_t m, uint64_t n, uint64_t k) {
   if (kind != 2) return 0;
   uint32_t s = skinny::splits_for(m, k);

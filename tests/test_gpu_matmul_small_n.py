@@ -34,3 +34,28 @@ def test_few_columns(m, n, k, tr):
     d.fsigmoid(out, both)
     assert torch.equal(act, both)
     assert d.device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(514, 7, 999), (1001, 10, 2000), (130, 16, 8192), (33, 3, 512), (2049, 16, 700), (514, 10, 300)])
+@pytest.mark.parametrize("tr", [0, 1])
+def test_few_columns_of_rows_that_are_no_vectors(m, n, k, tr):
+    import torch
+    import __graft_entry__ as ge
+    ge.load_package()
+    from polarai_framework_b200.device_builtins import DeviceBuiltins
+    d = DeviceBuiltins()
+    g = torch.Generator(device="cuda").manual_seed(m + n + k + tr)
+    left = torch.empty((k, m), device="cuda").uniform_(-1, 1, generator=g)
+    right = torch.empty((n, k) if tr else (k, n), device="cuda").uniform_(-1, 1, generator=g)
+    r = (right.t() if tr else right).double()
+    ref = left.double().t() @ r
+    out = torch.full((m, n), float("nan"), device="cuda")
+    d.fmatmul(1, tr, left, right, out)
+    assert float((out.double() - ref).norm() / ref.norm()) <= 3e-7
+    need = int(d.lib.cdll.polar_b200_fmatmul_workspace_bytes(1, tr, m, n, k))
+    ws = torch.empty(need + 16, dtype=torch.uint8, device="cuda")
+    again = torch.full((m, n), float("nan"), device="cuda")
+    rc = d.lib.cdll.polar_b200_fmatmul(1, tr, m, n, k, left.data_ptr(), right.data_ptr(), again.data_ptr(), ws.data_ptr(), need,
+                                       torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and torch.equal(out, again)
+    assert d.device_status() == 0
