@@ -659,8 +659,11 @@ dense_grad_kernel(const float* __restrict__ H, const float* __restrict__ dz, con
 inline int round_np(uint64_t n) { return n <= 1 ? 1 : n <= 2 ? 2 : n <= 4 ? 4 : n <= 8 ? 8 : n <= 10 ? 10 : 16; }
 
 // Into how many parts the k range of a small-n product with M-contiguous left is cut: about two CTAs per SM, parts of at
-// least KS rows - or of 16, as long as parts of KS rows leave SMs without a CTA.
-uint32_t splits_for(uint64_t m, uint64_t k) {
+// least KS rows - or of 32, as long as the partial sums stay below the 16 MiB that the entry point with built-in scratch
+// has (fdense_grad with 4096 columns and 10 outputs: 64 parts of 128 rows left 40 SMs with one CTA at 8192 rows, 16 parts the
+// chip half empty at 2048; the step of such a network 208 -> 202 us and 108 -> 102, at 4096 rows 149 -> 132) - or of 16, as
+// long as parts of KS rows leave SMs without a CTA.  n = 0: parts of KS rows.
+uint32_t splits_for(uint64_t m, uint64_t k, uint64_t n) {
   uint64_t m_blocks = (m + 4 * kThreads - 1) / (4 * kThreads);
   if (m_blocks < 1) m_blocks = 1;
   uint64_t want = ((uint64_t)sm_count() * 2 + m_blocks - 1) / m_blocks;   // about two CTAs per SM
@@ -672,6 +675,13 @@ uint32_t splits_for(uint64_t m, uint64_t k) {
     if (k <= kClusterRows) max_by_k = max_by_k < 8 ? max_by_k : 8;
   }
   uint64_t s = want < max_by_k ? want : max_by_k;
+  if (n && k > 8 * KS) {
+    const uint64_t by_scratch = (16ull << 20) / (m * n * sizeof(float)), fine = (k + 31) / 32;
+    uint64_t finer = want < fine ? want : fine;
+    if (finer > by_scratch) finer = by_scratch;
+    if (finer > KS) finer = KS;              // (the error of a sum of sums grows with the longer of the two)
+    if (finer > s) s = finer;
+  }
   if (s < 1) s = 1;
   if (s > 4096) s = 4096;
   return (uint32_t)s;
@@ -764,13 +774,13 @@ int launch_dense_grad_np(const float* H, const float* dz, const float* W, float*
 // `rem` rows of a t_f product, as the small-n product right^T . left_tail stored transposed.
 // Scratch: ragged_rows_workspace_bytes.  n a multiple of 4, right 16-byte aligned.
 uint64_t ragged_rows_workspace_bytes(uint64_t rem, uint64_t n, uint64_t k) {
-  return (uint64_t)skinny::splits_for(n, k) * n * rem * sizeof(float);
+  return (uint64_t)skinny::splits_for(n, k, 0) * n * rem * sizeof(float);
 }
 
 int launch_ragged_rows(const float* left_tail, uint64_t left_pitch, const float* right, float* out_tail,
                        float* ws, uint64_t rem, uint64_t n, uint64_t k, cudaStream_t st) {
   using namespace skinny;
-  const uint32_t splits = splits_for(n, k);
+  const uint32_t splits = splits_for(n, k, 0);
   uint64_t m_blocks = (n / 4 + kThreads - 1) / kThreads;
   uint64_t k_per_split = (k + splits - 1) / splits;
   k_per_split = (k_per_split + 3) & ~3ull;
@@ -831,7 +841,7 @@ double small_tn_estimate_us(uint64_t m, uint64_t n, uint64_t k) {
 
 uint64_t skinny_workspace_bytes(int kind, uint64_t m, uint64_t n, uint64_t k) {
   if (kind != 2) return 0;
-  uint32_t s = skinny::splits_for(m, k);
+  uint32_t s = skinny::splits_for(m, k, n);
   if (skinny::sum_in_cluster(k, n, s)) return 0;
   return s > 1 ? (uint64_t)s * m * n * sizeof(float) : 0;
 }
@@ -844,7 +854,7 @@ int launch_skinny(int kind, int tl, int tr, uint64_t m, uint64_t n, uint64_t k, 
   const uint64_t rsk = tr ? 1 : n, rsj = tr ? k : 1;
   if (kind == 1 || kind == 2) {
     const int np = round_np(n);
-    const uint32_t splits = kind == 2 ? splits_for(m, k) : 1;
+    const uint32_t splits = kind == 2 ? splits_for(m, k, n) : 1;
 #define POLAR_SKINNY_N(NP)                                                                   \
   case NP:                                                                                   \
     return kind == 1 ? launch_small_n_k<NP>(left, right, out, m, n, k, rsk, rsj, st, sigmoid_out) \
@@ -884,13 +894,13 @@ bool dense_grad_ok(uint64_t rows, uint64_t kh, uint64_t n, const float* H, const
   return n >= 1 && n <= 16 && rows >= 32 && kh >= 32 && (kh & 3) == 0 && aligned16(H) && aligned16(din);
 }
 uint64_t dense_grad_workspace_bytes(uint64_t rows, uint64_t kh, uint64_t n) {
-  const uint32_t s = skinny::splits_for(kh, rows);
+  const uint32_t s = skinny::splits_for(kh, rows, n);
   return s > 1 ? (uint64_t)s * kh * n * sizeof(float) : 0;
 }
 int launch_dense_grad(const float* H, const float* dz, const float* W, float* din, float* dw, float* ws,
                       uint64_t rows, uint64_t kh, uint64_t n, cudaStream_t st) {
   using namespace skinny;
-  const uint32_t splits = splits_for(kh, rows);
+  const uint32_t splits = splits_for(kh, rows, n);
   switch (round_np(n)) {
 #define POLAR_DENSE(NP) case NP: return launch_dense_grad_np<NP>(H, dz, W, din, dw, ws, splits, rows, kh, n, st);
     POLAR_DENSE(1) POLAR_DENSE(2) POLAR_DENSE(4) POLAR_DENSE(8) POLAR_DENSE(10) POLAR_DENSE(16)
