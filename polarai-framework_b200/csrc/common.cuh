@@ -164,6 +164,13 @@ __device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
   return v;
 }
+__device__ __forceinline__ double ld_cluster(const double* p, uint32_t rank) {
+  uint32_t remote;
+  double v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(remote) : "memory");
+  return v;
+}
 
 // fsigmoid's arithmetic, shared by the elementwise builtin and the fused matmul
 // epilogue so that both give the same bits: r = 1/(1+exp(-x)), then the reference's

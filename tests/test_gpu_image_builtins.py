@@ -51,3 +51,15 @@ def test_softmax_and_relu_sizes(gpu, oracle, n):
     lib.call("polar_b200_fsoftmax", X.data_ptr(), out.data_ptr(), n, ws.data_ptr(), 8, st)   # the smallest workspace it takes
     assert np.max(np.abs(out.cpu().numpy() - want) / want) <= 1e-5
     assert np.array_equal(bits(gpu.frelu(x)), bits(oracle.frelu(x)))
+
+
+@pytest.mark.parametrize("n", [31, 8191, 8193, 32_769, 262_143, 262_144, 262_145, 262_149])
+def test_softmax_around_the_limit_of_one_cluster(gpu, n):
+    import torch
+    x = np.random.default_rng(n).uniform(-4, 4, n).astype(np.float32)
+    e = np.exp(x.astype(np.float64))
+    want = e / e.sum()
+    X = torch.from_numpy(x).cuda()
+    st = torch.cuda.current_stream().cuda_stream
+    gpu.d.lib.call("polar_b200_fsoftmax", X.data_ptr(), X.data_ptr(), n, None, 0, st)       # in place
+    assert np.max(np.abs(X.cpu().numpy() - want) / want) <= 1e-5
