@@ -480,7 +480,11 @@ small_k_kernel(const float* __restrict__ left, const float* __restrict__ right, 
                uint64_t rsj, int vec_store, const float* __restrict__ sig) {
   __shared__ float as[RK][KP];
   pdl_enter();
-  const uint64_t j0 = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
+  // Four columns per thread: one vector, or - rows that are no vectors - a column out of each quarter of the warp's 128, so
+  // that a warp's scalar stores are consecutive (the MLP step 2000 x 77 x 1001 x 10, with one such product, 79 -> 68 us)
+  const bool vec = vec_store;                // (n is a multiple of four then)
+  const uint64_t j0 = (uint64_t)blockIdx.x * kThreads * 4 + (vec ? threadIdx.x * 4u : (threadIdx.x >> 5) * 128u + (threadIdx.x & 31));
+  const uint32_t step = vec ? 1 : 32;
   // Each thread's four columns of the small operand stay in registers while the CTA walks
   // over row blocks (gridDim.y CTAs share the rows of one column block).
   float b[4][KP];
@@ -488,8 +492,7 @@ small_k_kernel(const float* __restrict__ left, const float* __restrict__ right, 
   for (int c = 0; c < 4; ++c)
 #pragma unroll
     for (int kk = 0; kk < KP; ++kk)
-      b[c][kk] = (j0 + c < n && (uint64_t)kk < k) ? right[(uint64_t)kk * rsk + (j0 + c) * rsj] : 0.f;
-  const bool vec = vec_store && j0 + 4 <= n;
+      b[c][kk] = (j0 + c * step < n && (uint64_t)kk < k) ? right[(uint64_t)kk * rsk + (j0 + c * step) * rsj] : 0.f;
   // The gridDim.y CTAs of a column block split the rows evenly (contiguous ranges, a multiple
   // of four rows each) and stage them RK at a time.
   const uint64_t rows_per_cta = ((m + gridDim.y - 1) / gridDim.y + 3) & ~3ull;
@@ -519,9 +522,9 @@ small_k_kernel(const float* __restrict__ left, const float* __restrict__ right, 
             sv[u] = __ldcs(reinterpret_cast<const float4*>(sp));
           } else {
             sv[u].x = sp[0];
-            sv[u].y = (j0 + 1 < n) ? sp[1] : 0.f;
-            sv[u].z = (j0 + 2 < n) ? sp[2] : 0.f;
-            sv[u].w = (j0 + 3 < n) ? sp[3] : 0.f;
+            sv[u].y = (j0 + 32 < n) ? sp[32] : 0.f;
+            sv[u].z = (j0 + 64 < n) ? sp[64] : 0.f;
+            sv[u].w = (j0 + 96 < n) ? sp[96] : 0.f;
           }
         }
       }
@@ -548,9 +551,9 @@ small_k_kernel(const float* __restrict__ left, const float* __restrict__ right, 
           __stcs(reinterpret_cast<float4*>(dst), make_float4(c0, c1, c2, c3));
         } else {
           dst[0] = c0;
-          if (j0 + 1 < n) dst[1] = c1;
-          if (j0 + 2 < n) dst[2] = c2;
-          if (j0 + 3 < n) dst[3] = c3;
+          if (j0 + 32 < n) dst[32] = c1;
+          if (j0 + 64 < n) dst[64] = c2;
+          if (j0 + 96 < n) dst[96] = c3;
         }
       }
     }
