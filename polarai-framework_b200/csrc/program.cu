@@ -3,6 +3,8 @@
 // What a small program costs is not its arithmetic but its launches: on B200 about 2.5 us of host time
 // each and 3 us of GPU time from one short kernel to the next.  Two things take them out:
 //
+//  - Two neighbouring short chains (or single elementwise builtins) over different element counts share a launch where
+//    neither touches what the other writes.
 //  - Consecutive elementwise builtins over the same element count become ONE launch (chain_kernel): each
 //    thread carries four elements through the whole chain.  Every tensor a builtin of the chain names as its
 //    result is still written, with the bits its own launch gives; what goes away is reading a
@@ -52,6 +54,12 @@ struct ChainParams {
   ChainOp op[kChainOps];
 };
 
+template <int CHAINS>
+struct ChainLaunch {
+  ChainParams chain[CHAINS];
+  uint32_t first_blocks;
+};
+
 template <class Op>
 __device__ __forceinline__ float4 map4(Op op, float4 a, float4 b) {
   return make_float4(op(a.x, b.x), op(a.y, b.y), op(a.z, b.z), op(a.w, b.w));
@@ -64,10 +72,15 @@ __device__ __forceinline__ float4 map4(Op op, float4 a, float4 b) {
 // is no barrier, and consecutive lanes touch consecutive 16 bytes.
 // Measured, four-builtin chain, 32 bytes per element: 2^20 elements 18.4 us as four launches, 6.6 us as one;
 // 2^25 elements 158 us, 6.8 TB/s.
-__global__ void __launch_bounds__(kChainThreads) chain_kernel(const __grid_constant__ ChainParams p) {
+// CHAINS == 2: two short chains of different lengths that have nothing to do with each other, as the updates of two layers'
+// weights; the second one's blocks follow the first one's.  (The step 999 x 301 x 514 x 7 55.0 -> 53.7 us.)
+template <int CHAINS>
+__global__ void __launch_bounds__(kChainThreads) chain_kernel(const __grid_constant__ ChainLaunch<CHAINS> l) {
   extern __shared__ float4 slots[];
   pdl_enter();
-  const uint64_t e0 = ((uint64_t)blockIdx.x * kChainThreads + threadIdx.x) * 4;
+  const bool second = CHAINS == 2 && blockIdx.x >= l.first_blocks;
+  const ChainParams& p = l.chain[second];
+  const uint64_t e0 = ((uint64_t)(blockIdx.x - (second ? l.first_blocks : 0u)) * kChainThreads + threadIdx.x) * 4;
   if (e0 >= p.n) return;
   const bool full = e0 + 4 <= p.n;
   const int left = full ? 4 : (int)(p.n - e0);             // the last vector of an n that is no multiple of four
@@ -131,9 +144,9 @@ struct Op {                    // one builtin, its argument list owned by the pr
   std::vector<polar_b200_arg> args;
   std::vector<std::vector<uint64_t>> shapes;
 };
-struct Step {                  // one builtin, or a chain
+struct Step {                  // one builtin, a chain, or two chains
   int op = -1;
-  ChainParams chain;
+  ChainParams chain = {}, second = {};   // (one elementwise builtin is a chain of one, for pairing)
   size_t smem = 0;
 };
 struct Program {
@@ -291,18 +304,41 @@ private:
   std::vector<Entry> ops_;
 };
 
+// Whether two chains are short - longer ones outlast a launch, and a single builtin's own kernel has more loads in
+// flight - and neither touches a tensor that the other one writes: then their order does not matter.
+constexpr uint64_t kPairElements = 1ull << 19;
+bool may_pair(const ChainParams& a, const ChainParams& b) {
+  if (a.n > kPairElements || b.n > kPairElements) return false;
+  auto writes_into = [](const ChainParams& w, const ChainParams& o) {
+    for (uint32_t i = 0; i < w.ops; ++i) {
+      auto hits = [&](const float* t, uint64_t n) { return t && w.op[i].out < t + n && t < w.op[i].out + w.n; };
+      for (uint32_t j = 0; j < o.inputs; ++j)
+        if (hits(o.in[j], o.n)) return true;
+      for (uint32_t j = 0; j < o.ops; ++j)
+        if (hits(o.op[j].out, o.n) || hits(o.op[j].scalar, 1)) return true;
+    }
+    return false;
+  };
+  return !writes_into(a, b) && !writes_into(b, a);
+}
+
 void plan(Program* p) {
   ChainBuilder chain;
   int first = -1;                                          // the builtin a one-instruction chain stands for
   auto flush = [&] {
-    if (chain.size() == 1) {
-      Step s;
-      s.op = first;
-      p->steps.push_back(s);
-      chain = ChainBuilder();
-    } else if (chain.size() > 1) {
-      p->steps.push_back(chain.finish());
+    if (chain.size() == 0) return;
+    Step s = chain.finish();
+    if (s.chain.ops == 1) s.op = first;                    // (its own kernel, unless it finds a partner)
+    if (!p->steps.empty()) {
+      Step& last = p->steps.back();
+      if (last.chain.ops && !last.second.ops && may_pair(last.chain, s.chain)) {
+        last.op = -1;
+        last.second = s.chain;
+        if (s.smem > last.smem) last.smem = s.smem;
+        return;
+      }
     }
+    p->steps.push_back(s);
   };
   for (size_t i = 0; i < p->ops.size(); ++i) {
     Elementwise e;
@@ -328,9 +364,13 @@ int run_steps(Program* p, cudaStream_t stream) {
       const Op& op = p->ops[s.op];
       rc = polar_b200_launch_by_name(op.name.c_str(), op.args.data(), op.args.size(), p->workspace, p->workspace_bytes, stream);
     } else {
-      const uint64_t vectors = (s.chain.n + 3) / 4, grid = (vectors + kChainThreads - 1) / kChainThreads;
-      if (grid > 0x7fffffffull) return fail(POLAR_B200_ERR_INVALID, "element count too large");
-      rc = launch("chain of elementwise builtins", chain_kernel, (unsigned)grid, kChainThreads, s.smem, stream, s.chain);
+      auto blocks = [](uint64_t n) { return ((n + 3) / 4 + kChainThreads - 1) / kChainThreads; };
+      const uint64_t first = blocks(s.chain.n), second = s.second.ops ? blocks(s.second.n) : 0;
+      if (first + second > 0x7fffffffull) return fail(POLAR_B200_ERR_INVALID, "element count too large");
+      rc = second ? launch("two chains of elementwise builtins", chain_kernel<2>, (unsigned)(first + second), kChainThreads, s.smem,
+                           stream, ChainLaunch<2>{{s.chain, s.second}, (uint32_t)first})
+                  : launch("chain of elementwise builtins", chain_kernel<1>, (unsigned)first, kChainThreads, s.smem, stream,
+                           ChainLaunch<1>{{s.chain}, (uint32_t)first});
     }
     if (rc) return rc;
   }
