@@ -56,12 +56,12 @@ __device__ __forceinline__ void store_row_sums(const float (&acc)[ROWS_PER_WARP]
 }
 
 // Puts kt x n elements of the small operand into shared memory as [n][pitch], k contiguous.  Read in the order they are
-// stored in - whole lines - and kBatch at a time: one element per trip was one memory latency per trip, 15 us for the
-// 4096 x 10 of the MLP's output layer; eight, 7.  NP: columns the kernel is made for; few of them are staged in one trip as it is.
-template <int THREADS, int NP>
+// stored in - whole lines - and eight at a time: one element per trip was one memory latency per trip, 15 us for the
+// 4096 x 10 of the MLP's output layer.
+template <int THREADS>
 __device__ __forceinline__ void stage_small_operand(const float* __restrict__ right, float* bs, int kt, int n, int pitch,
                                                     uint64_t rsk, uint64_t rsj) {
-  constexpr int kBatch = NP >= 8 ? 20 : 8;   // (20: an eighth of 4096 x 10 over 256 threads in one trip)
+  constexpr int kBatch = 8;
   const bool by_k = rsk == 1;
   const uint32_t inner = by_k ? kt : n, total = (uint32_t)kt * (uint32_t)n;
   const uint32_t step_out = THREADS / inner, step_in = THREADS % inner;
@@ -120,7 +120,7 @@ small_n_rows_kernel(const float* __restrict__ left, const float* __restrict__ ri
   for (uint64_t k0 = kbeg; k0 < kend; k0 += KT) {
     const int kt = (int)((kend - k0 < KT) ? (kend - k0) : KT);
     __syncthreads();
-    stage_small_operand<kThreads, NP>(right + k0 * rsk, bs, kt, (int)n, KT_PAD, rsk, rsj);
+    stage_small_operand<kThreads>(right + k0 * rsk, bs, kt, (int)n, KT_PAD, rsk, rsj);
     __syncthreads();
     if (VEC) {
       for (int kk = (half * 32 + lane) * 4; kk < kt; kk += 256) {
@@ -231,7 +231,7 @@ small_n_kmajor_resident_kernel(const float* __restrict__ left, const float* __re
   if (n < NP)
     for (uint32_t e = threadIdx.x; e < (NP - (uint32_t)n) * (uint32_t)k; e += kResidentThreads)
       bs[((uint32_t)n + e / (uint32_t)k) * kpad + e % (uint32_t)k] = 0.f;
-  stage_small_operand<kResidentThreads, NP>(right, bs, (int)k, (int)n, (int)kpad, rsk, rsj);
+  stage_small_operand<kResidentThreads>(right, bs, (int)k, (int)n, (int)kpad, rsk, rsj);
   __syncthreads();
   for (; g < groups; g += warps_total) {
     const uint64_t row0 = g * ROWS_PER_WARP;
