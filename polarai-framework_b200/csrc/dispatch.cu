@@ -175,8 +175,9 @@ TcChoice tc_choose(uint64_t m, uint64_t n, uint64_t k, bool may_swap) {
         if (mt == 2 && rows < 256) continue;
         for (uint32_t splits = 0; splits <= 8; ++splits) {
           if (splits == 0 && (swap || tc_workspace_bytes(rows, cols, k, 0, mt) == 0)) continue;
-          // a unit of eight slabs at least, partial products of 256 MiB at most
-          if (splits > 1 && (k < 128 * splits || splits * m * n > (64ull << 20))) break;
+          // a unit of eight slabs at least, partial products of 256 MiB at most, and whole vectors of them: the summing
+          // kernel reads each at a stride of m * n / 4 vectors
+          if (splits > 1 && (k < 128 * splits || splits * m * n > (64ull << 20) || ((m * n) & 3) != 0)) break;
           const TcChoice c{mt, swap, splits};
           const double est = tc_estimate_us(m, n, k, c);
           if (best_est == 0.0 || est < best_est) {

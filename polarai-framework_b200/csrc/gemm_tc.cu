@@ -865,6 +865,7 @@ static int launch_cfg(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const 
     return check_launch("fmatmul_stream_reduce");
   }
   if (splits < 1 || !ws || splits > num_kb) splits = 1;
+  if (splits > 1 && ((m * n) & 3) != 0) return fail(POLAR_B200_ERR_UNSUPPORTED, "cuts of k: m * n must be a multiple of 4");
   if (TAIL && splits == 1) return fail(POLAR_B200_ERR_UNSUPPORTED, "rows past the tiles: cuts of k or stream mode only");
   p.splits = splits;
   p.partial = splits > 1 ? ws : nullptr;

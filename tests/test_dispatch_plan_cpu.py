@@ -119,3 +119,18 @@ def test_by_name_query_agrees_and_knows_the_fused_forms(lib):
     b, keep2 = args((65536, 4096), (4096, 10), (65536, 10))
     assert int(q(b"fmatmul_f_f", b, 3)) == 0 and int(q(b"fadd", b, 3)) == 0
     assert int(q(b"fmatmul_f_f_nonsense", b, 3)) == 0
+
+
+def test_results_that_are_no_vectors_are_not_cut_along_k(lib):
+    # the partial products of cuts are added as vectors of four, m * n / 4 of them apart: with m * n no multiple of four every
+    # cut after the first would land shifted.  Such shapes run whole, in clusters or in stream mode, whose scratch
+    # is whole tiles; only f_t reaches them here, since TMA takes its operands whenever k is a multiple of four
+    dims = [257, 513, 1025, 1281, 1537, 1793, 1999, 2049, 3001, 1026, 1538]
+    for m in dims:
+        for n in dims:
+            for k in (512, 1024, 1536, 1952, 2048, 4096, 65536):
+                if m * n % 4 == 0:
+                    continue
+                need = ws(lib, 0, 1, m, n, k)
+                assert all(need != s * m * n * 4 for s in range(2, 65)), (m, n, k)
+                assert need % (128 * 256 * 4) == 0, (m, n, k)
