@@ -153,6 +153,8 @@ int polar_b200_fslice(const float* in, uint64_t first_dim, uint64_t inner, uint6
  * Args of the builtin: T left, T right, T out; the transposes are part of the
  * kernel NAME (utils/dialects/include/PolarGraph/PolarGraphOps.td:342-352).
  * Replaces PolarGraph/kernels/MatMulOp.cpp:36-85 and opencl/kernels.h:80-117.
+ * A NaN in an operand makes NaN of every result whose sum it enters.  An infinity gives what IEEE arithmetic
+ * gives, except on the 256-column tensor-core tiles (the large products), where it gives NaN.
  *
  * `workspace` is device scratch of `workspace_bytes` bytes, 256-byte aligned;
  * polar_b200_fmatmul_workspace_bytes gives the size this call needs (0 = none;

@@ -32,6 +32,10 @@
 // The split: A's hi is rounded to the nearest TF32 (it is written anyway), B's is cut off; the dropped lo.lo is below
 // 2^-23 |a||b| and of either sign: 9e-8 of the norm for uniform operands, where four products with both cut off left 1.1e-7
 // and an FFMA sum has 1.0e-7 (32 terms) to 5.7e-7 (1000 terms).
+// A NaN or an infinity always reaches a product: in B as the raw word that is its hi part, in A as its hi part or through the
+// difference from it, which is a NaN then.  The sums that it enters come out as NaN or infinite,
+// though not always as the right one of the two (an infinity meets lo parts of 0), so a result that is not finite is
+// computed again in FFMA, in the order of k, when it is stored (plain_sum): the classes of every result are those of an FFMA kernel.
 // At the end the tile goes to shared memory in the layout of the result's rows; the cluster's CTAs each
 // add one share of it over all CTAs in rank order (the same bits run to run) and store whole lines.
 //
@@ -94,7 +98,18 @@ struct Params {
   int out_t, epilogue, vec_out;
   int* status;
   unsigned long long wait_ns;
+  // the operands in memory, for plain_sum: row i (column j) and term k of A (B) at i * a_row + k * a_k
+  const float *a, *b;
+  uint64_t k, a_row, a_k, b_col, b_k;
 };
+
+// The result at row i, column j of the product as the kernel sees it, in FFMA and ascending k.  Only for results that are not
+// finite, so a NaN ends it.
+__device__ __noinline__ float plain_sum(const float* a, uint64_t a_k, const float* b, uint64_t b_k, uint64_t k) {
+  float s = 0.f;
+  for (; k && s == s; --k, a += a_k, b += b_k) s = fmaf(*a, *b, s);
+  return s;
+}
 
 __device__ __forceinline__ float4 ld_shared_v4(uint32_t addr) {
   float4 v;
@@ -139,6 +154,16 @@ __device__ __forceinline__ void store_share(const Params& p, uint32_t base, uint
       float4 y = part[u][0];
 #pragma unroll
       for (int k = 1; k < CL; ++k) y.x += part[u][k].x, y.y += part[u][k].y, y.z += part[u][k].z, y.w += part[u][k].w;
+      // (0 * y is a NaN where y is not finite)
+      if (fmaf(0.f, y.x, fmaf(0.f, y.y, fmaf(0.f, y.z, 0.f * y.w))) != 0.f) {
+        float e[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint64_t row = p.out_t ? c + j : r, col = p.out_t ? r : c + j;
+          if (c + j < out_cols && 0.f * e[j] != 0.f) e[j] = plain_sum(p.a + row * p.a_row, p.a_k, p.b + col * p.b_col, p.b_k, p.k);
+        }
+        y = make_float4(e[0], e[1], e[2], e[3]);
+      }
       if (p.epilogue == 1) y = make_float4(sigmoid_clamped(y.x), sigmoid_clamped(y.y), sigmoid_clamped(y.z), sigmoid_clamped(y.w));
       float* dst = p.out + r * p.pitch + c;
       if (p.vec_out && c + 4 <= out_cols) {
@@ -292,13 +317,13 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const uint8_t* slab = gen + s * C::kRawBytes;
       const float4* raw = reinterpret_cast<const float4*>(slab + C::kABytes) + tid;
       float4* lo = reinterpret_cast<float4*>(gen + C::kLoBase + l * C::kBBytes) + tid;
-      // the tensor core ignores the low 13 bits: adding half of the last one it sees rounds to nearest.  The bound keeps what
-      // would round to infinity finite.
+      // the tensor core ignores the low 13 bits: adding half of the last one it sees rounds to nearest.  (The largest finite
+      // numbers become infinities: their results are computed again like those of an infinity.)
       auto nearest = [](float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); };
-      auto high = [&](float x) {
-        const float h = __uint_as_float(__float_as_uint(nearest(x)) & 0xFFFFE000u), top = __uint_as_float(0x7F7FE000u);
-        return fminf(fmaxf(h, -top), top);
-      };
+      auto high = [&](float x) { return __uint_as_float(__float_as_uint(nearest(x)) & 0xFFFFE000u); };
+      // the same for A's lo part, with the bound below the NaN that arithmetic returns (0x7fffffff), which the addition would make
+      // a zero of
+      auto nearest_or_nan = [](float x) { return (uint32_t)(min(__float_as_int(x), 0x7FFFEFFF) + 0x1000); };
       auto low = [&](float x) { return nearest(x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u)); };
       bool ok = true;
 #pragma unroll
@@ -329,7 +354,7 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         for (int j = 0; j < 16; ++j) part[j] = __float_as_uint(high(a[j]));
         tmem_st_32x16(at, part);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) part[j] = __float_as_uint(nearest(a[j] - __uint_as_float(part[j])));
+        for (int j = 0; j < 16; ++j) part[j] = nearest_or_nan(a[j] - __uint_as_float(part[j]));
         tmem_st_32x16(at + BK, part);
 #pragma unroll
         for (int i = 0; i < kVecs; ++i)
@@ -493,6 +518,13 @@ int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Pa
   if (rc) return rc;
   p.a_mn = a_mn;
   p.b_mn = b_mn;
+  p.a = left.p;
+  p.b = right.p;
+  p.k = k;
+  p.a_row = a_mn ? 1 : left.pitch;
+  p.a_k = a_mn ? left.pitch : 1;
+  p.b_col = b_mn ? 1 : right.pitch;
+  p.b_k = b_mn ? right.pitch : 1;
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(p.whole + (p.tiles_m * (uint32_t)((p.n + BN - 1) / BN) - p.whole) * p.cluster);
   c.blockDim = dim3(kThreads);
