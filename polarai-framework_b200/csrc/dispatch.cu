@@ -299,11 +299,13 @@ MidChoice mid_for_small_n(int kind, uint64_t m, uint64_t n, uint64_t k, uint64_t
   return c;
 }
 
+constexpr uint64_t kMaxDim = 1ull << 31;
+
 int check_mm(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
              const float* right, float* out) {
   if ((tl != 0 && tl != 1) || (tr != 0 && tr != 1))
     return fail(POLAR_B200_ERR_INVALID, "transpose flags must be 0 or 1");
-  if (m > (1ull << 31) || n > (1ull << 31) || k > (1ull << 31))
+  if (m > kMaxDim || n > kMaxDim || k > kMaxDim)
     return fail(POLAR_B200_ERR_INVALID, "matrix dimension too large");
   if (m * n != 0 && !out) return fail(POLAR_B200_ERR_INVALID, "null output pointer");
   if (m * n != 0 && k != 0 && (!left || !right)) return fail(POLAR_B200_ERR_INVALID, "null operand pointer");
@@ -321,6 +323,8 @@ extern "C" {
 // of the tensor-core kernel changes the answer: it keeps rows past a tile boundary on the
 // tensor cores).
 static uint64_t workspace_need(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, int fused, bool pitched = false) {
+  // empty products launch no matmul, larger ones are refused
+  if (m == 0 || n == 0 || k == 0 || m > kMaxDim || n > kMaxDim || k > kMaxDim) return 0;
   const float* al = reinterpret_cast<const float*>(256);   // allocator buffers are 256-byte aligned
   int kind = skinny_kind(tl, tr, m, n, k, al, al, al);
   if (kind == 1 || kind == 2) {
@@ -338,7 +342,6 @@ static uint64_t workspace_need(int tl, int tr, uint64_t m, uint64_t n, uint64_t 
     if (rem) need = align256(need) + ragged_rows_workspace_bytes(rem, n, k);
     return need;
   }
-  if (m == 0 || n == 0 || k == 0) return 0;
   const uint64_t pad = mid_workspace_bytes(tl, tr, m, n, k, al, al);
   return mid_for_rest(m, n, k, pad).bn ? pad : 0;
 }
@@ -381,6 +384,12 @@ int polar_b200_fmatmul_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k) 
 void polar_b200_fmatmul_tc_plan(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, int* tile_rows, int* exchanged,
                                 int* splits) {
   const float* al = reinterpret_cast<const float*>(256);
+  if (m == 0 || n == 0 || k == 0) {                        // nothing runs
+    if (tile_rows) *tile_rows = 0;
+    if (exchanged) *exchanged = 0;
+    if (splits) *splits = 0;
+    return;
+  }
   const uint64_t rem = ragged_rows(tl, tr, m, n, k, al, 0);
   const MidChoice mid = rem == 0 ? mid_for_tc(m, n, k, true) : MidChoice{};
   if (mid.bn) {
@@ -586,7 +595,7 @@ int polar_b200_fmatmul_t_f_rows(uint64_t m, uint64_t row0, uint64_t rows, uint64
   clear_error();
   if (rows == 0) return POLAR_B200_OK;
   if (!left || !right || !out) return fail(POLAR_B200_ERR_INVALID, "null device pointer");
-  if (row0 + rows > m || (row0 & 3) || m > (1ull << 31) || n > (1ull << 31) || k > (1ull << 31))
+  if (row0 + rows > m || (row0 & 3) || m > kMaxDim || n > kMaxDim || k > kMaxDim)
     return fail(POLAR_B200_ERR_INVALID, "fmatmul_t_f_rows: rows outside the result, or row0 not a multiple of 4");
   if (row0 == 0 && rows == m) return polar_b200_fmatmul(1, 0, m, n, k, left, right, out, workspace, workspace_bytes, stream);
   const float* l = left + row0;
@@ -619,6 +628,7 @@ int polar_b200_fmatmul_sigmoid_grad(int tl, int tr, uint64_t m, uint64_t n, uint
 
 uint64_t polar_b200_fdense_grad_workspace_bytes(uint64_t rows, uint64_t kh, uint64_t n) {
   const float* al = reinterpret_cast<const float*>(256);
+  if (rows > kMaxDim || kh > kMaxDim) return 0;            // refused
   if (dense_grad_ok(rows, kh, n, al, al)) return dense_grad_workspace_bytes(rows, kh, n);
   // the two builtins in sequence
   const uint64_t a = workspace_need(1, 0, kh, n, rows, 0), b = workspace_need(0, 1, rows, kh, n, 2);
@@ -631,7 +641,7 @@ int polar_b200_fdense_grad(uint64_t rows, uint64_t kh, uint64_t n, const float* 
   clear_error();
   if (rows == 0 || kh == 0 || n == 0) return fail(POLAR_B200_ERR_UNSUPPORTED, "fdense_grad: empty operand");
   if (!dz || !w || !h || !dw || !din) return fail(POLAR_B200_ERR_INVALID, "null device pointer");
-  if (rows > (1ull << 31) || kh > (1ull << 31)) return fail(POLAR_B200_ERR_INVALID, "matrix dimension too large");
+  if (rows > kMaxDim || kh > kMaxDim) return fail(POLAR_B200_ERR_INVALID, "matrix dimension too large");
   LaunchDeviceScope on(stream, din);
   if (!dense_grad_ok(rows, kh, n, h, din)) {
     // shapes the one-pass kernel does not serve: the two builtins it stands for, one after the other

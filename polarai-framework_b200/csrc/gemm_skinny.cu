@@ -678,8 +678,8 @@ uint32_t splits_for(uint64_t m, uint64_t k, uint64_t n) {
     if (k <= kClusterRows) max_by_k = max_by_k < 8 ? max_by_k : 8;
   }
   uint64_t s = want < max_by_k ? want : max_by_k;
-  if (n && k > 8 * KS) {
-    const uint64_t by_scratch = (16ull << 20) / (m * n * sizeof(float)), fine = (k + 31) / 32;
+  if (m && n && k > 8 * KS) {
+    const uint64_t by_scratch = (16ull << 20) / sizeof(float) / n / m, fine = (k + 31) / 32;
     uint64_t finer = want < fine ? want : fine;
     if (finer > by_scratch) finer = by_scratch;
     if (finer > KS) finer = KS;              // (the error of a sum of sums grows with the longer of the two)

@@ -134,3 +134,26 @@ def test_results_that_are_no_vectors_are_not_cut_along_k(lib):
                 need = ws(lib, 0, 1, m, n, k)
                 assert all(need != s * m * n * 4 for s in range(2, 65)), (m, n, k)
                 assert need % (128 * 256 * 4) == 0, (m, n, k)
+
+
+def test_size_queries_of_empty_and_of_refused_products():
+    # in a process of their own: a division by zero in a query would end it
+    import subprocess
+    code = """
+import ctypes, sys
+sys.path.insert(0, sys.argv[1])
+import __graft_entry__ as ge
+c = ge.load_package().lib().cdll
+x = [ctypes.c_int() for _ in range(3)]
+for a, b, k in ((0, 5, 2000), (2000, 0, 2000), (2000, 5, 0), (0, 0, 0), (0, 2000, 5), (1 << 62, 1, 2000), (1 << 60, 16, 1 << 20),
+                (2000, 1 << 62, 16), (16, 1 << 62, 2000), (2000, 2000, 1 << 63), (1 << 62, 4, 40)):
+    for tl, tr in ((0, 0), (0, 1), (1, 0), (1, 1)):
+        assert c.polar_b200_fmatmul_workspace_bytes(tl, tr, a, b, k) == 0, (a, b, k)
+        c.polar_b200_fmatmul_path(tl, tr, a, b, k)
+        c.polar_b200_fmatmul_tc_plan(tl, tr, a, b, k, *[ctypes.byref(v) for v in x])
+    assert c.polar_b200_fmatmul_t_f_rows_workspace_bytes(a, b, k) == 0, (a, b, k)
+    if not (a and b and k) or b > 1 << 31:
+        assert c.polar_b200_fdense_grad_workspace_bytes(a, b, k) == 0, (a, b, k)
+"""
+    r = subprocess.run([sys.executable, "-c", code, ROOT], capture_output=True, text=True)
+    assert r.returncode == 0, (r.returncode, r.stderr[-500:])
