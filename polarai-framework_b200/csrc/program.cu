@@ -18,6 +18,8 @@
 //    once or twice never pays for the instantiation; a run under the caller's own stream capture is
 //    always launched one by one.
 #include <cstring>
+#include <exception>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -377,6 +379,19 @@ int run_steps(Program* p, cudaStream_t stream) {
   return POLAR_B200_OK;
 }
 
+uint64_t kernel_nodes(cudaGraph_t g) {
+  size_t nodes = 0;
+  cudaGraphGetNodes(g, nullptr, &nodes);
+  std::unique_ptr<cudaGraphNode_t[]> list(new (std::nothrow) cudaGraphNode_t[nodes]);
+  if (!list || cudaGraphGetNodes(g, list.get(), &nodes) != cudaSuccess) return 0;
+  uint64_t kernels = 0;
+  for (size_t i = 0; i < nodes; ++i) {
+    cudaGraphNodeType type;
+    if (cudaGraphNodeGetType(list[i], &type) == cudaSuccess && type == cudaGraphNodeTypeKernel) kernels++;
+  }
+  return kernels;
+}
+
 // Captures one pass on a stream of the program's own and instantiates it.  Thread-local capture mode: other
 // threads may go on launching and allocating.
 bool make_graph(Program* p) {
@@ -394,15 +409,7 @@ bool make_graph(Program* p) {
     const bool ended = cudaStreamEndCapture(s, &g) == cudaSuccess && g;
     if (rc == POLAR_B200_OK && ended) {
       ok = cudaGraphInstantiate(&p->graph, g, 0) == cudaSuccess;
-      size_t nodes = 0;
-      cudaGraphGetNodes(g, nullptr, &nodes);
-      std::vector<cudaGraphNode_t> list(nodes);
-      cudaGraphGetNodes(g, list.data(), &nodes);
-      p->graph_launches = 0;
-      for (cudaGraphNode_t n : list) {
-        cudaGraphNodeType type;
-        if (cudaGraphNodeGetType(n, &type) == cudaSuccess && type == cudaGraphNodeTypeKernel) p->graph_launches++;
-      }
+      p->graph_launches = kernel_nodes(g);
       count_launch(0 - p->graph_launches);                 // captured, not launched
     }
     if (g) cudaGraphDestroy(g);
@@ -425,47 +432,39 @@ int polar_b200_program_create(const polar_b200_op* ops, uint64_t count, void* wo
   clear_error();
   if (!program || (count && !ops)) return fail(POLAR_B200_ERR_INVALID, "null program or operation list");
   *program = nullptr;
-  Program* p = new (std::nothrow) Program;
-  if (!p) return fail(POLAR_B200_ERR_INVALID, "out of host memory");
-  for (uint64_t i = 0; i < count; ++i) {
-    const polar_b200_op& o = ops[i];
-    if (!o.name || (o.argc && !o.args)) {
-      delete p;
-      return fail(POLAR_B200_ERR_INVALID, "null kernel name or argument list");
-    }
-    Op op;
-    op.name = o.name;
-    op.args.assign(o.args, o.args + o.argc);
-    op.shapes.resize(o.argc);
-    for (uint64_t a = 0; a < o.argc; ++a) {
-      if (!o.args[a].is_tensor) continue;
-      const polar_b200_tensor& t = o.args[a].tensor;
-      if (t.dims && !t.shape) {
-        delete p;
-        return fail(POLAR_B200_ERR_INVALID, "tensor without a shape");
+  try {
+    std::unique_ptr<Program> p(new Program);
+    for (uint64_t i = 0; i < count; ++i) {
+      const polar_b200_op& o = ops[i];
+      if (!o.name || (o.argc && !o.args)) return fail(POLAR_B200_ERR_INVALID, "null kernel name or argument list");
+      Op op;
+      op.name = o.name;
+      op.args.assign(o.args, o.args + o.argc);
+      op.shapes.resize(o.argc);
+      for (uint64_t a = 0; a < o.argc; ++a) {
+        if (!o.args[a].is_tensor) continue;
+        const polar_b200_tensor& t = o.args[a].tensor;
+        if (t.dims && !t.shape) return fail(POLAR_B200_ERR_INVALID, "tensor without a shape");
+        op.shapes[a].assign(t.shape, t.shape + t.dims);
+        if (!p->any_pointer) p->any_pointer = t.data;
+        if (elements(t) >= 2000000) p->short_launches = false;
       }
-      op.shapes[a].assign(t.shape, t.shape + t.dims);
-      if (!p->any_pointer) p->any_pointer = t.data;
-      if (elements(t) >= 2000000) p->short_launches = false;
+      p->ops.push_back(std::move(op));
+      Op& kept = p->ops.back();
+      for (uint64_t a = 0; a < o.argc; ++a)
+        if (kept.args[a].is_tensor) kept.args[a].tensor.shape = kept.shapes[a].data();
     }
-    p->ops.push_back(std::move(op));
-    Op& kept = p->ops.back();
-    for (uint64_t a = 0; a < o.argc; ++a)
-      if (kept.args[a].is_tensor) kept.args[a].tensor.shape = kept.shapes[a].data();
+    p->workspace = workspace;
+    p->workspace_bytes = workspace_bytes;
+    plan(p.get());
+    *program = p.release();
+  } catch (const std::exception&) {                        // (no exception may leave a C entry)
+    return fail(POLAR_B200_ERR_INVALID, "out of host memory");
   }
-  p->workspace = workspace;
-  p->workspace_bytes = workspace_bytes;
-  plan(p);
-  *program = p;
   return POLAR_B200_OK;
 }
 
-int polar_b200_program_run(void* program, void* stream) {
-  clear_error();
-  Program* p = static_cast<Program*>(program);
-  if (!p) return fail(POLAR_B200_ERR_INVALID, "null program");
-  cudaStream_t st = as_stream(stream);
-  LaunchDeviceScope on(stream, p->any_pointer);
+static int run_program(Program* p, cudaStream_t st) {
   if (p->steps.size() > 3 && p->short_launches) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     // (a query on the legacy stream fails while some other stream is capturing: then launch one by one)
@@ -491,6 +490,18 @@ int polar_b200_program_run(void* program, void* stream) {
     }
   }
   return run_steps(p, st);
+}
+
+int polar_b200_program_run(void* program, void* stream) {
+  clear_error();
+  Program* p = static_cast<Program*>(program);
+  if (!p) return fail(POLAR_B200_ERR_INVALID, "null program");
+  LaunchDeviceScope on(stream, p->any_pointer);
+  try {
+    return run_program(p, as_stream(stream));
+  } catch (const std::exception&) {
+    return fail(POLAR_B200_ERR_INVALID, "out of host memory");
+  }
 }
 
 uint64_t polar_b200_program_steps(const void* program) {

@@ -60,6 +60,28 @@ def test_launch_by_name_checks_argument_patterns(library):
     assert c.polar_b200_launch_by_name(b"fmatmul_f_f", args, 2, None, 0, None) == 3
 
 
+def test_a_program_that_no_host_can_hold_returns_status_not_abort(library):
+    # in a process of its own: an exception that left the C entry would end it
+    import subprocess
+    import sys
+    code = """
+import ctypes, sys
+sys.path.insert(0, sys.argv[1])
+import __graft_entry__ as ge
+c = ge.load_package().lib().cdll
+from polarai_framework_b200.capi import Arg, Op
+for argc, dims in ((1 << 57, 1), (2, 1 << 59)):
+    shape, args, handle = (ctypes.c_uint64 * 1)(4), (Arg * 2)(), ctypes.c_void_p(1)
+    for a in args:
+        a.is_tensor, a.tensor.dims, a.tensor.shape = 1, dims, shape
+    op = Op(b"fcopy", args, argc)
+    assert c.polar_b200_program_create(ctypes.byref(op), 1, None, 0, ctypes.byref(handle)) == 1
+    assert not handle.value and b"memory" in c.polar_b200_last_error()
+"""
+    r = subprocess.run([sys.executable, "-c", code, ROOT], capture_output=True, text=True)
+    assert r.returncode == 0, (r.returncode, r.stderr[-500:])
+
+
 def test_matmul_path_selection(library):
     c = library.cdll
     assert c.polar_b200_fmatmul_path(0, 0, 8192, 8192, 8192) == 0     # tensor cores
