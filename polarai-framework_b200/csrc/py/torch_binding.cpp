@@ -5,7 +5,9 @@
 //
 // Every function returns True when it has launched.  Anything out of the ordinary - an argument that is no
 // contiguous float32 CUDA tensor, sizes that do not agree, a status other than 0 - makes it return
-// False without an exception, and the caller takes its checked Python path, which raises what it always has.
+// False without an exception, and the caller takes its checked Python path, which raises what it always has.  That goes for
+// what torch throws as well (a tensor without storage, as tracing makes them, has no data pointer): a C++ exception must not
+// reach the interpreter, where it would end the process.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -15,6 +17,7 @@
 #include <polar_b200.h>
 
 #include <algorithm>
+#include <exception>
 #include <vector>
 
 namespace {
@@ -70,6 +73,27 @@ private:
 float* data(const at::Tensor* t) { return static_cast<float*>(t->data_ptr()); }
 uint64_t numel(const at::Tensor* t) { return (uint64_t)t->numel(); }
 PyObject* answer(bool launched) { return PyBool_FromLong(launched); }
+
+using Function = PyObject* (*)(PyObject*, PyObject* const*, Py_ssize_t);
+template <Function F>
+PyObject* declining(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  try {
+    return F(self, args, n);
+  } catch (const std::exception&) {
+    return answer(false);
+  }
+}
+template <Function F>
+PyObject* raising(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  try {
+    return F(self, args, n);
+  } catch (const c10::Error& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
 
 #define BUILTIN(name) PyObject* name(PyObject*, PyObject* const* args, Py_ssize_t n)
 
@@ -196,26 +220,26 @@ BUILTIN(run_program) {
   return PyLong_FromLong(polar_b200_program_run(handle, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream()));
 }
 
-#define ENTRY(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
+#define ENTRY(name, ...) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(__VA_ARGS__)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
-    ENTRY("ffill", ffill),
-    ENTRY("fcopy", unary<polar_b200_fcopy>),
-    ENTRY("fadd", fadd),
-    ENTRY("fmul", binary<polar_b200_fmul>),
-    ENTRY("fdivide", binary<polar_b200_fdivide>),
-    ENTRY("fsigmoid", unary<polar_b200_fsigmoid>),
-    ENTRY("fsigmoid_unclamped", unary<polar_b200_fsigmoid_unclamped>),
-    ENTRY("flogloss", binary<polar_b200_flogloss>),
-    ENTRY("fmulconcat", fmulconcat),
-    ENTRY("frelu", unary<polar_b200_frelu>),
-    ENTRY("fsoftmax", fsoftmax),
-    ENTRY("fpool", fpool),
-    ENTRY("fconv2d", fconv2d),
-    ENTRY("ftranspose", ftranspose),
-    ENTRY("fmatmul", fmatmul),
-    ENTRY("workspace_bytes", workspace_bytes),
-    ENTRY("create_program", create_program),
-    ENTRY("run_program", run_program),
+    ENTRY("ffill", declining<ffill>),
+    ENTRY("fcopy", declining<unary<polar_b200_fcopy>>),
+    ENTRY("fadd", declining<fadd>),
+    ENTRY("fmul", declining<binary<polar_b200_fmul>>),
+    ENTRY("fdivide", declining<binary<polar_b200_fdivide>>),
+    ENTRY("fsigmoid", declining<unary<polar_b200_fsigmoid>>),
+    ENTRY("fsigmoid_unclamped", declining<unary<polar_b200_fsigmoid_unclamped>>),
+    ENTRY("flogloss", declining<binary<polar_b200_flogloss>>),
+    ENTRY("fmulconcat", declining<fmulconcat>),
+    ENTRY("frelu", declining<unary<polar_b200_frelu>>),
+    ENTRY("fsoftmax", declining<fsoftmax>),
+    ENTRY("fpool", declining<fpool>),
+    ENTRY("fconv2d", declining<fconv2d>),
+    ENTRY("ftranspose", declining<ftranspose>),
+    ENTRY("fmatmul", declining<fmatmul>),
+    ENTRY("workspace_bytes", raising<workspace_bytes>),
+    ENTRY("create_program", raising<create_program>),
+    ENTRY("run_program", raising<run_program>),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "polar_b200_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

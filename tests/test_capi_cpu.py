@@ -82,6 +82,33 @@ for argc, dims in ((1 << 57, 1), (2, 1 << 59)):
     assert r.returncode == 0, (r.returncode, r.stderr[-500:])
 
 
+def test_the_binding_declines_tensors_without_data(library):
+    # in a process of its own: torch throws where such a tensor's data or an unknown device's stream is asked for
+    import subprocess
+    import sys
+    code = """
+import sys
+sys.path.insert(0, sys.argv[1])
+import torch
+import __graft_entry__ as ge
+ge.load_package()
+from polarai_framework_b200.capi import binding
+from torch._subclasses.fake_tensor import FakeTensorMode
+b = binding()
+with FakeTensorMode():
+    a, out = torch.empty(4, 4, device="cuda:0"), torch.empty(4, 4, device="cuda:0")
+assert not b.ffill(1.0, out) and not b.fcopy(a, out) and not b.fadd(a, 1.0, a, 1.0, out) and not b.fmul(a, a, out)
+assert not b.fmulconcat(a, a, out) and not b.fsoftmax(a, out) and not b.fpool(a, 1, 1, 1, 1, out)
+assert not b.fconv2d(a, out, out) and not b.ftranspose(a, out) and not b.fmatmul(0, 0, a, a, out)
+try:
+    b.run_program(0, 63)
+except RuntimeError:
+    print("raised")
+"""
+    r = subprocess.run([sys.executable, "-c", code, ROOT], capture_output=True, text=True)
+    assert r.returncode == 0 and "raised" in r.stdout, (r.returncode, r.stdout, r.stderr[-500:])
+
+
 def test_matmul_path_selection(library):
     c = library.cdll
     assert c.polar_b200_fmatmul_path(0, 0, 8192, 8192, 8192) == 0     # tensor cores
