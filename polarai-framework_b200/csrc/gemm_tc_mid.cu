@@ -35,7 +35,7 @@
 // A NaN or an infinity always reaches a product: in B as the raw word that is its hi part, in A as its hi part or through the
 // difference from it, which is a NaN then.  The sums that it enters come out as NaN or infinite,
 // though not always as the right one of the two (an infinity meets lo parts of 0), so a result that is not finite is
-// computed again in FFMA, in the order of k, when it is stored (plain_sum): the classes of every result are those of an FFMA kernel.
+// computed again in FFMA, in the order of k (repair_share): the classes of every result are those of an FFMA kernel.
 // At the end the tile goes to shared memory in the layout of the result's rows; the cluster's CTAs each
 // add one share of it over all CTAs in rank order (the same bits run to run) and store whole lines.
 //
@@ -87,29 +87,22 @@ template <int BN> struct Cfg {
   static_assert(BM * (BN + 4) * 4 <= (int)kTileBytes && BN * (BM + 4) * 4 <= (int)kTileBytes, "the tile must fit the rings");
 };
 
+// Kept small: a launch pays for every byte of its parameters, on the host and on the way to the SMs.  Extents are 2^31 at most.
 struct Params {
-  uint64_t m, n;            // of the product as the kernel sees it (rows = lanes)
   float* out;
-  uint64_t pitch;           // floats per row of the result
-  uint32_t tiles_m, slabs, cluster, chunk;
-  uint32_t whole;           // the first tiles, one CTA each whatever the cluster (even; see launch_mid)
-  int a_mn, b_mn;           // operand stored with m (n) contiguous
-  int b_whole;              // whole 32-element chunks of B's extent: tiles inside them come in one 3-D box
-  int out_t, epilogue, vec_out;
   int* status;
   unsigned long long wait_ns;
-  // the operands in memory, for plain_sum: row i (column j) and term k of A (B) at i * a_row + k * a_k
-  const float *a, *b;
-  uint64_t k, a_row, a_k, b_col, b_k;
+  const float *a, *b;       // the operands in memory, for repair_share
+  uint32_t a_pitch, b_pitch, k;
+  uint32_t m, n;            // of the product as the kernel sees it (rows = lanes)
+  uint32_t pitch;           // floats per row of the result
+  uint32_t tiles_m, slabs;
+  uint32_t whole;           // the first tiles, one CTA each whatever the cluster (even; see launch_mid)
+  uint32_t b_whole;         // whole 32-element chunks of B's extent: tiles inside them come in one 3-D box
+  uint32_t cluster, chunk;
+  uint8_t a_mn, b_mn;       // operand stored with m (n) contiguous
+  uint8_t out_t, epilogue, vec_out;
 };
-
-// The result at row i, column j of the product as the kernel sees it, in FFMA and ascending k.  Only for results that are not
-// finite, so a NaN ends it.
-__device__ __noinline__ float plain_sum(const float* a, uint64_t a_k, const float* b, uint64_t b_k, uint64_t k) {
-  float s = 0.f;
-  for (; k && s == s; --k, a += a_k, b += b_k) s = fmaf(*a, *b, s);
-  return s;
-}
 
 __device__ __forceinline__ float4 ld_shared_v4(uint32_t addr) {
   float4 v;
@@ -127,13 +120,17 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr, uint32_t rank) {
 
 // A CTA's share of the finished tile: the parts of all CTAs of the cluster, added in rank order, to the result.
 // Eight 128-bit reads of (distributed) shared memory are in flight per thread before the first is used.
+// True where one of the thread's results is not finite.
 template <int BN, int CL>
-__device__ __forceinline__ void store_share(const Params& p, uint32_t base, uint32_t rank, int m0, int n0) {
+__device__ __forceinline__ bool store_share(const Params& p, uint32_t base, uint32_t rank, int m0, int n0) {
   constexpr int kVecs = BM * BN / 4, kShare = kVecs / CL, kBatch = 8 / CL;
   const int shift = p.out_t ? 5 : (BN == 128 ? 5 : BN == 64 ? 4 : 3);       // log2 of the vectors in a row of the result
   const int width = 4 << shift;
-  const uint64_t out_rows = p.out_t ? p.n : p.m, out_cols = p.out_t ? p.m : p.n;
-  const uint64_t r0 = (uint64_t)(p.out_t ? n0 : m0), c0 = (uint64_t)(p.out_t ? m0 : n0);
+  const uint32_t out_rows = p.out_t ? p.n : p.m, out_cols = p.out_t ? p.m : p.n;
+  const uint32_t r0 = (uint32_t)(p.out_t ? n0 : m0), c0 = (uint32_t)(p.out_t ? m0 : n0);
+  // 0 * y is a NaN where y is not finite; what is stored for such a result is not finite either
+  auto act = [](float y) { return fmaf(0.f, y, sigmoid_clamped(y)); };
+  float probe = 0.f;
   for (int first = 0; first < kShare; first += kBatch * kThreads) {
     float4 part[kBatch][CL];
 #pragma unroll
@@ -149,23 +146,14 @@ __device__ __forceinline__ void store_share(const Params& p, uint32_t base, uint
     for (int u = 0; u < kBatch; ++u) {
       const int w = first + u * kThreads + (int)threadIdx.x, v = (int)rank * kShare + w;
       if (w >= kShare) continue;
-      const uint64_t r = r0 + (uint64_t)(v >> shift), c = c0 + (uint64_t)(v & ((1 << shift) - 1)) * 4;
+      const uint32_t r = r0 + (uint32_t)(v >> shift), c = c0 + (uint32_t)(v & ((1 << shift) - 1)) * 4;
       if (r >= out_rows || c >= out_cols) continue;
       float4 y = part[u][0];
 #pragma unroll
       for (int k = 1; k < CL; ++k) y.x += part[u][k].x, y.y += part[u][k].y, y.z += part[u][k].z, y.w += part[u][k].w;
-      // (0 * y is a NaN where y is not finite)
-      if (fmaf(0.f, y.x, fmaf(0.f, y.y, fmaf(0.f, y.z, 0.f * y.w))) != 0.f) {
-        float e[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint64_t row = p.out_t ? c + j : r, col = p.out_t ? r : c + j;
-          if (c + j < out_cols && 0.f * e[j] != 0.f) e[j] = plain_sum(p.a + row * p.a_row, p.a_k, p.b + col * p.b_col, p.b_k, p.k);
-        }
-        y = make_float4(e[0], e[1], e[2], e[3]);
-      }
-      if (p.epilogue == 1) y = make_float4(sigmoid_clamped(y.x), sigmoid_clamped(y.y), sigmoid_clamped(y.z), sigmoid_clamped(y.w));
-      float* dst = p.out + r * p.pitch + c;
+      probe = fmaf(0.f, y.x, fmaf(0.f, y.y, fmaf(0.f, y.z, fmaf(0.f, y.w, probe))));
+      if (p.epilogue == 1) y = make_float4(act(y.x), act(y.y), act(y.z), act(y.w));
+      float* dst = p.out + (uint64_t)r * p.pitch + c;
       if (p.vec_out && c + 4 <= out_cols) {
         *reinterpret_cast<float4*>(dst) = y;
       } else {
@@ -176,6 +164,45 @@ __device__ __forceinline__ void store_share(const Params& p, uint32_t base, uint
       }
     }
   }
+  return probe != 0.f;
+}
+
+// Computes what a thread has stored again where it is not finite: FFMA, ascending k.  A NaN ends a sum.  (Out of the loop
+// above, where it cost every launch 0.3 us.)
+__device__ __noinline__ void repair_share(const float* a, uint64_t a_row, uint64_t a_k, const float* b, uint64_t b_col, uint64_t b_k,
+                                          uint32_t terms, float* out, uint64_t pitch, uint32_t rows, uint32_t cols, uint32_t first_vec,
+                                          uint32_t end_vec, int shift, uint32_t r0, uint32_t c0, bool out_t, bool sigmoid) {
+  for (uint32_t v = first_vec + threadIdx.x; v < end_vec; v += kThreads) {
+    const uint32_t r = r0 + (v >> shift);
+    for (uint32_t c = c0 + (v & ((1u << shift) - 1)) * 4, end = c + 4; r < rows && c < cols && c < end; ++c) {
+      float* dst = out + r * pitch + c;
+      if (0.f * *dst == 0.f) continue;
+      const float *x = a + (out_t ? c : r) * a_row, *y = b + (out_t ? r : c) * b_col;
+      float s = 0.f;
+      for (uint32_t k = 0; k < terms && s == s; ++k, x += a_k, y += b_k) s = fmaf(*x, *y, s);
+      *dst = sigmoid ? sigmoid_clamped(s) : s;
+    }
+  }
+}
+
+// Two floats in one instruction each (sm_100).
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 template <int BN>
@@ -321,9 +348,6 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       // numbers become infinities: their results are computed again like those of an infinity.)
       auto nearest = [](float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); };
       auto high = [&](float x) { return __uint_as_float(__float_as_uint(nearest(x)) & 0xFFFFE000u); };
-      // the same for A's lo part, with the bound below the NaN that arithmetic returns (0x7fffffff), which the addition would make
-      // a zero of
-      auto nearest_or_nan = [](float x) { return (uint32_t)(min(__float_as_int(x), 0x7FFFEFFF) + 0x1000); };
       auto low = [&](float x) { return nearest(x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u)); };
       bool ok = true;
 #pragma unroll
@@ -353,8 +377,22 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
         for (int j = 0; j < 16; ++j) part[j] = __float_as_uint(high(a[j]));
         tmem_st_32x16(at, part);
+        // Two lo parts at a time, and their sum: a NaN, where one of the row's elements is not finite.  (Arithmetic returns the NaN
+        // 0x7fffffff, which the rounding makes a zero of; bounding every element below that with a minimum cost 2 % at
+        // 1024^3.)
+        unsigned long long lost = 0;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) part[j] = nearest_or_nan(a[j] - __uint_as_float(part[j]));
+        for (int j = 0; j < 16; j += 2) {
+          const unsigned long long rest = fma2(pack2(__uint_as_float(part[j]), __uint_as_float(part[j + 1])), pack2(-1.f, -1.f), pack2(a[j], a[j + 1]));
+          lost = add2(lost, rest);
+          float x, y;
+          unpack2(rest, x, y);
+          part[j] = __float_as_uint(nearest(x));
+          part[j + 1] = __float_as_uint(nearest(y));
+        }
+        float x, y;
+        unpack2(lost, x, y);
+        part[15] = __float_as_uint(fmaf(0.f, x + y, __uint_as_float(part[15])));
         tmem_st_32x16(at + BK, part);
 #pragma unroll
         for (int i = 0; i < kVecs; ++i)
@@ -439,13 +477,21 @@ fmatmul_mid_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
     tmem_dealloc(tmem, C::kTmemCols);
   }
+  bool repair;
   switch (cluster) {
-    case 1: store_share<BN, 1>(p, base, 0, m0, n0); break;
-    case 2: store_share<BN, 2>(p, base, rank, m0, n0); break;
-    case 4: store_share<BN, 4>(p, base, rank, m0, n0); break;
-    default: store_share<BN, 8>(p, base, rank, m0, n0);
+    case 1: repair = store_share<BN, 1>(p, base, 0, m0, n0); break;
+    case 2: repair = store_share<BN, 2>(p, base, rank, m0, n0); break;
+    case 4: repair = store_share<BN, 4>(p, base, rank, m0, n0); break;
+    default: repair = store_share<BN, 8>(p, base, rank, m0, n0);
   }
   if (cluster > 1) cluster_wait();   // nobody leaves while another CTA may still read its part
+  if (repair) {
+    constexpr uint32_t kVecs = BM * BN / 4;
+    const uint64_t a_pitch = p.a_pitch, b_pitch = p.b_pitch;
+    repair_share(p.a, p.a_mn ? 1 : a_pitch, p.a_mn ? a_pitch : 1, p.b, p.b_mn ? 1 : b_pitch, p.b_mn ? b_pitch : 1, p.k, p.out, p.pitch,
+                 p.out_t ? p.n : p.m, p.out_t ? p.m : p.n, rank * (kVecs / cluster), (rank + 1) * (kVecs / cluster),
+                 p.out_t ? 5 : (BN == 128 ? 5 : BN == 64 ? 4 : 3), p.out_t ? n0 : m0, p.out_t ? m0 : n0, p.out_t, p.epilogue == 1);
+  }
 }
 
 // Copies up to two matrices to scratch with their rows padded to `pitch` floats (a multiple of 32; the
@@ -508,7 +554,7 @@ int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Pa
     map_b3 = map_b;
   } else if (!rc) {
     const uint64_t cols = right.padded ? right.pitch : right.cols;
-    p.b_whole = (int)(cols / 32);
+    p.b_whole = (uint32_t)(cols / 32);
     const bool boxes_2d = (p.n + BN - 1) / BN * BN > 32ull * p.b_whole;
     if (p.b_whole) rc = make_map_chunks(&map_b3, right.p, p.b_whole, k, BK, BN / 32, right.pitch);
     if (!rc && (boxes_2d || !p.b_whole)) rc = make_map(&map_b, right.p, cols, k, 32, BK, true, BK, right.pitch);
@@ -520,11 +566,8 @@ int launch_cfg(const Stored& left, const Stored& right, bool a_mn, bool b_mn, Pa
   p.b_mn = b_mn;
   p.a = left.p;
   p.b = right.p;
-  p.k = k;
-  p.a_row = a_mn ? 1 : left.pitch;
-  p.a_k = a_mn ? left.pitch : 1;
-  p.b_col = b_mn ? 1 : right.pitch;
-  p.b_k = b_mn ? right.pitch : 1;
+  p.a_pitch = (uint32_t)left.pitch;
+  p.b_pitch = (uint32_t)right.pitch;
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(p.whole + (p.tiles_m * (uint32_t)((p.n + BN - 1) / BN) - p.whole) * p.cluster);
   c.blockDim = dim3(kThreads);
@@ -595,12 +638,13 @@ int launch_mid(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* 
   if (!p.status) return rc;
   p.wait_ns = wait_limit_ns(2000000000ull);
   p.out = out;
-  p.pitch = n;
+  p.pitch = (uint32_t)n;
+  p.k = (uint32_t)k;
   p.vec_out = (n & 3) == 0 && aligned16(out);
-  p.out_t = swap;
-  p.epilogue = epilogue;
-  p.m = swap ? n : m;
-  p.n = swap ? m : n;
+  p.out_t = swap != 0;
+  p.epilogue = (uint8_t)epilogue;
+  p.m = (uint32_t)(swap ? n : m);
+  p.n = (uint32_t)(swap ? m : n);
   p.tiles_m = (uint32_t)((p.m + BM - 1) / BM);
   p.slabs = (uint32_t)((k + BK - 1) / BK);
   p.cluster = (uint32_t)cluster;
