@@ -113,9 +113,33 @@ inline cudaError_t scratch_free(void* p, cudaStream_t stream) { return cudaFreeA
 // pdl_enter() before its first access to global memory, which waits until everything earlier in
 // the stream has finished and written its results.  Measured on B200 for back-to-back kernels of
 // 2^14 elements: 3.06 us each without, 1.97 us with (the host's launch rate).
+// "Before its first access" is something the compiler has to keep to as well, since the kernel before may still be writing
+// what this one reads.  So no pointer of such a kernel is __restrict__ (which would promise that nobody writes the data
+// while the kernel runs, and allow loads through the read-only path and above the wait), and loads and stores with a
+// cache hint are the volatile ones below instead of the intrinsics.
 __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Streaming (evict-first) loads and stores of data that is touched once; a load from L2, past L1.
+__device__ __forceinline__ float ld_stream(const float* p) {
+  float v;
+  asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_stream(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_stream(float4* p, float4 v) {
+  asm volatile("st.global.cs.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ float ld_l2(const float* p) {
+  float v;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
 }
 
 // `cluster`: CTAs per cluster along y (1: no clusters).

@@ -28,9 +28,6 @@ constexpr int kThreads = 256;
 constexpr int kCtasPerSm = 4;   // 1024 threads/SM: 64 registers per thread available
 constexpr int kUnroll = 4;      // float4 vectors in flight per input per thread
 
-__device__ __forceinline__ float4 ld_stream(const float4* p) { return __ldcs(p); }
-__device__ __forceinline__ void st_stream(float4* p, float4 v) { __stcs(p, v); }
-
 // Vectors in flight per input per thread: kUnroll for streams (flat between 2 and 8 for every
 // builtin), 1 for short vectors (short_vector below).
 // NIN = number of input streams (0, 1 or 2).

@@ -137,8 +137,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) softmax_cluster_kernel(con
 // One thread per output, a row of outputs per blockIdx.y (the grid is walked where there are more rows than that).  W > 0:
 // square window of that extent, unrolled.
 template <int W>
-__global__ void __launch_bounds__(kThreads) pool_kernel(const float* __restrict__ in, uint64_t w, uint32_t wh, uint32_t ww, uint64_t sh,
-                                                        uint64_t sw, float* __restrict__ out, uint64_t oh, uint64_t ow) {
+__global__ void __launch_bounds__(kThreads) pool_kernel(const float* in, uint64_t w, uint32_t wh, uint32_t ww, uint64_t sh,
+                                                        uint64_t sw, float* out, uint64_t oh, uint64_t ow) {
   pdl_enter();
   const uint64_t j = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
   if (j >= ow) return;
@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(kThreads) pool_kernel(const float* __restrict_
 }
 
 // Any kernel extents: one thread per output.
-__global__ void __launch_bounds__(kThreads) conv2d_kernel(const float* __restrict__ in, uint64_t w, const float* __restrict__ ker,
-                                                          uint32_t kh, uint32_t kw, float* __restrict__ out, uint64_t oh,
+__global__ void __launch_bounds__(kThreads) conv2d_kernel(const float* in, uint64_t w, const float* ker,
+                                                          uint32_t kh, uint32_t kw, float* out, uint64_t oh,
                                                           uint64_t ow) {
   pdl_enter();
   const uint64_t j = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -185,8 +185,8 @@ __global__ void __launch_bounds__(kThreads) conv2d_kernel(const float* __restric
 // K * K times through L1 and spent its time in 64-bit index arithmetic (1024 x 768, K = 5: 17 us, here 4.5).
 constexpr int kConvX = 128, kConvY = 8;
 template <int K>
-__global__ void __launch_bounds__(kThreads) conv2d_tile_kernel(const float* __restrict__ in, uint64_t h, uint64_t w,
-                                                               const float* __restrict__ ker, float* __restrict__ out, uint64_t oh,
+__global__ void __launch_bounds__(kThreads) conv2d_tile_kernel(const float* in, uint64_t h, uint64_t w,
+                                                               const float* ker, float* out, uint64_t oh,
                                                                uint64_t ow, int vec) {
   constexpr int kRows = kConvY + K - 1, kCols = kConvX + K - 1, kPitch = (kCols + 3) / 4 * 4, kVecs = (K + 3 + 3) / 4;
   __shared__ __align__(16) float tile[kRows][kPitch + 4];
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kThreads) conv2d_tile_kernel(const float* __re
 // out[c, r] = in[r, c] through a 32 x 33 shared-memory tile: both the reads and the writes
 // are coalesced rows of 32 floats.  One tile per CTA (32 x 8 threads, four rows each).
 constexpr int kTile = 32;
-__global__ void __launch_bounds__(kTile * 8) transpose_kernel(const float* __restrict__ in, float* __restrict__ out,
+__global__ void __launch_bounds__(kTile * 8) transpose_kernel(const float* in, float* out,
                                                               uint64_t rows, uint64_t cols, uint32_t tiles_c) {
   __shared__ float tile[kTile][kTile + 1];
   pdl_enter();

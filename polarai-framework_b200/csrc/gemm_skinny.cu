@@ -39,7 +39,7 @@ constexpr int ROWS_PER_WARP = 4;
 // rows are contiguous in `out` (n values each), so lane l stores flat elements l, l + 32, ...:
 // coalesced stores, and a fused sigmoid costs each lane one or two evaluations, not forty.
 template <int NP>
-__device__ __forceinline__ void store_row_sums(const float (&acc)[ROWS_PER_WARP][NP], float* __restrict__ out,
+__device__ __forceinline__ void store_row_sums(const float (&acc)[ROWS_PER_WARP][NP], float* out,
                                                uint64_t row0, uint64_t m, uint64_t n, int lane, int act) {
   if (row0 >= m) return;
   const uint32_t rows = (uint32_t)((m - row0 < ROWS_PER_WARP) ? (m - row0) : ROWS_PER_WARP);
@@ -59,7 +59,7 @@ __device__ __forceinline__ void store_row_sums(const float (&acc)[ROWS_PER_WARP]
 // stored in - whole lines - and eight at a time: one element per trip was one memory latency per trip, 15 us for the
 // 4096 x 10 of the MLP's output layer.
 template <int THREADS>
-__device__ __forceinline__ void stage_small_operand(const float* __restrict__ right, float* bs, int kt, int n, int pitch,
+__device__ __forceinline__ void stage_small_operand(const float* right, float* bs, int kt, int n, int pitch,
                                                     uint64_t rsk, uint64_t rsj) {
   constexpr int kBatch = 8;
   const bool by_k = rsk == 1;
@@ -92,7 +92,7 @@ __device__ __forceinline__ void stage_small_operand(const float* __restrict__ ri
 constexpr uint64_t kResidentRows = 4096;
 template <int NP, int RW, bool VEC>
 __global__ void __launch_bounds__(kThreads)
-small_n_rows_kernel(const float* __restrict__ left, const float* __restrict__ right, float* __restrict__ out, uint64_t m,
+small_n_rows_kernel(const float* left, const float* right, float* out, uint64_t m,
                     uint64_t n, uint64_t k, uint64_t rsk, uint64_t rsj, int act, uint32_t shares) {
   extern __shared__ float bs[];            // [NP][KT_PAD], k contiguous
   __shared__ float part[2][4 * RW][NP];    // the two k halves of this CTA
@@ -203,8 +203,8 @@ constexpr int kResidentThreads = 512;
 
 template <int NP>
 __global__ void __launch_bounds__(kResidentThreads, 1)
-small_n_kmajor_resident_kernel(const float* __restrict__ left, const float* __restrict__ right,
-                               float* __restrict__ out, uint64_t m, uint64_t n, uint64_t k, uint64_t rsk,
+small_n_kmajor_resident_kernel(const float* left, const float* right,
+                               float* out, uint64_t m, uint64_t n, uint64_t k, uint64_t rsk,
                                uint64_t rsj, int act) {
   pdl_enter();
   extern __shared__ float bs[];   // [NP][k + 4], k contiguous
@@ -222,8 +222,8 @@ small_n_kmajor_resident_kernel(const float* __restrict__ left, const float* __re
     for (int r = 0; r < ROWS_PER_WARP; ++r) {
       const uint64_t row = group * ROWS_PER_WARP + r;
       const float* src = left + (row < m ? row : m - 1) * k;   // clamped: results of padding rows are dropped
-      a0[r] = __ldcs(reinterpret_cast<const float4*>(src + kk));
-      a1[r] = (kk + 128 < (uint32_t)k) ? __ldcs(reinterpret_cast<const float4*>(src + kk + 128))
+      a0[r] = ld_stream(reinterpret_cast<const float4*>(src + kk));
+      a1[r] = (kk + 128 < (uint32_t)k) ? ld_stream(reinterpret_cast<const float4*>(src + kk + 128))
                                        : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
@@ -315,8 +315,8 @@ __device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& 
 // products of few k, where a second launch costs as much as the first.
 template <int NP, bool VEC>
 __global__ void __launch_bounds__(kThreads, 2)
-small_n_mnmajor_kernel(const float* __restrict__ left, const float* __restrict__ right,
-                       float* __restrict__ partial, uint64_t m, uint64_t n, uint64_t k, uint64_t rsk,
+small_n_mnmajor_kernel(const float* left, const float* right,
+                       float* partial, uint64_t m, uint64_t n, uint64_t k, uint64_t rsk,
                        uint64_t rsj, uint64_t k_per_split, uint32_t shares) {
   __shared__ __align__(16) float2 bs[KS][NP];   // every value twice: one 64-bit load yields the pair
   extern __shared__ float tile[];               // with shares: this CTA's sums, [1024 rows][n]
@@ -332,10 +332,10 @@ small_n_mnmajor_kernel(const float* __restrict__ left, const float* __restrict__
   const bool live = m0 < m;   // VEC: m is a multiple of 4
   auto load = [&](uint64_t kk) {
     const float* src = left + kk * m + m0;
-    if (VEC) return __ldcs(reinterpret_cast<const float4*>(src));
-    return make_float4(__ldcs(src), m0 + kThreads < m ? __ldcs(src + kThreads) : 0.f,
-                       m0 + 2 * kThreads < m ? __ldcs(src + 2 * kThreads) : 0.f,
-                       m0 + 3 * kThreads < m ? __ldcs(src + 3 * kThreads) : 0.f);
+    if (VEC) return ld_stream(reinterpret_cast<const float4*>(src));
+    return make_float4(ld_stream(src), m0 + kThreads < m ? ld_stream(src + kThreads) : 0.f,
+                       m0 + 2 * kThreads < m ? ld_stream(src + 2 * kThreads) : 0.f,
+                       m0 + 3 * kThreads < m ? ld_stream(src + 3 * kThreads) : 0.f);
   };
   auto multiply = [&](const float4& a, int kk) {
     const unsigned long long a01 = pack2(a.x, a.y), a23 = pack2(a.z, a.w);
@@ -423,31 +423,31 @@ small_n_mnmajor_kernel(const float* __restrict__ left, const float* __restrict__
 
 // Sum of one element over the splits, ascending split index (a fixed order); the loads of
 // up to 32 splits are issued together, the additions stay in order.
-__device__ __forceinline__ float sum_splits(const float* __restrict__ partial, uint64_t elems, uint64_t e,
+__device__ __forceinline__ float sum_splits(const float* partial, uint64_t elems, uint64_t e,
                                             uint32_t splits) {
   float s = 0.f;
   uint32_t sp = 0;
   for (; sp + 32 <= splits; sp += 32) {
     float v[32];
 #pragma unroll
-    for (int u = 0; u < 32; ++u) v[u] = __ldcg(partial + (uint64_t)(sp + u) * elems + e);
+    for (int u = 0; u < 32; ++u) v[u] = ld_l2(partial + (uint64_t)(sp + u) * elems + e);
 #pragma unroll
     for (int u = 0; u < 32; ++u) s += v[u];
   }
   for (; sp + 8 <= splits; sp += 8) {
     float v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = __ldcg(partial + (uint64_t)(sp + u) * elems + e);
+    for (int u = 0; u < 8; ++u) v[u] = ld_l2(partial + (uint64_t)(sp + u) * elems + e);
 #pragma unroll
     for (int u = 0; u < 8; ++u) s += v[u];
   }
-  for (; sp < splits; ++sp) s += __ldcg(partial + (uint64_t)sp * elems + e);
+  for (; sp < splits; ++sp) s += ld_l2(partial + (uint64_t)sp * elems + e);
   return s;
 }
 
 // out[e] = sum over splits, ascending split index: a fixed order.
 __global__ void __launch_bounds__(kThreads)
-reduce_splits_kernel(const float* __restrict__ partial, float* __restrict__ out, uint64_t elems,
+reduce_splits_kernel(const float* partial, float* out, uint64_t elems,
                      uint32_t splits) {
   pdl_enter();
   const uint64_t stride = (uint64_t)gridDim.x * kThreads;
@@ -459,7 +459,7 @@ reduce_splits_kernel(const float* __restrict__ partial, float* __restrict__ out,
 // last few rows of a product whose left operand is stored [k, rows]: they are computed as
 // the small-n product of the transposed problem and land as rows of the result.
 __global__ void __launch_bounds__(kThreads)
-reduce_splits_transposed_kernel(const float* __restrict__ partial, float* __restrict__ out, uint64_t m,
+reduce_splits_transposed_kernel(const float* partial, float* out, uint64_t m,
                                 uint64_t n, uint32_t splits) {
   pdl_enter();
   const uint64_t elems = m * n, stride = (uint64_t)gridDim.x * kThreads;
@@ -475,9 +475,9 @@ constexpr int RK = 64;   // rows of the left operand staged per CTA
 // L'(i,kk) = left[i*lsi + kk*lsk]; R'(kk,j) = right[kk*rsk + j*rsj]; k <= KP.
 template <int KP>
 __global__ void __launch_bounds__(kThreads)
-small_k_kernel(const float* __restrict__ left, const float* __restrict__ right, float* __restrict__ out,
+small_k_kernel(const float* left, const float* right, float* out,
                uint64_t m, uint64_t n, uint64_t k, uint64_t lsi, uint64_t lsk, uint64_t rsk,
-               uint64_t rsj, int vec_store, const float* __restrict__ sig) {
+               uint64_t rsj, int vec_store, const float* sig) {
   __shared__ float as[RK][KP];
   pdl_enter();
   // Four columns per thread: one vector, or - rows that are no vectors - a column out of each quarter of the warp's 128, so
@@ -519,7 +519,7 @@ small_k_kernel(const float* __restrict__ left, const float* __restrict__ right, 
           if (rb + u >= rows) continue;
           const float* sp = sig + (row0 + rb + u) * n + j0;
           if (vec) {
-            sv[u] = __ldcs(reinterpret_cast<const float4*>(sp));
+            sv[u] = ld_stream(reinterpret_cast<const float4*>(sp));
           } else {
             sv[u].x = sp[0];
             sv[u].y = (j0 + 32 < n) ? sp[32] : 0.f;
@@ -548,7 +548,7 @@ small_k_kernel(const float* __restrict__ left, const float* __restrict__ right, 
         }
         float* dst = out + (row0 + r) * n + j0;
         if (vec) {
-          __stcs(reinterpret_cast<float4*>(dst), make_float4(c0, c1, c2, c3));
+          st_stream(reinterpret_cast<float4*>(dst), make_float4(c0, c1, c2, c3));
         } else {
           dst[0] = c0;
           if (j0 + 32 < n) dst[32] = c1;
@@ -574,8 +574,8 @@ small_k_kernel(const float* __restrict__ left, const float* __restrict__ right, 
 // ascending order), so both results carry the bits of the separate launches.
 template <int NP>
 __global__ void __launch_bounds__(kThreads, NP > 10 ? 1 : 2)
-dense_grad_kernel(const float* __restrict__ H, const float* __restrict__ dz, const float* __restrict__ W,
-                  float* __restrict__ din, float* __restrict__ partial, uint64_t rows, uint64_t kh, uint64_t n,
+dense_grad_kernel(const float* H, const float* dz, const float* W,
+                  float* din, float* partial, uint64_t rows, uint64_t kh, uint64_t n,
                   uint64_t rows_per_split) {
   pdl_enter();
   __shared__ __align__(16) float2 bs[KS][NP];   // dZ rows, every value twice: one 64-bit load yields the pair
@@ -612,7 +612,7 @@ dense_grad_kernel(const float* __restrict__ H, const float* __restrict__ dz, con
       float4 h[kBatch];
 #pragma unroll
       for (int u = 0; u < kBatch; ++u)
-        if (rr + u < rs) h[u] = __ldcs(reinterpret_cast<const float4*>(H + (r0 + rr + u) * kh + m0));
+        if (rr + u < rs) h[u] = ld_stream(reinterpret_cast<const float4*>(H + (r0 + rr + u) * kh + m0));
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
         if (rr + u >= rs) continue;
@@ -636,7 +636,7 @@ dense_grad_kernel(const float* __restrict__ H, const float* __restrict__ dz, con
         unpack2(c23, c2, c3);
         const float4 o = make_float4(sigmoid_grad_chain(c0, h[u].x), sigmoid_grad_chain(c1, h[u].y),
                                      sigmoid_grad_chain(c2, h[u].z), sigmoid_grad_chain(c3, h[u].w));
-        __stcs(reinterpret_cast<float4*>(din + (r0 + rr + u) * kh + m0), o);
+        st_stream(reinterpret_cast<float4*>(din + (r0 + rr + u) * kh + m0), o);
       }
     }
   }
