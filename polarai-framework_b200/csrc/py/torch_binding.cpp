@@ -5,8 +5,8 @@
 //
 // Every function returns True when it has launched.  Anything out of the ordinary - an argument that is no
 // contiguous float32 CUDA tensor, sizes that do not agree, a status other than 0 - makes it return
-// False without an exception, and the caller takes its checked Python path, which raises what it always has.  That goes for
-// what torch throws as well (a tensor without storage, as tracing makes them, has no data pointer): a C++ exception must not
+// False without an exception, and the caller takes its checked Python path, which raises, or launches what it can read and
+// write within its tensors.  That goes for what torch throws as well (a tensor without storage, as tracing makes them, has no data pointer): a C++ exception must not
 // reach the interpreter, where it would end the process.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -146,20 +146,24 @@ BUILTIN(fpool) {
   const at::Tensor* out = c.tensor(5);
   if (c.ok()) c.require(a->dim() == 2);
   if (!c.ok()) return answer(false);
-  return answer(polar_b200_fpool(data(a), (uint64_t)a->size(0), (uint64_t)a->size(1), wh, ww, sh, sw, data(out), c.stream()) == 0);
+  const uint64_t h = (uint64_t)a->size(0), w = (uint64_t)a->size(1);
+  if (wh && ww && sh && sw && wh <= h && ww <= w && numel(out) < ((h - wh) / sh + 1) * ((w - ww) / sw + 1)) return answer(false);
+  return answer(polar_b200_fpool(data(a), h, w, wh, ww, sh, sw, data(out), c.stream()) == 0);
 }
 BUILTIN(fconv2d) {
   Call c(args, n, 3);
   const at::Tensor *a = c.tensor(0), *k = c.tensor(1), *out = c.tensor(2);
   if (c.ok()) c.require(a->dim() == 2 && k->dim() == 2);
   if (!c.ok()) return answer(false);
+  const int64_t oh = a->size(0) - k->size(0) + 1, ow = a->size(1) - k->size(1) + 1;
+  if (oh > 0 && ow > 0 && out->numel() < oh * ow) return answer(false);
   return answer(polar_b200_fconv2d(data(a), (uint64_t)a->size(0), (uint64_t)a->size(1), data(k), (uint64_t)k->size(0),
                                    (uint64_t)k->size(1), data(out), c.stream()) == 0);
 }
 BUILTIN(ftranspose) {
   Call c(args, n, 2);
   const at::Tensor *a = c.tensor(0), *out = c.tensor(1);
-  if (c.ok()) c.require(a->dim() == 2);
+  if (c.ok()) c.require(a->dim() == 2 && numel(a) <= numel(out));
   if (!c.ok()) return answer(false);
   return answer(polar_b200_ftranspose(data(a), (uint64_t)a->size(0), (uint64_t)a->size(1), data(out), c.stream()) == 0);
 }

@@ -7,7 +7,8 @@ torch is used for device memory and streams only.
 
 Each builtin first goes to the native binding (capi.binding), which checks its tensors
 and launches without the interpreter; what that declines - tensors it would reject, a failing
-call - runs the checked path below it, which raises.
+call - runs the checked path below it, which raises.  An input may be longer than the result and a result
+tensor larger than what is written; what would be read or written outside a tensor is a ValueError.
 """
 import numpy as np
 import torch
@@ -30,6 +31,12 @@ def _chk(*ts):
             raise ValueError("builtins take contiguous float32 CUDA tensors")
 
 
+def _long_enough(n, *ts):
+    for t in ts:
+        if t.numel() < n:
+            raise ValueError(f"a tensor of {t.numel()} elements where the builtin takes {n}")
+
+
 class DeviceBuiltins:
     def __init__(self):
         if not torch.cuda.is_available():
@@ -46,12 +53,14 @@ class DeviceBuiltins:
     def fcopy(self, a, out):
         if not self._native.fcopy(a, out):
             _chk(a, out)
+            _long_enough(out.numel(), a)
             self.lib.call("polar_b200_fcopy", _ptr(a), _ptr(out), out.numel(), _stream(out))
         return out
 
     def fadd(self, a, sa, b, sb, out):
         if not self._native.fadd(a, sa, b, sb, out):
             _chk(a, b, out)
+            _long_enough(out.numel(), a, b)
             self.lib.call("polar_b200_fadd", _ptr(a), float(sa), _ptr(b), float(sb), _ptr(out), out.numel(),
                           _stream(out))
         return out
@@ -59,18 +68,21 @@ class DeviceBuiltins:
     def fmul(self, a, b, out):
         if not self._native.fmul(a, b, out):
             _chk(a, b, out)
+            _long_enough(out.numel(), a, b)
             self.lib.call("polar_b200_fmul", _ptr(a), _ptr(b), _ptr(out), out.numel(), _stream(out))
         return out
 
     def fdivide(self, a, b, out):
         if not self._native.fdivide(a, b, out):
             _chk(a, b, out)
+            _long_enough(out.numel(), a, b)
             self.lib.call("polar_b200_fdivide", _ptr(a), _ptr(b), _ptr(out), out.numel(), _stream(out))
         return out
 
     def fsigmoid(self, a, out, clamp=True):
         if not (self._native.fsigmoid if clamp else self._native.fsigmoid_unclamped)(a, out):
             _chk(a, out)
+            _long_enough(out.numel(), a)
             name = "polar_b200_fsigmoid" if clamp else "polar_b200_fsigmoid_unclamped"
             self.lib.call(name, _ptr(a), _ptr(out), out.numel(), _stream(out))
         return out
@@ -78,6 +90,7 @@ class DeviceBuiltins:
     def flogloss(self, predicted, ground_truth, out):
         if not self._native.flogloss(predicted, ground_truth, out):
             _chk(predicted, ground_truth, out)
+            _long_enough(out.numel(), predicted, ground_truth)
             self.lib.call("polar_b200_flogloss", _ptr(predicted), _ptr(ground_truth), _ptr(out), out.numel(),
                           _stream(out))
         return out
@@ -85,18 +98,21 @@ class DeviceBuiltins:
     def fmulconcat(self, gradient, local, out):
         if not self._native.fmulconcat(gradient, local, out):
             _chk(gradient, local, out)
+            _long_enough(out.numel(), local)
             self.lib.call("polar_b200_fmulconcat", _ptr(gradient), _ptr(local), _ptr(out), out.numel(), _stream(out))
         return out
 
     def frelu(self, a, out):
         if not self._native.frelu(a, out):
             _chk(a, out)
+            _long_enough(out.numel(), a)
             self.lib.call("polar_b200_frelu", _ptr(a), _ptr(out), out.numel(), _stream(out))
         return out
 
     def fsoftmax(self, a, out):
         if not self._native.fsoftmax(a, out):
             _chk(a, out)
+            _long_enough(out.numel(), a)
             self.lib.call("polar_b200_fsoftmax", _ptr(a), _ptr(out), out.numel(), None, 0, _stream(out))
         return out
 
@@ -104,6 +120,8 @@ class DeviceBuiltins:
         if not self._native.fpool(a, window[0], window[1], stride[0], stride[1], out):
             _chk(a, out)
             h, w = a.shape
+            if 0 < window[0] <= h and 0 < window[1] <= w and stride[0] > 0 and stride[1] > 0:   # (else the library's error)
+                _long_enough(((h - window[0]) // stride[0] + 1) * ((w - window[1]) // stride[1] + 1), out)
             self.lib.call("polar_b200_fpool", _ptr(a), h, w, window[0], window[1], stride[0], stride[1], _ptr(out),
                           _stream(out))
         return out
@@ -113,6 +131,7 @@ class DeviceBuiltins:
             _chk(a, kernel, out)
             h, w = a.shape
             kh, kw = kernel.shape
+            _long_enough(max(h - kh + 1, 0) * max(w - kw + 1, 0), out)
             self.lib.call("polar_b200_fconv2d", _ptr(a), h, w, _ptr(kernel), kh, kw, _ptr(out), _stream(out))
         return out
 
@@ -120,11 +139,14 @@ class DeviceBuiltins:
         if not self._native.ftranspose(a, out):
             _chk(a, out)
             rows, cols = a.shape
+            _long_enough(rows * cols, out)
             self.lib.call("polar_b200_ftranspose", _ptr(a), rows, cols, _ptr(out), _stream(out))
         return out
 
     def fslice(self, a, index, out):
         _chk(a, out)
+        if 0 <= int(index) < a.shape[0]:                     # (else the library's error)
+            _long_enough((int(index) + 1) * out.numel(), a)
         self.lib.call("polar_b200_fslice", _ptr(a), a.shape[0], out.numel(), int(index), _ptr(out), _stream(out))
         return out
 
@@ -147,6 +169,7 @@ class DeviceBuiltins:
     def fmatmul_ffma(self, tl, tr, left, right, out):
         _chk(left, right, out)
         m, n, k = matmul_dims(tl, tr, left.shape, right.shape)
+        _long_enough(m * n, out)
         self.lib.call("polar_b200_fmatmul_ffma", int(tl), int(tr), m, n, k, _ptr(left), _ptr(right),
                       _ptr(out), _stream(out))
         return out
@@ -154,6 +177,7 @@ class DeviceBuiltins:
     def fmatmul_tc(self, tl, tr, left, right, out, tile_n=256, slab_k=16, passes=3, write_hi=0, splits=1):
         _chk(left, right, out)
         m, n, k = matmul_dims(tl, tr, left.shape, right.shape)
+        _long_enough(m * n, out)
         self.lib.call("polar_b200_fmatmul_tc", int(tl), int(tr), m, n, k, _ptr(left), _ptr(right),
                       _ptr(out), tile_n, slab_k, passes, write_hi, splits, _stream(out))
         return out
