@@ -8,6 +8,9 @@
 // False without an exception, and the caller takes its checked Python path, which raises, or launches what it can read and
 // write within its tensors.  That goes for what torch throws as well (a tensor without storage, as tracing makes them, has no data pointer): a C++ exception must not
 // reach the interpreter, where it would end the process.
+//
+// The C ABI is called without the interpreter's lock, as through ctypes: a launch waits when the GPU's queue is full,
+// which may take until another thread has launched what the kernels at its head wait for.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -70,9 +73,22 @@ private:
   int device_ = -1;
 };
 
+// Runs f without the interpreter's lock.  What f needs of Python objects is looked up before.
+template <class F>
+auto unlocked(F f) {
+  PyThreadState* state = PyEval_SaveThread();
+  auto r = f();
+  PyEval_RestoreThread(state);
+  return r;
+}
+
 float* data(const at::Tensor* t) { return static_cast<float*>(t->data_ptr()); }
 uint64_t numel(const at::Tensor* t) { return (uint64_t)t->numel(); }
 PyObject* answer(bool launched) { return PyBool_FromLong(launched); }
+template <class F, class... A>
+PyObject* launched(F f, A... args) {
+  return answer(unlocked([&] { return f(args...); }) == 0);
+}
 
 using Function = PyObject* (*)(PyObject*, PyObject* const*, Py_ssize_t);
 template <Function F>
@@ -101,7 +117,7 @@ BUILTIN(ffill) {
   Call c(args, n, 2);
   const float v = c.scalar(0);
   const at::Tensor* out = c.tensor(1);
-  return answer(c.ok() && polar_b200_ffill(v, data(out), numel(out), c.stream()) == 0);
+  return c.ok() ? launched(polar_b200_ffill, v, data(out), numel(out), c.stream()) : answer(false);
 }
 BUILTIN(fadd) {
   Call c(args, n, 5);
@@ -111,33 +127,33 @@ BUILTIN(fadd) {
   const float sb = c.scalar(3);
   const at::Tensor* out = c.tensor(4);
   if (c.ok()) c.require(numel(a) == numel(out) && numel(b) == numel(out));
-  return answer(c.ok() && polar_b200_fadd(data(a), sa, data(b), sb, data(out), numel(out), c.stream()) == 0);
+  return c.ok() ? launched(polar_b200_fadd, data(a), sa, data(b), sb, data(out), numel(out), c.stream()) : answer(false);
 }
 template <int (*F)(const float*, float*, uint64_t, void*)>
 BUILTIN(unary) {
   Call c(args, n, 2);
   const at::Tensor *a = c.tensor(0), *out = c.tensor(1);
   if (c.ok()) c.require(numel(a) == numel(out));
-  return answer(c.ok() && F(data(a), data(out), numel(out), c.stream()) == 0);
+  return c.ok() ? launched(F, data(a), data(out), numel(out), c.stream()) : answer(false);
 }
 template <int (*F)(const float*, const float*, float*, uint64_t, void*)>
 BUILTIN(binary) {
   Call c(args, n, 3);
   const at::Tensor *a = c.tensor(0), *b = c.tensor(1), *out = c.tensor(2);
   if (c.ok()) c.require(numel(a) == numel(out) && numel(b) == numel(out));
-  return answer(c.ok() && F(data(a), data(b), data(out), numel(out), c.stream()) == 0);
+  return c.ok() ? launched(F, data(a), data(b), data(out), numel(out), c.stream()) : answer(false);
 }
 BUILTIN(fmulconcat) {
   Call c(args, n, 3);
   const at::Tensor *g = c.tensor(0), *l = c.tensor(1), *out = c.tensor(2);
   if (c.ok()) c.require(numel(g) >= 1 && numel(l) == numel(out));
-  return answer(c.ok() && polar_b200_fmulconcat(data(g), data(l), data(out), numel(out), c.stream()) == 0);
+  return c.ok() ? launched(polar_b200_fmulconcat, data(g), data(l), data(out), numel(out), c.stream()) : answer(false);
 }
 BUILTIN(fsoftmax) {
   Call c(args, n, 2);
   const at::Tensor *a = c.tensor(0), *out = c.tensor(1);
   if (c.ok()) c.require(numel(a) == numel(out));
-  return answer(c.ok() && polar_b200_fsoftmax(data(a), data(out), numel(out), nullptr, 0, c.stream()) == 0);
+  return c.ok() ? launched(polar_b200_fsoftmax, data(a), data(out), numel(out), nullptr, 0, c.stream()) : answer(false);
 }
 BUILTIN(fpool) {
   Call c(args, n, 6);
@@ -148,7 +164,7 @@ BUILTIN(fpool) {
   if (!c.ok()) return answer(false);
   const uint64_t h = (uint64_t)a->size(0), w = (uint64_t)a->size(1);
   if (wh && ww && sh && sw && wh <= h && ww <= w && numel(out) < ((h - wh) / sh + 1) * ((w - ww) / sw + 1)) return answer(false);
-  return answer(polar_b200_fpool(data(a), h, w, wh, ww, sh, sw, data(out), c.stream()) == 0);
+  return launched(polar_b200_fpool, data(a), h, w, wh, ww, sh, sw, data(out), c.stream());
 }
 BUILTIN(fconv2d) {
   Call c(args, n, 3);
@@ -157,15 +173,15 @@ BUILTIN(fconv2d) {
   if (!c.ok()) return answer(false);
   const int64_t oh = a->size(0) - k->size(0) + 1, ow = a->size(1) - k->size(1) + 1;
   if (oh > 0 && ow > 0 && out->numel() < oh * ow) return answer(false);
-  return answer(polar_b200_fconv2d(data(a), (uint64_t)a->size(0), (uint64_t)a->size(1), data(k), (uint64_t)k->size(0),
-                                   (uint64_t)k->size(1), data(out), c.stream()) == 0);
+  return launched(polar_b200_fconv2d, data(a), (uint64_t)a->size(0), (uint64_t)a->size(1), data(k), (uint64_t)k->size(0),
+                  (uint64_t)k->size(1), data(out), c.stream());
 }
 BUILTIN(ftranspose) {
   Call c(args, n, 2);
   const at::Tensor *a = c.tensor(0), *out = c.tensor(1);
   if (c.ok()) c.require(a->dim() == 2 && numel(a) <= numel(out));
   if (!c.ok()) return answer(false);
-  return answer(polar_b200_ftranspose(data(a), (uint64_t)a->size(0), (uint64_t)a->size(1), data(out), c.stream()) == 0);
+  return launched(polar_b200_ftranspose, data(a), (uint64_t)a->size(0), (uint64_t)a->size(1), data(out), c.stream());
 }
 BUILTIN(fmatmul) {
   Call c(args, n, 5);
@@ -175,8 +191,8 @@ BUILTIN(fmatmul) {
   if (!c.ok()) return answer(false);
   const int64_t m = l->size(tl ? 1 : 0), k = l->size(tl ? 0 : 1), cols = r->size(tr ? 0 : 1);
   if (r->size(tr ? 1 : 0) != k || out->size(0) != m || out->size(1) != cols) return answer(false);
-  return answer(polar_b200_fmatmul((int)tl, (int)tr, (uint64_t)m, (uint64_t)cols, (uint64_t)k, data(l), data(r), data(out),
-                                   nullptr, 0, c.stream()) == 0);
+  return launched(polar_b200_fmatmul, (int)tl, (int)tr, (uint64_t)m, (uint64_t)cols, (uint64_t)k, data(l), data(r), data(out),
+                  nullptr, 0, c.stream());
 }
 
 // A program's operations as Python has them: a list of (native name, address of the argument structs, their count).
@@ -221,7 +237,8 @@ BUILTIN(run_program) {
   void* handle = PyLong_AsVoidPtr(args[0]);
   const long device = PyLong_AsLong(args[1]);
   if (PyErr_Occurred()) return nullptr;
-  return PyLong_FromLong(polar_b200_program_run(handle, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream()));
+  void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+  return PyLong_FromLong(unlocked([&] { return polar_b200_program_run(handle, stream); }));
 }
 
 #define ENTRY(name, ...) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(__VA_ARGS__)), METH_FASTCALL, nullptr}
