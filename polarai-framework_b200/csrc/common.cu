@@ -49,6 +49,7 @@ int* device_status_word(int* rc) {
   static std::once_flag once;
   static cudaError_t err = cudaSuccess;
   std::call_once(once, [] {
+    RelaxedCaptureMode relaxed;
     err = cudaHostAlloc(reinterpret_cast<void**>(&g_status_host), kMaxDevices * sizeof(int),
                         cudaHostAllocMapped | cudaHostAllocPortable);
     if (err == cudaSuccess) {
@@ -94,6 +95,7 @@ cudaError_t scratch_alloc(void** p, uint64_t bytes, cudaStream_t stream) {
   cudaError_t e = cudaStreamIsCapturing(stream, &capturing);
   if (e != cudaSuccess) return e;
   if (capturing != cudaStreamCaptureStatusNone) return cudaMallocAsync(p, bytes, stream);
+  RelaxedCaptureMode relaxed;
   int dev = 0;
   e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;

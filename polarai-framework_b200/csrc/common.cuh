@@ -94,6 +94,15 @@ private:
   bool switched_ = false;
 };
 
+// While it lives, the calling thread may allocate and create streams and graphs although another thread captures in the
+// global mode (torch.cuda.graph's default): in that mode such a call from any thread fails and ends the other's capture with
+// an error.  None of the calls that it is used for touches what that thread captures.
+struct RelaxedCaptureMode {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // ---- scratch ------------------------------------------------------------------------------
 // Device memory for the length of one launch sequence, when the caller hands in no workspace:
 // from a pool of the library's own (one per device, made on first use), so that blocks survive a
@@ -103,7 +112,10 @@ private:
 // gives the rest back too.  Stream-ordered, so it is safe with any number of threads and streams.
 constexpr uint64_t kScratchKeepBytes = 256ull << 20;
 cudaError_t scratch_alloc(void** p, uint64_t bytes, cudaStream_t stream);
-inline cudaError_t scratch_free(void* p, cudaStream_t stream) { return cudaFreeAsync(p, stream); }
+inline cudaError_t scratch_free(void* p, cudaStream_t stream) {
+  RelaxedCaptureMode relaxed;
+  return cudaFreeAsync(p, stream);
+}
 
 #ifdef __CUDACC__
 // ---- programmatic dependent launch -------------------------------------------------------------

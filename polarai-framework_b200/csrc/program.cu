@@ -392,15 +392,6 @@ uint64_t kernel_nodes(cudaGraph_t g) {
   return kernels;
 }
 
-// While it lives, the calling thread may create streams and graphs although another thread captures in the global
-// mode (torch.cuda.graph's default): in that mode such a call from any thread ends the other's capture with an error.  None of
-// them touches what that thread captures.
-struct RelaxedCaptureMode {
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  RelaxedCaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode); }
-  ~RelaxedCaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
-
 // Captures one pass on a stream of the program's own and instantiates it.  Thread-local capture mode: other
 // threads may go on launching and allocating.
 bool make_graph(Program* p) {
