@@ -163,6 +163,7 @@ struct Program {
   bool graph_failed = false;
   cudaGraphExec_t graph = nullptr;
   uint64_t graph_launches = 0;
+  unsigned long long graph_limit = 0;   // polar_b200_set_wait_limit_ns when the graph was made: its launches carry it
 };
 
 uint64_t elements(const polar_b200_tensor& t) {
@@ -474,9 +475,14 @@ static int run_program(Program* p, cudaStream_t st) {
       cudaGetLastError();
     } else {
       std::lock_guard<std::mutex> guard(p->mu);
+      if (p->graph && p->graph_limit != wait_limit_ns(0)) {
+        cudaGraphExecDestroy(p->graph);                    // (a run in flight is not disturbed)
+        p->graph = nullptr;
+      }
       if (p->runs < 2) {
         ++p->runs;
       } else if (!p->graph && !p->graph_failed) {
+        p->graph_limit = wait_limit_ns(0);
         p->graph_failed = !make_graph(p);
       }
       if (p->graph) {

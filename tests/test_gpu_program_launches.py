@@ -114,6 +114,26 @@ def test_steps_replayed_as_a_graph(env, fused):
         assert env.equal(ex.t[t].view(env.int32), want[t].view(env.int32)), t
 
 
+def test_a_changed_wait_limit_makes_the_graph_again(env):
+    # (the limit itself shows only where a wait runs out; here every wait ends)
+    from polarai_framework_b200.program import DeviceExecutor, mlp_program
+    prog = mlp_program(300, 65, 130, 7, 1e-3)
+    ins = inputs(env, prog, 6)
+    want = one_by_one(env, prog, ins, 9)
+    ex = DeviceExecutor(prog)
+    ex.set_inputs(**ins)
+    try:
+        for limit in (0, 500_000_000, 0):
+            ex.lib.cdll.polar_b200_set_wait_limit_ns(limit)
+            for _ in range(3):
+                ex.run()
+    finally:
+        ex.lib.cdll.polar_b200_set_wait_limit_ns(0)
+    env.cuda.synchronize()
+    for t in prog.outputs:
+        assert env.equal(ex.t[t].view(env.int32), want[t].view(env.int32)), t
+
+
 def test_bad_programs_are_statuses(env):
     from polarai_framework_b200.capi import Arg, Op, PolarB200Error, lib
     from polarai_framework_b200.program import DeviceExecutor, Program
