@@ -255,7 +255,8 @@ int polar_b200_fmatmul_tc(int transLeft, int transRight, uint64_t m, uint64_t n,
  * end, so a lost peer or a stuck pipeline never hangs the GPU.  The reference has no
  * counterpart: its runtimes terminate the process on any error
  * (src/backend/generic/runtime/cuda/utils.hpp:20-28).
- *  - Codes: 0 = none; 101..107 = which wait of the tensor-core matmul; 301 = a peer's
+ *  - Codes: 0 = none; 101..107 and 111..117 = which wait of the
+ *    tensor-core matmul or of its cluster form; 301 = a peer's
  *    gradients never became ready, 302 = a peer never finished its slice (in both cases no
  *    weight was updated).  The first code recorded since the last clear stays.
  *  - The words live in pinned host memory: reading them needs no CUDA call.  Read after
@@ -273,8 +274,9 @@ void polar_b200_set_wait_limit_ns(uint64_t ns);
 uint64_t polar_b200_wait_limit_ns(void);
 
 /* Which matmul path polar_b200_fmatmul would take for these sizes:
- * 0 = tcgen05 tensor-core tiles on the operands as they are stored, 1 = skinny
- * (bandwidth-bound CUDA-core) path, 2 = operands TMA cannot address as they are stored, or less
+ * 0 = tcgen05 tensor-core tiles on the operands as they are stored, 1 = one tiny
+ * dimension: bandwidth-bound CUDA-core kernels or, with up to 16 columns and where they are
+ * faster, 32-column tensor-core tiles, 2 = operands TMA cannot address as they are stored, or less
  * than a tile: clusters of tensor-core CTAs, on padded copies where needed (scratch), with the
  * accuracy of FFMA sums - or, for the smallest, FFMA tiles. */
 int polar_b200_fmatmul_path(int transLeft, int transRight, uint64_t m,

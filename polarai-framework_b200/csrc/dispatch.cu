@@ -39,9 +39,10 @@ namespace {
 
 enum Path { kPathTc = 0, kPathSkinny = 1, kPathFfma = 2 };
 
-// Tensor-core tiles are 128 x 256 (or 128 x 128): below one tile in either
-// output dimension, or with a k extent shorter than a slab, the CUDA-core
-// kernel does less wasted work.
+// kPathTc: operands that TMA addresses as they are stored and products of at least half a tile: the 256-column tiles, or
+// clusters of tensor-core CTAs where those are faster (mid_for_tc).  kPathFfma: the rest - unaligned operands, products below
+// that - which the cluster kernel takes as well but for the smallest (mid_for_rest).  kPathSkinny: one tiny dimension, on the
+// narrow kernels or the cluster kernel's 32-column tiles (mid_for_small_n).
 int choose_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const float* left,
                 const float* right, const float* out) {
   if (skinny_kind(tl, tr, m, n, k, left, right, out)) return kPathSkinny;
@@ -232,6 +233,12 @@ struct MidChoice {
   double us = 1e30;
 };
 
+// CTAs of clusters of `cluster` that run at a time.  Those of 4 and 8 leave SMs of a GPC unused: 33 and 15 clusters on 148 SMs.
+uint64_t ctas_at_once(int cluster) {
+  const uint64_t sms = (uint64_t)sm_count();
+  return cluster <= 2 ? sms : cluster == 4 ? sms * 132 / 148 : sms * 120 / 148;
+}
+
 MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact, int orientations = 2, int widths = 3) {
   MidChoice best;
   const uint64_t sms = (uint64_t)sm_count(), slabs = (k + 31) / 32;
@@ -242,8 +249,7 @@ MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact, int orienta
       static const double slab_us[2][3] = {{0.29, 0.36, 0.56}, {0.40, 0.42, 0.63}};
       const uint64_t tiles = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
       for (int cl = 1; cl <= 8 && (uint64_t)cl <= slabs; cl *= 2) {
-        // clusters of 4 and 8 leave SMs of a GPC unused: 33 and 15 of them run at a time on 148 SMs
-        const uint64_t at_once = cl <= 2 ? sms : cl == 4 ? sms * 132 / 148 : sms * 120 / 148;
+        const uint64_t at_once = ctas_at_once(cl);
         const uint64_t waves = (tiles * cl + at_once - 1) / at_once;
         const int log_cl = cl == 8 ? 3 : cl / 2;
         const double exchange = cl == 1 ? 0.0 : bn == 128 ? 1.5 + 0.6 * log_cl : 1.1 + 0.2 * log_cl;
@@ -289,11 +295,15 @@ MidChoice mid_for_rest(uint64_t m, uint64_t n, uint64_t k, uint64_t pad_bytes) {
 // 2048 x 10 x 4096 47 against 19, 8192 x 16 x 4096 110 against 33); at the largest, and for n of 1 to 4, by memory, which they
 // read faster.  Sums of 32 in tensor memory and two levels of them in registers: as close to float64 as the narrow kernels.
 // kind 2, an MN-major left operand: only where its rows are no vectors, since fdense_grad gives the bits of the narrow kernel
-// wherever they are.
+// wherever they are.  Both sides, in us: 301 x 10 x 512 7.1 against 6.6, 1001 x 16 x 1024 28.1 against 8.7, 1001 x 3 x 1024 7.2
+// against 8.8 (stays narrow).  Below 512 terms the estimate of the narrow kernel, fitted to its second launch, does not hold, so
+// all of them stay: 77 x 3 x 256 3.5 against 5.8, though from 10 columns and 300 rows on the tiles would be
+// faster there too (301 x 10 x 384 8.0 against 6.5).
 MidChoice mid_for_small_n(int kind, uint64_t m, uint64_t n, uint64_t k, uint64_t pad_bytes) {
   if (kind == 2 && ((m & 3) == 0 || k < 512)) return MidChoice{};
   MidChoice c = mid_choose(m, n, k, true, 1, 1);
-  // (with a wave or more of tiles the narrow kernel runs several groups of rows per warp, closer to the memory than estimated)
+  // (from half a wave of tiles on the narrow kernel runs several groups of rows per warp, closer to the memory than estimated: 20000 x
+  // 10 x 4096 88.8 against 89.0, 4736 x 10 x 4096 36.6 against 32.5 us; it keeps 4736 x 10 x 1024, 13.2 against 12.0)
   const double other = kind == 2 ? small_tn_estimate_us(m, n, k) : small_n_estimate_us(m, n, k) * (m > 128ull * sm_count() / 2 ? 0.9 : 1.0);
   if (c.us + (pad_bytes ? 2.0 + (double)pad_bytes * 2.0 / 4e6 : 0.0) >= other) c.bn = 0;
   return c;
@@ -405,7 +415,7 @@ void polar_b200_fmatmul_tc_plan(int tl, int tr, uint64_t m, uint64_t n, uint64_t
 }
 
 // The tensor-core path of one product: whole tiles on the tcgen05 kernel, rows just past a tile
-// boundary of a t_f product beside it on the bandwidth-bound kernel.  `pitch` (t_f only; 0 = m)
+// boundary of a t_f product in its split warps, or beside it on a kernel of their own.  `pitch` (t_f only; 0 = m)
 // is the number of floats between consecutive k rows of the stored left operand: a value above
 // m makes the product one over COLUMNS [0, m) of a wider stored matrix, i.e. over a block of
 // rows of the full result.
@@ -425,8 +435,8 @@ static int tc_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const flo
     return run_tc(tl, tr, m, n, k, left, right, out, 256, 16, 3, 0, c.splits, workspace,
                   workspace_bytes, as_stream(stream), fused == 1 ? 1 : 0, pitch, c.mt, c.swap);
   }
-  // whole tile rows on the tensor cores (left is stored [k, m]: the first m - rem columns
-  // of rows of pitch m), the last `rem` rows on the bandwidth-bound kernel, concurrently
+  // whole tile rows as tiles (left is stored [k, m]: the first m - rem columns of rows of pitch m), the last `rem` rows
+  // along with them or, on another stream, at the same time
   const uint64_t mm = m - rem;
   const TcChoice c = tc_choose(mm, n, k, false);
   const int mt = c.mt;
@@ -471,7 +481,7 @@ static int tc_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const flo
   // to the bandwidth of its one pass over `right` (280 us at k = 65536 against 300).
   if (k <= 32768) {
     const uint64_t tiles = (n + 127) / 128;
-    const int cluster = tiles * 8 <= 120 ? 8 : tiles * 4 <= 132 ? 4 : tiles * 2 <= (uint64_t)sm_count() ? 2 : 1;
+    const int cluster = tiles * 8 <= ctas_at_once(8) ? 8 : tiles * 4 <= ctas_at_once(4) ? 4 : tiles * 2 <= ctas_at_once(2) ? 2 : 1;
     rc = launch_mid(1, 0, rem, n, k, left + mm, right, out + mm * n, 32, cluster, 0, 1, 1, 0, nullptr, rag_stream, lp);
   } else {
     rc = launch_ragged_rows(left + mm, lp, right, out + mm * n, reinterpret_cast<float*>(ws + tc_need), rem, n, k,

@@ -289,7 +289,10 @@ small_n_kmajor_resident_kernel(const float* left, const float* right,
 // ---------------------------------------------------------------- small n, MN-major left (split k)
 
 constexpr int KS = 128;   // rows of R staged per pass
-constexpr uint64_t kClusterRows = 384;   // sums of at most this many terms are cut over the CTAs of one cluster
+// Sums of at most this many terms are cut over the CTAs of one cluster, longer ones over more CTAs and a second launch.  In a cluster
+// against in two launches, us: 784 x 10 x 384 8.8 and 9.5, x 512 10.1 and 10.2, x 768 12.8 and 12.3; 4096 x 10 x 384 9.4 and 19.9,
+// x 1024 16.1 and 16.5; 64 x 10 x 256 5.5 and 5.1, x 512 7.3 and 5.3.
+constexpr uint64_t kClusterRows = 384;
 
 // Two fused multiply-adds in one instruction (sm_100: fma.rn.f32x2 on register pairs), each
 // an IEEE fma like fmaf: (c.lo, c.hi) = (a.lo, a.hi) * (b.lo, b.hi) + (c.lo, c.hi).

@@ -13,10 +13,11 @@
 //  - From its third run on, a program of many short launches is replayed as a CUDA graph: one host call instead of 2 us
 //    of host time per launch.  Programs of up to three steps, and programs with tensors of two million elements or
 //    more, whose kernels outlast their launches, stay with launches: programmatic dependent launch overlaps them more
-//    closely in a stream than in a graph (inference on 16 rows, two launches: 17.3 us against 19.9; MLP step at batch
-//    8192 640 against 645; ragged MLP step 57 us of host time against 29 at the same 59 us in all).  The first two runs are launched one by one, so that a program run
-//    once or twice never pays for the instantiation; a run under the caller's own stream capture is
-//    always launched one by one.
+//    closely in a stream than in a graph (inference on 16 rows, two launches: 17.3 us against 19.9).  The 12-launch MLP step by its
+//    largest tensor, as a graph and launched: 0.8 M elements 63.3 and 66.0 us, 2.1 M 120.8 and 119.1, 8.4 M 255.7 and
+//    249.6; the ragged step takes 29 instead of 57 us of host time at the same 52 us in all.  The first two runs are
+//    launched one by one, so that a program run once or twice never pays for the instantiation; a run under the caller's
+//    own stream capture is always launched one by one.
 #include <cstring>
 #include <exception>
 #include <memory>
@@ -308,7 +309,8 @@ private:
 };
 
 // Whether two chains are short - longer ones outlast a launch, and a single builtin's own kernel has more loads in
-// flight - and neither touches a tensor that the other one writes: then their order does not matter.
+// flight - and neither touches a tensor that the other one writes: then their order does not matter.  Two fadds of n and n / 2
+// elements, together against apart: n = 2^18 2.5 against 4.6 us, 2^19 2.9 and 4.5, 2^20 4.4 and 4.6, 2^21 7.7 and 5.3.
 constexpr uint64_t kPairElements = 1ull << 19;
 bool may_pair(const ChainParams& a, const ChainParams& b) {
   if (a.n > kPairElements || b.n > kPairElements) return false;

@@ -1,7 +1,7 @@
 """The matmul dispatch's planning, checked without a GPU: which path a shape takes and how much
 scratch it asks for (the queries read shapes only; with no device they assume B200's 148 SMs).
 The expected values restate the plans: k cut into work units, stream-mode teams and slots,
-256-row tiles, rows past a tile boundary on the bandwidth-bound kernel."""
+256-row tiles, rows past a tile boundary beside them."""
 import ctypes
 import os
 import sys
@@ -70,8 +70,8 @@ def test_whole_waves_need_no_scratch(lib):
 
 def test_weight_gradient_of_the_full_batch(lib):
     # 784 = 3 * 256 + 16 rows, k = 65536: 768 rows on the tensor cores in 256-row tiles (48 tiles,
-    # three work units each fill 144 of 148 SMs), 16 rows on the split-k small-n kernel AT THE
-    # SAME TIME on the library's side stream: the two scratch areas follow one another
+    # three work units each fill 144 of 148 SMs), whose split warps take the 16 rows along.  Their scratch
+    # follows the tiles', of the size that the split-k small-n kernel would need for them
     tc = 3 * 768 * 4096 * 4
     splits_ragged = min((2 * SMS + 3) // 4, 65536 // 128)          # two CTAs per SM over 4 column blocks
     ragged = splits_ragged * 4096 * 16 * 4
@@ -87,7 +87,7 @@ def test_weight_gradient_of_an_eighth_of_the_batch(lib):
     tc = 3 * (teams + 16) * 256 * 256 * 4
     ragged = min((2 * SMS + 3) // 4, 8192 // 128) * 4096 * 16 * 4
     assert ws(lib, 1, 0, 784, 4096, 8192) == tc + ragged
-    # below 4096 the extra pass over the right operand would outlast the tiles: no division
+    # below 4096 terms no division
     assert ws(lib, 1, 0, 784, 4096, 2048) != 0
     assert ws(lib, 1, 0, 784, 4096, 2048) % (128 * 256 * 4) == 0
 
