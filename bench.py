@@ -441,7 +441,9 @@ def run_mlp(args):
 
     reset_weights()
     for _ in range(max(3, args.warmup)):                    # warm-up, eager (also primes NCCL)
+        n0 = lib.launch_count()
         dp.step()
+        launches_per_step = int(lib.launch_count() - n0)    # kernels of this library in one step
     torch.cuda.synchronize()
     if not args.no_graph and not dp.capture():
         if rank == 0:
@@ -451,7 +453,6 @@ def run_mlp(args):
         for _ in range(2):
             dp.step()
         torch.cuda.synchronize()
-    launches_per_step = program.launches()
     timed_step = dp.step
 
     # ---- device-resident throughput ----
@@ -618,7 +619,7 @@ def run_mlp(args):
                        "per_gpu_batch": per, "lr": LR, "parallelism": f"dp{world}",
                        "cuda_graph": graph is not None,
                        "builtins": "extended (fused launches, every output bit-identical to the builtin chain)"
-                       if fused else "the reference's builtin chain, one launch per builtin",
+                       if fused else "the reference's builtin chain",
                        "collective": dp.collective,
                        "data_seed": "numpy default_rng(0): X, labels, W1, W2 in that order; the same global batch "
                                     "at every N, sharded by rows",
@@ -627,7 +628,7 @@ def run_mlp(args):
             "flop_per_sample": FLOP_PER_SAMPLE, "tflops": value * FLOP_PER_SAMPLE / 1e12,
             "first_step_mean_loss": first_loss,
             "gpu_launches": int(launched) if graph is None else launches_per_step * args.steps,
-            "launches_per_step": launches_per_step,
+            "launches_per_step": launches_per_step, "builtins_per_step": program.launches(),
             "clocks": clocks, "e2e": e2e if e2e is not None else e2e_direct, "e2e_direct": e2e_direct,
             "roofline": roofline,
             "breakdown_ms": {k: round(v["ms"], 4) for k, v in sorted(by_kernel.items(), key=lambda kv: -kv[1]["ms"])}}
@@ -643,8 +644,8 @@ def run_mlp(args):
             line["exchange_phases_us_overlapped_part"] = {k: round(v, 1) for k, v in peers.phase_times_us(1).items()}
     line["device_status"] = dp.device_status()             # 0: no bounded device-side wait gave up
     if fused and not args.no_extras:
-        # The same step as the reference's own builtin chain, one launch per builtin (20 launches
-        # instead of 8-9) with NCCL all-reduces: same outputs bit for bit at one rank.  Every
+        # The same step as the reference's own builtin chain (20 builtins instead of 8-9, of which neighbouring
+        # elementwise ones share a launch) with NCCL all-reduces: same outputs bit for bit at one rank.  Every
         # rank runs it (its all-reduces are collective).
         cdp = DataParallelExecutor(lambda rows: mlp_program(rows, N_IN, N_HIDDEN, N_OUT, LR), GLOBAL_BATCH,
                                    ("X", "Y"), rank, world, dev, builtins="reference", collective="nccl")
@@ -652,12 +653,14 @@ def run_mlp(args):
         cex.t["X"].copy_(ex.t["X"]), cex.t["Y"].copy_(ex.t["Y"])
         cex.t["W1"].copy_(w1), cex.t["W2"].copy_(w2)
         for _ in range(3):
+            n0 = lib.launch_count()
             cex.run()
+            chain_launches = int(lib.launch_count() - n0)
         cms = time_region(torch, cex.run, args.steps, dist, world) / args.steps
         line["builtin_chain"] = {"value": GLOBAL_BATCH / (cms / 1e3), "unit": "samples/s", "ms_per_step": cms,
-                                 "launches_per_step": chain.launches(), "cuda_graph": False,
-                                 "note": "the unfused program: one launch per reference builtin, NCCL "
-                                         "all-reduce of dW2 and dW1, fadd updates"}
+                                 "launches_per_step": chain_launches, "builtins_per_step": chain.launches(), "cuda_graph": False,
+                                 "note": "the unfused program of reference builtins, NCCL all-reduce of dW2 and dW1, "
+                                         "fadd updates"}
         cdp.close()
         del cex, cdp
     if rank == 0 and world == 1 and not args.no_extras:
@@ -848,8 +851,8 @@ def elementwise_sweep(torch, lib, dev, peaks):
 
 def small_program_latencies(torch, dev="cuda:0", reps=200):
     """The two latency-bound configurations: microseconds per evaluation of the four-builtin
-    elementwise chain on 2^20 elements and of the logistic-regression step on 256 x 784, launched
-    builtin by builtin and replayed as a CUDA graph; inputs resident (both fit in L2)."""
+    elementwise chain on 2^20 elements and of the logistic-regression step on 256 x 784, as
+    prepared programs and captured in a CUDA graph by the caller; inputs resident (both fit in L2)."""
     import numpy as np
     from polarai_framework_b200.program import DeviceExecutor, elementwise_chain_program, fuse_program, logreg_program
     rng = np.random.default_rng(0)
@@ -866,6 +869,9 @@ def small_program_latencies(torch, dev="cuda:0", reps=200):
         ex = DeviceExecutor(prog, dev)
         ex.set_inputs(**inputs)
         eager_us = event_time(torch, ex.run, reps, warmup=10) * 1e3
+        n0 = ex.lib.launch_count()
+        ex.run()
+        launches = int(ex.lib.launch_count() - n0)          # kernels of this library
         side = torch.cuda.Stream(dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):
@@ -876,7 +882,7 @@ def small_program_latencies(torch, dev="cuda:0", reps=200):
                 ex.run()
         torch.cuda.synchronize()
         graph_us = event_time(torch, g.replay, reps, warmup=10) * 1e3
-        out[name] = {"launches": prog.launches(), "us_per_eval": eager_us, "us_per_eval_cuda_graph": graph_us}
+        out[name] = {"builtins": prog.launches(), "launches": launches, "us_per_eval": eager_us, "us_per_eval_cuda_graph": graph_us}
         del g, ex
     return out
 
