@@ -234,8 +234,7 @@ struct MidChoice {
 };
 
 // CTAs of clusters of `cluster` that run at a time.  Those of 4 and 8 leave SMs of a GPC unused: 33 and 15 clusters on 148 SMs.
-uint64_t ctas_at_once(int cluster) {
-  const uint64_t sms = (uint64_t)sm_count();
+uint64_t ctas_at_once(int cluster, uint64_t sms) {
   return cluster <= 2 ? sms : cluster == 4 ? sms * 132 / 148 : sms * 120 / 148;
 }
 
@@ -249,7 +248,7 @@ MidChoice mid_choose(uint64_t m, uint64_t n, uint64_t k, bool exact, int orienta
       static const double slab_us[2][3] = {{0.29, 0.36, 0.56}, {0.40, 0.42, 0.63}};
       const uint64_t tiles = ((rows + 127) / 128) * ((cols + bn - 1) / bn);
       for (int cl = 1; cl <= 8 && (uint64_t)cl <= slabs; cl *= 2) {
-        const uint64_t at_once = ctas_at_once(cl);
+        const uint64_t at_once = ctas_at_once(cl, sms);
         const uint64_t waves = (tiles * cl + at_once - 1) / at_once;
         const int log_cl = cl == 8 ? 3 : cl / 2;
         const double exchange = cl == 1 ? 0.0 : bn == 128 ? 1.5 + 0.6 * log_cl : 1.1 + 0.2 * log_cl;
@@ -481,7 +480,8 @@ static int tc_path(int tl, int tr, uint64_t m, uint64_t n, uint64_t k, const flo
   // to the bandwidth of its one pass over `right` (280 us at k = 65536 against 300).
   if (k <= 32768) {
     const uint64_t tiles = (n + 127) / 128;
-    const int cluster = tiles * 8 <= ctas_at_once(8) ? 8 : tiles * 4 <= ctas_at_once(4) ? 4 : tiles * 2 <= ctas_at_once(2) ? 2 : 1;
+    const uint64_t sms = (uint64_t)sm_count();
+    const int cluster = tiles * 8 <= ctas_at_once(8, sms) ? 8 : tiles * 4 <= ctas_at_once(4, sms) ? 4 : tiles * 2 <= ctas_at_once(2, sms) ? 2 : 1;
     rc = launch_mid(1, 0, rem, n, k, left + mm, right, out + mm * n, 32, cluster, 0, 1, 1, 0, nullptr, rag_stream, lp);
   } else {
     rc = launch_ragged_rows(left + mm, lp, right, out + mm * n, reinterpret_cast<float*>(ws + tc_need), rem, n, k,
