@@ -172,8 +172,9 @@ uint64_t polar_b200_fmatmul_workspace_bytes(int transLeft, int transRight,
                                             uint64_t m, uint64_t n, uint64_t k);
 
 /* A block of rows of fmatmul_t_f: out[row0 .. row0+rows, :] of out[m,n] = left^T . right with
- * left stored [k,m], right [k,n]; the other rows of `out` are not touched.  Bit for bit the
- * rows the product of the column block of `left` gives.  For a step that exchanges a weight
+ * left stored [k,m], right [k,n]; the other rows of `out` are not touched.  The rows agree with
+ * those of the whole product, and with the product of the column block of `left`, within the fmatmul
+ * tolerance: the sums may be cut differently.  For a step that exchanges a weight
  * gradient between GPUs while the rest of it is still being computed (see
  * polar_b200_allreduce_fadd_range).  row0 and m multiples of 4; the block must be one the
  * tensor-core path serves (rows >= 64, n >= 32, k >= 32, TMA-describable), else
